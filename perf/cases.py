@@ -198,18 +198,26 @@ def _host_view(ptr, count, dtype, owner):
     return np.frombuffer(buf, dtype)
 
 
+def _orbit(rng, info, w, h, *radius):
+    """Parameters of a camera that orbits the scene and sees its centre. swr_camera_init takes the pitch of the given
+    direction and swr_camera_update turns by it the other way (as the reference's camera does), so the target's height
+    is mirrored about the camera's."""
+    pos, at, fov, w, h, far = scenes.sphere_camera(rng, info, w, h, *radius)
+    return pos, (at[0], 2.0 * pos[1] - at[1], at[2]), fov, w, h, far
+
+
 def _frame_scene(case, seed):
     rng = np.random.default_rng(seed)
     w, h = case["width"], case["height"]
     if case["scene"] == "spheres":
         s = swr.Scene(scenes.spheres_scene(seed=seed, count=case["objects"], subdiv=case["subdiv"]))
-        cam = scenes.sphere_camera(rng, s.info(), w, h)
+        cam = _orbit(rng, s.info(), w, h)
     elif case["scene"] == "glass":
         sd = scenes.translucent_scene(seed=seed, count=case["objects"], subdiv=case["subdiv"], box=6.0, tex_size=256,
                                       cube_size=64)
         s = swr.Scene(sd)
         d = s.info().bounds_diagonal
-        cam = scenes.sphere_camera(rng, s.info(), w, h, 0.6 * d, 0.9 * d)
+        cam = _orbit(rng, s.info(), w, h, 0.6 * d, 0.9 * d)
     else:
         sd, cam = _stress_scene(seed, case["triangles"], w, h, case["textures"], case["tex"], case["slots"],
                                 voxel=32 if case["gi"] else 128)
@@ -234,7 +242,7 @@ def prepare(case, seed):
         if kind == "batch_views":
             s = swr.Scene(scenes.spheres_scene(seed=seed, count=case["objects"], subdiv=case["subdiv"]))
             sizes = _view_sizes(case, VIEW_SIZES)
-            items = [(s, swr.make_camera(*scenes.sphere_camera(rng, s.info(), w, h)), w, h) for w, h in sizes]
+            items = [(s, swr.make_camera(*_orbit(rng, s.info(), w, h)), w, h) for w, h in sizes]
         else:
             sizes = _view_sizes(case, SCENE_SIZES)
             items = []
@@ -262,13 +270,13 @@ def prepare(case, seed):
             k = i % len(ids)
             info = resident[k].info()
             d = info.bounds_diagonal
-            requests.append((ids[k], swr.make_camera(*scenes.sphere_camera(rng, info, w, h, 0.7 * d, 1.5 * d)), w, h))
+            requests.append((ids[k], swr.make_camera(*_orbit(rng, info, w, h, 0.7 * d, 1.5 * d)), w, h))
         return {"case": case, "scenes": resident, "server": srv, "requests": requests, "held": [], "seen": {}}
     if kind == "noalloc":
         w, h = case["width"], case["height"]
         scene = swr.Scene(scenes.spheres_scene(seed=seed, count=case["objects"], subdiv=case["subdiv"], box=4.0,
                                                voxel=64))
-        cam = swr.make_camera(*scenes.sphere_camera(rng, scene.info(), w, h, 8.0, 16.0))
+        cam = swr.make_camera(*_orbit(rng, scene.info(), w, h, 8.0, 16.0))
         return {"case": case, "scene": scene, "cam": cam,
                 "rgba": torch.zeros(h, w, dtype=torch.int32, device="cuda"),
                 "vis": torch.zeros(h, w, dtype=torch.int64, device="cuda")}
