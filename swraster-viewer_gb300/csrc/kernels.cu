@@ -87,11 +87,16 @@ __device__ __forceinline__ f3 interp3(const float* s, float b1, float b2) {
     return {(s[0] + b1 * s[3]) + b2 * s[6], (s[1] + b1 * s[4]) + b2 * s[7], (s[2] + b1 * s[5]) + b2 * s[8]};
 }
 
-__constant__ float c_unorm8[256];  // i / 255.0 (src/util.rs:83-89)
-
-__device__ __forceinline__ f3 unpack_rgb(uint32_t t) {
-    return {c_unorm8[(t >> 24) & 0xFFu], c_unorm8[(t >> 16) & 0xFFu], c_unorm8[(t >> 8) & 0xFFu]};
+// i / 255.0 of the byte at bits [15, 23) of `b` (src/util.rs:83-89). With
+// x = i / 256, exact from the mantissa, i / 255 = x + x / 255, and one fused
+// operation with the rounded 1/255 gives the correctly rounded quotient for
+// every byte (tests/test_unorm8.py). A 256-entry __constant__ table cost a
+// replay per distinct byte of the warp, 17 lookups a pixel.
+__device__ __forceinline__ float unorm8(uint32_t b) {
+    const float x = __uint_as_float(0x3F800000u | (b & 0x7F8000u)) - 1.0f;
+    return __fmaf_rn(x, 1.0f / 255.0f, x);
 }
+__device__ __forceinline__ f3 unpack_rgb(uint32_t t) { return {unorm8(t >> 9), unorm8(t >> 1), unorm8(t << 7)}; }
 
 // srgb_to_linear_fast (src/util.rs:111-113).
 __device__ __forceinline__ float srgb_fast(float x) { return x * (x * (x * 0.305306011f + 0.682171111f) + 0.012522878f); }
@@ -254,13 +259,24 @@ __device__ __forceinline__ void rebuild_bary(const RecRaster& r, int32_t px, int
     const Edge e01 = make_edge(r.p[0], r.p[1], r.p[2], r.p[3]);
     float w1 = edge_eval(e20, lx, ly);
     float w2 = edge_eval(e01, lx, ly);
-    for (int j = 0; j < qj; ++j) {
-        w1 += e20.sy;
-        w2 += e01.sy;
-    }
-    for (int i = 0; i < qi; ++i) {
-        w1 += e20.sx;
-        w2 += e01.sx;
+    // Closed form where every partial sum is an integer below 2^24 (see
+    // Regions below), else the additions themselves. The loops took up to
+    // 2 x 14 dependent additions per warp.
+    const float fi = (float)qi, fj = (float)qj;
+    const float m1 = __fadd_ru(__fadd_ru(fabsf(w1), __fmul_ru(fj, fabsf(e20.sy))), __fmul_ru(fi, fabsf(e20.sx)));
+    const float m2 = __fadd_ru(__fadd_ru(fabsf(w2), __fmul_ru(fj, fabsf(e01.sy))), __fmul_ru(fi, fabsf(e01.sx)));
+    if (fmaxf(m1, m2) <= 16777216.0f) {
+        w1 += e20.sy * fj + e20.sx * fi;
+        w2 += e01.sy * fj + e01.sx * fi;
+    } else {
+        for (int j = 0; j < qj; ++j) {
+            w1 += e20.sy;
+            w2 += e01.sy;
+        }
+        for (int i = 0; i < qi; ++i) {
+            w1 += e20.sx;
+            w2 += e01.sx;
+        }
     }
     b1 = w1 * r.ooa;
     b2 = w2 * r.ooa;
@@ -1128,7 +1144,7 @@ __device__ __forceinline__ bool alpha_pass(const DScene& sc, const DMaterial& m,
     const float u = interp(q.uow, b1, b2) * w;
     const float v = interp(q.vow, b1, b2) * w;
     const uint32_t tx = sample_texel(t, u, v, mip, m.wrap_s[TS_BASE], m.wrap_t[TS_BASE]);
-    return c_unorm8[tx & 0xFFu] >= m.alpha_cutoff;
+    return unorm8(tx << 15) >= m.alpha_cutoff;
 }
 
 // coarse_raster's block reject (src/tilerasterizer.rs:238-269): the block is
@@ -1860,16 +1876,19 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const D
     const float EPS = 1e-6f;
     const float INV_PI = 1.0f / 3.14159265358979f;
     const f3 in_n = normalize(interp3(q.nrm, b1, b2), md, tab);
-    const f3 in_t = normalize(interp3(q.tan, b1, b2), md, tab);
-    const float tsign = interp(q.tsign, b1, b2);
     const f3 pw = interp3(q.pww, b1, b2) * w;
     const float uvx = interp(q.uow, b1, b2) * w;
     const float uvy = interp(q.vow, b1, b2) * w;
-    const f3 tw = normalize(in_t - in_n * dot(in_n, in_t), md, tab);
-    const float hand = tsign >= 0.0f ? 1.0f : -1.0f;
-    const f3 bw = cross(in_n, tw) * hand;
-    f3 nw = normalize(in_n, md, tab);
-    if (m.tex[TS_NORMAL] >= 0) {
+    // The tangent frame only feeds the normal map: without one its two
+    // normalisations, interpolations and cross product are not evaluated.
+    f3 nw;
+    if (m.tex[TS_NORMAL] < 0) {
+        nw = normalize(in_n, md, tab);
+    } else {
+        const f3 in_t = normalize(interp3(q.tan, b1, b2), md, tab);
+        const f3 tw = normalize(in_t - in_n * dot(in_n, in_t), md, tab);
+        const float hand = interp(q.tsign, b1, b2) >= 0.0f ? 1.0f : -1.0f;
+        const f3 bw = cross(in_n, tw) * hand;
         const f3 s = unpack_rgb(sample_slot(sc, m, TS_NORMAL, uvx, uvy, du_dv));
         const f3 tsn = mk3(s.x * 2.0f - 1.0f, s.y * 2.0f - 1.0f, s.z * 2.0f - 1.0f);
         nw = (tw * tsn.x + bw * tsn.y) + in_n * tsn.z;
@@ -2021,13 +2040,28 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
         for (int i = 0; i < 5; ++i) dst[i] = __ldg(src + i);
         rebuild_bary(r, px, py, b1, b2);
     }
-    // bary1/bary2 of all four lanes of the quad (uncovered lanes hold 0, the
-    // contents of a fresh renderer's vbuffer; src/tilerasterizer.rs:114-118).
-    float qb1[4], qb2[4];
+    // 1 / w at each quad lane's barycentrics with this lane's triangle. A
+    // quad lane of the same triangle has computed that very value as its own
+    // w, so it is taken from there; only warps with a quad over several
+    // triangles exchange barycentrics (uncovered lanes hold 0, the contents of
+    // a fresh renderer's vbuffer; src/tilerasterizer.rs:114-118) and divide.
+    const uint32_t tri = writer ? slot : 0xFFFFFFFFu;
+    const float w_own = writer ? 1.0f / interp(r.oow, b1, b2) : 0.0f;
+    float wq[4];
+    uint32_t other = 0u;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        qb1[i] = __shfl_sync(0xFFFFFFFFu, b1, (int)((lane & ~3u) + (uint32_t)i));
-        qb2[i] = __shfl_sync(0xFFFFFFFFu, b2, (int)((lane & ~3u) + (uint32_t)i));
+        const int src = (int)((lane & ~3u) + (uint32_t)i);
+        wq[i] = __shfl_sync(0xFFFFFFFFu, w_own, src);
+        other |= __shfl_sync(0xFFFFFFFFu, tri, src) != tri ? 1u << i : 0u;
+    }
+    if (__any_sync(0xFFFFFFFFu, writer && other != 0u)) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int src = (int)((lane & ~3u) + (uint32_t)i);
+            const float ob1 = __shfl_sync(0xFFFFFFFFu, b1, src), ob2 = __shfl_sync(0xFFFFFFFFu, b2, src);
+            if (writer && (other & (1u << i))) wq[i] = 1.0f / interp(r.oow, ob1, ob2);
+        }
     }
     f3 col = mk3(0.0f, 0.0f, 0.0f);
     uint32_t vis_hi = 0xFFFFFFFFu, vis_fan = 0;
@@ -2040,15 +2074,9 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
 #pragma unroll
                 for (int i = 0; i < 11; ++i) dst[i] = __ldg(src + i);
             }
-            // 1 / w at each quad lane's bary with this lane's triangle; this
-            // lane's own entry is the w that shading uses (qb*[k] = b1, b2).
-            float wq[4], dd[4];
+            float dd[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                wq[i] = 1.0f / interp(r.oow, qb1[i], qb2[i]);
-                dd[i] = q.du_dv[i] * wq[i];
-            }
-            const float w_own = k == 0 ? wq[0] : (k == 1 ? wq[1] : (k == 2 ? wq[2] : wq[3]));
+            for (int i = 0; i < 4; ++i) dd[i] = q.du_dv[i] * wq[i];
             const DMaterial& m = sc.materials[r.material & kRecMaterialMask];
             col = pbr_lane<false, GI>(sc, v, m, q, w_own, b1, b2, dd, md, tab, col);
             vis_hi = q.static_id;
@@ -2366,10 +2394,7 @@ cudaError_t init_kernel_constants() {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 64 && (g_const_init_mask >> dev) & 1ull) return cudaSuccess;
-    float t[256];
-    for (int i = 0; i < 256; ++i) t[i] = (float)i / 255.0f;
-    e = cudaMemcpyToSymbol(c_unorm8, t, sizeof(t));
-    if (e == cudaSuccess) e = raster_smem_attr<8, true>();
+    e = raster_smem_attr<8, true>();
     if (e == cudaSuccess) e = raster_smem_attr<16, true>();
     if (e == cudaSuccess) e = raster_smem_attr<32, false>();
     if (e == cudaSuccess) e = raster_smem_attr<32, true>();
