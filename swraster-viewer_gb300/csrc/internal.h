@@ -203,7 +203,7 @@ struct alignas(16) RecRaster {
     uint32_t material;
     uint32_t view;
     uint32_t zfloor;           // orderable depth floor of the whole triangle (occlusion culling), 0 = none
-    uint32_t pad;
+    uint32_t wide;             // 1: binned from the wide queue (k_scatter's slot loop skips it)
 };
 static_assert(sizeof(RecRaster) == 80, "RecRaster layout");
 
@@ -250,7 +250,17 @@ struct alignas(16) DCounters {
     uint32_t draw_count;
     uint32_t culled;           // (triangle, tile) pairs the raster dropped as hidden
     uint32_t clip_path;        // triangles of draws whose sphere intersects the frustum (the clip path)
+    uint32_t wide_main;        // wide-queue segments appended by k_frontend
+    uint32_t wide_clip;        // ... and by k_clip (second half of the queue)
 };
+
+// Triangles over more than kWideTiles scheduling tiles are binned by whole
+// warps, kWideSegment tiles at a time, instead of by one thread: the wide
+// queue holds (record slot, segment) pairs. A triangle that finds the queue
+// full is binned by its thread.
+constexpr uint32_t kWideTiles = 32;
+constexpr uint32_t kWideSegment = 128;
+constexpr uint32_t kWideCap = 32768;   // entries per half of the queue
 
 // Per-frame counts, uploaded with the tables: kernels read them from device
 // memory so a launch sequence captured once (grids sized by capacity)
@@ -284,12 +294,13 @@ struct FrameArgs {
     uint32_t view_cap;
     uint64_t bin_cap;
     uint32_t sched_tile;       // S
-    uint32_t pad0;
+    uint32_t wide_cap;         // entries per half of wide_queue (0: no queue)
     uint8_t* tri_state;
     RecRaster* rec_r;
     RecShade* rec_s;
     uint32_t* fan_base;
     uint2* clip_queue;         // (g, draw)
+    uint2* wide_queue;         // 2 * wide_cap entries: k_frontend's, then k_clip's
     uint32_t* tile_count;      // n_bins; after k_scan, the raster tile order
     uint32_t* tile_offset;     // n_bins + 1
     uint32_t* tile_cursor;     // n_bins

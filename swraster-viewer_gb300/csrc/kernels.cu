@@ -355,28 +355,50 @@ __device__ __forceinline__ void agg_inc(uint32_t* counter, uint32_t idx) {
     if ((int)(threadIdx.x & 31) == leader) atomicAdd(counter + idx, (uint32_t)__popc(peers));
 }
 
-// Iterate the scheduling tiles a setup triangle touches. f(stile) is called
-// once per (triangle, scheduling tile) pair. Mirrors the bin loop of
-// bin_triangle (src/renderer.rs:756-830) restricted to real tiles (the
-// reference's x == tiles_x column aliases into the next row's tile 0 and only
-// ever yields an empty rect or an exact duplicate packet).
-template <typename F>
-__device__ __forceinline__ void for_each_stile(const DView& v, int32_t S, int32_t mnx, int32_t mny, int32_t mxx,
-                                               int32_t mxy, F f) {
-    const int32_t bx0 = mnx / kRefTile, by0 = mny / kRefTile;
-    const int32_t bx1 = min((mxx + kRefTile - 1) / kRefTile, v.tiles_x);
-    const int32_t by1 = min((mxy + kRefTile - 1) / kRefTile, v.tiles_y);
-    for (int32_t ty = by0; ty < by1; ++ty) {
-        for (int32_t tx = bx0; tx < bx1; ++tx) {
-            const int32_t x0 = max(mnx, tx * kRefTile), y0 = max(mny, ty * kRefTile);
-            const int32_t x1 = min(mxx, tx * kRefTile + kRefTile), y1 = min(mxy, ty * kRefTile + kRefTile);
-            if (x1 - x0 < 1 || y1 - y0 < 1) continue;
-            const int32_t sx0 = x0 / S, sx1 = (x1 - 1) / S;
-            const int32_t sy0 = y0 / S, sy1 = (y1 - 1) / S;
-            for (int32_t sy = sy0; sy <= sy1; ++sy)
-                for (int32_t sx = sx0; sx <= sx1; ++sx) f(v.stile_base + (uint32_t)(sy * v.stiles_x + sx));
-        }
+// Scheduling tiles a setup triangle touches: the bin loop of bin_triangle
+// (src/renderer.rs:756-830) restricted to real tiles (the reference's
+// x == tiles_x column aliases into the next row's tile 0 and only ever yields
+// an empty rect or an exact duplicate packet). The reference walks 64-px
+// tiles; a scheduling tile divides one, so over all of them the touched
+// scheduling tiles form one rectangle.
+struct TileRect {
+    uint32_t first;      // its top left tile's bin
+    uint32_t nx, ny;     // tiles per row, rows
+    uint32_t pitch;      // bins per row of the view
+    __device__ __forceinline__ uint32_t count() const { return nx * ny; }
+    __device__ __forceinline__ uint32_t tile(uint32_t k) const {
+        const uint32_t y = k / nx;
+        return first + y * pitch + (k - y * nx);
     }
+};
+__device__ __forceinline__ TileRect tile_rect(const DView& v, uint32_t S, uint32_t bin_off, int32_t mnx, int32_t mny,
+                                              int32_t mxx, int32_t mxy) {
+    const int32_t x1 = min(mxx, v.tiles_x * kRefTile), y1 = min(mxy, v.tiles_y * kRefTile);
+    TileRect t{0u, 0u, 0u, (uint32_t)v.stiles_x};
+    if (x1 <= mnx || y1 <= mny) return t;
+    const uint32_t sh = 31u - (uint32_t)__clz(S);  // S is a power of two; the corners are not negative
+    const uint32_t x0 = (uint32_t)mnx >> sh, y0 = (uint32_t)mny >> sh;
+    t.nx = ((uint32_t)(x1 - 1) >> sh) - x0 + 1u;
+    t.ny = ((uint32_t)(y1 - 1) >> sh) - y0 + 1u;
+    t.first = bin_off + v.stile_base + y0 * t.pitch + x0;
+    return t;
+}
+template <typename F>
+__device__ __forceinline__ void for_each_stile(const TileRect& t, F f) {
+    for (uint32_t y = 0; y < t.ny; ++y)
+        for (uint32_t x = 0; x < t.nx; ++x) f(t.first + y * t.pitch + x);
+}
+
+// Appends a wide triangle's segments to one half of the wide queue; false
+// when they do not fit (the entries taken are marked unused).
+__device__ __forceinline__ bool push_wide(const FrameArgs& a, uint32_t* counter, uint2* queue, uint32_t slot, uint32_t n) {
+    if (a.wide_cap == 0u) return false;
+    const uint32_t segs = (n + kWideSegment - 1u) / kWideSegment;
+    const uint32_t base = atomicAdd(counter, segs);
+    const bool ok = base <= a.wide_cap && segs <= a.wide_cap - base;
+    for (uint32_t s = 0; s < segs && base + s < a.wide_cap; ++s)
+        queue[base + s] = make_uint2(ok ? slot : 0xFFFFFFFFu, s);
+    return ok;
 }
 
 // Occlusion culling runs for scheduling tiles of at least this many pixels
@@ -385,11 +407,12 @@ __device__ __forceinline__ void for_each_stile(const DView& v, int32_t S, int32_
 #define SWR_CULL_MIN_TILE 64
 #endif
 
-// bin_triangle (src/renderer.rs:668-831): setup + count. Returns true when
-// the triangle covers at least one tile; its records are then in r and q.
+// bin_triangle (src/renderer.rs:668-831): setup. Returns true when the
+// triangle covers at least one tile; its records are then in r and q, its
+// tiles (still to be counted) in tiles.
 __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx& v0, const Vtx& v1, const Vtx& v2,
                                uint32_t seq8, uint32_t static_id, uint32_t material, uint32_t view_idx,
-                               RecRaster& r, RecShade& q) {
+                               RecRaster& r, RecShade& q, TileRect& tiles) {
     int32_t p0x, p0y, p1x, p1y, p2x, p2y;
     to_screen(v0, view.width_f, view.height_f, p0x, p0y);
     to_screen(v1, view.width_f, view.height_f, p1x, p1y);
@@ -405,10 +428,9 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     const int32_t mxx = wadd(mxs_x, kSubpixelScale) >> kSubpixelShift;
     const int32_t mxy = wadd(mxs_y, kSubpixelScale) >> kSubpixelShift;
 
-    uint32_t n = 0;
-    const int32_t S = (int32_t)a.sched_tile;
-    for_each_stile(view, S, mnx, mny, mxx, mxy, [&](uint32_t) { ++n; });
-    if (n == 0) return false;
+    const bool translucent = (material & kRecTransBit) != 0u;
+    tiles = tile_rect(view, a.sched_tile, translucent ? a.dyn->n_stiles : 0u, mnx, mny, mxx, mxy);
+    if (tiles.count() == 0u) return false;
 
     // Interpolator setup (src/renderer.rs:699-754).
     const float ooa = 1.0f / i2f(wabs(area));
@@ -434,7 +456,7 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     r.material = material;
     r.view = view_idx;
     r.zfloor = 0u;  // taken by k_scatter when the frame culls
-    r.pad = 0u;
+    r.wide = 0u;
     q.nrm[0] = v0.nx; q.nrm[1] = v0.ny; q.nrm[2] = v0.nz;
     q.nrm[3] = v1.nx - v0.nx; q.nrm[4] = v1.ny - v0.ny; q.nrm[5] = v1.nz - v0.nz;
     q.nrm[6] = v2.nx - v0.nx; q.nrm[7] = v2.ny - v0.ny; q.nrm[8] = v2.nz - v0.nz;
@@ -453,11 +475,8 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     q.du_dv[0] = du_dx * s; q.du_dv[1] = du_dy * s; q.du_dv[2] = dv_dx * s; q.du_dv[3] = dv_dy * s;
     q.static_id = static_id;
     // Average z for the per-tile translucency sort (src/renderer.rs:765-774).
-    const bool translucent = (material & kRecTransBit) != 0u;
     q.pad[0] = translucent ? __float_as_uint(((v0.cz + v1.cz) + v2.cz) / 3.0f) : 0u;
     q.pad[1] = q.pad[2] = 0;
-    const uint32_t bin_off = translucent ? a.dyn->n_stiles : 0u;
-    for_each_stile(view, S, mnx, mny, mxx, mxy, [&](uint32_t st) { agg_inc(a.tile_count, bin_off + st); });
     return true;
 }
 
@@ -758,6 +777,8 @@ __global__ void __launch_bounds__(256) k_reset(FrameArgs a) {
         a.counters->trans_packets = 0u;
         a.counters->culled = 0u;
         a.counters->clip_path = 0u;
+        a.counters->wide_main = 0u;
+        a.counters->wide_clip = 0u;
         a.counters->draw_tris = a.gpu_draws ? 0u : a.dyn->tri_total;
     }
     if (a.gpu_draws) draw_count_blocks(a);
@@ -832,8 +853,18 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
     const uint32_t mword = record_material(sc, d, pr.material);
     RecRaster r;
     RecShade q;
-    const bool ok = setup_triangle(a, view, v0, v1, v2, g << 3, d.static_base + local, mword, d.view, r, q);
-    if (ok) store_records(a, g, r, q);
+    TileRect tiles;
+    const bool ok = setup_triangle(a, view, v0, v1, v2, g << 3, d.static_base + local, mword, d.view, r, q, tiles);
+    if (ok) {
+        // A wide triangle's tiles are counted by k_clip's warps: one thread
+        // walking the 4,576 16-px tiles of a 1367x769 frame held the kernel
+        // for 79 us (150k triangles; 12 us without such triangles).
+        if (tiles.count() > kWideTiles && push_wide(a, &a.counters->wide_main, a.wide_queue, g, tiles.count()))
+            r.wide = 1u;
+        else
+            for_each_stile(tiles, [&](uint32_t st) { agg_inc(a.tile_count, st); });
+        store_records(a, g, r, q);
+    }
     a.tri_state[g] = ok ? 1 : 0;
     warp_count(&a.counters->setup_tris, ok);
 }
@@ -849,34 +880,55 @@ __global__ void __launch_bounds__(kChunkTris, SWR_FRONTEND_MIN_BLOCKS) k_fronten
     if (blockIdx.x < a.dyn->n_chunks) frontend_triangle(a, blockIdx.x);
 }
 
-// intersect (src/renderer.rs:598-609).
-__device__ __forceinline__ Vtx lerp_vtx(const Vtx& a, const Vtx& b, float t) {
-    Vtx o;
-    o.cx = a.cx + (b.cx - a.cx) * t; o.cy = a.cy + (b.cy - a.cy) * t;
-    o.cz = a.cz + (b.cz - a.cz) * t; o.cw = a.cw + (b.cw - a.cw) * t;
-    o.wx = a.wx + (b.wx - a.wx) * t; o.wy = a.wy + (b.wy - a.wy) * t; o.wz = a.wz + (b.wz - a.wz) * t;
-    o.nx = a.nx + (b.nx - a.nx) * t; o.ny = a.ny + (b.ny - a.ny) * t; o.nz = a.nz + (b.nz - a.nz) * t;
-    o.tx = a.tx + (b.tx - a.tx) * t; o.ty = a.ty + (b.ty - a.ty) * t;
-    o.tz = a.tz + (b.tz - a.tz) * t; o.tw = a.tw + (b.tw - a.tw) * t;
-    o.u = a.u + (b.u - a.u) * t; o.v = a.v + (b.v - a.v) * t;
-    return o;
-}
-__device__ __forceinline__ float plane_dist(const Vtx& v, int p) {
-    switch (p) {
-        case 0: return v.cz + v.cw;   // near:   z + w
-        case 1: return -v.cz + v.cw;  // far:   -z + w
-        case 2: return v.cx + v.cw;   // right:  x + w
-        case 3: return -v.cx + v.cw;  // left:  -x + w
-        case 4: return v.cy + v.cw;   // top:    y + w
-        default: return -v.cy + v.cw; // bottom: -y + w
-    }
+// Sutherland-Hodgman for the queued triangles, sixteen lanes per triangle.
+// A vertex (Vtx) is sixteen floats: lane i transforms, keeps and lerps float
+// i, and the polygon lives in shared memory; each fan triangle's setup is
+// then one lane's. One thread per triangle held two 16-vertex polygons in
+// 2 KB of local memory and filled 8 CTAs with a thousand clipped triangles.
+// The kernel also counts the tiles of k_frontend's wide triangles, a warp per
+// segment, and those of its own by all sixteen lanes.
+constexpr int kClipThreads = 128;
+constexpr int kClipMaxVerts = 16;  // a triangle cut by six planes has at most nine
+constexpr int kClipPoly = 2 * kClipMaxVerts * 16 + 16;  // two buffers; the pad spreads neighbouring groups over the banks
+__device__ __forceinline__ float plane_dist(const float* v, int p) {
+    // near z + w, far -z + w, right x + w, left -x + w, top y + w, bottom -y + w
+    // (src/renderer.rs:581-588; every product is by 0 or +-1).
+    const float c = v[p < 2 ? 2 : (p < 4 ? 0 : 1)];
+    return ((p & 1) ? -c : c) + v[3];
 }
 
-__global__ void __launch_bounds__(128) k_clip(FrameArgs a) {
+// Record of a queued wide segment, or null where the entry is unused.
+__device__ __forceinline__ const RecRaster* wide_record(const FrameArgs& a, uint2 e) {
+    return e.x == 0xFFFFFFFFu ? nullptr : a.rec_r + e.x;
+}
+__device__ __forceinline__ TileRect record_tiles(const FrameArgs& a, const RecRaster& r) {
+    return tile_rect(a.views[r.view], a.sched_tile, (r.material & kRecTransBit) ? a.dyn->n_stiles : 0u, r.bb[0],
+                     r.bb[1], r.bb[2], r.bb[3]);
+}
+
+__global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
+    __shared__ __align__(16) float poly_mem[kClipThreads / 16][kClipPoly];
+    const uint32_t lane = threadIdx.x & 31u;
+    {
+        const uint32_t n = min(a.counters->wide_main, a.wide_cap);
+        const uint32_t nw = gridDim.x * (kClipThreads / 32);
+        for (uint32_t e = blockIdx.x * (kClipThreads / 32) + (threadIdx.x >> 5); e < n; e += nw) {
+            const uint2 q = a.wide_queue[e];
+            const RecRaster* r = wide_record(a, q);
+            if (!r) continue;
+            const TileRect t = record_tiles(a, *r);
+            const uint32_t k1 = min(t.count(), (q.y + 1u) * kWideSegment);
+            for (uint32_t k = q.y * kWideSegment + lane; k < k1; k += 32u) atomicAdd(a.tile_count + t.tile(k), 1u);
+        }
+    }
     const uint32_t nq = min(a.counters->clip_queue, a.clip_cap);
     const uint32_t tri_total = a.dyn->tri_total;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const uint2 e = a.clip_queue[q];
+    const uint32_t grp = threadIdx.x >> 4, i = threadIdx.x & 15u;
+    const uint32_t gmask = 0xFFFFu << (lane & 16u);
+    const int lead = (int)(lane & 16u);
+    float* const buf = poly_mem[grp];
+    for (uint32_t qi = blockIdx.x * (kClipThreads / 16) + grp; qi < nq; qi += gridDim.x * (kClipThreads / 16)) {
+        const uint2 e = a.clip_queue[qi];
         const uint32_t g = e.x;
         const DDraw& d = a.draws[e.y];
         const uint32_t local = g - d.tri_begin;
@@ -884,60 +936,116 @@ __global__ void __launch_bounds__(128) k_clip(FrameArgs a) {
         const DView& view = a.views[d.view];
         const DPrimitive pr = sc.prims[d.prim];
         const uint32_t mword = record_material(sc, d, pr.material);
-        const float* model = sc.node_xform + 16u * d.node;
         const uint32_t* ib = sc.indices + pr.idx_base + 3u * local;
-        Vtx poly[16], np[16];
-        poly[0] = transform_vertex(sc.vertices, pr.vtx_base + __ldg(ib), model, d.mvp);
-        poly[1] = transform_vertex(sc.vertices, pr.vtx_base + __ldg(ib + 1), model, d.mvp);
-        poly[2] = transform_vertex(sc.vertices, pr.vtx_base + __ldg(ib + 2), model, d.mvp);
-        int len = 3;
-        for (int p = 0; p < 6 && len > 0; ++p) {
-            int nl = 0;
-            for (int i = 0; i < len; ++i) {
-                const Vtx& cur = poly[i];
-                const Vtx& prv = poly[(i + len - 1) % len];
-                const float dc = plane_dist(cur, p), dp = plane_dist(prv, p);
-                const bool cin = dc >= 0.0f, pin = dp >= 0.0f;
-                if (cin) {
-                    if (!pin) np[nl++] = lerp_vtx(prv, cur, dp / (dp - dc));
-                    np[nl++] = cur;
-                } else if (pin) {
-                    np[nl++] = lerp_vtx(prv, cur, dp / (dp - dc));
-                }
+        {
+            // Lane i's row of the vertex transform (transform_vertex): clip
+            // position, world position, normal, tangent, then copies.
+            const float* m = i < 4u ? d.mvp : sc.node_xform + 16u * d.node;
+            const uint32_t row = i < 4u ? i : (i < 7u ? i - 4u : (i < 10u ? i - 7u : i - 10u));
+            const uint32_t src = i < 7u ? 0u : (i < 10u ? 4u : 8u);
+            const uint32_t copy = i == 13u ? 11u : (i == 14u ? 3u : 7u);
+            float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;
+            if (i < 13u) {
+                c0 = m[row];
+                c1 = m[4u + row];
+                c2 = m[8u + row];
+                c3 = m[12u + row];
             }
-            for (int i = 0; i < nl; ++i) poly[i] = np[i];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float* v = reinterpret_cast<const float*>(sc.vertices + pr.vtx_base + __ldg(ib + k));
+                float o;
+                if (i < 13u) {
+                    o = (c0 * __ldg(v + src) + c1 * __ldg(v + src + 1)) + c2 * __ldg(v + src + 2);
+                    if (i < 7u) o = o + c3;
+                } else {
+                    o = __ldg(v + copy);
+                }
+                buf[k * 16 + i] = o;
+            }
+        }
+        __syncwarp(gmask);
+        int len = 3;
+        float* cur = buf;
+        float* nxt = buf + kClipMaxVerts * 16;
+        for (int p = 0; p < 6 && len > 0; ++p) {
+            // intersect (src/renderer.rs:598-609): prev + (cur - prev) * t.
+            int nl = 0;
+            const float* pv = cur + (len - 1) * 16;
+            float dp = plane_dist(pv, p);
+            for (int k = 0; k < len; ++k) {
+                const float* cv = cur + k * 16;
+                const float dc = plane_dist(cv, p);
+                const bool cin = dc >= 0.0f, pin = dp >= 0.0f;
+                if (cin != pin && nl < kClipMaxVerts) {
+                    const float t = dp / (dp - dc);
+                    nxt[nl++ * 16 + i] = pv[i] + (cv[i] - pv[i]) * t;
+                }
+                if (cin && nl < kClipMaxVerts) nxt[nl++ * 16 + i] = cv[i];
+                pv = cv;
+                dp = dc;
+            }
+            __syncwarp(gmask);
+            float* const x = cur;
+            cur = nxt;
+            nxt = x;
             len = nl;
         }
-        uint32_t any = 0;
-        if (len >= 3) {
-            const int fans = len - 2;
-            uint32_t base = 0;
-            if (fans > 1) {
-                base = atomicAdd(&a.counters->extra_used, (uint32_t)(fans - 1));
-                if (base + (uint32_t)(fans - 1) > a.extra_cap) {
+        const int fans = len - 2;
+        if (fans <= 0) {
+            if (i == 0u) a.tri_state[g] = 3;
+            __syncwarp(gmask);
+            continue;
+        }
+        uint32_t base = 0;
+        if (fans > 1) {
+            if (i == 0u) base = atomicAdd(&a.counters->extra_used, (uint32_t)(fans - 1));
+            base = __shfl_sync(gmask, base, lead);
+            if (base + (uint32_t)(fans - 1) > a.extra_cap) {
+                if (i == 0u) {
                     atomicOr(&a.counters->status, ST_CLIP_OVERFLOW);
                     a.tri_state[g] = 0;
-                    continue;
                 }
-                a.fan_base[g] = tri_total + base;
+                __syncwarp(gmask);
+                continue;
             }
-            for (int f = 0; f < fans; ++f) {
-                const uint32_t slot = f == 0 ? g : tri_total + base + (uint32_t)(f - 1);
-                RecRaster r;
-                RecShade q;
-                const bool ok = setup_triangle(a, view, poly[0], poly[f + 1], poly[f + 2], (g << 3) | (uint32_t)f,
-                                               d.static_base + local, mword, d.view, r, q);
-                if (ok) store_records(a, slot, r, q);
-                if (ok) {
-                    atomicAdd(&a.counters->setup_tris, 1u);
-                    if (f == 0) any = 1;
-                } else if (f > 0) {
-                    // Mark the unused extra slot so the scatter skips it.
-                    a.rec_r[slot].view = 0xFFFFFFFFu;
-                }
+            if (i == 0u) a.fan_base[g] = tri_total + base;
+        }
+        // Lane f sets up fan triangle f.
+        bool ok = false;
+        TileRect tiles{0u, 0u, 0u, 0u};
+        if ((int)i < fans) {
+            const uint32_t slot = i == 0u ? g : tri_total + base + i - 1u;
+            const Vtx* pl = reinterpret_cast<const Vtx*>(cur);
+            RecRaster r;
+            RecShade q;
+            ok = setup_triangle(a, view, pl[0], pl[i + 1], pl[i + 2], (g << 3) | i, d.static_base + local, mword,
+                                d.view, r, q, tiles);
+            if (ok) {
+                if (tiles.count() > kWideTiles &&
+                    push_wide(a, &a.counters->wide_clip, a.wide_queue + a.wide_cap, slot, tiles.count()))
+                    r.wide = 1u;
+                store_records(a, slot, r, q);
+            } else if (i > 0u) {
+                // Mark the unused extra slot so the scatter skips it.
+                a.rec_r[slot].view = 0xFFFFFFFFu;
             }
         }
-        a.tri_state[g] = any ? 1 : 3;
+        const uint32_t oks = __ballot_sync(gmask, ok);
+        for (uint32_t left = oks; left; left &= left - 1u) {
+            const int f = __ffs(left) - 1;
+            TileRect t;
+            t.first = __shfl_sync(gmask, tiles.first, f);
+            t.nx = __shfl_sync(gmask, tiles.nx, f);
+            t.ny = __shfl_sync(gmask, tiles.ny, f);
+            t.pitch = __shfl_sync(gmask, tiles.pitch, f);
+            for (uint32_t k = i; k < t.count(); k += 16u) atomicAdd(a.tile_count + t.tile(k), 1u);
+        }
+        if (i == 0u) {
+            if (oks) atomicAdd(&a.counters->setup_tris, (uint32_t)__popc(oks));
+            a.tri_state[g] = ((oks >> lead) & 1u) ? 1 : 3;
+        }
+        __syncwarp(gmask);
     }
 }
 
@@ -1089,8 +1197,6 @@ __device__ __forceinline__ void scatter_slot(const FrameArgs& a, uint32_t slot, 
         return;
     }
     const RecRaster& r = a.rec_r[slot];
-    const DView& view = a.views[r.view];
-    const uint32_t bin_off = (r.material & kRecTransBit) ? a.dyn->n_stiles : 0u;
     if ((int32_t)a.sched_tile >= SWR_CULL_MIN_TILE && !(r.material & kRecTransBit) &&
         (SWR_FLOOR_MIN_PX == 0 ||
          (uint32_t)(r.bb[2] - r.bb[0] + 1) * (uint32_t)(r.bb[3] - r.bb[1] + 1) >= (uint32_t)SWR_FLOOR_MIN_PX)) {
@@ -1102,8 +1208,8 @@ __device__ __forceinline__ void scatter_slot(const FrameArgs& a, uint32_t slot, 
         if (depth_floor(r.p, r.zow, r.oow, (int32_t)r.bb[2] * kSubpixelScale, (int32_t)r.bb[3] * kSubpixelScale, zl))
             a.rec_r[slot].zfloor = float_to_ordered(zl);
     }
-    for_each_stile(view, (int32_t)a.sched_tile, r.bb[0], r.bb[1], r.bb[2], r.bb[3], [&](uint32_t b) {
-        const uint32_t st = bin_off + b;
+    if (r.wide) return;  // scatter_wide
+    for_each_stile(record_tiles(a, r), [&](uint32_t st) {
         const uint32_t active = __activemask();
         const uint32_t peers = __match_any_sync(active, st);
         const int leader = __ffs(peers) - 1;
@@ -1116,10 +1222,34 @@ __device__ __forceinline__ void scatter_slot(const FrameArgs& a, uint32_t slot, 
     });
 }
 
+// One segment of a wide triangle: the warp's lanes take its tiles, each with
+// kWideSegment / 32 independent cursor additions in flight (one thread per
+// triangle waited for one after another, 145 us for the 106k triangles of a
+// 1367x769 frame).
+__device__ __forceinline__ void scatter_wide(const FrameArgs& a, uint2 q) {
+    const RecRaster* r = wide_record(a, q);
+    if (!r) return;
+    const TileRect t = record_tiles(a, *r);
+    const uint32_t n = t.count(), k0 = q.y * kWideSegment + (threadIdx.x & 31u);
+    uint32_t at[kWideSegment / 32];
+#pragma unroll
+    for (uint32_t j = 0; j < kWideSegment / 32; ++j)
+        if (k0 + 32u * j < n) at[j] = atomicAdd(a.tile_cursor + t.tile(k0 + 32u * j), 1u);
+#pragma unroll
+    for (uint32_t j = 0; j < kWideSegment / 32; ++j)
+        if (k0 + 32u * j < n) a.bins[at[j]] = q.x;
+}
+
 __global__ void k_scatter(FrameArgs a) {
     if (a.counters->status & (ST_BIN_OVERFLOW | ST_CLIP_OVERFLOW | ST_QUEUE_OVERFLOW)) return;
     const uint32_t tri_total = a.dyn->tri_total;
     const uint32_t n = tri_total + min(a.counters->extra_used, a.extra_cap);
+    for (uint32_t half = 0; half < 2u; ++half) {
+        const uint32_t nwide = min(half ? a.counters->wide_clip : a.counters->wide_main, a.wide_cap);
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        for (uint32_t e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); e < nwide; e += warps)
+            scatter_wide(a, a.wide_queue[half * a.wide_cap + e]);
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         scatter_slot(a, i, tri_total);
 }
@@ -2465,7 +2595,7 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
         launches++;
     }
     mark(2);
-    k_clip<<<num_sms * 4, 128, 0, s>>>(a);
+    k_clip<<<num_sms * 4, kClipThreads, 0, s>>>(a);
     mark(3);
     k_scan<<<1, 1024, 0, s>>>(a);
     launches += 2;

@@ -148,7 +148,7 @@ void FrameEngine::release() {
     graph_exec = nullptr;
     if (capture_stream) cudaStreamDestroy(capture_stream);
     capture_stream = nullptr;
-    for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &fan_base, &clip_queue, &tile_count, &tile_offset,
+    for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &fan_base, &clip_queue, &wide_queue, &tile_count, &tile_offset,
                     &tile_cursor, &bins, &keys, &counters, &rsqrt_tab, &color})
         b->release();
     for (int i = 0; i < kStageRing; ++i) {
@@ -251,6 +251,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     chk(rec_s.ensure(slots * sizeof(RecShade)));
     chk(fan_base.ensure((size_t)tri_cap * sizeof(uint32_t)));
     chk(clip_queue.ensure((size_t)tri_cap * sizeof(uint2)));
+    chk(wide_queue.ensure(2u * kWideCap * sizeof(uint2)));
     chk(tile_count.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
     chk(tile_offset.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
     chk(tile_cursor.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
@@ -326,6 +327,8 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     a.rec_s = rec_s.as<RecShade>();
     a.fan_base = fan_base.as<uint32_t>();
     a.clip_queue = clip_queue.as<uint2>();
+    a.wide_queue = wide_queue.as<uint2>();
+    a.wide_cap = kWideCap;
     a.tile_count = tile_count.as<uint32_t>();
     a.tile_offset = tile_offset.as<uint32_t>();
     a.tile_cursor = tile_cursor.as<uint32_t>();

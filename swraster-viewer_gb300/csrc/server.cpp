@@ -133,7 +133,7 @@ struct swr_server {
     static uint64_t one_engine_bytes(const Engine& e) {
         const FrameEngine& f = e.b->eng;
         uint64_t t = e.b->tile_lum.bytes;
-        for (const DBuf* d : {&f.tables, &f.tri_state, &f.rec_r, &f.rec_s, &f.fan_base, &f.clip_queue,
+        for (const DBuf* d : {&f.tables, &f.tri_state, &f.rec_r, &f.rec_s, &f.fan_base, &f.clip_queue, &f.wide_queue,
                               &f.tile_count, &f.tile_offset, &f.tile_cursor, &f.bins, &f.keys, &f.counters,
                               &f.rsqrt_tab, &f.color})
             t += d->bytes;
