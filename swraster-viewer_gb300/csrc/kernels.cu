@@ -1679,7 +1679,8 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
 // bin's packets go through rounds of one packet per thread: pass 1 stages
 // regions (a block-wide scan places them), pass 2 rasterizes the exact
 // regions' quads flattened over all lanes, pass 3 the sequential regions.
-template <int S, bool FUSE>
+// GI and MODE: the fused shading's variant (see k_shade); unused without FUSE.
+template <int S, bool FUSE, bool GI, int MODE>
 __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kMinBlocks) k_raster(FrameArgs a) {
     using Sh = RasterShared<S>;
     constexpr int NT = Sh::kThreads, R = Sh::kRegions, NW = NT / 32;
@@ -1864,7 +1865,7 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
             const bool needed = live && shade_needed(view, qx, qy);
             unsigned long long key = kEmptyKey;
             if (needed) key = s.sk[(2 * (ql / QS) + (k >> 1)) * S + 2 * (ql % QS) + (k & 1)];
-            shade_pixel<true, kModeAny>(a, s.tab, view, sc, qx, qy, k, needed, key);
+            shade_pixel<GI, MODE>(a, s.tab, view, sc, qx, qy, k, needed, key);
         }
         __syncthreads();
     }
@@ -2513,10 +2514,36 @@ __global__ void k_resolve(FrameArgs a) {
 // --------------------------------------------------------------------------
 static uint64_t g_const_init_mask = 0;  // one bit per device
 
-template <int S, bool FUSE>
+template <int S, bool FUSE, bool GI, int MODE>
 static cudaError_t raster_smem_attr() {
-    return cudaFuncSetAttribute(k_raster<S, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_raster<S, FUSE, GI, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(RasterShared<S>));
+}
+template <int S>
+static cudaError_t fused_smem_attr() {
+    cudaError_t e = raster_smem_attr<S, true, false, kModeArm>();
+    if (e == cudaSuccess) e = raster_smem_attr<S, true, false, kModeAny>();
+    if (e == cudaSuccess) e = raster_smem_attr<S, true, true, kModeArm>();
+    if (e == cudaSuccess) e = raster_smem_attr<S, true, true, kModeAny>();
+    return e;
+}
+template <int S, bool FUSE, bool GI, int MODE>
+static void launch_raster(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
+    k_raster<S, FUSE, GI, MODE><<<grid, RasterShared<S>::kThreads, sizeof(RasterShared<S>), s>>>(a);
+}
+// The fused shading compiled for what the frame needs: the variant for baked
+// grids of any rsqrt mode spills 250-450 B a thread against 0-130 B, and
+// every fused frame ran it (64 batched views 5% slower, 1280x720 2%).
+template <int S>
+static void launch_fused(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
+    const bool arm = a.rsqrt_uniform == 1u + kModeArm;
+    if (a.has_gi) {
+        if (arm) launch_raster<S, true, true, kModeArm>(a, grid, s);
+        else launch_raster<S, true, true, kModeAny>(a, grid, s);
+    } else {
+        if (arm) launch_raster<S, true, false, kModeArm>(a, grid, s);
+        else launch_raster<S, true, false, kModeAny>(a, grid, s);
+    }
 }
 
 cudaError_t init_kernel_constants() {
@@ -2524,11 +2551,11 @@ cudaError_t init_kernel_constants() {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 64 && (g_const_init_mask >> dev) & 1ull) return cudaSuccess;
-    e = raster_smem_attr<8, true>();
-    if (e == cudaSuccess) e = raster_smem_attr<16, true>();
-    if (e == cudaSuccess) e = raster_smem_attr<32, false>();
-    if (e == cudaSuccess) e = raster_smem_attr<32, true>();
-    if (e == cudaSuccess) e = raster_smem_attr<64, false>();
+    e = fused_smem_attr<8>();
+    if (e == cudaSuccess) e = fused_smem_attr<16>();
+    if (e == cudaSuccess) e = fused_smem_attr<32>();
+    if (e == cudaSuccess) e = raster_smem_attr<32, false, false, kModeAny>();
+    if (e == cudaSuccess) e = raster_smem_attr<64, false, false, kModeAny>();
     if (e == cudaSuccess && dev < 64) g_const_init_mask |= 1ull << dev;
     return e;
 }
@@ -2536,7 +2563,8 @@ cudaError_t init_kernel_constants() {
 template <int S, bool FUSE>
 static int raster_blocks_per_sm() {
     int rb = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rb, k_raster<S, FUSE>, RasterShared<S>::kThreads,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rb, k_raster<S, FUSE, false, FUSE ? kModeArm : kModeAny>,
+                                                  RasterShared<S>::kThreads,
                                                   sizeof(RasterShared<S>));
     return rb;
 }
@@ -2614,15 +2642,13 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
     const uint32_t rg = SWR_RASTER_PERSISTENT ? (a.raster_grid > 0 ? a.raster_grid : (uint32_t)num_sms)
                                               : (a.stile_cap > 0 ? a.stile_cap : 1u);
     switch (a.sched_tile) {
-        case 8: k_raster<8, true><<<rg, RasterShared<8>::kThreads, sizeof(RasterShared<8>), s>>>(a); break;
-        case 16: k_raster<16, true><<<rg, RasterShared<16>::kThreads, sizeof(RasterShared<16>), s>>>(a); break;
+        case 8: launch_fused<8>(a, rg, s); break;
+        case 16: launch_fused<16>(a, rg, s); break;
         case 32:
-            if (a.fused_shade)
-                k_raster<32, true><<<rg, RasterShared<32>::kThreads, sizeof(RasterShared<32>), s>>>(a);
-            else
-                k_raster<32, false><<<rg, RasterShared<32>::kThreads, sizeof(RasterShared<32>), s>>>(a);
+            if (a.fused_shade) launch_fused<32>(a, rg, s);
+            else launch_raster<32, false, false, kModeAny>(a, rg, s);
             break;
-        default: k_raster<64, false><<<rg, RasterShared<64>::kThreads, sizeof(RasterShared<64>), s>>>(a); break;
+        default: launch_raster<64, false, false, kModeAny>(a, rg, s); break;
     }
     launches++;
     mark(6);
