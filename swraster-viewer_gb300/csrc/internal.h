@@ -21,6 +21,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 namespace swr {
@@ -44,22 +45,22 @@ struct alignas(16) DPrimitive {
     uint32_t material;
 };
 
+// One mip of a texture, two 16-byte loads a sample.
+struct alignas(16) DMip {
+    float wf, hf;              // size
+    // 1 / wf (1 / hf) when that size is a power of two, else 0: a division
+    // by 2^k and a multiplication by 2^-k round the same exact value.
+    float rwf, rhf;
+    uint32_t offset;           // relative to DTexture.data
+    uint32_t w, h;
+    uint32_t stride;           // texels per array slice (cubemap face)
+};
 struct alignas(16) DTexture {
     const uint32_t* data;      // device pointer to mip 0 of this texture
-    uint32_t width, height;
     uint32_t max_mip;
-    uint32_t pad0;
+    uint32_t pad;
     float whv[4];              // width_height_vec
-    uint32_t mip_offset[16];   // relative to data
-    uint32_t mip_w[16];
-    uint32_t mip_h[16];
-    uint32_t array_stride[16];
-    float mip_wf[16];
-    float mip_hf[16];
-    // 1 / mip_wf (1 / mip_hf) when that size is a power of two, else 0: a
-    // division by 2^k and a multiplication by 2^-k round the same exact value.
-    float mip_rwf[16];
-    float mip_rhf[16];
+    DMip mip[16];
 };
 
 enum : uint32_t {
@@ -70,17 +71,17 @@ enum : uint32_t {
 // Texture slots inside DMaterial.tex.
 enum { TS_BASE = 0, TS_MR = 1, TS_NORMAL = 2, TS_EMISSIVE = 3, TS_OCCLUSION = 4, TS_TRANSMISSION = 5 };
 
+// Read as 16-byte vectors by the shading (load_material).
 struct alignas(16) DMaterial {
     float base_color[4];
     float metallic, roughness, occlusion_strength, alpha_cutoff;
     float emissive[3];
     uint32_t flags;
     int32_t tex[6];            // index into scene texture table, -1 none
-    uint32_t wrap_s[6];
-    uint32_t wrap_t[6];
+    uint32_t wrap;             // per slot four bits: wrap_s | wrap_t << 2
     float transmission;
-    uint32_t pad[1];
 };
+static_assert(sizeof(DMaterial) == 80, "DMaterial layout");
 
 // Draw-list inputs (render_node / render_mesh, src/renderer.rs:357-420),
 // laid out so one node needs two dependent reads: per node its world
@@ -105,28 +106,38 @@ struct alignas(16) DMeshEntry {
 // Scene-wide device constants. The per-voxel SH4 of the non-GI path is
 // the same for every voxel (src/gi.rs:123-149): rgb = irradiance_sh * scale,
 // w0 = light intensity (per voxel), w1 = sky visibility, w2 = w3 = 0.
+// The kernels that shade keep a copy in shared memory; the groups of four
+// floats are read as vectors.
 struct alignas(16) DScene {
+    float voxel_min[3];
+    uint32_t voxel_n;
+    float voxel_size_f[3];     // (max - min) / n per axis
+    float sky_visibility;
+    float gi_rgb[4][3];
+    float light_dir[3];
+    float spec_max_mip;        // specular->max_mip
+    float light_color[3];
+    uint32_t brdf_w;           // width of brdf_lut
+    float brdf_wf, brdf_hf;    // its size
+    float sky_wf, sky_hf;      // cubemap face size
+    uint32_t sky_w, sky_stride;
+    const uint32_t* brdf_lut;  // mip 0 texels
+    const uint32_t* sky;       // cubemap mip 0 texels
+    const DTexture* specular;  // prefiltered environment
+    const float* voxel_light;  // voxel_n^3
+    const float4* voxel_sh4;   // baked GI: voxel_n^3 x 4 (r, g, b, w), or null (constant SH form)
+    const DMaterial* materials;
+    const DTexture* textures;  // scene textures, then cubemap, specular, brdf lut
     const DVertex* vertices;
     const uint32_t* indices;
     const DPrimitive* prims;
     const float* node_xform;   // 16 floats per node
-    const DMaterial* materials;
-    const DTexture* textures;  // scene textures, then cubemap, specular, brdf lut
-    const float* voxel_light;  // voxel_n^3
     const DNodeInfo* node_info;
     const DMeshEntry* mesh_entries;
-    const float4* voxel_sh4;   // baked GI: voxel_n^3 x 4 (r, g, b, w), or null (constant SH form)
-    uint32_t tex_cubemap, tex_specular, tex_brdf_lut, voxel_n;
-    float voxel_min[3];
-    float voxel_size_f[3];     // (max - min) / n per axis
-    float gi_rgb[4][3];
-    float sky_visibility;
-    float light_dir[3];
-    float light_color[3];
-    float pad[3];
 };
 
-// One view (camera + resolution + outputs).
+// One view (camera + resolution + outputs); the kernels that shade keep the
+// part before cam_view in shared memory.
 struct alignas(16) DView {
     float skybox_t[16];        // RenderCamera::skybox_matrix_transposed
     float cam_pos[3];
@@ -151,15 +162,19 @@ struct alignas(16) DView {
     uint32_t out_pitch;
     uint32_t host_pitch;       // row pitch of rgba8_host
     uint32_t* rgba8_host;      // device-writable host copy of rgba8 (rows below height & ~1), or null
+    uint32_t tiles_x_magic;    // ceil(2^32 / tiles_x), 0 when tiles_x == 1 (quad row = (q >> 5) * magic >> 32)
+    uint32_t pad2[3];
     // Camera of the device draw-list build (RenderCamera, src/rendercamera.rs).
     float cam_view[16];
     float cam_view_project[16];
     float cam_planes[24];      // view_clip_planes, view space
     uint32_t order_base;       // this view's sorted nodes in FrameArgs.node_order
     uint32_t n_order;
-    uint32_t tiles_x_magic;    // ceil(2^32 / tiles_x), 0 when tiles_x == 1 (quad row = (q >> 5) * magic >> 32)
-    uint32_t pad3;
+    uint32_t pad3[2];
 };
+
+constexpr uint32_t kViewHead = offsetof(DView, cam_view);
+static_assert(kViewHead % 16 == 0 && sizeof(DScene) % 16 == 0, "copied as 16-byte vectors");
 
 // DView.flags
 constexpr uint32_t kViewLinear = 1u;       // caller wants linear colour (exposure applied later)

@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "depthfloor.cuh"
 #include "devmath.cuh"
@@ -132,13 +133,13 @@ __device__ __forceinline__ uint32_t mip_level(const DTexture& t, float d0, float
     return mip < t.max_mip ? mip : t.max_mip;
 }
 
-__device__ __forceinline__ uint32_t sample_texel(const DTexture& t, float u, float v, uint32_t mip, uint32_t ws,
-                                                 uint32_t wt) {
-    const float wf = t.mip_wf[mip], hf = t.mip_hf[mip];
-    const uint32_t x = f2u_sat(apply_wrap(floorf(u * wf), wf, t.mip_rwf[mip], ws));
-    const uint32_t y = f2u_sat(apply_wrap(floorf(v * hf), hf, t.mip_rhf[mip], wt));
-    const uint32_t idx = t.mip_offset[mip] + y * t.mip_w[mip] + x;
-    return __ldg(t.data + idx);
+// wrap: wrap_s | wrap_t << 2.
+__device__ __forceinline__ uint32_t sample_texel(const DTexture& t, float u, float v, uint32_t mip, uint32_t wrap) {
+    const float4 d = __ldg(reinterpret_cast<const float4*>(t.mip + mip));      // wf, hf, rwf, rhf
+    const uint2 o = __ldg(reinterpret_cast<const uint2*>(&t.mip[mip].offset));  // offset, w
+    const uint32_t x = f2u_sat(apply_wrap(floorf(u * d.x), d.x, d.z, wrap & 3u));
+    const uint32_t y = f2u_sat(apply_wrap(floorf(v * d.y), d.y, d.w, (wrap >> 2) & 3u));
+    return __ldg(t.data + (o.x + y * o.y + x));
 }
 
 // cubemap_uv_from_normal (src/texture.rs:593-644).
@@ -164,23 +165,24 @@ __device__ __forceinline__ void cube_uv(f3 n, float& uf, float& vf, uint32_t& sl
     slice = mx ? ix : (my ? iy : iz);
 }
 
-// sample_cubemap_rgb (src/texture.rs:646-663): nearest texel at one mip.
-__device__ __forceinline__ f3 sample_cube(const DTexture& t, float uf, float vf, uint32_t slice, uint32_t mip) {
-    if (mip > t.max_mip) mip = t.max_mip;
-    const float wf = t.mip_wf[mip], hf = t.mip_hf[mip];
-    const uint32_t off = t.mip_offset[mip] + slice * t.array_stride[mip];
+// sample_cubemap_rgb (src/texture.rs:646-663): nearest texel of one mip
+// (its texels, face size and stride).
+__device__ __forceinline__ f3 sample_cube(const uint32_t* data, float wf, float hf, uint32_t w, uint32_t stride,
+                                          float uf, float vf, uint32_t slice) {
     float x = round_away(uf * (wf - 1.0f));
     float y = round_away(vf * (hf - 1.0f));
     x = clampf(x, 0.0f, wf - 1.0f);
     y = clampf(y, 0.0f, hf - 1.0f);
-    const uint32_t idx = off + f2u_sat(y) * t.mip_w[mip] + f2u_sat(x);
-    return unpack_rgb(__ldg(t.data + idx));
+    return unpack_rgb(__ldg(data + (slice * stride + f2u_sat(y) * w + f2u_sat(x))));
+}
+__device__ __forceinline__ f3 sample_cube(const DTexture& t, float uf, float vf, uint32_t slice, uint32_t mip) {
+    const float2 d = __ldg(reinterpret_cast<const float2*>(t.mip + mip));
+    const uint4 o = __ldg(reinterpret_cast<const uint4*>(&t.mip[mip].offset));  // offset, w, h, stride
+    return sample_cube(t.data + o.x, d.x, d.y, o.y, o.w, uf, vf, slice);
 }
 
 // sample_bilinear_rgb at mip 0, slice 0 (src/texture.rs:730-790); ClampToEdge.
-__device__ __forceinline__ f3 sample_bilinear(const DTexture& t, float u, float v) {
-    const float wf = t.mip_wf[0], hf = t.mip_hf[0];
-    const uint32_t wi = t.mip_w[0];
+__device__ __forceinline__ f3 sample_bilinear(const uint32_t* data, float wf, float hf, uint32_t wi, float u, float v) {
     const float xf = u * wf - 0.5f;
     const float yf = v * hf - 0.5f;
     const float x0 = floorf(xf), y0 = floorf(yf);
@@ -191,11 +193,10 @@ __device__ __forceinline__ f3 sample_bilinear(const DTexture& t, float u, float 
     const uint32_t y0i = f2u_sat(apply_wrap(y0, hf, 0.0f, 2u));
     const uint32_t x1i = f2u_sat(apply_wrap(x1, wf, 0.0f, 2u));
     const uint32_t y1i = f2u_sat(apply_wrap(y1, hf, 0.0f, 2u));
-    const uint32_t off = t.mip_offset[0];
-    const f3 p00 = unpack_rgb(__ldg(t.data + off + y0i * wi + x0i));
-    const f3 p10 = unpack_rgb(__ldg(t.data + off + y0i * wi + x1i));
-    const f3 p01 = unpack_rgb(__ldg(t.data + off + y1i * wi + x0i));
-    const f3 p11 = unpack_rgb(__ldg(t.data + off + y1i * wi + x1i));
+    const f3 p00 = unpack_rgb(__ldg(data + (y0i * wi + x0i)));
+    const f3 p10 = unpack_rgb(__ldg(data + (y0i * wi + x1i)));
+    const f3 p01 = unpack_rgb(__ldg(data + (y1i * wi + x0i)));
+    const f3 p11 = unpack_rgb(__ldg(data + (y1i * wi + x1i)));
     const float w00 = ofx * ofy, w10 = fx * ofy, w01 = ofx * fy, w11 = fx * fy;
     return {((p00.x * w00 + p10.x * w10) + p01.x * w01) + p11.x * w11,
             ((p00.y * w00 + p10.y * w10) + p01.y * w01) + p11.y * w11,
@@ -1273,7 +1274,7 @@ __device__ __forceinline__ bool alpha_pass(const DScene& sc, const DMaterial& m,
     const DTexture& t = sc.textures[m.tex[TS_BASE]];
     const float u = interp(q.uow, b1, b2) * w;
     const float v = interp(q.vow, b1, b2) * w;
-    const uint32_t tx = sample_texel(t, u, v, mip, m.wrap_s[TS_BASE], m.wrap_t[TS_BASE]);
+    const uint32_t tx = sample_texel(t, u, v, mip, m.wrap >> (4 * TS_BASE));
     return unorm8(tx << 15) >= m.alpha_cutoff;
 }
 
@@ -1395,6 +1396,25 @@ __device__ __forceinline__ bool region_exact(const PacketCtx& c, const float w[1
     return ok;
 }
 
+// What shading reads of its view and scene, in shared memory: the compiler
+// read some forty of these fields from global memory again for every pixel
+// (stores to the frame might have changed them); now they are broadcast
+// vector loads.
+struct alignas(16) ShadeConst {
+    DScene scene;
+    unsigned char head[kViewHead];  // the part of the DView before cam_view
+    __device__ __forceinline__ const DView& view() const { return *reinterpret_cast<const DView*>(head); }
+};
+__device__ __forceinline__ void load_shade_const(ShadeConst& c, const FrameArgs& a, uint32_t vi, uint32_t t, uint32_t nt) {
+    const DView* v = a.views + vi;
+    const uint4* s0 = reinterpret_cast<const uint4*>(a.scenes + v->scene);
+    const uint4* s1 = reinterpret_cast<const uint4*>(v);
+    uint4* d0 = reinterpret_cast<uint4*>(&c.scene);
+    uint4* d1 = reinterpret_cast<uint4*>(c.head);
+    for (uint32_t i = t; i < sizeof(DScene) / 16; i += nt) d0[i] = s0[i];
+    for (uint32_t i = t; i < kViewHead / 16; i += nt) d1[i] = s1[i];
+}
+
 template <int S>
 struct RasterShared {
     static constexpr int kThreads = S <= 16 ? 128 : 256;
@@ -1417,8 +1437,16 @@ struct RasterShared {
     uint32_t scan[kThreads / 32][2];
     uint32_t cell_far[(S / 8) * (S / 8)];  // farthest key depth of each 8x8-px cell (orderable bits)
     uint32_t n_regions, n_quads, n_slow, cur_tile;
-    uint8_t tab[512];           // FRSQRTE table for the fused shading
 };
+// With the fused shading's FRSQRTE table, view and scene. (The 64-px kernel
+// shades apart, and three of its CTAs fill an SM's shared memory.)
+template <int S>
+struct FusedShared : RasterShared<S> {
+    uint8_t tab[512];
+    ShadeConst shade;
+};
+template <int S, bool FUSE>
+using RasterSmem = std::conditional_t<FUSE, FusedShared<S>, RasterShared<S>>;
 
 constexpr uint32_t kSlowRegion = 0x8000u;  // region replays the sequential additions
 
@@ -1682,7 +1710,7 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
 // GI and MODE: the fused shading's variant (see k_shade); unused without FUSE.
 template <int S, bool FUSE, bool GI, int MODE>
 __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kMinBlocks) k_raster(FrameArgs a) {
-    using Sh = RasterShared<S>;
+    using Sh = RasterSmem<S, FUSE>;
     constexpr int NT = Sh::kThreads, R = Sh::kRegions, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char raster_smem[];
     Sh& s = *reinterpret_cast<Sh*>(raster_smem);
@@ -1695,9 +1723,9 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
     // of packets, whole instead: 4K 718 against 728 frames/s).
     constexpr bool kCull = S >= SWR_CULL_MIN_TILE;
     constexpr uint32_t kFirst = (kCull && SWR_CULL_FIRST > 0 && SWR_CULL_FIRST < NT) ? SWR_CULL_FIRST : NT;
-    if (kFuse)
+    if constexpr (kFuse)
         for (int i = threadIdx.x; i < 512; i += NT) s.tab[i] = a.rsqrt_table[i];
-    uint32_t n_culled = 0;
+    uint32_t n_culled = 0, held = 0xFFFFFFFFu;
     for (uint32_t iter = 0;; ++iter) {
 #if SWR_RASTER_PERSISTENT
         if (threadIdx.x == 0) {
@@ -1718,6 +1746,10 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
         const int32_t sy0 = (int32_t)(local / (uint32_t)view.stiles_x) * S;
         const int32_t tx0 = (sx0 / kRefTile) * kRefTile, ty0 = (sy0 / kRefTile) * kRefTile;
         for (int i = threadIdx.x; i < S * S; i += NT) s.sk[i] = kEmptyKey;
+        if constexpr (kFuse) {
+            if (vi != held) load_shade_const(s.shade, a, vi, threadIdx.x, NT);  // read after the barrier before the shading
+            held = vi;
+        }
         const bool bad = (a.counters->status & (ST_BIN_OVERFLOW | ST_CLIP_OVERFLOW | ST_QUEUE_OVERFLOW)) != 0u;
         const uint32_t b0 = a.tile_offset[st], b1 = bad ? b0 : a.tile_offset[st + 1];
         const DScene& sc = a.scenes[view.scene];
@@ -1855,17 +1887,19 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
         constexpr int QS = S / 2;
         // Lanes read keys other threads initialised or wrote: a tile without
         // packets has had no barrier since the keys were reset.
-        if (kFuse) __syncthreads();
-        for (int base = 0; kFuse && base < S * S; base += NT) {
-            const int t = base + (int)threadIdx.x;
-            const bool live = t < S * S;
-            const int ql = live ? (t >> 2) : 0;
-            const int32_t k = t & 3;
-            const int32_t qx = (sx0 >> 1) + ql % QS, qy = (sy0 >> 1) + ql / QS;
-            const bool needed = live && shade_needed(view, qx, qy);
-            unsigned long long key = kEmptyKey;
-            if (needed) key = s.sk[(2 * (ql / QS) + (k >> 1)) * S + 2 * (ql % QS) + (k & 1)];
-            shade_pixel<GI, MODE>(a, s.tab, view, sc, qx, qy, k, needed, key);
+        if constexpr (kFuse) {
+            __syncthreads();
+            for (int base = 0; base < S * S; base += NT) {
+                const int t = base + (int)threadIdx.x;
+                const bool live = t < S * S;
+                const int ql = live ? (t >> 2) : 0;
+                const int32_t k = t & 3;
+                const int32_t qx = (sx0 >> 1) + ql % QS, qy = (sy0 >> 1) + ql / QS;
+                const bool needed = live && shade_needed(s.shade.view(), qx, qy);
+                unsigned long long key = kEmptyKey;
+                if (needed) key = s.sk[(2 * (ql / QS) + (k >> 1)) * S + 2 * (ql % QS) + (k & 1)];
+                shade_pixel<GI, MODE>(a, s.tab, s.shade.view(), s.shade.scene, qx, qy, k, needed, key);
+            }
         }
         __syncthreads();
     }
@@ -1901,7 +1935,7 @@ __device__ __forceinline__ f3 skybox(const DView& v, const DScene& sc, int32_t q
     float uf, vf;
     uint32_t slice;
     cube_uv(n, uf, vf, slice);
-    return srgb_fast3(sample_cube(sc.textures[sc.tex_cubemap], uf, vf, slice, 0u));
+    return srgb_fast3(sample_cube(sc.sky, sc.sky_wf, sc.sky_hf, sc.sky_w, sc.sky_stride, uf, vf, slice));
 }
 
 // get_filtered_gi_sh4_packed_vec over the baked grid: every coefficient's
@@ -1988,19 +2022,33 @@ __device__ void voxel_gi(const DScene& sc, f3 pos, f3 sh[4], float& w0, float& w
     }
 }
 
+// A material in registers, read as 16-byte vectors.
+struct MaterialLane {
+    float4 base, mr, em;  // base colour; metallic, roughness, occlusion strength, -; emissive
+    int4 t0, t1;          // tex[0..3]; tex[4], tex[5], wrap, transmission bits
+    __device__ __forceinline__ int32_t tex(int slot) const {
+        return slot == 0 ? t0.x : slot == 1 ? t0.y : slot == 2 ? t0.z : slot == 3 ? t0.w : slot == 4 ? t1.x : t1.y;
+    }
+};
+__device__ __forceinline__ MaterialLane load_material(const DMaterial* m) {
+    const float4* f = reinterpret_cast<const float4*>(m);
+    const int4* i = reinterpret_cast<const int4*>(m);
+    return MaterialLane{__ldg(f), __ldg(f + 1), __ldg(f + 2), __ldg(i + 3), __ldg(i + 4)};
+}
+
 // One material texture of a lane: quad mip (compute_mip_level) and point
 // sample (sample4_rgb / sample4_alpha lane, src/texture.rs:680-727).
-__device__ __forceinline__ uint32_t sample_slot(const DScene& sc, const DMaterial& m, int slot, float u, float v, const float* du_dv) {
-    const DTexture& t = sc.textures[m.tex[slot]];
+__device__ __forceinline__ uint32_t sample_slot(const DScene& sc, const MaterialLane& m, int slot, float u, float v, const float* du_dv) {
+    const DTexture& t = sc.textures[m.tex(slot)];
     const uint32_t mip = mip_level(t, du_dv[0], du_dv[1], du_dv[2], du_dv[3]);
-    return sample_texel(t, u, v, mip, m.wrap_s[slot], m.wrap_t[slot]);
+    return sample_texel(t, u, v, mip, (uint32_t)m.t1.z >> (4 * slot));
 }
 
 // pbr_shader<TRANS> for one lane (src/shader.rs:110-309). du_dv already holds
 // packet.du_dv * w with component i scaled by lane i's w (Q6 quirk). `cur` is
 // the colour under a translucent fragment. GI: read baked voxel grids.
 template <bool TRANS, bool GI>
-__device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const DMaterial& m, const RecShade& q,
+__device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const MaterialLane& m, const RecShade& q,
                                        float w, float b1, float b2, const float du_dv[4], uint32_t md,
                                        const uint8_t* tab, f3 cur) {
     const float PI = 3.14159265358979f;
@@ -2013,7 +2061,7 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const D
     // The tangent frame only feeds the normal map: without one its two
     // normalisations, interpolations and cross product are not evaluated.
     f3 nw;
-    if (m.tex[TS_NORMAL] < 0) {
+    if (m.tex(TS_NORMAL) < 0) {
         nw = normalize(in_n, md, tab);
     } else {
         const f3 in_t = normalize(interp3(q.tan, b1, b2), md, tab);
@@ -2039,10 +2087,10 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const D
     voxel_gi<GI>(sc, pw, sh, gw0, gw1);
     const float vli = clampf(gw0, 0.0f, 1.0f);
     const float skyv = clampf(gw1, 0.0f, 1.0f);
-    f3 bc = mk3(m.base_color[0], m.base_color[1], m.base_color[2]);
-    if (m.tex[TS_BASE] >= 0) bc = bc * srgb_fast3(unpack_rgb(sample_slot(sc, m, TS_BASE, uvx, uvy, du_dv)));
-    float rough = m.roughness, metal = m.metallic;
-    if (m.tex[TS_MR] >= 0) {
+    f3 bc = mk3(m.base.x, m.base.y, m.base.z);
+    if (m.tex(TS_BASE) >= 0) bc = bc * srgb_fast3(unpack_rgb(sample_slot(sc, m, TS_BASE, uvx, uvy, du_dv)));
+    float rough = m.mr.y, metal = m.mr.x;
+    if (m.tex(TS_MR) >= 0) {
         const f3 s = unpack_rgb(sample_slot(sc, m, TS_MR, uvx, uvy, du_dv));
         rough = rough * s.y;
         metal = metal * s.z;
@@ -2050,9 +2098,9 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const D
     rough = clampf(rough, 0.045f, 1.0f);
     metal = clampf(metal, 0.0f, 1.0f);
     float ao = 1.0f;
-    if (m.tex[TS_OCCLUSION] >= 0) {
+    if (m.tex(TS_OCCLUSION) >= 0) {
         ao = unpack_rgb(sample_slot(sc, m, TS_OCCLUSION, uvx, uvy, du_dv)).x;
-        ao = 1.0f + (ao - 1.0f) * m.occlusion_strength;
+        ao = 1.0f + (ao - 1.0f) * m.mr.z;
     }
     const f3 c004 = mk3(0.04f, 0.04f, 0.04f);
     const f3 f0 = c004 + (bc - c004) * metal;
@@ -2084,11 +2132,10 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const D
     // reflect: self - normal * self.dot(normal) * 2 (src/math.rs:118-120).
     const f3 iv = vn * -1.0f;
     const f3 rd = iv - (nw * dot(iv, nw)) * 2.0f;
-    const DTexture& spec = sc.textures[sc.tex_specular];
-    const float spec_mip = rough * (float)spec.max_mip;
+    const float spec_mip = rough * sc.spec_max_mip;
     f3 env;
     {
-        const float mx = (float)spec.max_mip;
+        const float mx = sc.spec_max_mip;
         const float mp = clampf(spec_mip, 0.0f, mx);
         const float m0 = floorf(mp);
         const float m1 = fminf(m0 + 1.0f, mx);
@@ -2096,19 +2143,19 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const D
         float uf, vf;
         uint32_t slice;
         cube_uv(rd, uf, vf, slice);
-        const f3 c0 = sample_cube(spec, uf, vf, slice, f2u_sat(m0));
-        const f3 c1 = sample_cube(spec, uf, vf, slice, f2u_sat(m1));
+        const f3 c0 = sample_cube(*sc.specular, uf, vf, slice, f2u_sat(m0));
+        const f3 c1 = sample_cube(*sc.specular, uf, vf, slice, f2u_sat(m1));
         env = c0 + (c1 - c0) * t;
     }
-    const f3 lut = sample_bilinear(sc.textures[sc.tex_brdf_lut], clampf(ndv, 0.0f, 1.0f), clampf(rough, 0.0f, 1.0f));
+    const f3 lut = sample_bilinear(sc.brdf_lut, sc.brdf_wf, sc.brdf_hf, sc.brdf_w, clampf(ndv, 0.0f, 1.0f), clampf(rough, 0.0f, 1.0f));
     const f3 bsf = f0 * lut.x + mk3(lut.y, lut.y, lut.y);
     f3 cis = env * bsf;
     const float ao_spec = 1.0f + (ao - 1.0f) * 0.5f;
     cis = cis * (ao_spec * skyv);
     f3 col;
     if (TRANS) {
-        float tr = m.transmission;
-        if (m.tex[TS_TRANSMISSION] >= 0) tr = tr * unpack_rgb(sample_slot(sc, m, TS_TRANSMISSION, uvx, uvy, du_dv)).x;
+        float tr = __int_as_float(m.t1.w);
+        if (m.tex(TS_TRANSMISSION) >= 0) tr = tr * unpack_rgb(sample_slot(sc, m, TS_TRANSMISSION, uvx, uvy, du_dv)).x;
         tr = clampf(tr, 0.0f, 1.0f);
         const float inv = 1.0f - tr;
         col = (((cur * bc) * tr + (cdd + cid) * inv) + cds) + cis;
@@ -2116,8 +2163,8 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const D
         col = ((cdd + cds) + cid) + cis;
     }
     f3 em = one;
-    if (m.tex[TS_EMISSIVE] >= 0) em = srgb_fast3(unpack_rgb(sample_slot(sc, m, TS_EMISSIVE, uvx, uvy, du_dv)));
-    col = col + em * mk3(m.emissive[0], m.emissive[1], m.emissive[2]);
+    if (m.tex(TS_EMISSIVE) >= 0) em = srgb_fast3(unpack_rgb(sample_slot(sc, m, TS_EMISSIVE, uvx, uvy, du_dv)));
+    col = col + em * mk3(m.em.x, m.em.y, m.em.z);
     return col;
 }
 
@@ -2208,7 +2255,7 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
             float dd[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) dd[i] = q.du_dv[i] * wq[i];
-            const DMaterial& m = sc.materials[r.material & kRecMaterialMask];
+            const MaterialLane m = load_material(sc.materials + (r.material & kRecMaterialMask));
             col = pbr_lane<false, GI>(sc, v, m, q, w_own, b1, b2, dd, md, tab, col);
             vis_hi = q.static_id;
             vis_fan = r.seq8 & 7u;
@@ -2263,19 +2310,16 @@ __device__ __forceinline__ void quad_xy(const DView& v, uint32_t lq, int32_t& qx
 
 // One lane of the shading pass over the padded quad grid of every view.
 template <bool GI, int MODE>
-__device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* tab, uint32_t gt, uint32_t total) {
-    const uint32_t gq = gt >> 2;
-    const bool live = gq < total;
-    const uint32_t vi = find_view_by_quad(a, live ? gq : 0u);
-    const DView& v = a.views[vi];
+__device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* tab, const ShadeConst& c, uint32_t gt) {
+    const DView& v = c.view();
     int32_t qx, qy;
-    quad_xy(v, gq - v.quad_base, qx, qy);
+    quad_xy(v, (gt >> 2) - v.quad_base, qx, qy);
     const int32_t k = (int32_t)(gt & 3u);
-    const bool needed = live && shade_needed(v, qx, qy);
+    const bool needed = shade_needed(v, qx, qy);
     unsigned long long key = kEmptyKey;
     if (needed)
         key = a.keys[v.key_offset + (uint64_t)(2 * qy + (k >> 1)) * v.key_pitch + (uint64_t)(2 * qx + (k & 1))];
-    shade_pixel<GI, MODE>(a, tab, v, a.scenes[v.scene], qx, qy, k, needed, key);
+    shade_pixel<GI, MODE>(a, tab, v, c.scene, qx, qy, k, needed, key);
 }
 
 // CTA shape of the grid-stride shading kernel. Without voxel GI, seven
@@ -2291,14 +2335,23 @@ template <bool GI> struct ShadeShape {
 template <bool GI, int MODE>
 __global__ void __launch_bounds__(ShadeShape<GI>::kThreads, ShadeShape<GI>::kMinBlocks) k_shade(FrameArgs a) {
     __shared__ uint8_t tab[512];
+    __shared__ ShadeConst sc;
     for (int i = threadIdx.x; i < 512; i += blockDim.x) tab[i] = a.rsqrt_table[i];
-    __syncthreads();
-    // Every view's quad count is a multiple of 32, so each warp's lanes are
-    // either all live or all past the end (warp-uniform loop).
+    // Every view's quad count is a multiple of 1024 (a 64-px tile), so the
+    // CTA's 32 or 64 quads are one view's and all live.
     const uint32_t total = a.dyn->total_quads;
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < total * 4u; base += stride)
-        shade_thread<GI, MODE>(a, tab, base + threadIdx.x, total);
+    uint32_t held = 0xFFFFFFFFu;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < total * 4u; base += stride) {
+        const uint32_t vi = find_view_by_quad(a, base >> 2);
+        if (vi != held) {
+            __syncthreads();
+            load_shade_const(sc, a, vi, threadIdx.x, blockDim.x);
+            __syncthreads();
+            held = vi;
+        }
+        shade_thread<GI, MODE>(a, tab, sc, base + threadIdx.x);
+    }
 }
 
 __global__ void k_rsqrt_selftest(const float* in, float* out, uint64_t n, uint32_t mode, const uint8_t* table) {
@@ -2464,7 +2517,7 @@ __global__ void __launch_bounds__(kTransThreads) k_translucent(FrameArgs a) {
                 float dd[4];
 #pragma unroll
                 for (int l = 0; l < 4; ++l) dd[l] = qs.du_dv[l] * wl[l];
-                const DMaterial& m = sc.materials[c.r.material & kRecMaterialMask];
+                const MaterialLane m = load_material(sc.materials + (c.r.material & kRecMaterialMask));
 #pragma unroll
                 for (int l = 0; l < 4; ++l)
                     if (mask & (1u << l))
@@ -2517,7 +2570,7 @@ static uint64_t g_const_init_mask = 0;  // one bit per device
 template <int S, bool FUSE, bool GI, int MODE>
 static cudaError_t raster_smem_attr() {
     return cudaFuncSetAttribute(k_raster<S, FUSE, GI, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(RasterShared<S>));
+                                (int)sizeof(RasterSmem<S, FUSE>));
 }
 template <int S>
 static cudaError_t fused_smem_attr() {
@@ -2529,7 +2582,7 @@ static cudaError_t fused_smem_attr() {
 }
 template <int S, bool FUSE, bool GI, int MODE>
 static void launch_raster(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
-    k_raster<S, FUSE, GI, MODE><<<grid, RasterShared<S>::kThreads, sizeof(RasterShared<S>), s>>>(a);
+    k_raster<S, FUSE, GI, MODE><<<grid, RasterShared<S>::kThreads, sizeof(RasterSmem<S, FUSE>), s>>>(a);
 }
 // The fused shading compiled for what the frame needs: the variant for baked
 // grids of any rsqrt mode spills 250-450 B a thread against 0-130 B, and
@@ -2564,8 +2617,7 @@ template <int S, bool FUSE>
 static int raster_blocks_per_sm() {
     int rb = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rb, k_raster<S, FUSE, false, FUSE ? kModeArm : kModeAny>,
-                                                  RasterShared<S>::kThreads,
-                                                  sizeof(RasterShared<S>));
+                                                  RasterShared<S>::kThreads, sizeof(RasterSmem<S, FUSE>));
     return rb;
 }
 

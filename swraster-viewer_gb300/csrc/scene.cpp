@@ -1324,20 +1324,19 @@ struct Arena {
 DTexture to_dtex(const HTexture& t, uintptr_t addr) {
     DTexture d{};
     d.data = reinterpret_cast<const uint32_t*>(addr);
-    d.width = t.width;
-    d.height = t.height;
     d.max_mip = t.max_mip;
     for (int k = 0; k < 4; ++k) d.whv[k] = t.whv[k];
     for (uint32_t m = 0; m <= t.max_mip && m < 16; ++m) {
-        d.mip_offset[m] = t.mip_offsets[m];
-        d.mip_w[m] = t.mip_widths[m];
-        d.mip_h[m] = t.mip_heights[m];
-        d.array_stride[m] = t.array_stride[m];
-        d.mip_wf[m] = t.mip_widths_f[m];
-        d.mip_hf[m] = t.mip_heights_f[m];
+        DMip& k = d.mip[m];
         const uint32_t w = t.mip_widths[m], h = t.mip_heights[m];
-        d.mip_rwf[m] = (w > 0 && (w & (w - 1)) == 0 && (float)w == d.mip_wf[m]) ? 1.0f / (float)w : 0.0f;
-        d.mip_rhf[m] = (h > 0 && (h & (h - 1)) == 0 && (float)h == d.mip_hf[m]) ? 1.0f / (float)h : 0.0f;
+        k.offset = t.mip_offsets[m];
+        k.w = w;
+        k.h = h;
+        k.stride = t.array_stride[m];
+        k.wf = t.mip_widths_f[m];
+        k.hf = t.mip_heights_f[m];
+        k.rwf = (w > 0 && (w & (w - 1)) == 0 && (float)w == k.wf) ? 1.0f / (float)w : 0.0f;
+        k.rhf = (h > 0 && (h & (h - 1)) == 0 && (float)h == k.hf) ? 1.0f / (float)h : 0.0f;
     }
     return d;
 }
@@ -1423,8 +1422,7 @@ swr_status upload_scene(SceneImpl* s, std::string& err, bool to_device) {
         d.flags = (m.is_alpha_tested ? MAT_ALPHA_TESTED : 0u) | (m.is_translucent ? MAT_TRANSLUCENT : 0u);
         for (int k = 0; k < 6; ++k) {
             d.tex[k] = m.tex[k];
-            d.wrap_s[k] = m.wrap_s[k];
-            d.wrap_t[k] = m.wrap_t[k];
+            d.wrap |= (std::min(m.wrap_s[k], 2u) | (std::min(m.wrap_t[k], 2u) << 2)) << (4 * k);
         }
         d.transmission = m.transmission;
         mats.push_back(d);
@@ -1475,9 +1473,19 @@ swr_status upload_scene(SceneImpl* s, std::string& err, bool to_device) {
     ds.voxel_sh4 = s->voxel_sh4.empty() ? nullptr : reinterpret_cast<const float4*>(at(o_sh4));
     ds.node_info = reinterpret_cast<const DNodeInfo*>(at(o_ninfo));
     ds.mesh_entries = reinterpret_cast<const DMeshEntry*>(at(o_entries));
-    ds.tex_cubemap = (uint32_t)s->textures.size();
-    ds.tex_specular = ds.tex_cubemap + 1;
-    ds.tex_brdf_lut = ds.tex_cubemap + 2;
+    const size_t nt = s->textures.size();
+    const DTexture &cube = dtex[nt], &lut = dtex[nt + 2];
+    ds.specular = ds.textures + nt + 1;
+    ds.spec_max_mip = (float)dtex[nt + 1].max_mip;
+    ds.sky = cube.data + cube.mip[0].offset;
+    ds.sky_w = cube.mip[0].w;
+    ds.sky_stride = cube.mip[0].stride;
+    ds.sky_wf = cube.mip[0].wf;
+    ds.sky_hf = cube.mip[0].hf;
+    ds.brdf_lut = lut.data + lut.mip[0].offset;
+    ds.brdf_w = lut.mip[0].w;
+    ds.brdf_wf = lut.mip[0].wf;
+    ds.brdf_hf = lut.mip[0].hf;
     ds.voxel_n = s->voxel_n;
     const V3 wsz = sub(s->voxel_max, s->voxel_min);
     ds.voxel_min[0] = s->voxel_min.x;
