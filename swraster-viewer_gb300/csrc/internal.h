@@ -13,7 +13,8 @@
 //   chunks     DChunk[]     256-triangle slices of draws, one CTA each
 //   tri_state  u8[T]        0 none, 1 record in slot g, 2 clipped
 //   rec_r      RecRaster[T + extra]   80 B: screen vertices, bbox, z/w, 1/w, depth floor
-//   rec_s      RecShade [T + extra]  176 B: shading interpolators
+//   rec_s      RecShade [T + extra]  128 B: shading interpolators
+//   rec_t      RecTangent[T + extra]  48 B: tangents, written under a normal map only
 //   fan_base   u32[T]       first extra slot of a clipped triangle's fans 1..6
 //   bins       u32[cap]     record indices grouped by scheduling tile
 //   keys       u64[pitch*rows] per view: orderable(z) << 32 | ~(seq8 + 1)
@@ -66,6 +67,7 @@ struct alignas(16) DTexture {
 enum : uint32_t {
     MAT_ALPHA_TESTED = 1u,
     MAT_TRANSLUCENT = 2u,
+    MAT_NORMAL_MAP = 4u,
 };
 
 // Texture slots inside DMaterial.tex.
@@ -201,8 +203,7 @@ struct DChunk {
 };
 
 // RecRaster.material carries the alpha-test flag in its top bit and the
-// translucent flag below it; RecShade.pad[0] holds a translucent record's
-// average clip-space z (the sort key).
+// translucent flag below it.
 constexpr uint32_t kRecAlphaBit = 0x80000000u;
 constexpr uint32_t kRecTransBit = 0x40000000u;
 constexpr uint32_t kRecMaterialMask = 0x3FFFFFFFu;
@@ -222,19 +223,25 @@ struct alignas(16) RecRaster {
 };
 static_assert(sizeof(RecRaster) == 80, "RecRaster layout");
 
-// Shading-side record.
-struct alignas(16) RecShade {
+// Shading-side record, one 128-byte line.
+struct alignas(128) RecShade {
     float nrm[9];              // normals a.xyz, da.xyz, db.xyz
-    float tan[9];
-    float tsign[3];
     float uow[3];
     float vow[3];
     float pww[9];              // pos_world_over_w
     float du_dv[4];
     uint32_t static_id;
-    uint32_t pad[3];
+    uint32_t avg_z;            // a translucent record's average clip-space z (float bits, the sort key)
+    uint32_t pad[2];
 };
-static_assert(sizeof(RecShade) == 176, "RecShade layout");
+static_assert(sizeof(RecShade) == 128, "RecShade layout");
+// Tangent interpolators of triangles whose material has a normal map, the
+// only reader.
+struct alignas(16) RecTangent {
+    float tan[9];
+    float tsign[3];
+};
+static_assert(sizeof(RecTangent) == 48, "RecTangent layout");
 
 // Device status word bits.
 enum : uint32_t {
@@ -313,6 +320,7 @@ struct FrameArgs {
     uint8_t* tri_state;
     RecRaster* rec_r;
     RecShade* rec_s;
+    RecTangent* rec_t;
     uint32_t* fan_base;
     uint2* clip_queue;         // (g, draw)
     uint2* wide_queue;         // 2 * wide_cap entries: k_frontend's, then k_clip's

@@ -294,11 +294,11 @@ struct Vtx {
     float u, v;
 };
 
+// tangent: whether the tangent is wanted (only a normal map reads it).
 __device__ __forceinline__ Vtx transform_vertex(const DVertex* __restrict__ vb, uint32_t vi, const float* model,
-                                                const float* mvp) {
+                                                const float* mvp, bool tangent) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(vb + vi));
     const float4 b = __ldg(reinterpret_cast<const float4*>(vb + vi) + 1);
-    const float4 c = __ldg(reinterpret_cast<const float4*>(vb + vi) + 2);
     Vtx o;
     // Mat4 * Vec4 with w = 1: ((c0*x + c1*y) + c2*z) + c3*1 (src/renderer.rs:504-511).
     o.cx = ((mvp[0] * a.x + mvp[4] * a.y) + mvp[8] * a.z) + mvp[12];
@@ -312,10 +312,14 @@ __device__ __forceinline__ Vtx transform_vertex(const DVertex* __restrict__ vb, 
     o.nx = (model[0] * b.x + model[4] * b.y) + model[8] * b.z;
     o.ny = (model[1] * b.x + model[5] * b.y) + model[9] * b.z;
     o.nz = (model[2] * b.x + model[6] * b.y) + model[10] * b.z;
-    o.tx = (model[0] * c.x + model[4] * c.y) + model[8] * c.z;
-    o.ty = (model[1] * c.x + model[5] * c.y) + model[9] * c.z;
-    o.tz = (model[2] * c.x + model[6] * c.y) + model[10] * c.z;
-    o.tw = c.w;
+    o.tx = o.ty = o.tz = o.tw = 0.0f;
+    if (tangent) {
+        const float4 c = __ldg(reinterpret_cast<const float4*>(vb + vi) + 2);
+        o.tx = (model[0] * c.x + model[4] * c.y) + model[8] * c.z;
+        o.ty = (model[1] * c.x + model[5] * c.y) + model[9] * c.z;
+        o.tz = (model[2] * c.x + model[6] * c.y) + model[10] * c.z;
+        o.tw = c.w;
+    }
     o.u = a.w;
     o.v = b.w;
     return o;
@@ -461,10 +465,6 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     q.nrm[0] = v0.nx; q.nrm[1] = v0.ny; q.nrm[2] = v0.nz;
     q.nrm[3] = v1.nx - v0.nx; q.nrm[4] = v1.ny - v0.ny; q.nrm[5] = v1.nz - v0.nz;
     q.nrm[6] = v2.nx - v0.nx; q.nrm[7] = v2.ny - v0.ny; q.nrm[8] = v2.nz - v0.nz;
-    q.tan[0] = v0.tx; q.tan[1] = v0.ty; q.tan[2] = v0.tz;
-    q.tan[3] = v1.tx - v0.tx; q.tan[4] = v1.ty - v0.ty; q.tan[5] = v1.tz - v0.tz;
-    q.tan[6] = v2.tx - v0.tx; q.tan[7] = v2.ty - v0.ty; q.tan[8] = v2.tz - v0.tz;
-    q.tsign[0] = v0.tw; q.tsign[1] = v1.tw - v0.tw; q.tsign[2] = v2.tw - v0.tw;
     q.uow[0] = u0; q.uow[1] = u1 - u0; q.uow[2] = u2 - u0;
     q.vow[0] = w0; q.vow[1] = w1 - w0; q.vow[2] = w2 - w0;
     const float px0 = v0.wx * oow0, py0 = v0.wy * oow0, pz0 = v0.wz * oow0;
@@ -476,8 +476,8 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     q.du_dv[0] = du_dx * s; q.du_dv[1] = du_dy * s; q.du_dv[2] = dv_dx * s; q.du_dv[3] = dv_dy * s;
     q.static_id = static_id;
     // Average z for the per-tile translucency sort (src/renderer.rs:765-774).
-    q.pad[0] = translucent ? __float_as_uint(((v0.cz + v1.cz) + v2.cz) / 3.0f) : 0u;
-    q.pad[1] = q.pad[2] = 0;
+    q.avg_z = translucent ? __float_as_uint(((v0.cz + v1.cz) + v2.cz) / 3.0f) : 0u;
+    q.pad[0] = q.pad[1] = 0u;
     return true;
 }
 
@@ -490,7 +490,14 @@ __device__ __forceinline__ void store_records(const FrameArgs& a, uint32_t slot,
     const float4* sq = reinterpret_cast<const float4*>(&q);
     float4* dq = reinterpret_cast<float4*>(a.rec_s + slot);
 #pragma unroll
-    for (int i = 0; i < 11; ++i) dq[i] = sq[i];
+    for (int i = 0; i < 8; ++i) dq[i] = sq[i];
+}
+__device__ __forceinline__ void store_tangents(const FrameArgs& a, uint32_t slot, const Vtx& v0, const Vtx& v1,
+                                               const Vtx& v2) {
+    float4* d = reinterpret_cast<float4*>(a.rec_t + slot);
+    d[0] = make_float4(v0.tx, v0.ty, v0.tz, v1.tx - v0.tx);
+    d[1] = make_float4(v1.ty - v0.ty, v1.tz - v0.tz, v2.tx - v0.tx, v2.ty - v0.ty);
+    d[2] = make_float4(v2.tz - v0.tz, v0.tw, v1.tw - v0.tw, v2.tw - v0.tw);
 }
 
 // --------------------------------------------------------------------------
@@ -805,9 +812,9 @@ __device__ __forceinline__ bool clip_rejects_all(const Vtx& a, const Vtx& b, con
 
 // Record material word: translucent primitives (no alpha test on their path,
 // src/shader.rs:66-76) or opaque ones with the alpha-test flag.
-__device__ __forceinline__ uint32_t record_material(const DScene& sc, const DDraw& d, uint32_t material) {
+__device__ __forceinline__ uint32_t record_material(uint32_t flags, const DDraw& d, uint32_t material) {
     if (d.translucent) return material | kRecTransBit;
-    return material | ((sc.materials[material].flags & MAT_ALPHA_TESTED) ? kRecAlphaBit : 0u);
+    return material | ((flags & MAT_ALPHA_TESTED) ? kRecAlphaBit : 0u);
 }
 
 __device__ __forceinline__ bool vtx_inside_all(const Vtx& v) {
@@ -833,9 +840,11 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
     const float* model = sc.node_xform + 16u * d.node;
     const uint32_t* ib = sc.indices + pr.idx_base + 3u * local;
     const uint32_t i0 = __ldg(ib), i1 = __ldg(ib + 1), i2 = __ldg(ib + 2);
-    const Vtx v0 = transform_vertex(sc.vertices, pr.vtx_base + i0, model, d.mvp);
-    const Vtx v1 = transform_vertex(sc.vertices, pr.vtx_base + i1, model, d.mvp);
-    const Vtx v2 = transform_vertex(sc.vertices, pr.vtx_base + i2, model, d.mvp);
+    const uint32_t flags = sc.materials[pr.material].flags;
+    const bool tangents = (flags & MAT_NORMAL_MAP) != 0u;
+    const Vtx v0 = transform_vertex(sc.vertices, pr.vtx_base + i0, model, d.mvp, tangents);
+    const Vtx v1 = transform_vertex(sc.vertices, pr.vtx_base + i1, model, d.mvp, tangents);
+    const Vtx v2 = transform_vertex(sc.vertices, pr.vtx_base + i2, model, d.mvp, tangents);
     if (d.clip && !(vtx_inside_all(v0) && vtx_inside_all(v1) && vtx_inside_all(v2))) {
         if (clip_rejects_all(v0, v1, v2)) {  // the clipper would return an empty polygon
             a.tri_state[g] = 3;
@@ -851,7 +860,7 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
         return;
     }
     // All three vertices inside: the clipper would return the triangle unchanged.
-    const uint32_t mword = record_material(sc, d, pr.material);
+    const uint32_t mword = record_material(flags, d, pr.material);
     RecRaster r;
     RecShade q;
     TileRect tiles;
@@ -865,6 +874,7 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
         else
             for_each_stile(tiles, [&](uint32_t st) { agg_inc(a.tile_count, st); });
         store_records(a, g, r, q);
+        if (tangents) store_tangents(a, g, v0, v1, v2);
     }
     a.tri_state[g] = ok ? 1 : 0;
     warp_count(&a.counters->setup_tris, ok);
@@ -936,7 +946,8 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
         const DScene& sc = a.scenes[d.scene];
         const DView& view = a.views[d.view];
         const DPrimitive pr = sc.prims[d.prim];
-        const uint32_t mword = record_material(sc, d, pr.material);
+        const uint32_t flags = sc.materials[pr.material].flags;
+        const uint32_t mword = record_material(flags, d, pr.material);
         const uint32_t* ib = sc.indices + pr.idx_base + 3u * local;
         {
             // Lane i's row of the vertex transform (transform_vertex): clip
@@ -1027,6 +1038,7 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
                     push_wide(a, &a.counters->wide_clip, a.wide_queue + a.wide_cap, slot, tiles.count()))
                     r.wide = 1u;
                 store_records(a, slot, r, q);
+                if (flags & MAT_NORMAL_MAP) store_tangents(a, slot, pl[0], pl[i + 1], pl[i + 2]);
             } else if (i > 0u) {
                 // Mark the unused extra slot so the scatter skips it.
                 a.rec_r[slot].view = 0xFFFFFFFFu;
@@ -2049,6 +2061,7 @@ __device__ __forceinline__ uint32_t sample_slot(const DScene& sc, const Material
 // the colour under a translucent fragment. GI: read baked voxel grids.
 template <bool TRANS, bool GI>
 __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const MaterialLane& m, const RecShade& q,
+                                       const RecTangent* qt,
                                        float w, float b1, float b2, const float du_dv[4], uint32_t md,
                                        const uint8_t* tab, f3 cur) {
     const float PI = 3.14159265358979f;
@@ -2064,9 +2077,16 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const M
     if (m.tex(TS_NORMAL) < 0) {
         nw = normalize(in_n, md, tab);
     } else {
-        const f3 in_t = normalize(interp3(q.tan, b1, b2), md, tab);
+        RecTangent t;
+        {
+            const float4* src = reinterpret_cast<const float4*>(qt);
+            float4* dst = reinterpret_cast<float4*>(&t);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) dst[i] = __ldg(src + i);
+        }
+        const f3 in_t = normalize(interp3(t.tan, b1, b2), md, tab);
         const f3 tw = normalize(in_t - in_n * dot(in_n, in_t), md, tab);
-        const float hand = interp(q.tsign, b1, b2) >= 0.0f ? 1.0f : -1.0f;
+        const float hand = interp(t.tsign, b1, b2) >= 0.0f ? 1.0f : -1.0f;
         const f3 bw = cross(in_n, tw) * hand;
         const f3 s = unpack_rgb(sample_slot(sc, m, TS_NORMAL, uvx, uvy, du_dv));
         const f3 tsn = mk3(s.x * 2.0f - 1.0f, s.y * 2.0f - 1.0f, s.z * 2.0f - 1.0f);
@@ -2250,13 +2270,13 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
                 const float4* src = reinterpret_cast<const float4*>(a.rec_s + slot);
                 float4* dst = reinterpret_cast<float4*>(&q);
 #pragma unroll
-                for (int i = 0; i < 11; ++i) dst[i] = __ldg(src + i);
+                for (int i = 0; i < 8; ++i) dst[i] = __ldg(src + i);
             }
             float dd[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) dd[i] = q.du_dv[i] * wq[i];
             const MaterialLane m = load_material(sc.materials + (r.material & kRecMaterialMask));
-            col = pbr_lane<false, GI>(sc, v, m, q, w_own, b1, b2, dd, md, tab, col);
+            col = pbr_lane<false, GI>(sc, v, m, q, a.rec_t + slot, w_own, b1, b2, dd, md, tab, col);
             vis_hi = q.static_id;
             vis_fan = r.seq8 & 7u;
         } else {
@@ -2436,7 +2456,7 @@ __global__ void __launch_bounds__(kTransThreads) k_translucent(FrameArgs a) {
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
             const uint32_t slot = a.bins[b0 + i];
             tslot[i] = slot;
-            tkey[i] = trans_key(__uint_as_float(a.rec_s[slot].pad[0]), a.rec_r[slot].seq8);
+            tkey[i] = trans_key(__uint_as_float(a.rec_s[slot].avg_z), a.rec_r[slot].seq8);
         }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {  // keys are unique: rank = position
@@ -2512,7 +2532,7 @@ __global__ void __launch_bounds__(kTransThreads) k_translucent(FrameArgs a) {
                     const float4* src = reinterpret_cast<const float4*>(a.rec_s + slot);
                     float4* dst = reinterpret_cast<float4*>(&qs);
 #pragma unroll
-                    for (int t = 0; t < 11; ++t) dst[t] = __ldg(src + t);
+                    for (int t = 0; t < 8; ++t) dst[t] = __ldg(src + t);
                 }
                 float dd[4];
 #pragma unroll
@@ -2521,7 +2541,7 @@ __global__ void __launch_bounds__(kTransThreads) k_translucent(FrameArgs a) {
 #pragma unroll
                 for (int l = 0; l < 4; ++l)
                     if (mask & (1u << l))
-                        col[l] = pbr_lane<true, true>(sc, view, m, qs, wl[l], b1[l], b2[l], dd, view.rsqrt_mode,
+                        col[l] = pbr_lane<true, true>(sc, view, m, qs, a.rec_t + slot, wl[l], b1[l], b2[l], dd, view.rsqrt_mode,
                                                       tab, col[l]);
                 touched = true;
             }

@@ -60,7 +60,8 @@ constexpr size_t oChunks = oDraws + al(sizeof(DDraw) * kNaMaxDraws);
 constexpr size_t oState = oChunks + al(sizeof(DChunk) * kNaMaxChunks);
 constexpr size_t oRecR = oState + al(kNaMaxTris);
 constexpr size_t oRecS = oRecR + al(sizeof(RecRaster) * (kNaMaxTris + kNaExtra));
-constexpr size_t oFan = oRecS + al(sizeof(RecShade) * (kNaMaxTris + kNaExtra));
+constexpr size_t oRecT = oRecS + al(sizeof(RecShade) * (kNaMaxTris + kNaExtra));
+constexpr size_t oFan = oRecT + al(sizeof(RecTangent) * (kNaMaxTris + kNaExtra));
 constexpr size_t oClipQ = oFan + al(sizeof(uint32_t) * kNaMaxTris);
 constexpr size_t oCount = oClipQ + al(sizeof(uint2) * kNaMaxTris);
 constexpr size_t oOffset = oCount + al(sizeof(uint32_t) * (kNaTiles + 1));
@@ -284,6 +285,7 @@ extern "C" swr_status swr_render_frame_noalloc(const swr_scene* scene, const swr
     a.tri_state = base + oState;
     a.rec_r = reinterpret_cast<RecRaster*>(base + oRecR);
     a.rec_s = reinterpret_cast<RecShade*>(base + oRecS);
+    a.rec_t = reinterpret_cast<RecTangent*>(base + oRecT);
     a.fan_base = reinterpret_cast<uint32_t*>(base + oFan);
     a.clip_queue = reinterpret_cast<uint2*>(base + oClipQ);
     a.tile_count = reinterpret_cast<uint32_t*>(base + oCount);

@@ -148,7 +148,7 @@ void FrameEngine::release() {
     graph_exec = nullptr;
     if (capture_stream) cudaStreamDestroy(capture_stream);
     capture_stream = nullptr;
-    for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &fan_base, &clip_queue, &wide_queue, &tile_count, &tile_offset,
+    for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &rec_t, &fan_base, &clip_queue, &wide_queue, &tile_count, &tile_offset,
                     &tile_cursor, &bins, &keys, &counters, &rsqrt_tab, &color})
         b->release();
     for (int i = 0; i < kStageRing; ++i) {
@@ -249,6 +249,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     chk(tri_state.ensure(tri_cap));
     chk(rec_r.ensure(slots * sizeof(RecRaster)));
     chk(rec_s.ensure(slots * sizeof(RecShade)));
+    chk(rec_t.ensure(slots * sizeof(RecTangent)));
     chk(fan_base.ensure((size_t)tri_cap * sizeof(uint32_t)));
     chk(clip_queue.ensure((size_t)tri_cap * sizeof(uint2)));
     chk(wide_queue.ensure(2u * kWideCap * sizeof(uint2)));
@@ -325,6 +326,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     a.tri_state = tri_state.as<uint8_t>();
     a.rec_r = rec_r.as<RecRaster>();
     a.rec_s = rec_s.as<RecShade>();
+    a.rec_t = rec_t.as<RecTangent>();
     a.fan_base = fan_base.as<uint32_t>();
     a.clip_queue = clip_queue.as<uint2>();
     a.wide_queue = wide_queue.as<uint2>();

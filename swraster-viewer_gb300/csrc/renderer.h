@@ -85,7 +85,7 @@ struct FrameEngine {
     uint32_t raster_cta_cap = 0, grid_cap = 0;  // raster CTAs per SM (0: as many as fit; batch autotuner's choice)
     bool fuse32 = false;        // 32-px tiles shade inside the raster kernel (batch autotuner's choice)
     bool grid_fused32 = false;
-    DBuf tables, tri_state, rec_r, rec_s, fan_base, clip_queue, wide_queue;
+    DBuf tables, tri_state, rec_r, rec_s, rec_t, fan_base, clip_queue, wide_queue;
     DBuf tile_count, tile_offset, tile_cursor, bins, keys, counters, rsqrt_tab;
     DBuf color;                // linear colour of views that need it (padded tile grids)
     bool defer_resolve = false;// the caller resolves (renderer frames with dt > 0)

@@ -125,7 +125,7 @@ struct swr_server {
             // (a quarter more), per-slot state, fan bases, clip queue and two
             // bin entries per slot.
             const uint64_t T = tris[i] * 5 / 4 + 16;
-            t += (T + T / 4) * (80 + 176) + T * (1 + 4 + 8) + T * 2 * 4;
+            t += (T + T / 4) * (sizeof(RecRaster) + sizeof(RecShade) + sizeof(RecTangent)) + T * (1 + 4 + 8) + T * 2 * 4;
         }
         return t + (1u << 20);
     }
@@ -133,7 +133,7 @@ struct swr_server {
     static uint64_t one_engine_bytes(const Engine& e) {
         const FrameEngine& f = e.b->eng;
         uint64_t t = e.b->tile_lum.bytes;
-        for (const DBuf* d : {&f.tables, &f.tri_state, &f.rec_r, &f.rec_s, &f.fan_base, &f.clip_queue, &f.wide_queue,
+        for (const DBuf* d : {&f.tables, &f.tri_state, &f.rec_r, &f.rec_s, &f.rec_t, &f.fan_base, &f.clip_queue, &f.wide_queue,
                               &f.tile_count, &f.tile_offset, &f.tile_cursor, &f.bins, &f.keys, &f.counters,
                               &f.rsqrt_tab, &f.color})
             t += d->bytes;
