@@ -68,7 +68,10 @@ enum : uint32_t {
     MAT_ALPHA_TESTED = 1u,
     MAT_TRANSLUCENT = 2u,
     MAT_NORMAL_MAP = 4u,
+    MAT_BOUNDED = 8u,  // base colour finite, at most kBoundedColor
 };
+
+constexpr float kBoundedColor = 1.0e6f;
 
 // Texture slots inside DMaterial.tex.
 enum { TS_BASE = 0, TS_MR = 1, TS_NORMAL = 2, TS_EMISSIVE = 3, TS_OCCLUSION = 4, TS_TRANSMISSION = 5 };

@@ -2098,13 +2098,12 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const M
     const f3 vd = mk3(v.cam_pos[0], v.cam_pos[1], v.cam_pos[2]) - pw;
     const f3 vn = normalize(vd, md, tab);
     const float ndl = fmaxf(dot(nw, ld), 0.0f);
-    const f3 hv = normalize(ld + vn, md, tab);
-    const float ndh = fmaxf(dot(nw, hv), 0.0f);
     const float ndv = fmaxf(dot(nw, vn), 1.0e-4f);
-    const float vdh = fmaxf(dot(vn, hv), 0.0f);
     f3 sh[4];
     float gw0, gw1;
     voxel_gi<GI>(sc, pw, sh, gw0, gw1);
+    f3 irr = ((sh[0] + sh[1] * nw.y) + sh[2] * nw.z) + sh[3] * nw.x;
+    irr = mk3(fmaxf(irr.x, 0.0f), fmaxf(irr.y, 0.0f), fmaxf(irr.z, 0.0f));
     const float vli = clampf(gw0, 0.0f, 1.0f);
     const float skyv = clampf(gw1, 0.0f, 1.0f);
     f3 bc = mk3(m.base.x, m.base.y, m.base.z);
@@ -2124,30 +2123,38 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const M
     }
     const f3 c004 = mk3(0.04f, 0.04f, 0.04f);
     const f3 f0 = c004 + (bc - c004) * metal;
-    const float omvh = 1.0f - vdh;
-    const float omvh2 = omvh * omvh;
-    const float omvh4 = omvh2 * omvh2;
-    const float omvh5 = omvh4 * omvh;
     const f3 one = mk3(1.0f, 1.0f, 1.0f);
-    const f3 fd = f0 + (one - f0) * omvh5;
-    const float alpha = rough * rough;
-    const float alpha2 = alpha * alpha;
-    const float ndh2 = ndh * ndh;
-    const float den_d = ndh2 * (alpha2 - 1.0f) + 1.0f;
-    const float brdf_d = alpha2 / (PI * (den_d * den_d) + EPS);
-    float k = rough + 1.0f;
-    k = (k * k) * 0.125f;
-    const float gv = ndv / ((ndv * (1.0f - k) + k) + EPS);
-    const float gl = ndl / ((ndl * (1.0f - k) + k) + EPS);
-    const float brdf_g = gv * gl;
-    const float spec_dg = (brdf_d * brdf_g) / ((4.0f * ndl) * ndv + EPS);
-    const f3 kd = (one - fd) * (1.0f - metal);
-    const f3 lambert = bc * INV_PI;
-    const f3 cdd = (((lc * kd) * lambert) * ndl) * vli;
-    const f3 cds = (((lc * fd) * spec_dg) * ndl) * vli;
+    // Sunlight. Both terms end in a product with n.l and the sun visibility,
+    // so where one of these is 0 (faces turned away, shadow: whole warps of a
+    // frame) and every other factor is finite (MAT_BOUNDED; the dot products
+    // are clamped, roughness >= 0.045, denominators >= EPS) they are 0.
+    f3 cdd = mk3(0.0f, 0.0f, 0.0f), cds = cdd;
+    if ((ndl > 0.0f && vli > 0.0f) || !(__float_as_uint(m.em.w) & MAT_BOUNDED)) {
+        const f3 hv = normalize(ld + vn, md, tab);
+        const float ndh = fmaxf(dot(nw, hv), 0.0f);
+        const float vdh = fmaxf(dot(vn, hv), 0.0f);
+        const float omvh = 1.0f - vdh;
+        const float omvh2 = omvh * omvh;
+        const float omvh4 = omvh2 * omvh2;
+        const float omvh5 = omvh4 * omvh;
+        const f3 fd = f0 + (one - f0) * omvh5;
+        const float alpha = rough * rough;
+        const float alpha2 = alpha * alpha;
+        const float ndh2 = ndh * ndh;
+        const float den_d = ndh2 * (alpha2 - 1.0f) + 1.0f;
+        const float brdf_d = alpha2 / (PI * (den_d * den_d) + EPS);
+        float k = rough + 1.0f;
+        k = (k * k) * 0.125f;
+        const float gv = ndv / ((ndv * (1.0f - k) + k) + EPS);
+        const float gl = ndl / ((ndl * (1.0f - k) + k) + EPS);
+        const float brdf_g = gv * gl;
+        const float spec_dg = (brdf_d * brdf_g) / ((4.0f * ndl) * ndv + EPS);
+        const f3 kd = (one - fd) * (1.0f - metal);
+        const f3 lambert = bc * INV_PI;
+        cdd = (((lc * kd) * lambert) * ndl) * vli;
+        cds = (((lc * fd) * spec_dg) * ndl) * vli;
+    }
     const f3 kdi = (one - f0) * (1.0f - metal);
-    f3 irr = ((sh[0] + sh[1] * nw.y) + sh[2] * nw.z) + sh[3] * nw.x;
-    irr = mk3(fmaxf(irr.x, 0.0f), fmaxf(irr.y, 0.0f), fmaxf(irr.z, 0.0f));
     const f3 cid = ((irr * bc) * kdi) * INV_PI;
     // reflect: self - normal * self.dot(normal) * 2 (src/math.rs:118-120).
     const f3 iv = vn * -1.0f;

@@ -1419,8 +1419,10 @@ swr_status upload_scene(SceneImpl* s, std::string& err, bool to_device) {
         d.occlusion_strength = m.occlusion_strength;
         d.alpha_cutoff = m.alpha_cutoff;
         for (int k = 0; k < 3; ++k) d.emissive[k] = m.emissive_factor[k];
+        bool bounded = true;  // false for NaN too
+        for (int k = 0; k < 3; ++k) bounded = bounded && std::fabs(d.base_color[k]) <= kBoundedColor;
         d.flags = (m.is_alpha_tested ? MAT_ALPHA_TESTED : 0u) | (m.is_translucent ? MAT_TRANSLUCENT : 0u) |
-                  (m.tex[TS_NORMAL] >= 0 ? MAT_NORMAL_MAP : 0u);
+                  (m.tex[TS_NORMAL] >= 0 ? MAT_NORMAL_MAP : 0u) | (bounded ? MAT_BOUNDED : 0u);
         for (int k = 0; k < 6; ++k) {
             d.tex[k] = m.tex[k];
             d.wrap |= (std::min(m.wrap_s[k], 2u) | (std::min(m.wrap_t[k], 2u) << 2)) << (4 * k);
