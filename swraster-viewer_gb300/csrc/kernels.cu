@@ -2393,7 +2393,7 @@ __global__ void k_rsqrt_selftest(const float* in, float* out, uint64_t n, uint32
 // Translucent forward pass (render_tile, src/tilerasterizer.rs:92-101)
 // --------------------------------------------------------------------------
 constexpr int kTransCap = 2048;  // translucent packets one scheduling tile can sort
-constexpr int kTransThreads = 256;
+constexpr int kTransThreads = 128;
 
 // Sort key of a translucent packet: OrderedFloat avg_z back to front (NaN is
 // the largest value, -0 equals +0), then submission order. The reference's
@@ -2405,47 +2405,90 @@ __device__ __forceinline__ unsigned long long trans_key(float avg_z, uint32_t se
     return ((unsigned long long)(0xFFFFFFFFu - o) << 32) | (unsigned long long)seq8;
 }
 
-// Edge values of a quad's four lanes at quad (i, j) of a region with origin
-// (ox, oy), as fine_raster reaches them: step_y added j times to the origin
-// value, then step_x i times. Closed form where every partial sum is an
-// integer below 2^24 (then exact), else the additions themselves.
-__device__ __forceinline__ void quad_edge_values(const Edge& e, int32_t ox, int32_t oy, int32_t i, int32_t j,
-                                                 float out[4]) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float v = edge_eval(e, i2f(ox + ((k & 1) ? 24 : 8)), i2f(oy + ((k >> 1) ? 24 : 8)));
-        const float b = ru_add(ru_add(fabsf(v), ru_mul((float)j, fabsf(e.sy))), ru_mul((float)i, fabsf(e.sx)));
-        if (b <= 16777216.0f) {
-            v = v + (e.sy * (float)j + e.sx * (float)i);
-        } else {
-            for (int32_t t = 0; t < j; ++t) v += e.sy;
-            for (int32_t t = 0; t < i; ++t) v += e.sx;
-        }
-        out[k] = v;
-    }
+// Edge value of lane k of quad (i, j) of a region with origin (ox, oy), as
+// fine_raster reaches it: step_y added j times to the origin value, then
+// step_x i times. Closed form where every partial sum is an integer below
+// 2^24 (then exact), else the additions themselves.
+__device__ __forceinline__ float lane_edge_value(const Edge& e, int32_t ox, int32_t oy, int32_t i, int32_t j, int32_t k) {
+    float v = edge_eval(e, i2f(ox + ((k & 1) ? 24 : 8)), i2f(oy + ((k >> 1) ? 24 : 8)));
+    const float b = ru_add(ru_add(fabsf(v), ru_mul((float)j, fabsf(e.sy))), ru_mul((float)i, fabsf(e.sx)));
+    if (b <= 16777216.0f) return v + (e.sy * (float)j + e.sx * (float)i);
+    for (int32_t t = 0; t < j; ++t) v += e.sy;
+    for (int32_t t = 0; t < i; ++t) v += e.sx;
+    return v;
 }
 
-// Per scheduling tile, after opaque shading: sort the tile's translucent
-// packets back to front, then every thread walks its own quads through the
-// sorted packets (fine_raster coverage, depth test against the opaque depth,
-// TranslucentForwardShader blend over the current colour; no depth write).
-// Quads are disjoint, so the per-pixel order is the sorted order.
-template <int S>
-__global__ void __launch_bounds__(kTransThreads) k_translucent(FrameArgs a) {
-    __shared__ unsigned long long tkey[kTransCap];
+// Ascending bitonic sort of n distinct keys and their slots in shared memory;
+// m is n's power of two, entries past n are already the largest key.
+template <int NT>
+__device__ __forceinline__ void bitonic_sort(unsigned long long* key, uint32_t* slot, uint32_t m) {
+    for (uint32_t size = 2; size <= m; size *= 2)
+        for (uint32_t d = size / 2; d > 0; d /= 2) {
+            for (uint32_t t = threadIdx.x; t < m / 2; t += NT) {
+                const uint32_t i = 2u * t - (t & (d - 1u)), j = i + d;
+                const bool up = (i & size) == 0u;
+                const unsigned long long x = key[i], y = key[j];
+                if ((x > y) == up) {
+                    key[i] = y;
+                    key[j] = x;
+                    const uint32_t u = slot[i];
+                    slot[i] = slot[j];
+                    slot[j] = u;
+                }
+            }
+            __syncthreads();
+        }
+}
+
+// Per 16x16-px part of a scheduling tile (or the whole 8-px tile), after
+// opaque shading: the bin's translucent packets that reach the part are
+// sorted back to front, then each warp takes 8x4-pixel blocks, a lane per
+// pixel, and walks the sorted packets that reach its block (fine_raster
+// coverage, depth test against the opaque depth, TranslucentForwardShader
+// blend over the current colour; no depth write). Parts, blocks and lanes are
+// disjoint pixels, so the per-pixel order is the sorted order.
+//
+// Issue-bound shading, so the lanes are what counts: a thread per quad that
+// shaded its four pixels one after another ran at 196 registers, one CTA an
+// SM, and walked every packet of the tile (1600x900, 24 glass objects:
+// 1,750 us).
+constexpr int kTransPart = 16;
+constexpr uint32_t kTransRankMax = 256;  // up to this many packets a rank count beats the bitonic passes
+// Rectangle of a packet's quads in a part, five bits a side: x0 | y0 << 5 | x1 << 10 | y1 << 15.
+__device__ __forceinline__ uint32_t part_rect(const RecRaster& r, int32_t tx0, int32_t ty0, int32_t ux, int32_t uy,
+                                              int32_t part) {
+    int32_t x0, y0, x1, y1;
+    clipped_rect(r, tx0, ty0, x0, y0, x1, y1);
+    x0 = max((x0 & ~1) - ux, 0), y0 = max((y0 & ~1) - uy, 0);
+    x1 = min(x1 - ux, part), y1 = min(y1 - uy, part);
+    return x1 > x0 && y1 > y0 ? (uint32_t)(x0 | (y0 << 5) | (x1 << 10) | (y1 << 15)) : 0u;
+}
+
+template <bool GI, int MODE>
+__global__ void __launch_bounds__(kTransThreads, 4) k_translucent(FrameArgs a) {
+    __shared__ unsigned long long tkey[kTransCap];  // sort keys, then (rectangle, blocks) in sorted order
     __shared__ uint32_t tslot[kTransCap];
     __shared__ uint32_t tsorted[kTransCap];
-    __shared__ uint32_t tblk[kTransCap];
     __shared__ uint8_t tab[512];
-    __shared__ uint32_t cur_tile;
-    for (int i = threadIdx.x; i < 512; i += blockDim.x) tab[i] = a.rsqrt_table[i];
+    __shared__ ShadeConst shade;
+    __shared__ uint32_t cur_item, kept;
+    for (int i = threadIdx.x; i < 512; i += kTransThreads) tab[i] = a.rsqrt_table[i];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t S = a.sched_tile;
+    const int32_t part = min((int32_t)S, kTransPart);
+    const uint32_t ppr = S / (uint32_t)part, parts = ppr * ppr;  // parts per tile row, per tile
     const uint32_t n_st = a.dyn->n_stiles;
     const bool bad = (a.counters->status & (ST_BIN_OVERFLOW | ST_CLIP_OVERFLOW | ST_QUEUE_OVERFLOW)) != 0u;
+    uint32_t held = 0xFFFFFFFFu;
+    uint2* const tinfo = reinterpret_cast<uint2*>(tkey);
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) cur_tile = atomicAdd(&a.counters->trans_next, 1u);
+        if (threadIdx.x == 0) {
+            cur_item = atomicAdd(&a.counters->trans_next, 1u);
+            kept = 0u;
+        }
         __syncthreads();
-        const uint32_t st = cur_tile;
+        const uint32_t st = cur_item / parts, sub = cur_item - st * parts;
         if (st >= n_st || bad) break;
         const uint32_t b0 = a.tile_offset[n_st + st], n = a.tile_offset[n_st + st + 1] - b0;
         if (n == 0u) continue;
@@ -2454,119 +2497,139 @@ __global__ void __launch_bounds__(kTransThreads) k_translucent(FrameArgs a) {
             continue;
         }
         const uint32_t vi = find_view_by_stile(a, st);
-        const DView& view = a.views[vi];
-        const DScene& sc = a.scenes[view.scene];
-        const uint32_t local = st - view.stile_base;
-        const int32_t sx0 = (int32_t)(local % (uint32_t)view.stiles_x) * S;
-        const int32_t sy0 = (int32_t)(local / (uint32_t)view.stiles_x) * S;
-        const int32_t tx0 = (sx0 / kRefTile) * kRefTile, ty0 = (sy0 / kRefTile) * kRefTile;
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        if (vi != held) load_shade_const(shade, a, vi, threadIdx.x, kTransThreads);  // read after the barriers below
+        held = vi;
+        const DView& gv = a.views[vi];
+        const uint32_t local = st - gv.stile_base;
+        const int32_t ux = (int32_t)((local % (uint32_t)gv.stiles_x) * S + (sub % ppr) * (uint32_t)part);
+        const int32_t uy = (int32_t)((local / (uint32_t)gv.stiles_x) * S + (sub / ppr) * (uint32_t)part);
+        const int32_t tx0 = (ux / kRefTile) * kRefTile, ty0 = (uy / kRefTile) * kRefTile;
+        for (uint32_t i = threadIdx.x; i < n; i += kTransThreads) {
             const uint32_t slot = a.bins[b0 + i];
-            tslot[i] = slot;
-            tkey[i] = trans_key(__uint_as_float(a.rec_s[slot].avg_z), a.rec_r[slot].seq8);
+            const RecRaster& r = a.rec_r[slot];
+            if (part_rect(r, tx0, ty0, ux, uy, part) == 0u) continue;
+            const uint32_t at = atomicAdd(&kept, 1u);
+            tslot[at] = slot;
+            tkey[at] = trans_key(__uint_as_float(a.rec_s[slot].avg_z), r.seq8);
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {  // keys are unique: rank = position
-            const unsigned long long k = tkey[i];
-            uint32_t rank = 0;
-            for (uint32_t j = 0; j < n; ++j) rank += tkey[j] < k ? 1u : 0u;
-            tsorted[rank] = tslot[i];
+        const uint32_t m = kept;
+        if (m == 0u) continue;
+        if (m <= kTransRankMax) {
+            for (uint32_t i = threadIdx.x; i < m; i += kTransThreads) {  // keys are unique: rank = position
+                const unsigned long long k = tkey[i];
+                uint32_t rank = 0;
+                for (uint32_t j = 0; j < m; ++j) rank += tkey[j] < k ? 1u : 0u;
+                tsorted[rank] = tslot[i];
+            }
+        } else {
+            uint32_t m2 = kTransRankMax;
+            while (m2 < m) m2 *= 2u;
+            for (uint32_t i = m + threadIdx.x; i < m2; i += kTransThreads) tkey[i] = ~0ull;
+            __syncthreads();
+            bitonic_sort<kTransThreads>(tkey, tslot, m2);
+            for (uint32_t i = threadIdx.x; i < m; i += kTransThreads) tsorted[i] = tslot[i];
         }
         __syncthreads();
-        // Coarse flag and accepted 16-px blocks (coarse_raster's reject) per packet.
-        for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
+        // Rectangle, coarse flag and accepted 16-px blocks (coarse_raster's reject) per packet.
+        for (uint32_t k = threadIdx.x; k < m; k += kTransThreads) {
             PacketCtx c;
-            load_packet(a, sc, tsorted[k], tx0, ty0, c);
-            uint32_t m = 0;
+            load_packet(a, shade.scene, tsorted[k], tx0, ty0, c);
+            uint32_t blk = 0;
             if (c.coarse) {
-                m = 0x80000000u;
+                blk = 0x80000000u;
                 for (int32_t by = 0; by * 256 < c.ye - c.ys; ++by)
                     for (int32_t bx = 0; bx * 256 < c.xe - c.xs; ++bx)
                         if (!block_rejected(c.e12, c.e20, c.e01, c.xs + 256 * bx, c.ys + 256 * by))
-                            m |= 1u << (by * 5 + bx);
+                            blk |= 1u << (by * 5 + bx);
             }
-            tblk[k] = m;
+            tinfo[k] = make_uint2(part_rect(c.r, tx0, ty0, ux, uy, part), blk);
         }
         __syncthreads();
-        for (int32_t q = threadIdx.x; q < (S / 2) * (S / 2); q += blockDim.x) {
-            const int32_t px0 = sx0 + 2 * (q % (S / 2)), py0 = sy0 + 2 * (q / (S / 2));
-            float zop[4];
-            f3 col[4];
+        const DView& view = shade.view();
+        const int32_t kq = (int32_t)(lane & 3u), quad = (int32_t)(lane >> 2);
+        const int32_t nblk = (part / 8) * (part / 4);
+        for (int32_t blk = (int32_t)warp; blk < nblk; blk += kTransThreads / 32) {
+            const int32_t bx = (blk % (part / 8)) * 8, by = (blk / (part / 8)) * 4;
+            const int32_t qx = bx + 2 * (quad & 3), qy = by + 2 * (quad >> 2);  // this lane's quad in the part
+            const int32_t X = (ux + qx) * kSubpixelScale, Y = (uy + qy) * kSubpixelScale;
+            const uint64_t pi = (uint64_t)(uy + qy + (kq >> 1)) * view.key_pitch + (uint64_t)(ux + qx + (kq & 1));
+            float* const cp = view.color + pi * 3u;
+            float zop = 0.0f;
+            f3 col = mk3(0.0f, 0.0f, 0.0f);
+            bool loaded = false, touched = false;
+            for (uint32_t base = 0; base < m; base += 32u) {
+                const uint32_t rc = base + lane < m ? tinfo[base + lane].x : 0u;
+                const bool hit = bx + 6 >= (int32_t)(rc & 31u) && bx < (int32_t)((rc >> 10) & 31u) &&
+                                 by + 2 >= (int32_t)((rc >> 5) & 31u) && by < (int32_t)((rc >> 15) & 31u);
+                for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, hit); todo; todo &= todo - 1u) {
+                    const uint32_t k = base + (uint32_t)(__ffs(todo) - 1);
+                    if (!loaded) {
+                        zop = ordered_to_float((uint32_t)(a.keys[view.key_offset + pi] >> 32));
+                        col = mk3(cp[0], cp[1], cp[2]);
+                        loaded = true;
+                    }
+                    const uint32_t slot = tsorted[k];
+                    const uint2 info = tinfo[k];
+                    bool in = qx >= (int32_t)(info.x & 31u) && qx < (int32_t)((info.x >> 10) & 31u) &&
+                              qy >= (int32_t)((info.x >> 5) & 31u) && qy < (int32_t)((info.x >> 15) & 31u);
+                    PacketCtx c;
+                    load_packet(a, shade.scene, slot, tx0, ty0, c);
+                    int32_t ox = c.xs, oy = c.ys;
+                    if (info.y >> 31) {
+                        const int32_t cx = (X - c.xs) >> 8, cy = (Y - c.ys) >> 8;
+                        in = in && ((info.y >> (cy * 5 + cx)) & 1u);
+                        ox = c.xs + 256 * cx;
+                        oy = c.ys + 256 * cy;
+                    }
+                    float b1 = 0.0f, b2 = 0.0f, w = 0.0f;
+                    bool pass = false;
+                    if (in) {
+                        const int32_t i = (X - ox) >> 5, j = (Y - oy) >> 5;
+                        const float w0 = lane_edge_value(c.e12, ox, oy, i, j, kq);
+                        const float w1 = lane_edge_value(c.e20, ox, oy, i, j, kq);
+                        const float w2 = lane_edge_value(c.e01, ox, oy, i, j, kq);
+                        b1 = w1 * c.r.ooa;
+                        b2 = w2 * c.r.ooa;
+                        w = 1.0f / interp(c.r.oow, b1, b2);
+                        const float z = interp(c.r.zow, b1, b2) * w;
+                        pass = w0 >= 0.0f && w1 >= 0.0f && w2 >= 0.0f && z <= zop;
+                    }
+                    if (!__any_sync(0xFFFFFFFFu, pass)) continue;
+                    float wq[4];
 #pragma unroll
-            for (int l = 0; l < 4; ++l) {
-                const uint64_t pi = (uint64_t)(py0 + (l >> 1)) * view.key_pitch + (uint64_t)(px0 + (l & 1));
-                zop[l] = ordered_to_float((uint32_t)(a.keys[view.key_offset + pi] >> 32));
-                const float* cp = view.color + pi * 3u;
-                col[l] = mk3(cp[0], cp[1], cp[2]);
+                    for (int l = 0; l < 4; ++l) wq[l] = __shfl_sync(0xFFFFFFFFu, w, (int)((lane & ~3u) + (uint32_t)l));
+                    if (pass) {
+                        RecShade q;
+                        {
+                            const float4* src = reinterpret_cast<const float4*>(a.rec_s + slot);
+                            float4* dst = reinterpret_cast<float4*>(&q);
+#pragma unroll
+                            for (int t = 0; t < 8; ++t) dst[t] = __ldg(src + t);
+                        }
+                        float dd[4];
+#pragma unroll
+                        for (int l = 0; l < 4; ++l) dd[l] = q.du_dv[l] * wq[l];
+                        const MaterialLane mat = load_material(shade.scene.materials + (c.r.material & kRecMaterialMask));
+                        const uint32_t md = MODE == kModeAny ? view.rsqrt_mode : (uint32_t)MODE;
+                        col = pbr_lane<true, GI>(shade.scene, view, mat, q, a.rec_t + slot, w, b1, b2, dd, md, tab, col);
+                        touched = true;
+                    }
+                }
             }
-            const int32_t X = px0 * kSubpixelScale, Y = py0 * kSubpixelScale;
-            bool touched = false;
-            for (uint32_t k = 0; k < n; ++k) {
-                const uint32_t slot = tsorted[k];
-                const RecRaster& rr = a.rec_r[slot];
-                int32_t x0, y0, x1, y1;
-                clipped_rect(rr, tx0, ty0, x0, y0, x1, y1);
-                const int32_t xs = (x0 & ~1) * kSubpixelScale, ys = (y0 & ~1) * kSubpixelScale;
-                if (X < xs || X >= x1 * kSubpixelScale || Y < ys || Y >= y1 * kSubpixelScale) continue;
-                int32_t ox = xs, oy = ys;
-                const uint32_t blk = tblk[k];
-                if (blk >> 31) {
-                    const int32_t bx = (X - xs) >> 8, by = (Y - ys) >> 8;
-                    if (!((blk >> (by * 5 + bx)) & 1u)) continue;
-                    ox = xs + 256 * bx;
-                    oy = ys + 256 * by;
-                }
-                const int32_t i = (X - ox) >> 5, j = (Y - oy) >> 5;
-                PacketCtx c;
-                load_packet(a, sc, slot, tx0, ty0, c);
-                float w0[4], w1[4], w2[4];
-                quad_edge_values(c.e12, ox, oy, i, j, w0);
-                quad_edge_values(c.e20, ox, oy, i, j, w1);
-                quad_edge_values(c.e01, ox, oy, i, j, w2);
-                float b1[4], b2[4], wl[4];
-                uint32_t mask = 0;
-#pragma unroll
-                for (int l = 0; l < 4; ++l) {
-                    b1[l] = w1[l] * c.r.ooa;
-                    b2[l] = w2[l] * c.r.ooa;
-                    wl[l] = 1.0f / interp(c.r.oow, b1[l], b2[l]);
-                    const float z = interp(c.r.zow, b1[l], b2[l]) * wl[l];
-                    if (w0[l] >= 0.0f && w1[l] >= 0.0f && w2[l] >= 0.0f && z <= zop[l]) mask |= 1u << l;
-                }
-                if (mask == 0u) continue;
-                RecShade qs;
-                {
-                    const float4* src = reinterpret_cast<const float4*>(a.rec_s + slot);
-                    float4* dst = reinterpret_cast<float4*>(&qs);
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) dst[t] = __ldg(src + t);
-                }
-                float dd[4];
-#pragma unroll
-                for (int l = 0; l < 4; ++l) dd[l] = qs.du_dv[l] * wl[l];
-                const MaterialLane m = load_material(sc.materials + (c.r.material & kRecMaterialMask));
-#pragma unroll
-                for (int l = 0; l < 4; ++l)
-                    if (mask & (1u << l))
-                        col[l] = pbr_lane<true, true>(sc, view, m, qs, a.rec_t + slot, wl[l], b1[l], b2[l], dd, view.rsqrt_mode,
-                                                      tab, col[l]);
-                touched = true;
-            }
-            if (!touched) continue;
-#pragma unroll
-            for (int l = 0; l < 4; ++l) {
-                const uint64_t pi = (uint64_t)(py0 + (l >> 1)) * view.key_pitch + (uint64_t)(px0 + (l & 1));
-                float* cp = view.color + pi * 3u;
-                cp[0] = col[l].x;
-                cp[1] = col[l].y;
-                cp[2] = col[l].z;
+            if (touched) {
+                cp[0] = col.x;
+                cp[1] = col.y;
+                cp[2] = col.z;
             }
             // Centre luminance of the reference tile (src/tilerasterizer.rs:103-106): quad (0, 16).
-            if ((px0 & (kRefTile - 1)) == 0 && (py0 & (kRefTile - 1)) == kRefTile / 2) {
-                float l4[4];
+            const float lum = (col.x * 0.2126f + col.y * 0.7152f) + col.z * 0.0722f;
+            float l4[4];
 #pragma unroll
-                for (int l = 0; l < 4; ++l) l4[l] = (col[l].x * 0.2126f + col[l].y * 0.7152f) + col[l].z * 0.0722f;
-                const uint32_t tile = (uint32_t)(py0 / kRefTile) * (uint32_t)view.tiles_x + (uint32_t)(px0 / kRefTile);
+            for (int l = 0; l < 4; ++l) l4[l] = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + (uint32_t)l));
+            const uint32_t quad_touched = (__ballot_sync(0xFFFFFFFFu, touched) >> (lane & ~3u)) & 0xFu;
+            if (quad_touched && kq == 0 && ((ux + qx) & (kRefTile - 1)) == 0 && ((uy + qy) & (kRefTile - 1)) == kRefTile / 2) {
+                const uint32_t tile = (uint32_t)((uy + qy) / kRefTile) * (uint32_t)view.tiles_x + (uint32_t)((ux + qx) / kRefTile);
                 view.tile_lum[tile] = (((l4[0] + l4[1]) + l4[2]) + l4[3]) * 0.25f;
             }
         }
@@ -2757,12 +2820,14 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
     }
     mark(7);
     if (a.has_translucent) {
-        const uint32_t tg = (uint32_t)num_sms * 2u;
-        switch (a.sched_tile) {
-            case 8: k_translucent<8><<<tg, kTransThreads, 0, s>>>(a); break;
-            case 16: k_translucent<16><<<tg, kTransThreads, 0, s>>>(a); break;
-            case 32: k_translucent<32><<<tg, kTransThreads, 0, s>>>(a); break;
-            default: k_translucent<64><<<tg, kTransThreads, 0, s>>>(a); break;
+        const uint32_t tg = (uint32_t)num_sms * 4u;
+        const bool arm = a.rsqrt_uniform == 1u + kModeArm;
+        if (a.has_gi) {
+            if (arm) k_translucent<true, kModeArm><<<tg, kTransThreads, 0, s>>>(a);
+            else k_translucent<true, kModeAny><<<tg, kTransThreads, 0, s>>>(a);
+        } else {
+            if (arm) k_translucent<false, kModeArm><<<tg, kTransThreads, 0, s>>>(a);
+            else k_translucent<false, kModeAny><<<tg, kTransThreads, 0, s>>>(a);
         }
         launches++;
         if (!a.defer_resolve) {
