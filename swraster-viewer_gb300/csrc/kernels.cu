@@ -2636,20 +2636,34 @@ __global__ void __launch_bounds__(kTransThreads, 4) k_translucent(FrameArgs a) {
     }
 }
 
-// Exposure applied after the host's update_auto_exposure (dt > 0 path).
-__global__ void k_resolve(FrameArgs a) {
+// Exposure applied after the host's update_auto_exposure (dt > 0 path). The
+// exposure lies in mapped host memory: one read per CTA, which then walks
+// 256-pixel row pieces (one read per warp over NVLink-C2C and a thread per
+// pixel took 54 us for 1367x769, most of it waiting for those reads).
+constexpr int kResolveThreads = 256;
+__global__ void __launch_bounds__(kResolveThreads) k_resolve(FrameArgs a) {
+    __shared__ float exposure;
     const uint32_t vi = blockIdx.y;
     if (vi >= a.dyn->n_views) return;
     const DView& v = a.views[vi];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!v.flags) return;
+    if (threadIdx.x == 0) exposure = a.exposure_dev ? *a.exposure_dev : v.exposure;
+    __syncthreads();
+    const float e = exposure;
     const uint32_t w = (uint32_t)v.width, h = (uint32_t)(v.height & ~1);
-    if (i >= w * h || !v.flags) return;
-    const uint32_t x = i % w, y = i / w;
-    const float* c = v.color + ((uint64_t)y * v.key_pitch + x) * 3u;
-    const float e = a.exposure_dev ? *a.exposure_dev : v.exposure;
-    const uint32_t p = tonemap_pack(mk3(c[0], c[1], c[2]), e);
-    v.rgba8[(uint64_t)y * v.out_pitch + x] = p;
-    if (v.rgba8_host) v.rgba8_host[(uint64_t)y * v.host_pitch + x] = p;
+    const uint32_t per_row = (w + kResolveThreads - 1u) / kResolveThreads, n = per_row * h;
+    const float* const color = v.color;
+    uint32_t* const out = v.rgba8;
+    uint32_t* const host = v.rgba8_host;
+    const uint64_t pitch = v.key_pitch, out_pitch = v.out_pitch, host_pitch = v.host_pitch;
+    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+        const uint32_t y = i / per_row, x = (i - y * per_row) * kResolveThreads + threadIdx.x;
+        if (x >= w) continue;
+        const float* c = color + (y * pitch + x) * 3u;
+        const uint32_t p = tonemap_pack(mk3(__ldg(c), __ldg(c + 1), __ldg(c + 2)), e);
+        out[y * out_pitch + x] = p;
+        if (host) host[y * host_pitch + x] = p;
+    }
 }
 
 // --------------------------------------------------------------------------
@@ -2851,8 +2865,11 @@ cudaError_t launch_rsqrt_selftest(const float* in, float* out, uint64_t n, uint3
 void launch_resolve(const FrameArgs& a, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t maxpx = a.pixel_cap > 0 ? a.pixel_cap : 1u;
-    dim3 grid((maxpx + 255) / 256, a.view_cap > 0 ? a.view_cap : 1u);
-    k_resolve<<<grid, 256, 0, s>>>(a);
+    // About eight CTAs an SM when one view is resolved, fewer each for more.
+    const uint32_t views = a.view_cap > 0 ? a.view_cap : 1u;
+    const uint32_t most = std::max(1216u / views, 64u);
+    dim3 grid(std::min((maxpx + kResolveThreads - 1) / kResolveThreads, most), views);
+    k_resolve<<<grid, kResolveThreads, 0, s>>>(a);
 }
 
 }  // namespace swr
