@@ -86,6 +86,13 @@ swr_status BatchImpl::enqueue(const swr_view_desc* vd, int32_t n, cudaStream_t s
     cudaEventRecord(ev_start, stream);
     st = eng.launch(stream, nullptr, err);
     cudaEventRecord(ev_end, stream);
+    if (st == SWR_OK && (h_counters.ensure(sizeof(DCounters)) != cudaSuccess ||
+                         cudaMemcpyAsync(h_counters.p, eng.counters.p, sizeof(DCounters), cudaMemcpyDeviceToHost,
+                                         stream) != cudaSuccess)) {
+        cudaGetLastError();
+        err = "counter readback failed";
+        st = SWR_CUDA_ERROR;
+    }
     last_stream = stream;
     return st;
 }
@@ -99,12 +106,7 @@ swr_status BatchImpl::sync(std::string& err) {
             cudaGetLastError();
             return SWR_CUDA_ERROR;
         }
-        DCounters c{};
-        e = cudaMemcpy(&c, eng.counters.p, sizeof(c), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) {
-            err = "counter readback failed";
-            return SWR_CUDA_ERROR;
-        }
+        const DCounters c = *static_cast<const DCounters*>(h_counters.p);
         eng.last = c;
         if (!(c.status & kStRetry)) {
             pending = false;
@@ -240,6 +242,7 @@ void swr_batch_destroy(swr_batch* b) {
         o.vis.release();
     }
     b->impl.tile_lum.release();
+    b->impl.h_counters.release();
     if (b->impl.ev_start) cudaEventDestroy(b->impl.ev_start);
     if (b->impl.ev_end) cudaEventDestroy(b->impl.ev_end);
     delete b;

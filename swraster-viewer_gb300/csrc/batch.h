@@ -33,6 +33,7 @@ struct BatchImpl {
     cudaEvent_t ev_start = nullptr, ev_end = nullptr;
     cudaStream_t last_stream = nullptr;
     bool pending = false;
+    HBuf h_counters;                     // the batch's counters, copied back behind its kernels
 
     swr_status render(const swr_view_desc* vd, int32_t n, cudaStream_t stream, std::string& err);
     swr_status enqueue(const swr_view_desc* vd, int32_t n, cudaStream_t stream, std::string& err);

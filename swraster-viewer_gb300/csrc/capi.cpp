@@ -230,7 +230,6 @@ swr_status swr_renderer_create(int32_t width, int32_t height, const swr_renderer
     chk(r->tile_lum.ensure((size_t)r->tiles_x * r->tiles_y * sizeof(float)));
     chk(cudaHostAlloc((void**)&r->h_lum, (size_t)r->tiles_x * r->tiles_y * sizeof(float), cudaHostAllocDefault));
     chk(cudaHostAlloc((void**)&r->h_expo, sizeof(float), cudaHostAllocMapped));
-    chk(cudaHostAlloc((void**)&r->h_status, sizeof(uint32_t), cudaHostAllocDefault));
     if (e == cudaSuccess) chk(cudaHostGetDevicePointer((void**)&r->d_expo, r->h_expo, 0));
     chk(cudaEventCreateWithFlags(&r->expo_done, cudaEventDisableTiming));
     chk(cudaHostAlloc((void**)&r->h_counters, sizeof(DCounters), cudaHostAllocDefault));
@@ -253,7 +252,6 @@ void swr_renderer_destroy(swr_renderer* r) {
     r->tile_lum.release();
     if (r->h_lum) cudaFreeHost(r->h_lum);
     if (r->h_expo) cudaFreeHost(r->h_expo);
-    if (r->h_status) cudaFreeHost(r->h_status);
     if (r->expo_done) cudaEventDestroy(r->expo_done);
     if (r->h_counters) cudaFreeHost(r->h_counters);
     if (r->status_ev) cudaEventDestroy(r->status_ev);
@@ -287,7 +285,7 @@ void CUDART_CB exposure_callback(void* p) {
     swr_renderer* r = static_cast<swr_renderer*>(p);
     // A frame that overflowed its bins is re-rendered; it must not advance
     // the exposure state.
-    if (*r->h_status & kStRetry) return;
+    if (r->h_counters->status & kStRetry) return;
     r->expo.update(r->h_lum, (size_t)r->tiles_x * r->tiles_y, r->pending_dt);
     *r->h_expo = r->expo.exposure;
 }
@@ -338,10 +336,11 @@ swr_status enqueue_frame(swr_renderer* r, const swr_scene* scene, const swr_came
     FrameArgs a{};
     swr_status st = r->eng.run(scenes, views, cams, stream, &a, err, ev);
     if (st != SWR_OK) return fail(st, err);
+    // The counters are final here (the resolve does not touch them).
+    cudaMemcpyAsync(r->h_counters, r->eng.counters.p, sizeof(DCounters), cudaMemcpyDeviceToHost, stream);
     if (deferred) {
         const size_t nt = (size_t)r->tiles_x * r->tiles_y;
         cudaMemcpyAsync(r->h_lum, r->tile_lum.p, nt * sizeof(float), cudaMemcpyDeviceToHost, stream);
-        cudaMemcpyAsync(r->h_status, r->eng.counters.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
         r->pending_dt = dt;
         cudaLaunchHostFunc(stream, exposure_callback, r);
         a.exposure_dev = r->d_expo;
@@ -352,7 +351,6 @@ swr_status enqueue_frame(swr_renderer* r, const swr_scene* scene, const swr_came
         cudaEventRecord(r->expo_done, stream);
         r->expo_pending = true;
     }
-    cudaMemcpyAsync(r->h_counters, r->eng.counters.p, sizeof(DCounters), cudaMemcpyDeviceToHost, stream);
     cudaEventRecord(r->status_ev, stream);
     r->status_pending = true;
     cudaError_t e = cudaGetLastError();
@@ -391,9 +389,10 @@ swr_status check_frame(swr_renderer* r) {
     for (int attempt = 0; attempt < 6; ++attempt) {
         cudaError_t e = cudaStreamSynchronize(r->last_stream);
         if (e != cudaSuccess) return cuda_fail(e, "frame execution");
-        DCounters c{};
-        e = cudaMemcpy(&c, r->eng.counters.p, sizeof(c), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return cuda_fail(e, "counter readback");
+        // The frame's own copy of the counters (a second, blocking copy here
+        // cost a render-blit loop about 8 us a frame).
+        const DCounters c = *r->h_counters;
+        r->status_pending = false;
         r->eng.last = c;
         if (!(c.status & kStRetry)) {
             r->checked = true;
@@ -437,12 +436,14 @@ swr_status swr_renderer_sync(swr_renderer* r) {
 swr_status swr_blit(swr_renderer* r, uint32_t* pixels, size_t row_stride, void* stream) {
     if (!r || !pixels) return fail(SWR_INVALID_ARG, "null argument");
     if (!r->have_frame) return fail(SWR_INVALID_ARG, "no frame rendered");
+    const bool waited = !r->checked && (cudaStream_t)stream == r->last_stream;  // check_frame waits for that stream
     swr_status st = check_frame(r);
     if (st != SWR_OK) return st;
     if (row_stride == 0) row_stride = (size_t)r->width;
     if (row_stride < (size_t)r->width) return fail(SWR_INVALID_ARG, "row_stride smaller than width");
     if (pixels == r->frame_target && row_stride == r->frame_stride) {
         // The shading pass already wrote this frame into `pixels`.
+        if (waited) return SWR_OK;
         const cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
         if (e != cudaSuccess) return cuda_fail(e, "blit wait");
         return SWR_OK;

@@ -167,7 +167,6 @@ struct swr_renderer {
     swr::ExposureState expo;
     // Mapped pinned memory for the dt > 0 exposure step.
     float* h_lum = nullptr;
-    uint32_t* h_status = nullptr;
     float* h_expo = nullptr;
     float* d_expo = nullptr;
     cudaEvent_t expo_done = nullptr;

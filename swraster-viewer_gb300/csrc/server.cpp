@@ -349,6 +349,7 @@ void swr_server_destroy(swr_server* s) {
     for (auto& e : s->engines) {
         e->b->eng.release();
         e->b->tile_lum.release();
+        e->b->h_counters.release();
         for (auto& o : e->b->owned) {
             o.rgba8.release();
             o.vis.release();
