@@ -537,7 +537,7 @@ swr_status swr_renderer_get_stats(swr_renderer* r, swr_frame_stats* o) {
     o->triangles_in = c.draw_tris;
     o->triangles_clipped = c.clip_queue;
     o->setup_triangles = c.setup_tris;
-    o->bin_pairs = c.pairs;
+    o->bin_pairs = c.pairs + c.unsampled;
     o->bin_capacity = r->eng.bin_cap;
     o->tiles = r->tiles_x * r->tiles_y;
     o->overflow_retries = r->eng.retries;

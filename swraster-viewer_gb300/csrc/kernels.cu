@@ -352,6 +352,13 @@ __device__ __forceinline__ void warp_count(uint32_t* counter, bool pred) {
     if ((int)(threadIdx.x & 31u) == __ffs(active) - 1 && b) atomicAdd(counter, (uint32_t)__popc(b));
 }
 
+// One atomic per warp: adds the active lanes' values.
+__device__ __forceinline__ void warp_sum(uint32_t* counter, uint32_t v) {
+    const uint32_t active = __activemask();
+    const uint32_t s = __reduce_add_sync(active, v);
+    if ((int)(threadIdx.x & 31u) == __ffs(active) - 1 && s) atomicAdd(counter, s);
+}
+
 // Warp-aggregated atomicAdd of 1 on counter[idx].
 __device__ __forceinline__ void agg_inc(uint32_t* counter, uint32_t idx) {
     const uint32_t active = __activemask();
@@ -412,10 +419,44 @@ __device__ __forceinline__ bool push_wide(const FrameArgs& a, uint32_t* counter,
 #define SWR_CULL_MIN_TILE 64
 #endif
 
-// bin_triangle (src/renderer.rs:668-831): setup. Returns true when the
-// triangle covers at least one tile; its records are then in r and q, its
-// tiles (still to be counted) in tiles.
-__device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx& v0, const Vtx& v1, const Vtx& v2,
+// Whether no pixel centre can pass the raster's edge tests for a front-facing
+// triangle with subpixel vertices (x0, y0) .. (x2, y2) inside the screen,
+// whose bounding box holds at most 2x2 centres. Claimed only where every value
+// the raster's f32 edge arithmetic forms is an integer below 2^24 (the bound
+// of depthfloor.cuh), so that its tests are the integer ones; a centre outside
+// the bounding box is then outside an edge, and a triangle of no area covers
+// nothing (of opposite edges one has the top-left bias -1).
+__device__ __forceinline__ bool covers_no_centre(int32_t x0, int32_t y0, int32_t x1, int32_t y1, int32_t x2, int32_t y2,
+                                                 int32_t w, int32_t h) {
+    const int32_t lx = min(min(x0, x1), x2), hx = max(max(x0, x1), x2);
+    const int32_t ly = min(min(y0, y1), y2), hy = max(max(y0, y1), y2);
+    if (lx < 0 || ly < 0 || hx > w || hy > h) return false;
+    const int32_t cx0 = (lx + 7) >> 4, cx1 = (hx - 8) >> 4, cy0 = (ly + 7) >> 4, cy1 = (hy - 8) >> 4;
+    if (cx1 - cx0 > 1 || cy1 - cy0 > 1) return false;  // so hx - lx and hy - ly are below 64
+    const int32_t ex = hx - lx, ey = hy - ly;
+    if (2 * (ey * (hx + 64) + ex * (hy + 64)) + 1 + 256 * (ex + ey) > 16777216) return false;
+    // Edge i -> j at (x, y): (yj - yi) (x - xi) + (xi - xj) (y - yi) + bias.
+    const int32_t a0 = y1 - y0, b0 = x0 - x1, a1 = y2 - y1, b1 = x1 - x2, a2 = y0 - y2, b2 = x2 - x0;
+    const int32_t t0 = top_left_bias(a0, b0), t1 = top_left_bias(a1, b1), t2 = top_left_bias(a2, b2);
+    bool any = false;
+    for (int32_t cy = cy0; cy <= cy1; ++cy)
+        for (int32_t cx = cx0; cx <= cx1; ++cx) {
+            const int32_t x = cx * 16 + 8, y = cy * 16 + 8;
+            const int32_t e0 = a0 * (x - x0) + b0 * (y - y0) + t0;
+            const int32_t e1 = a1 * (x - x1) + b1 * (y - y1) + t1;
+            const int32_t e2 = a2 * (x - x2) + b2 * (y - y2) + t2;
+            any = any || (e0 | e1 | e2) >= 0;
+        }
+    return !any;
+}
+
+// bin_triangle (src/renderer.rs:668-831): setup. kSetupRecord when the
+// triangle has records (then in r and q), kSetupNone when it is culled or
+// covers no tile, kSetupUnsampled when the reference bins it but no pixel
+// centre is in it: it cannot change the frame, so it is only counted. Its
+// tiles (still to be counted) are in tiles.
+enum : uint32_t { kSetupNone = 0, kSetupRecord = 1, kSetupUnsampled = 2 };
+__device__ uint32_t setup_triangle(const FrameArgs& a, const DView& view, const Vtx& v0, const Vtx& v1, const Vtx& v2,
                                uint32_t seq8, uint32_t static_id, uint32_t material, uint32_t view_idx,
                                RecRaster& r, RecShade& q, TileRect& tiles) {
     int32_t p0x, p0y, p1x, p1y, p2x, p2y;
@@ -423,7 +464,7 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     to_screen(v1, view.width_f, view.height_f, p1x, p1y);
     to_screen(v2, view.width_f, view.height_f, p2x, p2y);
     const int32_t area = wsub(wmul(wsub(p1x, p0x), wsub(p2y, p0y)), wmul(wsub(p2x, p0x), wsub(p1y, p0y)));
-    if (area > 0) return false;  // back-facing (CW front faces after the y flip)
+    if (area > 0) return kSetupNone;  // back-facing (CW front faces after the y flip)
     const int32_t wsub_px = view.width * kSubpixelScale, hsub_px = view.height * kSubpixelScale;
     const int32_t mns_x = max(min(min(p0x, p1x), p2x), 0);
     const int32_t mns_y = max(min(min(p0y, p1y), p2y), 0);
@@ -435,7 +476,9 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
 
     const bool translucent = (material & kRecTransBit) != 0u;
     tiles = tile_rect(view, a.sched_tile, translucent ? a.dyn->n_stiles : 0u, mnx, mny, mxx, mxy);
-    if (tiles.count() == 0u) return false;
+    if (tiles.count() == 0u) return kSetupNone;
+    if (a.skip_unsampled && !translucent && covers_no_centre(p0x, p0y, p1x, p1y, p2x, p2y, wsub_px, hsub_px))
+        return kSetupUnsampled;
 
     // Interpolator setup (src/renderer.rs:699-754).
     const float ooa = 1.0f / i2f(wabs(area));
@@ -460,7 +503,13 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     r.seq8 = seq8;
     r.material = material;
     r.view = view_idx;
-    r.zfloor = 0u;  // taken by k_scatter when the frame culls
+    r.zfloor = 0u;
+    if ((int32_t)a.sched_tile >= SWR_CULL_MIN_TILE && !translucent) {
+        const float zc[3] = {v0.cz, v1.cz, v2.cz}, wc[3] = {v0.cw, v1.cw, v2.cw};
+        float zl;
+        if (depth_floor(r.p, area, r.zow, r.oow, zc, wc, mxx * kSubpixelScale, mxy * kSubpixelScale, zl))
+            r.zfloor = float_to_ordered(zl);
+    }
     r.wide = 0u;
     q.nrm[0] = v0.nx; q.nrm[1] = v0.ny; q.nrm[2] = v0.nz;
     q.nrm[3] = v1.nx - v0.nx; q.nrm[4] = v1.ny - v0.ny; q.nrm[5] = v1.nz - v0.nz;
@@ -478,7 +527,7 @@ __device__ bool setup_triangle(const FrameArgs& a, const DView& view, const Vtx&
     // Average z for the per-tile translucency sort (src/renderer.rs:765-774).
     q.avg_z = translucent ? __float_as_uint(((v0.cz + v1.cz) + v2.cz) / 3.0f) : 0u;
     q.pad[0] = q.pad[1] = 0u;
-    return true;
+    return kSetupRecord;
 }
 
 __device__ __forceinline__ void store_records(const FrameArgs& a, uint32_t slot, const RecRaster& r,
@@ -785,6 +834,7 @@ __global__ void __launch_bounds__(256) k_reset(FrameArgs a) {
         a.counters->trans_packets = 0u;
         a.counters->culled = 0u;
         a.counters->clip_path = 0u;
+        a.counters->unsampled = 0u;
         a.counters->wide_main = 0u;
         a.counters->wide_clip = 0u;
         a.counters->draw_tris = a.gpu_draws ? 0u : a.dyn->tri_total;
@@ -864,8 +914,8 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
     RecRaster r;
     RecShade q;
     TileRect tiles;
-    const bool ok = setup_triangle(a, view, v0, v1, v2, g << 3, d.static_base + local, mword, d.view, r, q, tiles);
-    if (ok) {
+    const uint32_t res = setup_triangle(a, view, v0, v1, v2, g << 3, d.static_base + local, mword, d.view, r, q, tiles);
+    if (res == kSetupRecord) {
         // A wide triangle's tiles are counted by k_clip's warps: one thread
         // walking the 4,576 16-px tiles of a 1367x769 frame held the kernel
         // for 79 us (150k triangles; 12 us without such triangles).
@@ -876,8 +926,9 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
         store_records(a, g, r, q);
         if (tangents) store_tangents(a, g, v0, v1, v2);
     }
-    a.tri_state[g] = ok ? 1 : 0;
-    warp_count(&a.counters->setup_tris, ok);
+    a.tri_state[g] = res == kSetupRecord ? 1 : 0;
+    warp_count(&a.counters->setup_tris, res != kSetupNone);
+    warp_sum(&a.counters->unsampled, res == kSetupUnsampled ? tiles.count() : 0u);
 }
 
 // Thread per triangle of a 256-triangle chunk, CTA per chunk (a loop over
@@ -1031,8 +1082,13 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
             const Vtx* pl = reinterpret_cast<const Vtx*>(cur);
             RecRaster r;
             RecShade q;
-            ok = setup_triangle(a, view, pl[0], pl[i + 1], pl[i + 2], (g << 3) | i, d.static_base + local, mword,
-                                d.view, r, q, tiles);
+            const uint32_t res = setup_triangle(a, view, pl[0], pl[i + 1], pl[i + 2], (g << 3) | i,
+                                                d.static_base + local, mword, d.view, r, q, tiles);
+            ok = res == kSetupRecord;
+            if (res == kSetupUnsampled) {
+                atomicAdd(&a.counters->setup_tris, 1u);
+                atomicAdd(&a.counters->unsampled, tiles.count());
+            }
             if (ok) {
                 if (tiles.count() > kWideTiles &&
                     push_wide(a, &a.counters->wide_clip, a.wide_queue + a.wide_cap, slot, tiles.count()))
@@ -1192,15 +1248,6 @@ __global__ void __launch_bounds__(1024) k_scan(FrameArgs a) {
     }
 }
 
-// Triangles whose bounding box spans fewer pixels than this take no depth
-// floor, so their packets are never culled (0: every triangle takes one).
-// Small triangles are most of what culling drops: on the 4K frame, raster +
-// scatter took 0.394 + 0.075 ms with a floor for every triangle, 0.421 +
-// 0.077 from 16 px, 0.467 + 0.061 from 64 px and 0.506 + 0.058 from 256 px.
-#ifndef SWR_FLOOR_MIN_PX
-#define SWR_FLOOR_MIN_PX 0
-#endif
-
 // Record slots are the frame's main slots [0, T) and the clipper's extra
 // slots right after them.
 __device__ __forceinline__ void scatter_slot(const FrameArgs& a, uint32_t slot, uint32_t tri_total) {
@@ -1210,17 +1257,6 @@ __device__ __forceinline__ void scatter_slot(const FrameArgs& a, uint32_t slot, 
         return;
     }
     const RecRaster& r = a.rec_r[slot];
-    if ((int32_t)a.sched_tile >= SWR_CULL_MIN_TILE && !(r.material & kRecTransBit) &&
-        (SWR_FLOOR_MIN_PX == 0 ||
-         (uint32_t)(r.bb[2] - r.bb[0] + 1) * (uint32_t)(r.bb[3] - r.bb[1] + 1) >= (uint32_t)SWR_FLOOR_MIN_PX)) {
-        // The depth floor of the whole triangle for the raster's occlusion
-        // culling: every packet's sample coordinates lie below the bbox end,
-        // so one floor bounds the depths of all its packets; taken once here
-        // instead of per packet and round in the raster.
-        float zl;
-        if (depth_floor(r.p, r.zow, r.oow, (int32_t)r.bb[2] * kSubpixelScale, (int32_t)r.bb[3] * kSubpixelScale, zl))
-            a.rec_r[slot].zfloor = float_to_ordered(zl);
-    }
     if (r.wide) return;  // scatter_wide
     for_each_stile(record_tiles(a, r), [&](uint32_t st) {
         const uint32_t active = __activemask();
@@ -2853,7 +2889,18 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
 }
 
 bool depth_floor_host(const int32_t p[6], const float zow[3], const float oow[3], int32_t xe, int32_t ye, float& zlo) {
-    return depth_floor(p, zow, oow, xe, ye, zlo);
+    // Vertex depths and w from the interpolants' corners, the area wrapped as
+    // the front end's.
+    float zc[3], wc[3];
+    for (int v = 0; v < 3; ++v) {
+        const float o = v == 0 ? oow[0] : oow[0] + oow[v], z = v == 0 ? zow[0] : zow[0] + zow[v];
+        if (!(o > 0.0f)) return false;
+        zc[v] = z / o;
+        wc[v] = 1.0f / o;
+    }
+    auto d = [&](int i, int j) { return (uint32_t)p[i] - (uint32_t)p[j]; };
+    const int32_t area = (int32_t)(d(2, 0) * d(5, 1) - d(4, 0) * d(3, 1));
+    return depth_floor(p, area, zow, oow, zc, wc, xe, ye, zlo);
 }
 
 cudaError_t launch_rsqrt_selftest(const float* in, float* out, uint64_t n, uint32_t mode, const uint8_t* table) {
