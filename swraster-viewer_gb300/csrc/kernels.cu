@@ -414,9 +414,9 @@ __device__ __forceinline__ bool push_wide(const FrameArgs& a, uint32_t* counter,
 }
 
 // Occlusion culling runs for scheduling tiles of at least this many pixels
-// (the raster drops packets hidden behind the depths of earlier rounds).
+// a side (the raster drops packets hidden behind the depths of earlier rounds).
 #ifndef SWR_CULL_MIN_TILE
-#define SWR_CULL_MIN_TILE 64
+#define SWR_CULL_MIN_TILE 32
 #endif
 
 // Whether no pixel centre can pass the raster's edge tests for a front-facing
@@ -1737,15 +1737,19 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
                                             const DScene& sc, int32_t qx, int32_t qy, int32_t k, bool needed,
                                             unsigned long long key);
 
-// Occlusion culling is on for 64-px scheduling tiles, the choice for large
-// single views. It pays where many packets of a tile lie behind near
-// geometry drawn first (the 2M-triangle 4K frame: 640 -> 728 frames/s) and
-// costs where triangles are small and seldom hidden: on the served mix of
-// orbiting cameras, culling in every tile size took the plain loop from
-// 1,210 to 1,030 frames/s and the served batches (32-px tiles) from 4,980
-// to 4,460; for the 16-px tiles of the 1280x720 small frame it cost 6%.
+// Occlusion culling is on for 64-px scheduling tiles and for the 32-px tiles
+// that take more than one round (SWR_CULL_FROM packets). It pays where many
+// packets of a tile lie behind near geometry drawn first: eight uneven scenes
+// in a batch, 32-px raster 1,454 -> 1,080 us with the fused shading, 830 ->
+// 442 apart. From 100, 192, 256, 320 or 384 packets on, that raster takes
+// 448, 443, 442, 442 and 443 us, and the fused one of 64 batched views (small
+// spheres, seldom hidden) 2,373, 2,333, 2,323, 2,320 and 2,315. Lighter tiles
+// would pay a short first round's barriers for it.
 // A first round of 64 packets: 4K raster 0.444 ms, against 0.461 (32),
 // 0.460 (128) and 0.477 (a full round of 256).
+#ifndef SWR_CULL_FROM
+#define SWR_CULL_FROM 256
+#endif
 #ifndef SWR_CULL_FIRST
 #define SWR_CULL_FIRST 64
 #endif
@@ -1771,6 +1775,7 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
     // of packets, whole instead: 4K 718 against 728 frames/s).
     constexpr bool kCull = S >= SWR_CULL_MIN_TILE;
     constexpr uint32_t kFirst = (kCull && SWR_CULL_FIRST > 0 && SWR_CULL_FIRST < NT) ? SWR_CULL_FIRST : NT;
+    constexpr uint32_t kCullFrom = S >= 64 ? 0u : SWR_CULL_FROM;
     if constexpr (kFuse)
         for (int i = threadIdx.x; i < 512; i += NT) s.tab[i] = a.rsqrt_table[i];
     uint32_t n_culled = 0, held = 0xFFFFFFFFu;
@@ -1805,14 +1810,15 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
         // hold another tile's, or nothing); they are taken again after a
         // round that had regions.
         bool keys_changed = false, cells_valid = false;
+        const bool cull = kCull && b1 - b0 > kCullFrom;
         for (uint32_t cursor = b0; cursor < b1;) {
             // The keys the previous rounds left, per cell, for occlusion culling.
-            if (kCull && keys_changed) {
+            if (cull && keys_changed) {
                 cell_depths<S>(s);
                 keys_changed = false;
                 cells_valid = true;
             }
-            const uint32_t lim = cursor == b0 ? kFirst : (uint32_t)NT;
+            const uint32_t lim = cull && cursor == b0 ? kFirst : (uint32_t)NT;
             // Pass 1: count this thread's regions and quads.
             const uint32_t pidx = cursor + threadIdx.x;
             PacketCtx c;
@@ -1830,7 +1836,7 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(np + sizeof(RecRaster) - 1));
                 }
 #endif
-                if (kCull && cells_valid) {
+                if (cull && cells_valid) {
                     const uint32_t far = cells_far<S>(s, c.xs >> kSubpixelShift, c.xe >> kSubpixelShift,
                                                       c.ys >> kSubpixelShift, c.ye >> kSubpixelShift, sx0, sy0);
                     hidden = far < 0xFF800000u && packet_floor(c) > far;

@@ -133,8 +133,8 @@ void sort_nodes_by_distance(const SceneImpl& s, const swr_camera& cam, std::vect
 void init_view(DView& v, const swr_camera& cam, int32_t width, int32_t height, uint32_t sched_tile);
 
 // Scheduling tile for views of the given sizes when the caller leaves it to
-// the library: the largest of 64, 32, 16 that still gives the raster kernel
-// at least 8 tiles per SM (16 when none does).
+// the library: 64 where that gives the raster kernel at least 8 tiles per SM,
+// else 32 where that gives it at least 7, else 16.
 uint32_t auto_sched_tile(const int32_t* widths, const int32_t* heights, int32_t n, int num_sms);
 
 // Sets the calling thread's swr_last_error() message.

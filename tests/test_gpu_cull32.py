@@ -1,0 +1,37 @@
+"""Occlusion culling in 32-px scheduling tiles: bins of more than one round
+(256 packets) are culled against the depths of earlier rounds, lighter ones are
+not. Stacks of screen-filling quads with a tie that arrives last, with bins on
+both sides of the line, shaded apart and in the raster kernel, against the
+oracle: visibility must be equal and the last of the tied quads must win."""
+import numpy as np
+import pytest
+
+import oracle
+import swr
+from test_gpu_parity import tie_across_rounds_scene
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [40, 110, 130, 300])
+@pytest.mark.parametrize("fused", [False, True])
+def test_ties_and_culling_in_32px_tiles(n, fused):
+    s = swr.Scene(tie_across_rounds_scene(n))
+    w, h = 190, 127
+    cam = swr.make_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 1.0, w, h, 40.0)
+    orgba, ovis, _, _ = oracle.render(s, cam, w, h, rsqrt_mode=swr.RSQRT_AARCH64, threads=1)
+    b = swr.Batch(sched_tile=32, fused_shade=fused)
+    b.render(swr.Batch.views([(s, cam, w, h, 2.0, swr.RSQRT_AARCH64)] * 2))
+    for i in range(2):
+        rgba, vis = b.output(i, w, h)
+        assert np.array_equal(vis, ovis)
+        d = np.abs(rgba[:h & ~1].view(np.uint8).astype(np.int32) - orgba[:h & ~1].view(np.uint8).astype(np.int32))
+        assert d.max() <= 1
+    b.close()
+    r = swr.Renderer(w, h, sched_tile=32)
+    r.render(s, cam)
+    assert np.array_equal(r.visbuffer(), ovis)
+    if n in (40, 300):
+        assert (r.stats().culled_pairs > 0) == (n == 300)
+    r.close()
+    s.close()
