@@ -122,10 +122,12 @@ struct alignas(16) DScene {
     float light_dir[3];
     float spec_max_mip;        // specular->max_mip
     float light_color[3];
-    uint32_t brdf_w;           // width of brdf_lut
-    float brdf_wf, brdf_hf;    // its size
-    float sky_wf, sky_hf;      // cubemap face size
-    uint32_t sky_w, sky_stride;
+    uint32_t brdf_w;           // brdf_lut's size
+    float brdf_wf, brdf_hf;
+    uint32_t brdf_h;
+    uint32_t sky_stride;       // cubemap texels per face, its face size
+    float sky_wf, sky_hf;
+    uint32_t sky_w, sky_h;
     const uint32_t* brdf_lut;  // mip 0 texels
     const uint32_t* sky;       // cubemap mip 0 texels
     const DTexture* specular;  // prefiltered environment

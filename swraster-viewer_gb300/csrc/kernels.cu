@@ -136,9 +136,20 @@ __device__ __forceinline__ uint32_t mip_level(const DTexture& t, float d0, float
 // wrap: wrap_s | wrap_t << 2.
 __device__ __forceinline__ uint32_t sample_texel(const DTexture& t, float u, float v, uint32_t mip, uint32_t wrap) {
     const float4 d = __ldg(reinterpret_cast<const float4*>(t.mip + mip));      // wf, hf, rwf, rhf
-    const uint2 o = __ldg(reinterpret_cast<const uint2*>(&t.mip[mip].offset));  // offset, w
-    const uint32_t x = f2u_sat(apply_wrap(floorf(u * d.x), d.x, d.z, wrap & 3u));
-    const uint32_t y = f2u_sat(apply_wrap(floorf(v * d.y), d.y, d.w, (wrap >> 2) & 3u));
+    const uint4 o = __ldg(reinterpret_cast<const uint4*>(&t.mip[mip].offset));  // offset, w, h
+    const float uw = u * d.x, vh = v * d.y;
+    uint32_t x, y;
+    if ((wrap & 0xFu) == 0u && d.z != 0.0f && d.w != 0.0f && fmaxf(fabsf(uw), fabsf(vh)) < 2147483648.0f &&
+        uw == uw && vh == vh) {
+        // Repeat over power-of-two sizes: floor(uw) - floor(floor(uw) / w) * w
+        // is exact and equals the integer's low bits, one conversion a side
+        // instead of three.
+        x = (uint32_t)__float2int_rd(uw) & (o.y - 1u);
+        y = (uint32_t)__float2int_rd(vh) & (o.z - 1u);
+    } else {
+        x = f2u_sat(apply_wrap(floorf(uw), d.x, d.z, wrap & 3u));
+        y = f2u_sat(apply_wrap(floorf(vh), d.y, d.w, (wrap >> 2) & 3u));
+    }
     return __ldg(t.data + (o.x + y * o.y + x));
 }
 
@@ -166,33 +177,35 @@ __device__ __forceinline__ void cube_uv(f3 n, float& uf, float& vf, uint32_t& sl
 }
 
 // sample_cubemap_rgb (src/texture.rs:646-663): nearest texel of one mip
-// (its texels, face size and stride).
-__device__ __forceinline__ f3 sample_cube(const uint32_t* data, float wf, float hf, uint32_t w, uint32_t stride,
-                                          float uf, float vf, uint32_t slice) {
-    float x = round_away(uf * (wf - 1.0f));
-    float y = round_away(vf * (hf - 1.0f));
-    x = clampf(x, 0.0f, wf - 1.0f);
-    y = clampf(y, 0.0f, hf - 1.0f);
-    return unpack_rgb(__ldg(data + (slice * stride + f2u_sat(y) * w + f2u_sat(x))));
+// (its texels, face size and stride). cube_uv's coordinates are in [0, 1] or
+// NaN (a quotient by the largest component), so x is not negative: rounding
+// half away is the floor of x + 1/2, which an addition rounded toward zero
+// cannot carry past the next integer; NaN becomes 0 as by the clamp.
+__device__ __forceinline__ f3 sample_cube(const uint32_t* data, float wf, float hf, uint32_t w, uint32_t h,
+                                          uint32_t stride, float uf, float vf, uint32_t slice) {
+    const uint32_t x = min(f2u_sat(__fadd_rz(uf * (wf - 1.0f), 0.5f)), w - 1u);
+    const uint32_t y = min(f2u_sat(__fadd_rz(vf * (hf - 1.0f), 0.5f)), h - 1u);
+    return unpack_rgb(__ldg(data + (slice * stride + y * w + x)));
 }
 __device__ __forceinline__ f3 sample_cube(const DTexture& t, float uf, float vf, uint32_t slice, uint32_t mip) {
     const float2 d = __ldg(reinterpret_cast<const float2*>(t.mip + mip));
     const uint4 o = __ldg(reinterpret_cast<const uint4*>(&t.mip[mip].offset));  // offset, w, h, stride
-    return sample_cube(t.data + o.x, d.x, d.y, o.y, o.w, uf, vf, slice);
+    return sample_cube(t.data + o.x, d.x, d.y, o.y, o.z, o.w, uf, vf, slice);
 }
 
 // sample_bilinear_rgb at mip 0, slice 0 (src/texture.rs:730-790); ClampToEdge.
-__device__ __forceinline__ f3 sample_bilinear(const uint32_t* data, float wf, float hf, uint32_t wi, float u, float v) {
+__device__ __forceinline__ f3 sample_bilinear(const uint32_t* data, float wf, float hf, uint32_t wi, uint32_t hi, float u,
+                                              float v) {
     const float xf = u * wf - 0.5f;
     const float yf = v * hf - 0.5f;
     const float x0 = floorf(xf), y0 = floorf(yf);
-    const float x1 = x0 + 1.0f, y1 = y0 + 1.0f;
     const float fx = xf - x0, fy = yf - y0;
     const float ofx = 1.0f - fx, ofy = 1.0f - fy;
-    const uint32_t x0i = f2u_sat(apply_wrap(x0, wf, 0.0f, 2u));
-    const uint32_t y0i = f2u_sat(apply_wrap(y0, hf, 0.0f, 2u));
-    const uint32_t x1i = f2u_sat(apply_wrap(x1, wf, 0.0f, 2u));
-    const uint32_t y1i = f2u_sat(apply_wrap(y1, hf, 0.0f, 2u));
+    // u and v are clamped to [0, 1], so x0 and y0 are integers from -1 to the
+    // last texel: the clamped neighbours are integer arithmetic.
+    const int32_t xi = __float2int_rz(x0), yi = __float2int_rz(y0);
+    const uint32_t x0i = (uint32_t)max(xi, 0), x1i = (uint32_t)min(xi + 1, (int32_t)wi - 1);
+    const uint32_t y0i = (uint32_t)max(yi, 0), y1i = (uint32_t)min(yi + 1, (int32_t)hi - 1);
     const f3 p00 = unpack_rgb(__ldg(data + (y0i * wi + x0i)));
     const f3 p10 = unpack_rgb(__ldg(data + (y0i * wi + x1i)));
     const f3 p01 = unpack_rgb(__ldg(data + (y1i * wi + x0i)));
@@ -1989,7 +2002,7 @@ __device__ __forceinline__ f3 skybox(const DView& v, const DScene& sc, int32_t q
     float uf, vf;
     uint32_t slice;
     cube_uv(n, uf, vf, slice);
-    return srgb_fast3(sample_cube(sc.sky, sc.sky_wf, sc.sky_hf, sc.sky_w, sc.sky_stride, uf, vf, slice));
+    return srgb_fast3(sample_cube(sc.sky, sc.sky_wf, sc.sky_hf, sc.sky_w, sc.sky_h, sc.sky_stride, uf, vf, slice));
 }
 
 // get_filtered_gi_sh4_packed_vec over the baked grid: every coefficient's
@@ -2216,7 +2229,7 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const M
         const f3 c1 = sample_cube(*sc.specular, uf, vf, slice, f2u_sat(m1));
         env = c0 + (c1 - c0) * t;
     }
-    const f3 lut = sample_bilinear(sc.brdf_lut, sc.brdf_wf, sc.brdf_hf, sc.brdf_w, clampf(ndv, 0.0f, 1.0f), clampf(rough, 0.0f, 1.0f));
+    const f3 lut = sample_bilinear(sc.brdf_lut, sc.brdf_wf, sc.brdf_hf, sc.brdf_w, sc.brdf_h, clampf(ndv, 0.0f, 1.0f), clampf(rough, 0.0f, 1.0f));
     const f3 bsf = f0 * lut.x + mk3(lut.y, lut.y, lut.y);
     f3 cis = env * bsf;
     const float ao_spec = 1.0f + (ao - 1.0f) * 0.5f;
@@ -2292,22 +2305,25 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
     // w, so it is taken from there; only warps with a quad over several
     // triangles exchange barycentrics (uncovered lanes hold 0, the contents of
     // a fresh renderer's vbuffer; src/tilerasterizer.rs:114-118) and divide.
-    const uint32_t tri = writer ? slot : 0xFFFFFFFFu;
-    const float w_own = writer ? 1.0f / interp(r.oow, b1, b2) : 0.0f;
-    float wq[4];
-    uint32_t other = 0u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int src = (int)((lane & ~3u) + (uint32_t)i);
-        wq[i] = __shfl_sync(0xFFFFFFFFu, w_own, src);
-        other |= __shfl_sync(0xFFFFFFFFu, tri, src) != tri ? 1u << i : 0u;
-    }
-    if (__any_sync(0xFFFFFFFFu, writer && other != 0u)) {
+    // A warp of sky skips all of it.
+    float w_own = 0.0f, wq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (__any_sync(0xFFFFFFFFu, writer)) {
+        const uint32_t tri = writer ? slot : 0xFFFFFFFFu;
+        if (writer) w_own = 1.0f / interp(r.oow, b1, b2);
+        uint32_t other = 0u;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int src = (int)((lane & ~3u) + (uint32_t)i);
-            const float ob1 = __shfl_sync(0xFFFFFFFFu, b1, src), ob2 = __shfl_sync(0xFFFFFFFFu, b2, src);
-            if (writer && (other & (1u << i))) wq[i] = 1.0f / interp(r.oow, ob1, ob2);
+            wq[i] = __shfl_sync(0xFFFFFFFFu, w_own, src);
+            other |= __shfl_sync(0xFFFFFFFFu, tri, src) != tri ? 1u << i : 0u;
+        }
+        if (__any_sync(0xFFFFFFFFu, writer && other != 0u)) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int src = (int)((lane & ~3u) + (uint32_t)i);
+                const float ob1 = __shfl_sync(0xFFFFFFFFu, b1, src), ob2 = __shfl_sync(0xFFFFFFFFu, b2, src);
+                if (writer && (other & (1u << i))) wq[i] = 1.0f / interp(r.oow, ob1, ob2);
+            }
         }
     }
     f3 col = mk3(0.0f, 0.0f, 0.0f);
@@ -2333,18 +2349,21 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
         }
     }
     // Tile-centre luminance (src/tilerasterizer.rs:103-106): quad (0, 16).
-    const float lum = (col.x * 0.2126f + col.y * 0.7152f) + col.z * 0.0722f;
-    const float l0 = __shfl_sync(0xFFFFFFFFu, lum, (int)(lane & ~3u));
-    const float l1 = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + 1u));
-    const float l2 = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + 2u));
-    const float l3 = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + 3u));
-    if (needed && centre && k == 0) {
-        const uint32_t tile = (uint32_t)(qy >> 5) * (uint32_t)v.tiles_x + (uint32_t)(qx >> 5);
-        v.tile_lum[tile] = (((l0 + l1) + l2) + l3) * 0.25f;
+    if (__any_sync(0xFFFFFFFFu, centre)) {  // one warp in 128 has one
+        const float lum = (col.x * 0.2126f + col.y * 0.7152f) + col.z * 0.0722f;
+        const float l0 = __shfl_sync(0xFFFFFFFFu, lum, (int)(lane & ~3u));
+        const float l1 = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + 1u));
+        const float l2 = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + 2u));
+        const float l3 = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + 3u));
+        if (needed && centre && k == 0) {
+            const uint32_t tile = (uint32_t)(qy >> 5) * (uint32_t)v.tiles_x + (uint32_t)(qx >> 5);
+            v.tile_lum[tile] = (((l0 + l1) + l2) + l3) * 0.25f;
+        }
     }
     if (!needed) return;
+    // Pixel indices stay below 2^30 (32768 x 32768).
     if (px < v.width && py < v.height) {
-        v.vis[(uint64_t)py * (uint64_t)v.width + (uint64_t)px] =
+        v.vis[(uint32_t)py * (uint32_t)v.width + (uint32_t)px] =
             covered ? (((unsigned long long)vis_hi << 3) | vis_fan) : ~0ull;
     }
     if (v.flags) {
@@ -2356,7 +2375,7 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
         c[2] = col.z;
     } else if (px < v.width && py < (v.height & ~1)) {
         const uint32_t c = tonemap_pack(col, v.exposure);
-        v.rgba8[(uint64_t)py * v.out_pitch + (uint64_t)px] = c;
+        v.rgba8[(uint32_t)py * v.out_pitch + (uint32_t)px] = c;
         if (v.rgba8_host) v.rgba8_host[(uint64_t)py * v.host_pitch + (uint64_t)px] = c;
     }
 }
@@ -2387,7 +2406,7 @@ __device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* 
     const bool needed = shade_needed(v, qx, qy);
     unsigned long long key = kEmptyKey;
     if (needed)
-        key = a.keys[v.key_offset + (uint64_t)(2 * qy + (k >> 1)) * v.key_pitch + (uint64_t)(2 * qx + (k & 1))];
+        key = (a.keys + v.key_offset)[(uint32_t)(2 * qy + (k >> 1)) * (uint32_t)v.key_pitch + (uint32_t)(2 * qx + (k & 1))];
     shade_pixel<GI, MODE>(a, tab, v, c.scene, qx, qy, k, needed, key);
 }
 
@@ -2410,14 +2429,19 @@ __global__ void __launch_bounds__(ShadeShape<GI>::kThreads, ShadeShape<GI>::kMin
     // CTA's 32 or 64 quads are one view's and all live.
     const uint32_t total = a.dyn->total_quads;
     const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t held = 0xFFFFFFFFu;
+    // Quads [q0, q1) are the held view's (a search per iteration took six
+    // dependent loads for each pixel of a 64-view batch).
+    uint32_t q0 = 0u, q1 = 0u;
     for (uint32_t base = blockIdx.x * blockDim.x; base < total * 4u; base += stride) {
-        const uint32_t vi = find_view_by_quad(a, base >> 2);
-        if (vi != held) {
+        const uint32_t q = base >> 2;
+        if (q < q0 || q >= q1) {
+            const uint32_t vi = find_view_by_quad(a, q);
             __syncthreads();
             load_shade_const(sc, a, vi, threadIdx.x, blockDim.x);
             __syncthreads();
-            held = vi;
+            const DView& v = sc.view();
+            q0 = v.quad_base;
+            q1 = q0 + v.quad_pitch * (uint32_t)v.tiles_y * 32u;
         }
         shade_thread<GI, MODE>(a, tab, sc, base + threadIdx.x);
     }

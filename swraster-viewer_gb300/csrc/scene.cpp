@@ -1482,11 +1482,13 @@ swr_status upload_scene(SceneImpl* s, std::string& err, bool to_device) {
     ds.spec_max_mip = (float)dtex[nt + 1].max_mip;
     ds.sky = cube.data + cube.mip[0].offset;
     ds.sky_w = cube.mip[0].w;
+    ds.sky_h = cube.mip[0].h;
     ds.sky_stride = cube.mip[0].stride;
     ds.sky_wf = cube.mip[0].wf;
     ds.sky_hf = cube.mip[0].hf;
     ds.brdf_lut = lut.data + lut.mip[0].offset;
     ds.brdf_w = lut.mip[0].w;
+    ds.brdf_h = lut.mip[0].h;
     ds.brdf_wf = lut.mip[0].wf;
     ds.brdf_hf = lut.mip[0].hf;
     ds.voxel_n = s->voxel_n;
