@@ -160,13 +160,13 @@ uint32_t BatchImpl::tuned_tile(const swr_view_desc* vd, int32_t n) const {
         h[(size_t)i] = vd[i].height;
     }
     const uint32_t S = auto_sched_tile(w.data(), h.data(), n, eng.num_sms);
-    // Several views: at most 32-px tiles, shaded inside the raster kernel.
-    // Tiles of uneven views balance better over the persistent CTAs, and the
-    // keys stay in shared memory: a burst of 24 requests takes 1,190 us,
-    // against 1,330 with 32-px tiles shaded apart and 1,460 with 64-px tiles
-    // (64 views of one scene 2,817, 2,988 and 2,730; eight uneven scenes
-    // 1,497, 1,445 and 1,400).
-    if (n > 1 && S >= 32u) return 32u | 0x100u;
+    // Several views: at most 32-px tiles, which balance better over the
+    // persistent CTAs where views and tiles are uneven. Shaded apart they take
+    // 2,364 us for 64 views of one scene, 1,374 for eight uneven scenes and
+    // 1,093 for a burst of 24 requests, fused into the raster kernel (the
+    // autotuner's other form) 2,631, 1,504 and 1,083; 64-px tiles took 2,377,
+    // 1,340 and 1,359 (before tiles without packets were left out).
+    if (n > 1 && S >= 32u) return 32u;
     return S;
 }
 

@@ -261,6 +261,9 @@ enum : uint32_t {
 constexpr uint32_t kStRetry =
     ST_BIN_OVERFLOW | ST_CLIP_OVERFLOW | ST_QUEUE_OVERFLOW | ST_TRANS_OVERFLOW | ST_DRAW_OVERFLOW;
 
+// Size buckets of the raster's visiting order: two per octave of a bin's packets, and empty bins.
+constexpr int kOrderBuckets = 66;
+
 // Frame-level counters (device).
 struct alignas(16) DCounters {
     uint32_t status;
@@ -278,6 +281,9 @@ struct alignas(16) DCounters {
     uint32_t culled;           // (triangle, tile) pairs the raster dropped as hidden
     uint32_t clip_path;        // triangles of draws whose sphere intersects the frustum (the clip path)
     uint32_t unsampled;        // (triangle, tile) pairs of triangles that hold no pixel centre (not binned)
+    uint32_t scan_done;        // k_scan's CTAs done
+    uint32_t filled;           // scheduling tiles with opaque packets, first in the visiting order
+    uint32_t bucket[kOrderBuckets];  // opaque bins per size bucket; then the next place in the visiting order
     uint32_t wide_main;        // wide-queue segments appended by k_frontend
     uint32_t wide_clip;        // ... and by k_clip (second half of the queue)
 };
@@ -330,8 +336,9 @@ struct FrameArgs {
     uint32_t* fan_base;
     uint2* clip_queue;         // (g, draw)
     uint2* wide_queue;         // 2 * wide_cap entries: k_frontend's, then k_clip's
-    uint32_t* tile_count;      // n_bins; after k_scan, the raster tile order
-    uint32_t* tile_offset;     // n_bins + 1
+    uint32_t* tile_count;      // n_bins
+    uint32_t* tile_offset;     // n_bins
+    uint4* work;               // n_stiles raster work items in visiting order (k_scatter)
     uint32_t* tile_cursor;     // n_bins
     uint32_t* bins;
     unsigned long long* keys;

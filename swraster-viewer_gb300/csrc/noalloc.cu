@@ -66,7 +66,8 @@ constexpr size_t oClipQ = oFan + al(sizeof(uint32_t) * kNaMaxTris);
 constexpr size_t oCount = oClipQ + al(sizeof(uint2) * kNaMaxTris);
 constexpr size_t oOffset = oCount + al(sizeof(uint32_t) * (kNaTiles + 1));
 constexpr size_t oCursor = oOffset + al(sizeof(uint32_t) * (kNaTiles + 1));
-constexpr size_t oBins = oCursor + al(sizeof(uint32_t) * (kNaTiles + 1));
+constexpr size_t oWork = oCursor + al(sizeof(uint32_t) * (kNaTiles + 1));
+constexpr size_t oBins = oWork + al(sizeof(uint4) * kNaTiles);
 constexpr size_t oKeys = oBins + al(sizeof(uint32_t) * kNaBinCap);
 constexpr size_t oCounters = oKeys + al(sizeof(unsigned long long) * kNaMaxDim * kNaMaxDim);
 constexpr size_t oTab = oCounters + al(sizeof(DCounters));
@@ -290,6 +291,7 @@ extern "C" swr_status swr_render_frame_noalloc(const swr_scene* scene, const swr
     a.clip_queue = reinterpret_cast<uint2*>(base + oClipQ);
     a.tile_count = reinterpret_cast<uint32_t*>(base + oCount);
     a.tile_offset = reinterpret_cast<uint32_t*>(base + oOffset);
+    a.work = reinterpret_cast<uint4*>(base + oWork);
     a.tile_cursor = reinterpret_cast<uint32_t*>(base + oCursor);
     a.bins = reinterpret_cast<uint32_t*>(base + oBins);
     a.keys = reinterpret_cast<unsigned long long*>(base + oKeys);
