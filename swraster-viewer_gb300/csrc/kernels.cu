@@ -2421,14 +2421,14 @@ __device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* 
     shade_pixel<GI, MODE>(a, tab, v, c.scene, qx, qy, k, needed, key);
 }
 
-// CTA shape of the grid-stride shading kernel. Without voxel GI, seven
-// 128-thread CTAs per SM (<= 72 registers): 4K frame shade 0.604 ms, against
-// 0.612 ms at three 256-thread CTAs (80 registers), 0.741 ms at two (95) and
-// 0.663 ms at four (64). The GI variant keeps three 256-thread CTAs: at 72
-// registers its cone-tracing loop spills 216 B per thread.
+// CTA shape of the grid-stride shading kernel. Without voxel GI, eight
+// 128-thread CTAs per SM (64 registers): 4K shade 442 us, against 451 at seven
+// (72), 450 at six and 471 at five; 64 views 1,478, 1,490, 1,555 and 1,720.
+// The GI variant keeps three 256-thread CTAs: at 72 registers its cone-tracing
+// loop spills 216 B per thread.
 template <bool GI> struct ShadeShape {
     static constexpr int kThreads = GI ? 256 : 128;
-    static constexpr int kMinBlocks = GI ? 3 : 7;
+    static constexpr int kMinBlocks = GI ? 3 : 8;
 };
 // GI: the frame has scenes with a baked voxel grid. MODE: see shade_pixel.
 template <bool GI, int MODE>
