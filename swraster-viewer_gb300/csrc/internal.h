@@ -338,6 +338,7 @@ struct FrameArgs {
     uint2* wide_queue;         // 2 * wide_cap entries: k_frontend's, then k_clip's
     uint32_t* tile_count;      // n_bins
     uint32_t* tile_offset;     // n_bins
+    uint8_t* sky_tab;          // 256 per view: RGBA8 value of a sky texel's byte (k_scatter)
     uint4* work;               // n_stiles raster work items in visiting order (k_scatter)
     uint32_t* tile_cursor;     // n_bins
     uint32_t* bins;

@@ -98,6 +98,17 @@ __device__ __forceinline__ f3 unpack_rgb(uint32_t t) { return {unorm8(t >> 9), u
 __device__ __forceinline__ float srgb_fast(float x) { return x * (x * (x * 0.305306011f + 0.682171111f) + 0.012522878f); }
 __device__ __forceinline__ f3 srgb_fast3(f3 c) { return {srgb_fast(c.x), srgb_fast(c.y), srgb_fast(c.z)}; }
 
+// One channel of blit_to_buffer (src/renderer.rs:325-348) and tonemap
+// (src/util.rs:37-41).
+__device__ __forceinline__ uint32_t tonemap_u8(float c, float exposure) {
+    const float k = 0.2f;
+    c = c * exposure;
+    return f2u8_sat(((c / (c + k)) * (1.0f + k)) * 255.0f);
+}
+__device__ __forceinline__ uint32_t tonemap_pack(f3 c, float exposure) {
+    return (tonemap_u8(c.x, exposure) << 24) | (tonemap_u8(c.y, exposure) << 16) | (tonemap_u8(c.z, exposure) << 8) | 0xFFu;
+}
+
 // --------------------------------------------------------------------------
 // Texture sampling (src/texture.rs:578-863)
 // --------------------------------------------------------------------------
@@ -176,16 +187,16 @@ __device__ __forceinline__ void cube_uv(f3 n, float& uf, float& vf, uint32_t& sl
 // NaN (a quotient by the largest component), so x is not negative: rounding
 // half away is the floor of x + 1/2, which an addition rounded toward zero
 // cannot carry past the next integer; NaN becomes 0 as by the clamp.
-__device__ __forceinline__ f3 sample_cube(const uint32_t* data, float wf, float hf, uint32_t w, uint32_t h,
-                                          uint32_t stride, float uf, float vf, uint32_t slice) {
+__device__ __forceinline__ uint32_t sample_cube(const uint32_t* data, float wf, float hf, uint32_t w, uint32_t h,
+                                                uint32_t stride, float uf, float vf, uint32_t slice) {
     const uint32_t x = min(f2u_sat(__fadd_rz(uf * (wf - 1.0f), 0.5f)), w - 1u);
     const uint32_t y = min(f2u_sat(__fadd_rz(vf * (hf - 1.0f), 0.5f)), h - 1u);
-    return unpack_rgb(__ldg(data + (slice * stride + y * w + x)));
+    return __ldg(data + (slice * stride + y * w + x));
 }
 __device__ __forceinline__ f3 sample_cube(const DTexture& t, float uf, float vf, uint32_t slice, uint32_t mip) {
     const float2 d = __ldg(reinterpret_cast<const float2*>(t.mip + mip));
     const uint4 o = __ldg(reinterpret_cast<const uint4*>(&t.mip[mip].offset));  // offset, w, h, stride
-    return sample_cube(t.data + o.x, d.x, d.y, o.y, o.z, o.w, uf, vf, slice);
+    return unpack_rgb(sample_cube(t.data + o.x, d.x, d.y, o.y, o.z, o.w, uf, vf, slice));
 }
 
 // sample_bilinear_rgb at mip 0, slice 0 (src/texture.rs:730-790); ClampToEdge.
@@ -1247,7 +1258,14 @@ __device__ __forceinline__ uint32_t find_view_by_stile(const FrameArgs& a, uint3
 // threads; the raster then reads one item a tile instead of an order entry,
 // two offsets, a search for the view and its tile pitch one after another).
 // After an overflow (the frame is rendered again) every bin is empty.
+//
+// Also each view's table from a sky texel's byte to its RGBA8 value, which
+// depends on nothing else: a sky pixel then takes three lookups instead of
+// the colour and three divisions of the tone map (a fifth of its
+// instructions).
 __device__ __forceinline__ void place_work(const FrameArgs& a, bool bad) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.dyn->n_views * 256u; i += gridDim.x * blockDim.x)
+        a.sky_tab[i] = (uint8_t)tonemap_u8(srgb_fast(unorm8((i & 0xFFu) << 15)), a.views[i >> 8].exposure);
     const uint32_t n_st = a.dyn->n_stiles, lane = threadIdx.x & 31u;
     const bool order = a.sched_tile >= kOrderMinTile;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -1470,6 +1488,7 @@ __device__ __forceinline__ bool region_exact(const PacketCtx& c, const float w[1
 struct alignas(16) ShadeConst {
     DScene scene;
     unsigned char head[kViewHead];  // the part of the DView before cam_view
+    uint8_t sky[256];               // the view's sky_tab
     __device__ __forceinline__ const DView& view() const { return *reinterpret_cast<const DView*>(head); }
 };
 __device__ __forceinline__ void load_shade_const(ShadeConst& c, const FrameArgs& a, uint32_t vi, uint32_t t, uint32_t nt) {
@@ -1480,6 +1499,8 @@ __device__ __forceinline__ void load_shade_const(ShadeConst& c, const FrameArgs&
     uint4* d1 = reinterpret_cast<uint4*>(c.head);
     for (uint32_t i = t; i < sizeof(DScene) / 16; i += nt) d0[i] = s0[i];
     for (uint32_t i = t; i < kViewHead / 16; i += nt) d1[i] = s1[i];
+    const uint4* s2 = reinterpret_cast<const uint4*>(a.sky_tab + 256u * vi);
+    if (t < 16u) reinterpret_cast<uint4*>(c.sky)[t] = s2[t];
 }
 
 template <int S>
@@ -1753,9 +1774,8 @@ __device__ __forceinline__ bool shade_needed(const DView& v, int32_t qx, int32_t
 // SWR_RSQRT_AARCH64, or any (read per view).
 constexpr int kModeIeee = 0, kModeArm = 1, kModeAny = 2;
 template <bool GI, int MODE>
-__device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* tab, const DView& v,
-                                            const DScene& sc, int32_t qx, int32_t qy, int32_t k, bool needed,
-                                            unsigned long long key);
+__device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* tab, const ShadeConst& c, int32_t qx,
+                                            int32_t qy, int32_t k, bool needed, unsigned long long key);
 
 // Occlusion culling is on for 64-px scheduling tiles and for the 32-px tiles
 // that take more than one round (SWR_CULL_FROM packets). It pays where many
@@ -1974,7 +1994,7 @@ __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kM
                 const bool needed = live && shade_needed(s.shade.view(), qx, qy);
                 unsigned long long key = kEmptyKey;
                 if (needed && !no_keys) key = s.sk[(2 * (ql / QS) + (k >> 1)) * S + 2 * (ql % QS) + (k & 1)];
-                shade_pixel<GI, MODE>(a, s.tab, s.shade.view(), s.shade.scene, qx, qy, k, needed, key);
+                shade_pixel<GI, MODE>(a, s.tab, s.shade, qx, qy, k, needed, key);
             }
         }
         if (kAhead && threadIdx.x == 0) fetch(wnext, &s.item[(iter + 1u) & 1u]);
@@ -1995,8 +2015,9 @@ __device__ __forceinline__ uint32_t find_view_by_quad(const FrameArgs& a, uint32
     return lo;
 }
 
-// compute_skybox for one lane (src/tilerasterizer.rs:478-508).
-__device__ __forceinline__ f3 skybox(const DView& v, const DScene& sc, int32_t qx_screen, int32_t qy_screen,
+// compute_skybox for one lane (src/tilerasterizer.rs:478-508): the texel, whose
+// colour is srgb_fast3 of its bytes.
+__device__ __forceinline__ uint32_t skybox_texel(const DView& v, const DScene& sc, int32_t qx_screen, int32_t qy_screen,
                                      int32_t kx, int32_t ky, uint32_t md, const uint8_t* tab) {
     const float pxf = i2f(qx_screen) + (kx ? 1.5f : 0.5f);
     const float pyf = i2f(qy_screen) + (ky ? 1.5f : 0.5f);
@@ -2011,7 +2032,7 @@ __device__ __forceinline__ f3 skybox(const DView& v, const DScene& sc, int32_t q
     float uf, vf;
     uint32_t slice;
     cube_uv(n, uf, vf, slice);
-    return srgb_fast3(sample_cube(sc.sky, sc.sky_wf, sc.sky_hf, sc.sky_w, sc.sky_h, sc.sky_stride, uf, vf, slice));
+    return sample_cube(sc.sky, sc.sky_wf, sc.sky_hf, sc.sky_w, sc.sky_h, sc.sky_stride, uf, vf, slice);
 }
 
 // get_filtered_gi_sh4_packed_vec over the baked grid: every coefficient's
@@ -2259,18 +2280,6 @@ __device__ __forceinline__ f3 pbr_lane(const DScene& sc, const DView& v, const M
     return col;
 }
 
-__device__ __forceinline__ uint32_t tonemap_pack(f3 c, float exposure) {
-    // blit_to_buffer (src/renderer.rs:325-348) and tonemap (src/util.rs:37-41).
-    const float k = 0.2f;
-    const float kk = 1.0f + k;
-    c = c * exposure;
-    const f3 d = c + mk3(k, k, k);
-    c = mk3(c.x / d.x, c.y / d.y, c.z / d.z) * kk;
-    c = c * 255.0f;
-    const uint32_t r = f2u8_sat(c.x), g = f2u8_sat(c.y), b = f2u8_sat(c.z);
-    return (r << 24) | (g << 16) | (b << 8) | 0xFFu;
-}
-
 // One lane of the shading pass; all 32 lanes of a warp call it together
 // (quad barycentrics and luminance are exchanged with warp shuffles).
 // Whether pixel lane k of quad (qx, qy) of view v is shaded: inside the
@@ -2285,9 +2294,10 @@ __device__ __forceinline__ bool shade_needed(const DView& v, int32_t qx, int32_t
 // the reciprocal square root of every view of the launch, so only that one
 // is compiled in, or kModeAny to read it from the view.
 template <bool GI, int MODE>
-__device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* tab, const DView& v,
-                                            const DScene& sc, int32_t qx, int32_t qy, int32_t k, bool needed,
-                                            unsigned long long key) {
+__device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* tab, const ShadeConst& c, int32_t qx,
+                                            int32_t qy, int32_t k, bool needed, unsigned long long key) {
+    const DView& v = c.view();
+    const DScene& sc = c.scene;
     const uint32_t md = MODE == kModeAny ? v.rsqrt_mode : (uint32_t)MODE;
     const uint32_t lane = threadIdx.x & 31u;
     const int32_t kx = k & 1, ky = k >> 1;
@@ -2336,7 +2346,8 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
         }
     }
     f3 col = mk3(0.0f, 0.0f, 0.0f);
-    uint32_t vis_hi = 0xFFFFFFFFu, vis_fan = 0;
+    uint32_t vis_hi = 0xFFFFFFFFu, vis_fan = 0, sky = 0;
+    const bool meter = __any_sync(0xFFFFFFFFu, centre);  // one warp in 128 has a centre quad
     if (needed) {
         if (covered) {
             RecShade q;
@@ -2354,11 +2365,14 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
             vis_hi = q.static_id;
             vis_fan = r.seq8 & 7u;
         } else {
-            col = skybox(v, sc, 2 * qx, 2 * qy, kx, ky, md, tab);
+            // The colour itself is only wanted by the luminance meter and
+            // for a later resolve.
+            sky = skybox_texel(v, sc, 2 * qx, 2 * qy, kx, ky, md, tab);
+            if (meter || v.flags) col = srgb_fast3(unpack_rgb(sky));
         }
     }
     // Tile-centre luminance (src/tilerasterizer.rs:103-106): quad (0, 16).
-    if (__any_sync(0xFFFFFFFFu, centre)) {  // one warp in 128 has one
+    if (meter) {
         const float lum = (col.x * 0.2126f + col.y * 0.7152f) + col.z * 0.0722f;
         const float l0 = __shfl_sync(0xFFFFFFFFu, lum, (int)(lane & ~3u));
         const float l1 = __shfl_sync(0xFFFFFFFFu, lum, (int)((lane & ~3u) + 1u));
@@ -2378,14 +2392,19 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
     if (v.flags) {
         // Linear colour over the padded tile grid (the translucent pass may
         // blend into the off-screen centre quad the luminance meter reads).
-        float* c = v.color + ((uint64_t)py * v.key_pitch + (uint64_t)px) * 3u;
-        c[0] = col.x;
-        c[1] = col.y;
-        c[2] = col.z;
+        float* out = v.color + ((uint64_t)py * v.key_pitch + (uint64_t)px) * 3u;
+        out[0] = col.x;
+        out[1] = col.y;
+        out[2] = col.z;
     } else if (px < v.width && py < (v.height & ~1)) {
-        const uint32_t c = tonemap_pack(col, v.exposure);
-        v.rgba8[(uint32_t)py * v.out_pitch + (uint32_t)px] = c;
-        if (v.rgba8_host) v.rgba8_host[(uint64_t)py * v.host_pitch + (uint64_t)px] = c;
+        uint32_t p;
+        if (covered)
+            p = tonemap_pack(col, v.exposure);
+        else
+            p = ((uint32_t)c.sky[sky >> 24] << 24) | ((uint32_t)c.sky[(sky >> 16) & 0xFFu] << 16) |
+                ((uint32_t)c.sky[(sky >> 8) & 0xFFu] << 8) | 0xFFu;
+        v.rgba8[(uint32_t)py * v.out_pitch + (uint32_t)px] = p;
+        if (v.rgba8_host) v.rgba8_host[(uint64_t)py * v.host_pitch + (uint64_t)px] = p;
     }
 }
 
@@ -2418,7 +2437,7 @@ __device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* 
     const uint32_t st = v.stile_base + ((uint32_t)qy >> sh) * (uint32_t)v.stiles_x + ((uint32_t)qx >> sh);
     if (needed && tile_filled(a, st))
         key = (a.keys + v.key_offset)[(uint32_t)(2 * qy + (k >> 1)) * (uint32_t)v.key_pitch + (uint32_t)(2 * qx + (k & 1))];
-    shade_pixel<GI, MODE>(a, tab, v, c.scene, qx, qy, k, needed, key);
+    shade_pixel<GI, MODE>(a, tab, c, qx, qy, k, needed, key);
 }
 
 // CTA shape of the grid-stride shading kernel. Without voxel GI, eight

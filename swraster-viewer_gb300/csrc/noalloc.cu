@@ -67,7 +67,8 @@ constexpr size_t oCount = oClipQ + al(sizeof(uint2) * kNaMaxTris);
 constexpr size_t oOffset = oCount + al(sizeof(uint32_t) * (kNaTiles + 1));
 constexpr size_t oCursor = oOffset + al(sizeof(uint32_t) * (kNaTiles + 1));
 constexpr size_t oWork = oCursor + al(sizeof(uint32_t) * (kNaTiles + 1));
-constexpr size_t oBins = oWork + al(sizeof(uint4) * kNaTiles);
+constexpr size_t oSky = oWork + al(sizeof(uint4) * kNaTiles);
+constexpr size_t oBins = oSky + al(256);
 constexpr size_t oKeys = oBins + al(sizeof(uint32_t) * kNaBinCap);
 constexpr size_t oCounters = oKeys + al(sizeof(unsigned long long) * kNaMaxDim * kNaMaxDim);
 constexpr size_t oTab = oCounters + al(sizeof(DCounters));
@@ -292,6 +293,7 @@ extern "C" swr_status swr_render_frame_noalloc(const swr_scene* scene, const swr
     a.tile_count = reinterpret_cast<uint32_t*>(base + oCount);
     a.tile_offset = reinterpret_cast<uint32_t*>(base + oOffset);
     a.work = reinterpret_cast<uint4*>(base + oWork);
+    a.sky_tab = base + oSky;
     a.tile_cursor = reinterpret_cast<uint32_t*>(base + oCursor);
     a.bins = reinterpret_cast<uint32_t*>(base + oBins);
     a.keys = reinterpret_cast<unsigned long long*>(base + oKeys);

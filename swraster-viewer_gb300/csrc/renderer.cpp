@@ -179,7 +179,7 @@ void FrameEngine::release() {
     if (capture_stream) cudaStreamDestroy(capture_stream);
     capture_stream = nullptr;
     for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &rec_t, &fan_base, &clip_queue, &wide_queue, &tile_count, &tile_offset,
-                    &tile_cursor, &work, &bins, &keys, &counters, &rsqrt_tab, &color})
+                    &tile_cursor, &work, &sky_tab, &bins, &keys, &counters, &rsqrt_tab, &color})
         b->release();
     for (int i = 0; i < kStageRing; ++i) {
         h_stage[i].release();
@@ -286,6 +286,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     chk(tile_count.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
     chk(tile_offset.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
     chk(tile_cursor.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
+    chk(sky_tab.ensure((size_t)view_cap * 256));
     chk(work.ensure((size_t)(stile_cap / 2 + 1) * sizeof(uint4)));
     chk(bins.ensure(bin_cap * sizeof(uint32_t)));
     chk(keys.ensure(std::max<uint64_t>(1, key_cap) * sizeof(unsigned long long)));
@@ -366,6 +367,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     a.tile_count = tile_count.as<uint32_t>();
     a.tile_offset = tile_offset.as<uint32_t>();
     a.work = work.as<uint4>();
+    a.sky_tab = sky_tab.as<uint8_t>();
     a.tile_cursor = tile_cursor.as<uint32_t>();
     a.bins = bins.as<uint32_t>();
     a.keys = keys.as<unsigned long long>();

@@ -86,7 +86,7 @@ struct FrameEngine {
     bool fuse32 = false;        // 32-px tiles shade inside the raster kernel (batch autotuner's choice)
     bool grid_fused32 = false;
     DBuf tables, tri_state, rec_r, rec_s, rec_t, fan_base, clip_queue, wide_queue;
-    DBuf tile_count, tile_offset, tile_cursor, work, bins, keys, counters, rsqrt_tab;
+    DBuf tile_count, tile_offset, tile_cursor, work, sky_tab, bins, keys, counters, rsqrt_tab;
     DBuf color;                // linear colour of views that need it (padded tile grids)
     bool defer_resolve = false;// the caller resolves (renderer frames with dt > 0)
     static constexpr int kStageRing = 4;
