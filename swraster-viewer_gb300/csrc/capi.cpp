@@ -210,6 +210,7 @@ swr_status swr_renderer_create(int32_t width, int32_t height, const swr_renderer
     r->height = height;
     r->opts = o;
     r->eng.bin_cap = o.bin_capacity;
+    r->eng.auto_graph = true;
     std::string err;
     swr_status st = r->eng.init(err);
     if (st != SWR_OK) {

@@ -402,8 +402,12 @@ swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string
         stage_pending[slot] = true;
         stage_slot = (slot + 1) % kStageRing;
     }
-    if (e == cudaSuccess && use_graph && !ev) {
-        const bool same = graph_exec && std::memcmp(&graph_args, &args, sizeof(args)) == 0;
+    const bool same = graph_exec && std::memcmp(&graph_args, &args, sizeof(args)) == 0;
+    if (auto_graph) {
+        same_frames = std::memcmp(&prev_args, &args, sizeof(args)) == 0 ? same_frames + 1 : 0;
+        prev_args = args;
+    }
+    if (e == cudaSuccess && !ev && (use_graph || (auto_graph && (same || same_frames >= kGraphAfter)))) {
         if (!same) {
             if (graph_exec) cudaGraphExecDestroy(graph_exec);
             graph_exec = nullptr;

@@ -105,6 +105,13 @@ struct FrameEngine {
     FrameArgs args{};
     // Graph replay.
     bool use_graph = false;
+    // Renderer frames: capture once a frame's arguments (pointers, capacities,
+    // kernel variants) have stayed the same for kGraphAfter frames, so that
+    // neither a first frame nor alternating scenes pay for a capture.
+    bool auto_graph = false;
+    static constexpr uint32_t kGraphAfter = 4;
+    uint32_t same_frames = 0;
+    FrameArgs prev_args{};
     cudaGraphExec_t graph_exec = nullptr;
     FrameArgs graph_args{};
     cudaStream_t graph_stream = nullptr;
