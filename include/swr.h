@@ -651,7 +651,7 @@ swr_status swr_selftest_depth_floor(const int32_t* p, const float* zow, const fl
  * caller's device buffers rgba8 (width*height, row pitch width; an odd last
  * row is left untouched) and vis (width*height), with a fixed `exposure`
  * (2.0 is a fresh renderer's) and without allocating anything: all per-frame
- * work buffers live in one fixed __device__ array of about 9 MB that every
+ * work buffers live in one fixed __device__ array of about 10 MB that every
  * GPU loading the library holds until exit. Limits: width, height <= 512, at
  * most 16384 triangles passing the frustum test, 4096 nodes, 4096 draws,
  * 65536 (triangle, tile) pairs, no translucent primitives; larger inputs

@@ -280,6 +280,7 @@ struct alignas(16) DCounters {
     uint32_t draw_count;
     uint32_t culled;           // (triangle, tile) pairs the raster dropped as hidden
     uint32_t clip_path;        // triangles of draws whose sphere intersects the frustum (the clip path)
+    uint32_t ref_pairs;        // (triangle, 64-px tile) pairs of a frame with a pair limit
     uint32_t unsampled;        // (triangle, tile) pairs of triangles that hold no pixel centre (not binned)
     uint32_t scan_done;        // k_scan's CTAs done
     uint32_t filled;           // scheduling tiles with opaque packets, first in the visiting order
@@ -357,6 +358,7 @@ struct FrameArgs {
     uint32_t fused_shade;      // 32-px tiles: shade inside the raster kernel (8 and 16 px always do)
     uint32_t has_gi;           // some scene of the frame has a baked voxel grid
     uint32_t gpu_draws;        // build draws and chunks on the device (else the host staged them)
+    uint32_t pair_limit;       // (triangle, 64-px tile) pairs past which a frame counts as overflowed, 0 = none
     uint32_t skip_unsampled;   // triangles that hold no pixel centre are not binned
     uint32_t rsqrt_uniform;    // 1 + the rsqrt mode all views share, 0 = per view
 };

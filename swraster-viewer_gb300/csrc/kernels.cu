@@ -414,6 +414,10 @@ __device__ __forceinline__ TileRect tile_rect(const DView& v, uint32_t S, uint32
     t.first = bin_off + v.stile_base + y0 * t.pitch + x0;
     return t;
 }
+// A record's (triangle, 64-px tile) pairs.
+__device__ __forceinline__ uint32_t ref_pairs(const DView& v, const RecRaster& r) {
+    return tile_rect(v, (uint32_t)kRefTile, 0u, r.bb[0], r.bb[1], r.bb[2], r.bb[3]).count();
+}
 template <typename F>
 __device__ __forceinline__ void for_each_stile(const TileRect& t, F f) {
     for (uint32_t y = 0; y < t.ny; ++y)
@@ -854,6 +858,7 @@ __global__ void __launch_bounds__(256) k_reset(FrameArgs a) {
         a.counters->trans_packets = 0u;
         a.counters->culled = 0u;
         a.counters->clip_path = 0u;
+        a.counters->ref_pairs = 0u;
         a.counters->unsampled = 0u;
         a.counters->scan_done = 0u;
         a.counters->wide_main = 0u;
@@ -950,6 +955,7 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
     a.tri_state[g] = res == kSetupRecord ? 1 : 0;
     warp_count(&a.counters->setup_tris, res != kSetupNone);
     warp_sum(&a.counters->unsampled, res == kSetupUnsampled ? tiles.count() : 0u);
+    if (a.pair_limit) warp_sum(&a.counters->ref_pairs, res == kSetupRecord ? ref_pairs(view, r) : 0u);
 }
 
 // Thread per triangle of a 256-triangle chunk, CTA per chunk (a loop over
@@ -1114,6 +1120,7 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
                 if (tiles.count() > kWideTiles &&
                     push_wide(a, &a.counters->wide_clip, a.wide_queue + a.wide_cap, slot, tiles.count()))
                     r.wide = 1u;
+                if (a.pair_limit) atomicAdd(&a.counters->ref_pairs, ref_pairs(view, r));
                 store_records(a, slot, r, q);
                 if (flags & MAT_NORMAL_MAP) store_tangents(a, slot, pl[0], pl[i + 1], pl[i + 2]);
             } else if (i > 0u) {
@@ -1226,7 +1233,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(FrameArgs a) {
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (threadIdx.x == 0 && __ldcg(&a.counters->pairs) > a.bin_cap) atomicOr(&a.counters->status, ST_BIN_OVERFLOW);
+    if (threadIdx.x == 0 && (__ldcg(&a.counters->pairs) > a.bin_cap || (a.pair_limit && a.counters->ref_pairs > a.pair_limit)))
+        atomicOr(&a.counters->status, ST_BIN_OVERFLOW);
     if (!order) return;
     for (int i = threadIdx.x; i < kOrderBuckets; i += kScanThreads) hist[i] = __ldcg(&a.counters->bucket[i]);
     __syncthreads();

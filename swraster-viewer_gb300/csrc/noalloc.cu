@@ -15,7 +15,7 @@
 // clipped triangles exceed the fixed capacity on the device returns
 // SWR_OVERFLOW.
 //
-// The array (about 9 MB) stays allocated on every GPU that loads the library
+// The array (about 10 MB) stays allocated on every GPU that loads the library
 // until the process exits. Its device address is looked up with
 // cudaGetSymbolAddress on the first call on each device. All calls on a
 // device share that device's array and it keeps the last call's contents:
@@ -47,8 +47,15 @@ constexpr uint32_t kNaExtra = 8192;
 constexpr uint32_t kNaMaxNodes = 4096;
 constexpr uint32_t kNaMaxDraws = 4096;
 constexpr uint32_t kNaMaxChunks = kNaMaxTris / kChunkTris + kNaMaxDraws;
-constexpr uint32_t kNaBinCap = 65536;
-constexpr uint32_t kNaTiles = (kNaMaxDim / kRefTile) * (kNaMaxDim / kRefTile);
+// The pair limit counts 64-px tiles; the raster runs on 32-px ones (a 500x281
+// frame has 40 of the former for 152 SMs: raster 63 us, frame 122 -> 93), of which one 64-px
+// pair makes at most four.
+constexpr uint32_t kNaPairLimit = 65536;
+constexpr int32_t kNaTile = 32;
+constexpr uint32_t kNaBinCap = 4 * kNaPairLimit;
+constexpr uint32_t kNaRefTiles = (kNaMaxDim / kRefTile) * (kNaMaxDim / kRefTile);
+constexpr uint32_t kNaTiles = (kNaMaxDim / kNaTile) * (kNaMaxDim / kNaTile);
+constexpr uint32_t kNaWideCap = 2048;
 
 constexpr size_t al(size_t x) { return (x + 255) & ~size_t(255); }
 // Scratch layout (byte offsets).
@@ -63,7 +70,8 @@ constexpr size_t oRecS = oRecR + al(sizeof(RecRaster) * (kNaMaxTris + kNaExtra))
 constexpr size_t oRecT = oRecS + al(sizeof(RecShade) * (kNaMaxTris + kNaExtra));
 constexpr size_t oFan = oRecT + al(sizeof(RecTangent) * (kNaMaxTris + kNaExtra));
 constexpr size_t oClipQ = oFan + al(sizeof(uint32_t) * kNaMaxTris);
-constexpr size_t oCount = oClipQ + al(sizeof(uint2) * kNaMaxTris);
+constexpr size_t oWide = oClipQ + al(sizeof(uint2) * kNaMaxTris);
+constexpr size_t oCount = oWide + al(sizeof(uint2) * 2 * kNaWideCap);
 constexpr size_t oOffset = oCount + al(sizeof(uint32_t) * (kNaTiles + 1));
 constexpr size_t oCursor = oOffset + al(sizeof(uint32_t) * (kNaTiles + 1));
 constexpr size_t oWork = oCursor + al(sizeof(uint32_t) * (kNaTiles + 1));
@@ -73,7 +81,7 @@ constexpr size_t oKeys = oBins + al(sizeof(uint32_t) * kNaBinCap);
 constexpr size_t oCounters = oKeys + al(sizeof(unsigned long long) * kNaMaxDim * kNaMaxDim);
 constexpr size_t oTab = oCounters + al(sizeof(DCounters));
 constexpr size_t oLum = oTab + al(512);
-constexpr size_t kNaScratchBytes = oLum + al(sizeof(float) * kNaTiles);
+constexpr size_t kNaScratchBytes = oLum + al(sizeof(float) * kNaRefTiles);
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNaScratchBytes];
 
@@ -167,7 +175,7 @@ extern "C" swr_status swr_render_frame_noalloc(const swr_scene* scene, const swr
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         g_dev_sms[dev] = sms > 0 ? sms : 148;
-        frame_grids(g_dev_sms[dev], 64, false, &g_raster_grid[dev], &g_shade_grid[dev]);
+        frame_grids(g_dev_sms[dev], kNaTile, false, &g_raster_grid[dev], &g_shade_grid[dev]);
         g_dev_ptr[dev] = static_cast<unsigned char*>(p);
     }
     unsigned char* base = g_dev_ptr[dev];
@@ -237,7 +245,7 @@ extern "C" swr_status swr_render_frame_noalloc(const swr_scene* scene, const swr
     }
     DView* v = reinterpret_cast<DView*>(g_stage + oView);
     std::memset(v, 0, sizeof(DView));
-    init_view(*v, *cam, width, height, 64);
+    init_view(*v, *cam, width, height, kNaTile);
     v->scene = 0;
     v->rsqrt_mode = rsqrt_mode;
     v->exposure = exposure;
@@ -283,7 +291,10 @@ extern "C" swr_status swr_render_frame_noalloc(const swr_scene* scene, const swr
     a.pixel_cap = dyn->max_view_pixels;
     a.view_cap = 1;
     a.bin_cap = kNaBinCap;
-    a.sched_tile = 64;
+    a.sched_tile = kNaTile;
+    a.pair_limit = kNaPairLimit;
+    a.wide_queue = reinterpret_cast<uint2*>(base + oWide);
+    a.wide_cap = kNaWideCap;
     a.tri_state = base + oState;
     a.rec_r = reinterpret_cast<RecRaster*>(base + oRecR);
     a.rec_s = reinterpret_cast<RecShade*>(base + oRecS);
