@@ -313,17 +313,22 @@ struct Vtx {
     float u, v;
 };
 
-// tangent: whether the tangent is wanted (only a normal map reads it).
-__device__ __forceinline__ Vtx transform_vertex(const DVertex* __restrict__ vb, uint32_t vi, const float* model,
-                                                const float* mvp, bool tangent) {
+// A vertex in two steps, so that triangles that are clipped away, face away or
+// hold no pixel centre never load a normal or form a world position: first
+// its position and u (the vertex's first vector) and clip position, then the
+// rest. tangent: whether the tangent is wanted (only a normal map reads it).
+__device__ __forceinline__ float4 transform_position(const DVertex* __restrict__ vb, uint32_t vi, const float* mvp, Vtx& o) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(vb + vi));
-    const float4 b = __ldg(reinterpret_cast<const float4*>(vb + vi) + 1);
-    Vtx o;
     // Mat4 * Vec4 with w = 1: ((c0*x + c1*y) + c2*z) + c3*1 (src/renderer.rs:504-511).
     o.cx = ((mvp[0] * a.x + mvp[4] * a.y) + mvp[8] * a.z) + mvp[12];
     o.cy = ((mvp[1] * a.x + mvp[5] * a.y) + mvp[9] * a.z) + mvp[13];
     o.cz = ((mvp[2] * a.x + mvp[6] * a.y) + mvp[10] * a.z) + mvp[14];
     o.cw = ((mvp[3] * a.x + mvp[7] * a.y) + mvp[11] * a.z) + mvp[15];
+    return a;
+}
+__device__ __forceinline__ void transform_attributes(const DVertex* __restrict__ vb, uint32_t vi, float4 a,
+                                                     const float* model, bool tangent, Vtx& o) {
+    const float4 b = __ldg(reinterpret_cast<const float4*>(vb + vi) + 1);
     o.wx = ((model[0] * a.x + model[4] * a.y) + model[8] * a.z) + model[12];
     o.wy = ((model[1] * a.x + model[5] * a.y) + model[9] * a.z) + model[13];
     o.wz = ((model[2] * a.x + model[6] * a.y) + model[10] * a.z) + model[14];
@@ -341,7 +346,6 @@ __device__ __forceinline__ Vtx transform_vertex(const DVertex* __restrict__ vb, 
     }
     o.u = a.w;
     o.v = b.w;
-    return o;
 }
 
 // clip_to_screen_subpixels (src/renderer.rs:834-846).
@@ -414,10 +418,6 @@ __device__ __forceinline__ TileRect tile_rect(const DView& v, uint32_t S, uint32
     t.first = bin_off + v.stile_base + y0 * t.pitch + x0;
     return t;
 }
-// A record's (triangle, 64-px tile) pairs.
-__device__ __forceinline__ uint32_t ref_pairs(const DView& v, const RecRaster& r) {
-    return tile_rect(v, (uint32_t)kRefTile, 0u, r.bb[0], r.bb[1], r.bb[2], r.bb[3]).count();
-}
 template <typename F>
 __device__ __forceinline__ void for_each_stile(const TileRect& t, F f) {
     for (uint32_t y = 0; y < t.ny; ++y)
@@ -473,96 +473,94 @@ __device__ __forceinline__ bool covers_no_centre(int32_t x0, int32_t y0, int32_t
     return !any;
 }
 
-// bin_triangle (src/renderer.rs:668-831): setup. kSetupRecord when the
-// triangle has records (then in r and q), kSetupNone when it is culled or
-// covers no tile, kSetupUnsampled when the reference bins it but no pixel
-// centre is in it: it cannot change the frame, so it is only counted. Its
-// tiles (still to be counted) are in tiles.
+// bin_triangle (src/renderer.rs:668-831) up to its tiles, from clip positions:
+// kSetupRecord when the triangle gets records, kSetupNone when it is culled
+// or covers no tile, kSetupUnsampled when the reference bins it but no pixel
+// centre is in it: it cannot change the frame, so it is only counted.
 enum : uint32_t { kSetupNone = 0, kSetupRecord = 1, kSetupUnsampled = 2 };
-__device__ uint32_t setup_triangle(const FrameArgs& a, const DView& view, const Vtx& v0, const Vtx& v1, const Vtx& v2,
-                               uint32_t seq8, uint32_t static_id, uint32_t material, uint32_t view_idx,
-                               RecRaster& r, RecShade& q, TileRect& tiles) {
-    int32_t p0x, p0y, p1x, p1y, p2x, p2y;
-    to_screen(v0, view.width_f, view.height_f, p0x, p0y);
-    to_screen(v1, view.width_f, view.height_f, p1x, p1y);
-    to_screen(v2, view.width_f, view.height_f, p2x, p2y);
-    const int32_t area = wsub(wmul(wsub(p1x, p0x), wsub(p2y, p0y)), wmul(wsub(p2x, p0x), wsub(p1y, p0y)));
-    if (area > 0) return kSetupNone;  // back-facing (CW front faces after the y flip)
+struct ScreenTri {
+    int32_t p0x, p0y, p1x, p1y, p2x, p2y;  // screen subpixels
+    int32_t area;
+    int32_t mnx, mny, mxx, mxy;            // bounding box in pixels
+    TileRect tiles;                        // still to be counted
+};
+__device__ __forceinline__ uint32_t screen_triangle(const FrameArgs& a, const DView& view, const Vtx& v0, const Vtx& v1,
+                                                    const Vtx& v2, bool translucent, ScreenTri& t) {
+    to_screen(v0, view.width_f, view.height_f, t.p0x, t.p0y);
+    to_screen(v1, view.width_f, view.height_f, t.p1x, t.p1y);
+    to_screen(v2, view.width_f, view.height_f, t.p2x, t.p2y);
+    t.area = wsub(wmul(wsub(t.p1x, t.p0x), wsub(t.p2y, t.p0y)), wmul(wsub(t.p2x, t.p0x), wsub(t.p1y, t.p0y)));
+    if (t.area > 0) return kSetupNone;  // back-facing (CW front faces after the y flip)
     const int32_t wsub_px = view.width * kSubpixelScale, hsub_px = view.height * kSubpixelScale;
-    const int32_t mns_x = max(min(min(p0x, p1x), p2x), 0);
-    const int32_t mns_y = max(min(min(p0y, p1y), p2y), 0);
-    const int32_t mxs_x = min(max(max(p0x, p1x), p2x), wsub_px);
-    const int32_t mxs_y = min(max(max(p0y, p1y), p2y), hsub_px);
-    const int32_t mnx = mns_x >> kSubpixelShift, mny = mns_y >> kSubpixelShift;
-    const int32_t mxx = wadd(mxs_x, kSubpixelScale) >> kSubpixelShift;
-    const int32_t mxy = wadd(mxs_y, kSubpixelScale) >> kSubpixelShift;
-
-    const bool translucent = (material & kRecTransBit) != 0u;
-    tiles = tile_rect(view, a.sched_tile, translucent ? a.dyn->n_stiles : 0u, mnx, mny, mxx, mxy);
-    if (tiles.count() == 0u) return kSetupNone;
-    if (a.skip_unsampled && !translucent && covers_no_centre(p0x, p0y, p1x, p1y, p2x, p2y, wsub_px, hsub_px))
+    const int32_t mns_x = max(min(min(t.p0x, t.p1x), t.p2x), 0);
+    const int32_t mns_y = max(min(min(t.p0y, t.p1y), t.p2y), 0);
+    const int32_t mxs_x = min(max(max(t.p0x, t.p1x), t.p2x), wsub_px);
+    const int32_t mxs_y = min(max(max(t.p0y, t.p1y), t.p2y), hsub_px);
+    t.mnx = mns_x >> kSubpixelShift, t.mny = mns_y >> kSubpixelShift;
+    t.mxx = wadd(mxs_x, kSubpixelScale) >> kSubpixelShift;
+    t.mxy = wadd(mxs_y, kSubpixelScale) >> kSubpixelShift;
+    t.tiles = tile_rect(view, a.sched_tile, translucent ? a.dyn->n_stiles : 0u, t.mnx, t.mny, t.mxx, t.mxy);
+    if (t.tiles.count() == 0u) return kSetupNone;
+    if (a.skip_unsampled && !translucent && covers_no_centre(t.p0x, t.p0y, t.p1x, t.p1y, t.p2x, t.p2y, wsub_px, hsub_px))
         return kSetupUnsampled;
+    return kSetupRecord;
+}
 
-    // Interpolator setup (src/renderer.rs:699-754).
-    const float ooa = 1.0f / i2f(wabs(area));
-    const float oow0 = 1.0f / v0.cw, oow1 = 1.0f / v1.cw, oow2 = 1.0f / v2.cw;
-    const float zow0 = v0.cz * oow0, zow1 = v1.cz * oow1, zow2 = v2.cz * oow2;
-    const float u0 = v0.u * oow0, u1 = v1.u * oow1, u2 = v2.u * oow2;
-    const float w0 = v0.v * oow0, w1 = v1.v * oow1, w2 = v2.v * oow2;
-    const float dx1 = i2f(wsub(p1x, p0x)), dx2 = i2f(wsub(p2x, p0x));
-    const float dy1 = i2f(wsub(p1y, p0y)), dy2 = i2f(wsub(p2y, p0y));
-    const float du1 = u1 - u0, du2 = u2 - u0, dv1 = w1 - w0, dv2 = w2 - w0;
-    const float du_dx = du1 * dy2 - du2 * dy1;
-    const float du_dy = du2 * dx1 - du1 * dx2;
-    const float dv_dx = dv1 * dy2 - dv2 * dy1;
-    const float dv_dy = dv2 * dx1 - dv1 * dx2;
-    const float s = ooa * 16.0f;
+// Its (triangle, 64-px tile) pairs.
+__device__ __forceinline__ uint32_t ref_pairs(const DView& v, const ScreenTri& t) {
+    return tile_rect(v, (uint32_t)kRefTile, 0u, t.mnx, t.mny, t.mxx, t.mxy).count();
+}
 
-    r.p[0] = p0x; r.p[1] = p0y; r.p[2] = p1x; r.p[3] = p1y; r.p[4] = p2x; r.p[5] = p2y;
-    r.bb[0] = (uint16_t)mnx; r.bb[1] = (uint16_t)mny; r.bb[2] = (uint16_t)mxx; r.bb[3] = (uint16_t)mxy;
+// Its records (src/renderer.rs:699-754), stored as they are formed: the raster
+// record from clip positions, then the shading record.
+__device__ __forceinline__ void store_raster(const FrameArgs& a, uint32_t slot, const Vtx& v0, const Vtx& v1,
+                                             const Vtx& v2, const ScreenTri& t, const float oow[3], float ooa,
+                                             uint32_t seq8, uint32_t material, uint32_t view_idx, bool wide) {
+    const float zow0 = v0.cz * oow[0], zow1 = v1.cz * oow[1], zow2 = v2.cz * oow[2];
+    RecRaster r;
+    r.p[0] = t.p0x; r.p[1] = t.p0y; r.p[2] = t.p1x; r.p[3] = t.p1y; r.p[4] = t.p2x; r.p[5] = t.p2y;
+    r.bb[0] = (uint16_t)t.mnx; r.bb[1] = (uint16_t)t.mny; r.bb[2] = (uint16_t)t.mxx; r.bb[3] = (uint16_t)t.mxy;
     r.ooa = ooa;
     r.zow[0] = zow0; r.zow[1] = zow1 - zow0; r.zow[2] = zow2 - zow0;
-    r.oow[0] = oow0; r.oow[1] = oow1 - oow0; r.oow[2] = oow2 - oow0;
+    r.oow[0] = oow[0]; r.oow[1] = oow[1] - oow[0]; r.oow[2] = oow[2] - oow[0];
     r.seq8 = seq8;
     r.material = material;
     r.view = view_idx;
     r.zfloor = 0u;
-    if ((int32_t)a.sched_tile >= SWR_CULL_MIN_TILE && !translucent) {
+    if ((int32_t)a.sched_tile >= SWR_CULL_MIN_TILE && !(material & kRecTransBit)) {
         const float zc[3] = {v0.cz, v1.cz, v2.cz}, wc[3] = {v0.cw, v1.cw, v2.cw};
         float zl;
-        if (depth_floor(r.p, area, r.zow, r.oow, zc, wc, mxx * kSubpixelScale, mxy * kSubpixelScale, zl))
+        if (depth_floor(r.p, t.area, r.zow, r.oow, zc, wc, t.mxx * kSubpixelScale, t.mxy * kSubpixelScale, zl))
             r.zfloor = float_to_ordered(zl);
     }
-    r.wide = 0u;
-    q.nrm[0] = v0.nx; q.nrm[1] = v0.ny; q.nrm[2] = v0.nz;
-    q.nrm[3] = v1.nx - v0.nx; q.nrm[4] = v1.ny - v0.ny; q.nrm[5] = v1.nz - v0.nz;
-    q.nrm[6] = v2.nx - v0.nx; q.nrm[7] = v2.ny - v0.ny; q.nrm[8] = v2.nz - v0.nz;
-    q.uow[0] = u0; q.uow[1] = u1 - u0; q.uow[2] = u2 - u0;
-    q.vow[0] = w0; q.vow[1] = w1 - w0; q.vow[2] = w2 - w0;
-    const float px0 = v0.wx * oow0, py0 = v0.wy * oow0, pz0 = v0.wz * oow0;
-    const float px1 = v1.wx * oow1, py1 = v1.wy * oow1, pz1 = v1.wz * oow1;
-    const float px2 = v2.wx * oow2, py2 = v2.wy * oow2, pz2 = v2.wz * oow2;
-    q.pww[0] = px0; q.pww[1] = py0; q.pww[2] = pz0;
-    q.pww[3] = px1 - px0; q.pww[4] = py1 - py0; q.pww[5] = pz1 - pz0;
-    q.pww[6] = px2 - px0; q.pww[7] = py2 - py0; q.pww[8] = pz2 - pz0;
-    q.du_dv[0] = du_dx * s; q.du_dv[1] = du_dy * s; q.du_dv[2] = dv_dx * s; q.du_dv[3] = dv_dy * s;
-    q.static_id = static_id;
-    // Average z for the per-tile translucency sort (src/renderer.rs:765-774).
-    q.avg_z = translucent ? __float_as_uint(((v0.cz + v1.cz) + v2.cz) / 3.0f) : 0u;
-    q.pad[0] = q.pad[1] = 0u;
-    return kSetupRecord;
+    r.wide = wide ? 1u : 0u;
+    const float4* src = reinterpret_cast<const float4*>(&r);
+    float4* dst = reinterpret_cast<float4*>(a.rec_r + slot);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) dst[i] = src[i];
 }
-
-__device__ __forceinline__ void store_records(const FrameArgs& a, uint32_t slot, const RecRaster& r,
-                                              const RecShade& q) {
-    const float4* sr = reinterpret_cast<const float4*>(&r);
-    float4* dr = reinterpret_cast<float4*>(a.rec_r + slot);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) dr[i] = sr[i];
-    const float4* sq = reinterpret_cast<const float4*>(&q);
-    float4* dq = reinterpret_cast<float4*>(a.rec_s + slot);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) dq[i] = sq[i];
+__device__ __forceinline__ void store_shade(const FrameArgs& a, uint32_t slot, const Vtx& v0, const Vtx& v1,
+                                            const Vtx& v2, const ScreenTri& t, const float oow[3], float ooa,
+                                            uint32_t static_id, uint32_t material) {
+    float4* d = reinterpret_cast<float4*>(a.rec_s + slot);
+    d[0] = make_float4(v0.nx, v0.ny, v0.nz, v1.nx - v0.nx);
+    d[1] = make_float4(v1.ny - v0.ny, v1.nz - v0.nz, v2.nx - v0.nx, v2.ny - v0.ny);
+    const float u0 = v0.u * oow[0], u1 = v1.u * oow[1], u2 = v2.u * oow[2];
+    const float w0 = v0.v * oow[0], w1 = v1.v * oow[1], w2 = v2.v * oow[2];
+    const float du1 = u1 - u0, du2 = u2 - u0, dv1 = w1 - w0, dv2 = w2 - w0;
+    d[2] = make_float4(v2.nz - v0.nz, u0, du1, du2);
+    const float px0 = v0.wx * oow[0], py0 = v0.wy * oow[0], pz0 = v0.wz * oow[0];
+    d[3] = make_float4(w0, dv1, dv2, px0);
+    d[4] = make_float4(py0, pz0, v1.wx * oow[1] - px0, v1.wy * oow[1] - py0);
+    d[5] = make_float4(v1.wz * oow[1] - pz0, v2.wx * oow[2] - px0, v2.wy * oow[2] - py0, v2.wz * oow[2] - pz0);
+    const float dx1 = i2f(wsub(t.p1x, t.p0x)), dx2 = i2f(wsub(t.p2x, t.p0x));
+    const float dy1 = i2f(wsub(t.p1y, t.p0y)), dy2 = i2f(wsub(t.p2y, t.p0y));
+    const float s = ooa * 16.0f;
+    d[6] = make_float4((du1 * dy2 - du2 * dy1) * s, (du2 * dx1 - du1 * dx2) * s, (dv1 * dy2 - dv2 * dy1) * s,
+                       (dv2 * dx1 - dv1 * dx2) * s);
+    // Average z for the per-tile translucency sort (src/renderer.rs:765-774).
+    const uint32_t avg_z = (material & kRecTransBit) ? __float_as_uint(((v0.cz + v1.cz) + v2.cz) / 3.0f) : 0u;
+    d[7] = make_float4(__uint_as_float(static_id), __uint_as_float(avg_z), 0.0f, 0.0f);
 }
 __device__ __forceinline__ void store_tangents(const FrameArgs& a, uint32_t slot, const Vtx& v0, const Vtx& v1,
                                                const Vtx& v2) {
@@ -918,9 +916,10 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
     const uint32_t i0 = __ldg(ib), i1 = __ldg(ib + 1), i2 = __ldg(ib + 2);
     const uint32_t flags = sc.materials[pr.material].flags;
     const bool tangents = (flags & MAT_NORMAL_MAP) != 0u;
-    const Vtx v0 = transform_vertex(sc.vertices, pr.vtx_base + i0, model, d.mvp, tangents);
-    const Vtx v1 = transform_vertex(sc.vertices, pr.vtx_base + i1, model, d.mvp, tangents);
-    const Vtx v2 = transform_vertex(sc.vertices, pr.vtx_base + i2, model, d.mvp, tangents);
+    Vtx v0, v1, v2;
+    const float4 a0 = transform_position(sc.vertices, pr.vtx_base + i0, d.mvp, v0);
+    const float4 a1 = transform_position(sc.vertices, pr.vtx_base + i1, d.mvp, v1);
+    const float4 a2 = transform_position(sc.vertices, pr.vtx_base + i2, d.mvp, v2);
     if (d.clip && !(vtx_inside_all(v0) && vtx_inside_all(v1) && vtx_inside_all(v2))) {
         if (clip_rejects_all(v0, v1, v2)) {  // the clipper would return an empty polygon
             a.tri_state[g] = 3;
@@ -937,31 +936,36 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
     }
     // All three vertices inside: the clipper would return the triangle unchanged.
     const uint32_t mword = record_material(flags, d, pr.material);
-    RecRaster r;
-    RecShade q;
-    TileRect tiles;
-    const uint32_t res = setup_triangle(a, view, v0, v1, v2, g << 3, d.static_base + local, mword, d.view, r, q, tiles);
+    ScreenTri t;
+    const uint32_t res = screen_triangle(a, view, v0, v1, v2, d.translucent != 0u, t);
+    uint32_t pairs64 = 0u;
     if (res == kSetupRecord) {
         // A wide triangle's tiles are counted by k_clip's warps: one thread
         // walking the 4,576 16-px tiles of a 1367x769 frame held the kernel
         // for 79 us (150k triangles; 12 us without such triangles).
-        if (tiles.count() > kWideTiles && push_wide(a, &a.counters->wide_main, a.wide_queue, g, tiles.count()))
-            r.wide = 1u;
-        else
-            for_each_stile(tiles, [&](uint32_t st) { agg_inc(a.tile_count, st); });
-        store_records(a, g, r, q);
+        const bool wide = t.tiles.count() > kWideTiles &&
+                          push_wide(a, &a.counters->wide_main, a.wide_queue, g, t.tiles.count());
+        if (!wide) for_each_stile(t.tiles, [&](uint32_t st) { agg_inc(a.tile_count, st); });
+        if (a.pair_limit) pairs64 = ref_pairs(view, t);
+        const float ooa = 1.0f / i2f(wabs(t.area));
+        const float oow[3] = {1.0f / v0.cw, 1.0f / v1.cw, 1.0f / v2.cw};
+        store_raster(a, g, v0, v1, v2, t, oow, ooa, g << 3, mword, d.view, wide);
+        transform_attributes(sc.vertices, pr.vtx_base + i0, a0, model, tangents, v0);
+        transform_attributes(sc.vertices, pr.vtx_base + i1, a1, model, tangents, v1);
+        transform_attributes(sc.vertices, pr.vtx_base + i2, a2, model, tangents, v2);
+        store_shade(a, g, v0, v1, v2, t, oow, ooa, d.static_base + local, mword);
         if (tangents) store_tangents(a, g, v0, v1, v2);
     }
     a.tri_state[g] = res == kSetupRecord ? 1 : 0;
     warp_count(&a.counters->setup_tris, res != kSetupNone);
-    warp_sum(&a.counters->unsampled, res == kSetupUnsampled ? tiles.count() : 0u);
-    if (a.pair_limit) warp_sum(&a.counters->ref_pairs, res == kSetupRecord ? ref_pairs(view, r) : 0u);
+    warp_sum(&a.counters->unsampled, res == kSetupUnsampled ? t.tiles.count() : 0u);
+    if (a.pair_limit) warp_sum(&a.counters->ref_pairs, pairs64);
 }
 
 // Thread per triangle of a 256-triangle chunk, CTA per chunk (a loop over
 // chunks per CTA made the kernel spill).
-// Four CTAs per SM (64 registers, a few spilled): 4K front end 0.161 ms,
-// against 0.164 at three (80 registers) and 0.204 at two (108 registers).
+// Four CTAs per SM (64 registers, a few spilled): 4K front end 126 us, 64 views
+// 222, against 139 and 245 at three (80 registers) and 140 and 244 at five.
 #ifndef SWR_FRONTEND_MIN_BLOCKS
 #define SWR_FRONTEND_MIN_BLOCKS 4
 #endif
@@ -1028,7 +1032,7 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
         const uint32_t mword = record_material(flags, d, pr.material);
         const uint32_t* ib = sc.indices + pr.idx_base + 3u * local;
         {
-            // Lane i's row of the vertex transform (transform_vertex): clip
+            // Lane i's row of the vertex transform (transform_position, transform_attributes): clip
             // position, world position, normal, tangent, then copies.
             const float* m = i < 4u ? d.mvp : sc.node_xform + 16u * d.node;
             const uint32_t row = i < 4u ? i : (i < 7u ? i - 4u : (i < 10u ? i - 7u : i - 10u));
@@ -1107,22 +1111,24 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
         if ((int)i < fans) {
             const uint32_t slot = i == 0u ? g : tri_total + base + i - 1u;
             const Vtx* pl = reinterpret_cast<const Vtx*>(cur);
-            RecRaster r;
-            RecShade q;
-            const uint32_t res = setup_triangle(a, view, pl[0], pl[i + 1], pl[i + 2], (g << 3) | i,
-                                                d.static_base + local, mword, d.view, r, q, tiles);
+            ScreenTri t;
+            const uint32_t res = screen_triangle(a, view, pl[0], pl[i + 1], pl[i + 2], d.translucent != 0u, t);
+            tiles = t.tiles;
             ok = res == kSetupRecord;
             if (res == kSetupUnsampled) {
                 atomicAdd(&a.counters->setup_tris, 1u);
                 atomicAdd(&a.counters->unsampled, tiles.count());
             }
             if (ok) {
-                if (tiles.count() > kWideTiles &&
-                    push_wide(a, &a.counters->wide_clip, a.wide_queue + a.wide_cap, slot, tiles.count()))
-                    r.wide = 1u;
-                if (a.pair_limit) atomicAdd(&a.counters->ref_pairs, ref_pairs(view, r));
-                store_records(a, slot, r, q);
-                if (flags & MAT_NORMAL_MAP) store_tangents(a, slot, pl[0], pl[i + 1], pl[i + 2]);
+                const Vtx &v0 = pl[0], &v1 = pl[i + 1], &v2 = pl[i + 2];
+                const bool wide = tiles.count() > kWideTiles &&
+                                  push_wide(a, &a.counters->wide_clip, a.wide_queue + a.wide_cap, slot, tiles.count());
+                if (a.pair_limit) atomicAdd(&a.counters->ref_pairs, ref_pairs(view, t));
+                const float ooa = 1.0f / i2f(wabs(t.area));
+                const float oow[3] = {1.0f / v0.cw, 1.0f / v1.cw, 1.0f / v2.cw};
+                store_raster(a, slot, v0, v1, v2, t, oow, ooa, (g << 3) | i, mword, d.view, wide);
+                store_shade(a, slot, v0, v1, v2, t, oow, ooa, d.static_base + local, mword);
+                if (flags & MAT_NORMAL_MAP) store_tangents(a, slot, v0, v1, v2);
             } else if (i > 0u) {
                 // Mark the unused extra slot so the scatter skips it.
                 a.rec_r[slot].view = 0xFFFFFFFFu;
