@@ -2776,18 +2776,40 @@ __global__ void __launch_bounds__(kResolveThreads) k_resolve(FrameArgs a) {
     __syncthreads();
     const float e = exposure;
     const uint32_t w = (uint32_t)v.width, h = (uint32_t)(v.height & ~1);
-    const uint32_t per_row = (w + kResolveThreads - 1u) / kResolveThreads, n = per_row * h;
+    // A thread takes four pixels, placed so that their host (or, without a
+    // host copy, device) addresses are one 16-byte vector; the pieces of a row
+    // start up to three pixels left of it.
+    constexpr uint32_t kPiece = 4u * kResolveThreads;
+    const uint32_t per_row = (w + 3u + kPiece - 1u) / kPiece, n = per_row * h;
     const float* const color = v.color;
     uint32_t* const out = v.rgba8;
     uint32_t* const host = v.rgba8_host;
     const uint64_t pitch = v.key_pitch, out_pitch = v.out_pitch, host_pitch = v.host_pitch;
     for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-        const uint32_t y = i / per_row, x = (i - y * per_row) * kResolveThreads + threadIdx.x;
-        if (x >= w) continue;
-        const float* c = color + (y * pitch + x) * 3u;
-        const uint32_t p = tonemap_pack(mk3(__ldg(c), __ldg(c + 1), __ldg(c + 2)), e);
-        out[y * out_pitch + x] = p;
-        if (host) host[y * host_pitch + x] = p;
+        const uint32_t y = i / per_row;
+        uint32_t* const o = out + y * out_pitch;
+        uint32_t* const ho = host ? host + y * host_pitch : nullptr;
+        const int32_t lead = (int32_t)((reinterpret_cast<uintptr_t>(host ? ho : o) >> 2) & 3u);
+        const int32_t x = (int32_t)((i - y * per_row) * kPiece + 4u * threadIdx.x) - lead;
+        if (x >= (int32_t)w || x + 4 <= 0) continue;
+        const float* c = color + (int64_t)(y * pitch) * 3 + (int64_t)x * 3;
+        uint32_t p[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (x + k >= 0 && x + k < (int32_t)w)
+                p[k] = tonemap_pack(mk3(__ldg(c + 3 * k), __ldg(c + 3 * k + 1), __ldg(c + 3 * k + 2)), e);
+        const bool whole = x >= 0 && x + 4 <= (int32_t)w;
+        auto store = [&](uint32_t* d) {
+            if (whole && (reinterpret_cast<uintptr_t>(d + x) & 15u) == 0u) {
+                *reinterpret_cast<uint4*>(d + x) = make_uint4(p[0], p[1], p[2], p[3]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (x + k >= 0 && x + k < (int32_t)w) d[x + k] = p[k];
+            }
+        };
+        store(o);
+        if (ho) store(ho);
     }
 }
 
