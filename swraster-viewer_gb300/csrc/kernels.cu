@@ -899,14 +899,19 @@ __device__ __forceinline__ bool vtx_inside_all(const Vtx& v) {
 }
 
 // Thread per triangle of a 256-triangle chunk of one draw.
-__device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t chunk) {
-    const DChunk ch = a.chunks[chunk];
+// CTAs of 128 triangles, two per chunk, start and end with less idle time
+// than one of 256: 64 views 222 -> 210 us, 4K 126 -> 122 (64: 214 and 123).
+constexpr int kFrontThreads = 128;
+constexpr uint32_t kFrontParts = kChunkTris / kFrontThreads;
+__device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t part) {
+    DChunk ch = a.chunks[part / kFrontParts];
+    ch.tri_start += (part % kFrontParts) * kFrontThreads;
     const DDraw& d = a.draws[ch.draw];
     // The CTA's triangles are one draw's: count the chunk once for the
     // reference's clip path (every triangle of an intersecting primitive).
-    if (threadIdx.x == 0 && d.clip) atomicAdd(&a.counters->clip_path, min((uint32_t)kChunkTris, d.tri_count - ch.tri_start));
     const uint32_t local = ch.tri_start + threadIdx.x;
     if (local >= d.tri_count) return;
+    if (threadIdx.x == 0 && d.clip) atomicAdd(&a.counters->clip_path, min((uint32_t)kFrontThreads, d.tri_count - ch.tri_start));
     const uint32_t g = d.tri_begin + local;
     const DScene& sc = a.scenes[d.scene];
     const DView& view = a.views[d.view];
@@ -962,15 +967,15 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t c
     if (a.pair_limit) warp_sum(&a.counters->ref_pairs, pairs64);
 }
 
-// Thread per triangle of a 256-triangle chunk, CTA per chunk (a loop over
-// chunks per CTA made the kernel spill).
-// Four CTAs per SM (64 registers, a few spilled): 4K front end 126 us, 64 views
+// Thread per triangle, CTA per half chunk (a loop over chunks per CTA: 64
+// views 222 -> 292 us at one resident set of CTAs, 257 at four).
+// Four times 256 threads per SM (64 registers, a few spilled): 4K front end 126 us, 64 views
 // 222, against 139 and 245 at three (80 registers) and 140 and 244 at five.
 #ifndef SWR_FRONTEND_MIN_BLOCKS
 #define SWR_FRONTEND_MIN_BLOCKS 4
 #endif
-__global__ void __launch_bounds__(kChunkTris, SWR_FRONTEND_MIN_BLOCKS) k_frontend(FrameArgs a) {
-    if (blockIdx.x < a.dyn->n_chunks) frontend_triangle(a, blockIdx.x);
+__global__ void __launch_bounds__(kFrontThreads, SWR_FRONTEND_MIN_BLOCKS * kFrontParts) k_frontend(FrameArgs a) {
+    if (blockIdx.x < a.dyn->n_chunks * kFrontParts) frontend_triangle(a, blockIdx.x);
 }
 
 // Sutherland-Hodgman for the queued triangles, sixteen lanes per triangle.
@@ -2922,7 +2927,7 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
     if (a.chunk_cap > 0) {
         // Host-built draw lists (no-alloc frames) size chunk_cap exactly.
         const uint64_t most = a.gpu_draws ? (uint64_t)a.tri_cap / kChunkTris + a.draw_cap + 1u : a.chunk_cap;
-        k_frontend<<<(uint32_t)std::min<uint64_t>(a.chunk_cap, most), kChunkTris, 0, s>>>(a);
+        k_frontend<<<(uint32_t)(std::min<uint64_t>(a.chunk_cap, most) * kFrontParts), kFrontThreads, 0, s>>>(a);
         launches++;
     }
     mark(2);
