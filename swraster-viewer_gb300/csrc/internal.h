@@ -358,6 +358,11 @@ struct FrameArgs {
     uint32_t fused_shade;      // 32-px tiles: shade inside the raster kernel (8 and 16 px always do)
     uint32_t has_gi;           // some scene of the frame has a baked voxel grid
     uint32_t gpu_draws;        // build draws and chunks on the device (else the host staged them)
+    // Kernels are launched to overlap their predecessor's end: for small frames
+    // launched directly (the allocation-free frame, 96 -> 87 us). Replayed
+    // graphs gain nothing (1280x720 124 -> 126) and frames of large kernels lose
+    // (4K 1062 -> 1088: the next kernel's waiting CTAs take up places).
+    uint32_t overlap;
     uint32_t pair_limit;       // (triangle, 64-px tile) pairs past which a frame counts as overflowed, 0 = none
     uint32_t skip_unsampled;   // triangles that hold no pixel centre are not binned
     uint32_t rsqrt_uniform;    // 1 + the rsqrt mode all views share, 0 = per view

@@ -98,6 +98,14 @@ __device__ __forceinline__ f3 unpack_rgb(uint32_t t) { return {unorm8(t >> 9), u
 __device__ __forceinline__ float srgb_fast(float x) { return x * (x * (x * 0.305306011f + 0.682171111f) + 0.012522878f); }
 __device__ __forceinline__ f3 srgb_fast3(f3 c) { return {srgb_fast(c.x), srgb_fast(c.y), srgb_fast(c.z)}; }
 
+// Entry of a frame kernel launched to overlap its predecessor's end
+// (FrameArgs.overlap): waits until the predecessor is complete, then lets the
+// next kernel's CTAs come in. Without that launch attribute both do nothing.
+__device__ __forceinline__ void frame_kernel_entry() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // One channel of blit_to_buffer (src/renderer.rs:325-348) and tonemap
 // (src/util.rs:37-41).
 __device__ __forceinline__ uint32_t tonemap_u8(float c, float exposure) {
@@ -822,6 +830,7 @@ __device__ void draw_count_blocks(const FrameArgs& a) {
 }
 
 __global__ void __launch_bounds__(kSlotBlock) k_draw_emit(FrameArgs a) {
+    frame_kernel_entry();
     __shared__ uint32_t sm[3 * (kSlotBlock / 32)];
     if (blockIdx.x == 0 && threadIdx.x == 0) a.counters->draw_done = 0u;  // for the next frame
     const uint32_t n = a.dyn->n_slots;
@@ -841,6 +850,7 @@ __global__ void __launch_bounds__(kSlotBlock) k_draw_emit(FrameArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_reset(FrameArgs a) {
+    frame_kernel_entry();
     const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n = a.dyn->n_bins;
     for (uint32_t i = i0; i < n; i += gridDim.x * blockDim.x) a.tile_count[i] = 0u;
@@ -975,6 +985,7 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t p
 #define SWR_FRONTEND_MIN_BLOCKS 4
 #endif
 __global__ void __launch_bounds__(kFrontThreads, SWR_FRONTEND_MIN_BLOCKS * kFrontParts) k_frontend(FrameArgs a) {
+    frame_kernel_entry();
     if (blockIdx.x < a.dyn->n_chunks * kFrontParts) frontend_triangle(a, blockIdx.x);
 }
 
@@ -1005,6 +1016,7 @@ __device__ __forceinline__ TileRect record_tiles(const FrameArgs& a, const RecRa
 }
 
 __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
+    frame_kernel_entry();
     __shared__ __align__(16) float poly_mem[kClipThreads / 16][kClipPoly];
     const uint32_t lane = threadIdx.x & 31u;
     {
@@ -1190,6 +1202,7 @@ __device__ __forceinline__ uint32_t order_bucket(uint32_t c) {
 // bins of 64 batched views and 7 us for a 4K frame's 2,040.
 constexpr int kScanThreads = 256, kScanBins = 1024;
 __global__ void __launch_bounds__(kScanThreads) k_scan(FrameArgs a) {
+    frame_kernel_entry();
     __shared__ uint32_t wsum[kScanThreads / 32];
     __shared__ uint32_t hist[kOrderBuckets];
     __shared__ uint32_t base;
@@ -1364,6 +1377,7 @@ __device__ __forceinline__ void scatter_wide(const FrameArgs& a, uint2 q) {
 }
 
 __global__ void k_scatter(FrameArgs a) {
+    frame_kernel_entry();
     const bool bad = (a.counters->status & (ST_BIN_OVERFLOW | ST_CLIP_OVERFLOW | ST_QUEUE_OVERFLOW)) != 0u;
     place_work(a, bad);
     if (bad) return;
@@ -1835,6 +1849,7 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
 // GI and MODE: the fused shading's variant (see k_shade); unused without FUSE.
 template <int S, bool FUSE, bool GI, int MODE>
 __global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kMinBlocks) k_raster(FrameArgs a) {
+    frame_kernel_entry();
     using Sh = RasterSmem<S, FUSE>;
     constexpr int NT = Sh::kThreads, R = Sh::kRegions, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char raster_smem[];
@@ -2485,6 +2500,7 @@ template <bool GI> struct ShadeShape {
 // GI: the frame has scenes with a baked voxel grid. MODE: see shade_pixel.
 template <bool GI, int MODE>
 __global__ void __launch_bounds__(ShadeShape<GI>::kThreads, ShadeShape<GI>::kMinBlocks) k_shade(FrameArgs a) {
+    frame_kernel_entry();
     __shared__ uint8_t tab[512];
     __shared__ ShadeConst sc;
     for (int i = threadIdx.x; i < 512; i += blockDim.x) tab[i] = a.rsqrt_table[i];
@@ -2595,6 +2611,7 @@ __device__ __forceinline__ uint32_t part_rect(const RecRaster& r, int32_t tx0, i
 
 template <bool GI, int MODE>
 __global__ void __launch_bounds__(kTransThreads, 4) k_translucent(FrameArgs a) {
+    frame_kernel_entry();
     __shared__ unsigned long long tkey[kTransCap];  // sort keys, then (rectangle, blocks) in sorted order
     __shared__ uint32_t tslot[kTransCap];
     __shared__ uint32_t tsorted[kTransCap];
@@ -2836,9 +2853,25 @@ static cudaError_t fused_smem_attr() {
     if (e == cudaSuccess) e = raster_smem_attr<S, true, true, kModeAny>();
     return e;
 }
+// Launches a frame kernel, with FrameArgs.overlap as a programmatic dependent
+// of the kernel before it in the stream.
+static void launch_kernel(void (*k)(FrameArgs), uint32_t grid, uint32_t threads, size_t smem, const FrameArgs& a, cudaStream_t s) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = a.overlap ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, a);
+}
+
 template <int S, bool FUSE, bool GI, int MODE>
 static void launch_raster(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
-    k_raster<S, FUSE, GI, MODE><<<grid, RasterShared<S>::kThreads, sizeof(RasterSmem<S, FUSE>), s>>>(a);
+    launch_kernel(k_raster<S, FUSE, GI, MODE>, grid, RasterShared<S>::kThreads, sizeof(RasterSmem<S, FUSE>), a, s);
 }
 // The fused shading compiled for what the frame needs: the variant for baked
 // grids of any rsqrt mode spills 250-450 B a thread against 0-130 B, and
@@ -2916,7 +2949,7 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
     if (a.gpu_draws) {
         const uint32_t sg = (a.slot_cap + kSlotBlock - 1u) / kSlotBlock;
         if (sg > 1u) {
-            k_draw_emit<<<sg, kSlotBlock, 0, s>>>(a);
+            launch_kernel(k_draw_emit, sg, kSlotBlock, 0, a, s);
             launches++;
         }
     }
@@ -2927,13 +2960,13 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
     if (a.chunk_cap > 0) {
         // Host-built draw lists (no-alloc frames) size chunk_cap exactly.
         const uint64_t most = a.gpu_draws ? (uint64_t)a.tri_cap / kChunkTris + a.draw_cap + 1u : a.chunk_cap;
-        k_frontend<<<(uint32_t)(std::min<uint64_t>(a.chunk_cap, most) * kFrontParts), kFrontThreads, 0, s>>>(a);
+        launch_kernel(k_frontend, (uint32_t)(std::min<uint64_t>(a.chunk_cap, most) * kFrontParts), kFrontThreads, 0, a, s);
         launches++;
     }
     mark(2);
-    k_clip<<<num_sms * 4, kClipThreads, 0, s>>>(a);
+    launch_kernel(k_clip, (uint32_t)num_sms * 4u, kClipThreads, 0, a, s);
     mark(3);
-    k_scan<<<(a.stile_cap + kScanBins - 1u) / kScanBins, kScanThreads, 0, s>>>(a);
+    launch_kernel(k_scan, (a.stile_cap + kScanBins - 1u) / kScanBins, kScanThreads, 0, a, s);
     launches += 2;
     mark(4);
     {
@@ -2942,7 +2975,7 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
         // loads stay coalesced (a grid-stride loop here made k_raster 2% slower).
         const uint64_t n = (uint64_t)a.tri_cap + a.extra_cap;
         if (n > 0) {
-            k_scatter<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
+            launch_kernel(k_scatter, (uint32_t)((n + 255) / 256), 256, 0, a, s);
             launches++;
         }
     }
@@ -2971,15 +3004,15 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
             }();
             const uint32_t sg = (uint32_t)num_sms * gi_blocks;
             const uint32_t T = ShadeShape<true>::kThreads;
-            if (a.rsqrt_uniform == 1u + kModeArm) k_shade<true, kModeArm><<<sg, T, 0, s>>>(a);
-            else if (a.rsqrt_uniform == 1u + kModeIeee) k_shade<true, kModeIeee><<<sg, T, 0, s>>>(a);
-            else k_shade<true, kModeAny><<<sg, T, 0, s>>>(a);
+            if (a.rsqrt_uniform == 1u + kModeArm) launch_kernel(k_shade<true, kModeArm>, sg, T, 0, a, s);
+            else if (a.rsqrt_uniform == 1u + kModeIeee) launch_kernel(k_shade<true, kModeIeee>, sg, T, 0, a, s);
+            else launch_kernel(k_shade<true, kModeAny>, sg, T, 0, a, s);
         } else {
             const uint32_t sg = a.shade_grid > 0 ? a.shade_grid : (uint32_t)num_sms;
             const uint32_t T = ShadeShape<false>::kThreads;
-            if (a.rsqrt_uniform == 1u + kModeArm) k_shade<false, kModeArm><<<sg, T, 0, s>>>(a);
-            else if (a.rsqrt_uniform == 1u + kModeIeee) k_shade<false, kModeIeee><<<sg, T, 0, s>>>(a);
-            else k_shade<false, kModeAny><<<sg, T, 0, s>>>(a);
+            if (a.rsqrt_uniform == 1u + kModeArm) launch_kernel(k_shade<false, kModeArm>, sg, T, 0, a, s);
+            else if (a.rsqrt_uniform == 1u + kModeIeee) launch_kernel(k_shade<false, kModeIeee>, sg, T, 0, a, s);
+            else launch_kernel(k_shade<false, kModeAny>, sg, T, 0, a, s);
         }
         launches++;
     }
@@ -2988,11 +3021,11 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
         const uint32_t tg = (uint32_t)num_sms * 4u;
         const bool arm = a.rsqrt_uniform == 1u + kModeArm;
         if (a.has_gi) {
-            if (arm) k_translucent<true, kModeArm><<<tg, kTransThreads, 0, s>>>(a);
-            else k_translucent<true, kModeAny><<<tg, kTransThreads, 0, s>>>(a);
+            if (arm) launch_kernel(k_translucent<true, kModeArm>, tg, kTransThreads, 0, a, s);
+            else launch_kernel(k_translucent<true, kModeAny>, tg, kTransThreads, 0, a, s);
         } else {
-            if (arm) k_translucent<false, kModeArm><<<tg, kTransThreads, 0, s>>>(a);
-            else k_translucent<false, kModeAny><<<tg, kTransThreads, 0, s>>>(a);
+            if (arm) launch_kernel(k_translucent<false, kModeArm>, tg, kTransThreads, 0, a, s);
+            else launch_kernel(k_translucent<false, kModeAny>, tg, kTransThreads, 0, a, s);
         }
         launches++;
         if (!a.defer_resolve) {

@@ -293,6 +293,7 @@ extern "C" swr_status swr_render_frame_noalloc(const swr_scene* scene, const swr
     a.bin_cap = kNaBinCap;
     a.sched_tile = kNaTile;
     a.pair_limit = kNaPairLimit;
+    a.overlap = 1u;
     a.wide_queue = reinterpret_cast<uint2*>(base + oWide);
     a.wide_cap = kNaWideCap;
     a.tri_state = base + oState;

@@ -345,6 +345,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     a.draw_cap = draw_cap;
     a.gpu_draws = 1u;
     a.skip_unsampled = 1u;
+    a.overlap = 0u;
     a.fused_shade = fused32 ? 1u : 0u;
     a.chunk_cap = chunk_cap;
     a.tri_cap = tri_cap;
