@@ -48,7 +48,20 @@ __device__ __forceinline__ V normalize(V a) { return a * (1.0f / __fsqrt_rn(dot(
 __device__ __forceinline__ V vmax0(V a) { return V{fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f), fmaxf(a.z, 0.0f)}; }
 __device__ __forceinline__ V ld3(const float* p) { return V{p[0], p[1], p[2]}; }
 
+// A triangle as the traversal reads it, in leaf order: vertex 0 and whether
+// its material is translucent, the edges from vertex 0 and its index.
+struct alignas(16) LeafTri {
+    float p0[3];
+    uint32_t translucent;
+    float e1[3];
+    uint32_t index;
+    float e2[3];
+    uint32_t pad;
+};
+
 struct Dev {
+    LeafTri* leaf;
+    uint32_t n_tris;
     const BakeTri* tris;
     const BakeNode* nodes;
     const uint32_t* order;
@@ -71,11 +84,20 @@ struct Dev {
     float* out;  // n^3 x 16 before the blur
 };
 
+__device__ __forceinline__ LeafTri load_leaf(const LeafTri* p) {
+    LeafTri t;
+    const float4* src = reinterpret_cast<const float4*>(p);
+    float4* dst = reinterpret_cast<float4*>(&t);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dst[i] = __ldg(src + i);
+    return t;
+}
+
 // ray_triangle_intersect (src/raytracer.rs:225-260).
-__device__ __forceinline__ bool ray_tri(V o, V d, const BakeTri& t, float tmin, float tmax, float& th, float& bu,
+__device__ __forceinline__ bool ray_tri(V o, V d, const LeafTri& t, float tmin, float tmax, float& th, float& bu,
                                         float& bv) {
     const V p0 = ld3(t.p0);
-    const V e1 = ld3(t.p1) - p0, e2 = ld3(t.p2) - p0;
+    const V e1 = ld3(t.e1), e2 = ld3(t.e2);
     const V pv = cross(d, e2);
     const float det = dot(e1, pv);
     if (fabsf(det) <= 1.0e-8f) return false;
@@ -101,66 +123,96 @@ __device__ __forceinline__ bool hit_before(float ta, uint32_t ia, float tb, uint
     return ia < ib;
 }
 
-// Ray / node box (slab test from t = 0); returns the entry distance or -1.
-__device__ __forceinline__ float box_entry(const BakeNode& nd, V o, const float inv[3]) {
+// Ray / box (slab test from t = 0); returns the entry distance or -1.
+__device__ __forceinline__ float box_entry(const float mn[3], const float mx[3], V o, const float inv[3]) {
     const float oo[3] = {o.x, o.y, o.z};
     float t0 = 0.0f, t1 = INFINITY;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        float ta = (nd.mn[k] - oo[k]) * inv[k];
-        float tb = (nd.mx[k] - oo[k]) * inv[k];
+        float ta = (mn[k] - oo[k]) * inv[k];
+        float tb = (mx[k] - oo[k]) * inv[k];
         if (ta != ta) ta = -INFINITY;
         if (tb != tb) tb = INFINITY;
-        if (ta > tb) {
-            const float s = ta;
-            ta = tb;
-            tb = s;
-        }
-        t0 = fmaxf(t0, ta);
-        t1 = fminf(t1, tb);
-        if (t0 > t1) return -1.0f;
+        t0 = fmaxf(t0, fminf(ta, tb));
+        t1 = fminf(t1, fmaxf(ta, tb));
     }
-    return t0;
+    return t0 > t1 ? -1.0f : t0;
+}
+__device__ __forceinline__ BakeNode load_node(const Dev& D, uint32_t i) {
+    BakeNode nd;
+    const float4* src = reinterpret_cast<const float4*>(D.nodes + i);
+    float4* dst = reinterpret_cast<float4*>(&nd);
+    dst[0] = __ldg(src);
+    dst[1] = __ldg(src + 1);
+    return nd;
 }
 
+// Walks the leaves whose boxes the ray enters, nearer child first, and stops
+// when leaf(first, count) returns true. Both children of a node are tested
+// where it is (they are neighbours in memory), so only entered boxes are
+// pushed; a box is left out when beyond(entry) holds, at the push and again
+// when it is popped. The results do not depend on the order: they are minima
+// or "any" over the triangles hit. (Popping and loading every child before
+// its test, leaf triangles through an index: 11.2 + 4.2 ms for the bake of a
+// 61k-triangle scene's 64^3 grid.)
 constexpr int kStack = 64;
+template <typename Beyond, typename Leaf>
+__device__ __forceinline__ void walk_bvh(const Dev& D, V o, V d, Beyond beyond, Leaf leaf) {
+    if (D.n_nodes == 0) return;
+    const float inv[3] = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
+    uint2 stack[kStack];  // node, entry distance
+    int sp = 0;
+    BakeNode nd = load_node(D, 0);
+    if (box_entry(nd.mn, nd.mx, o, inv) < 0.0f) return;
+    for (;;) {
+        bool down = false;
+        if (nd.count) {
+            if (leaf(nd.left, nd.count)) return;
+        } else {
+            BakeNode l = load_node(D, nd.left), r = load_node(D, nd.left + 1);
+            const float tl = box_entry(l.mn, l.mx, o, inv), tr = box_entry(r.mn, r.mx, o, inv);
+            const bool hl = tl >= 0.0f && !beyond(tl), hr = tr >= 0.0f && !beyond(tr);
+            const bool left_first = hl && (!hr || tl <= tr);
+            if (hl && hr && sp < kStack)
+                stack[sp++] = left_first ? make_uint2(nd.left + 1, __float_as_uint(tr)) : make_uint2(nd.left, __float_as_uint(tl));
+            if (hl || hr) {
+                nd = left_first ? l : r;
+                down = true;
+            }
+        }
+        while (!down) {
+            if (sp == 0) return;
+            const uint2 e = stack[--sp];
+            if (beyond(__uint_as_float(e.y))) continue;
+            nd = load_node(D, e.x);
+            down = true;
+        }
+    }
+}
 
 // trace_nearest (src/raytracer.rs:134-170): the hit of smallest
 // (t, triangle). Boxes entered well beyond the best hit are skipped.
 __device__ bool trace_nearest(const Dev& D, V o, V d, float tmin, uint32_t& tri, float& th, float& bu, float& bv) {
-    const float inv[3] = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
-    uint32_t stack[kStack];
-    int sp = 0;
-    stack[sp++] = 0;
     bool found = false;
     float best = INFINITY;
-    if (D.n_nodes == 0) return false;
-    while (sp > 0) {
-        const BakeNode nd = D.nodes[stack[--sp]];
-        const float t0 = box_entry(nd, o, inv);
-        if (t0 < 0.0f) continue;
-        if (found && t0 > best + (fabsf(best) * 1.0e-3f + 1.0e-5f)) continue;
-        if (nd.count == 0) {
-            if (sp + 2 <= kStack) {
-                stack[sp++] = nd.left;
-                stack[sp++] = nd.left + 1;
+    walk_bvh(
+        D, o, d, [&](float t0) { return found && t0 > best + (fabsf(best) * 1.0e-3f + 1.0e-5f); },
+        [&](uint32_t first, uint32_t count) {
+            for (uint32_t i = 0; i < count; ++i) {
+                const LeafTri lt = load_leaf(D.leaf + first + i);
+                float t, u, v;
+                if (!ray_tri(o, d, lt, tmin, INFINITY, t, u, v)) continue;
+                if (!found || hit_before(t, lt.index, th, tri)) {
+                    found = true;
+                    tri = lt.index;
+                    th = t;
+                    bu = u;
+                    bv = v;
+                    best = t;
+                }
             }
-            continue;
-        }
-        for (uint32_t i = 0; i < nd.count; ++i) {
-            const uint32_t ti = D.order[nd.left + i];
-            float t, u, v;
-            if (!ray_tri(o, d, D.tris[ti], tmin, INFINITY, t, u, v)) continue;
-            if (!found || hit_before(t, ti, th, tri)) {
-                found = true;
-                tri = ti;
-                th = t;
-                bu = u;
-                bv = v;
-                best = t;
-            }
-        }
-    }
+            return false;
+        });
     return found;
 }
 
@@ -168,39 +220,31 @@ __device__ bool trace_nearest(const Dev& D, V o, V d, float tmin, uint32_t& tri,
 // last_i) (all hits when first); returns false at an opaque hit.
 __device__ bool next_translucent(const Dev& D, V o, V d, float tmin, bool first, float last_t, uint32_t last_i,
                                  bool& found, float& bt, uint32_t& bi, uint32_t& count) {
-    const float inv[3] = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
-    uint32_t stack[kStack];
-    int sp = 0;
-    stack[sp++] = 0;
+    bool clear = true;
     found = false;
     count = 0;
-    if (D.n_nodes == 0) return true;
-    while (sp > 0) {
-        const BakeNode nd = D.nodes[stack[--sp]];
-        if (box_entry(nd, o, inv) < 0.0f) continue;
-        if (nd.count == 0) {
-            if (sp + 2 <= kStack) {
-                stack[sp++] = nd.left;
-                stack[sp++] = nd.left + 1;
+    walk_bvh(
+        D, o, d, [](float) { return false; },
+        [&](uint32_t begin, uint32_t n) {
+            for (uint32_t i = 0; i < n; ++i) {
+                const LeafTri lt = load_leaf(D.leaf + begin + i);
+                float th, u, v;
+                if (!ray_tri(o, d, lt, tmin, INFINITY, th, u, v)) continue;
+                if (!lt.translucent) {
+                    clear = false;
+                    return true;
+                }
+                ++count;
+                if (!first && !hit_before(last_t, last_i, th, lt.index)) continue;
+                if (!found || hit_before(th, lt.index, bt, bi)) {
+                    found = true;
+                    bt = th;
+                    bi = lt.index;
+                }
             }
-            continue;
-        }
-        for (uint32_t i = 0; i < nd.count; ++i) {
-            const uint32_t ti = D.order[nd.left + i];
-            const BakeTri& t = D.tris[ti];
-            float th, u, v;
-            if (!ray_tri(o, d, t, tmin, INFINITY, th, u, v)) continue;
-            if (!D.mats[t.material].translucent) return false;
-            ++count;
-            if (!first && !hit_before(last_t, last_i, th, ti)) continue;
-            if (!found || hit_before(th, ti, bt, bi)) {
-                found = true;
-                bt = th;
-                bi = ti;
-            }
-        }
-    }
-    return true;
+            return false;
+        });
+    return clear;
 }
 
 // trace_transmittance (src/raytracer.rs:172-207).
@@ -484,6 +528,17 @@ __global__ void __launch_bounds__(128) k_gi_accum(Dev D, uint32_t k0, uint32_t k
     }
 }
 
+// The traversal's triangles in leaf order.
+__global__ void k_gi_pack(Dev D) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < D.n_tris; i += gridDim.x * blockDim.x) {
+        const uint32_t ti = D.order[i];
+        const BakeTri& t = D.tris[ti];
+        const V p0 = ld3(t.p0), e1 = ld3(t.p1) - p0, e2 = ld3(t.p2) - p0;
+        D.leaf[i] = LeafTri{{p0.x, p0.y, p0.z}, D.mats[t.material].translucent, {e1.x, e1.y, e1.z}, ti,
+                            {e2.x, e2.y, e2.z}, 0u};
+    }
+}
+
 // initialize_voxel_gi_from_scene(scale 1, sky 1) for voxels the bake skips.
 __global__ void k_gi_init(Dev D) {
     const uint64_t total = (uint64_t)D.n * D.n * D.n;
@@ -583,6 +638,7 @@ swr_status gi_bake_device(const BakeInput& in, float* out, std::string& err) {
     BakeTexture* texs = nullptr;
     float *lut = nullptr, *dirs = nullptr, *sun = nullptr, *raw = nullptr, *blur = nullptr;
     uint8_t* active = nullptr;
+    LeafTri* leaf = nullptr;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) {
         if (x != cudaSuccess && e == cudaSuccess) e = x;
@@ -599,9 +655,12 @@ swr_status gi_bake_device(const BakeInput& in, float* out, std::string& err) {
     chk(m.put(&active, in.active, nvox));
     chk(m.put(&sun, in.sun, nvox));
     chk(m.put(&alist, active_list.data(), active_list.size()));
+    chk(m.put(&leaf, (const LeafTri*)nullptr, in.ntris));
     chk(m.put(&raw, (const float*)nullptr, nvox * 16));
     chk(m.put(&blur, (const float*)nullptr, nvox * 16));
     if (e == cudaSuccess) {
+        D.leaf = leaf;
+        D.n_tris = (uint32_t)in.ntris;
         D.tris = tris;
         D.nodes = nodes;
         D.order = order;
@@ -628,6 +687,7 @@ swr_status gi_bake_device(const BakeInput& in, float* out, std::string& err) {
         D.n = n;
         D.out = raw;
         const uint32_t vg = (uint32_t)std::min<uint64_t>((nvox + 255) / 256, (uint64_t)sms * 16);
+        if (D.n_tris) k_gi_pack<<<(uint32_t)std::min<uint64_t>((D.n_tris + 255u) / 256u, (uint64_t)sms * 8), 256>>>(D);
         k_gi_init<<<vg, 256>>>(D);
         e = cudaGetLastError();
         // The active voxels in chunks: the texture samples of a chunk's rays

@@ -37,7 +37,7 @@ struct BakeTri {
     uint32_t material;
 };
 // BVH node over BakeTri indices (leaves: triangles order[left .. left+count)).
-struct BakeNode {
+struct alignas(16) BakeNode {
     float mn[3], mx[3];
     uint32_t left, count;
 };
