@@ -363,6 +363,7 @@ struct FrameArgs {
     // graphs gain nothing (1280x720 124 -> 126) and frames of large kernels lose
     // (4K 1062 -> 1088: the next kernel's waiting CTAs take up places).
     uint32_t overlap;
+    uint32_t narrow_raster;    // 32-px tiles shaded apart: rasterized by 128-thread CTAs
     uint32_t pair_limit;       // (triangle, 64-px tile) pairs past which a frame counts as overflowed, 0 = none
     uint32_t skip_unsampled;   // triangles that hold no pixel centre are not binned
     uint32_t rsqrt_uniform;    // 1 + the rsqrt mode all views share, 0 = per view
@@ -382,7 +383,7 @@ bool depth_floor_host(const int32_t p[6], const float zow[3], const float oow[3]
 // Per-device constant tables; call once per device outside stream capture.
 cudaError_t init_kernel_constants();
 // Persistent raster / grid-stride shading grid sizes for this device.
-void frame_grids(int num_sms, uint32_t sched_tile, bool fuse32, uint32_t* raster_grid, uint32_t* shade_grid);
+void frame_grids(int num_sms, uint32_t sched_tile, bool fuse32, bool narrow, uint32_t* raster_grid, uint32_t* shade_grid);
 // Whether frames with this scheduling tile shade inside the raster kernel.
 bool shade_fused(uint32_t sched_tile, bool fuse32);
 

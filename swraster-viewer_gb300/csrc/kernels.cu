@@ -1547,13 +1547,19 @@ __device__ __forceinline__ void load_shade_const(ShadeConst& c, const FrameArgs&
     if (t < 16u) reinterpret_cast<uint4*>(c.sky)[t] = s2[t];
 }
 
-template <int S>
+// T threads per CTA. Tiles of 8 and 16 px take 128 and larger ones 256 (64
+// and 256 views' small frames: a heavy tile of a small frame is one CTA's
+// latency), but 32-px tiles shaded apart 128 where there are many tiles per
+// SM: less of the CTA waits at each round's barriers (64 views, 32-px raster
+// 479 -> 411 us, eight scenes 424 -> 368, 1080p 138 -> 135; 1367x769 with 7
+// tiles an SM 67 -> 103).
+template <int S, int T = (S <= 16 ? 128 : 256)>
 struct RasterShared {
-    static constexpr int kThreads = S <= 16 ? 128 : 256;
+    static constexpr int kThreads = T;
     // CTAs per SM the register budget allows. Five of 128 threads (96
     // registers): 1280x720 with fused 16-px tiles 118.5 us a frame, against
     // 121.6 at six (80, spilling more) and 121.4 at four.
-    static constexpr int kMinBlocks = S <= 16 ? 5 : 3;
+    static constexpr int kMinBlocks = T == 128 ? 5 : 3;
     static constexpr int kRegions = kThreads + kThreads / 2;  // regions staged per round
     unsigned long long sk[S * S];                             // depth keys of the scheduling tile
     // Regions of the round, in packet order.
@@ -1581,8 +1587,8 @@ struct FusedShared : RasterShared<S> {
     uint8_t tab[512];
     ShadeConst shade;
 };
-template <int S, bool FUSE>
-using RasterSmem = std::conditional_t<FUSE, FusedShared<S>, RasterShared<S>>;
+template <int S, bool FUSE, int T>
+using RasterSmem = std::conditional_t<FUSE, FusedShared<S>, RasterShared<S, T>>;
 
 constexpr uint32_t kSlowRegion = 0x8000u;  // region replays the sequential additions
 
@@ -1592,8 +1598,8 @@ struct PacketLanes {
     uint32_t seq8, mat;
 };
 
-template <int S>
-__device__ __forceinline__ PacketLanes packet_lanes(const RasterShared<S>& s, uint32_t pk) {
+template <int S, int T>
+__device__ __forceinline__ PacketLanes packet_lanes(const RasterShared<S, T>& s, uint32_t pk) {
     PacketLanes L;
     const float4 o = s.p_o[pk], z = s.p_z[pk];
     L.ooa = o.x;
@@ -1611,8 +1617,8 @@ __device__ __forceinline__ PacketLanes packet_lanes(const RasterShared<S>& s, ui
 // Depth test of one covered lane: bary, w, z as fine_raster computes them,
 // then the canonical-order key (atomicMin keeps the lowest z, ties broken by
 // submission order).
-template <int S>
-__device__ __forceinline__ void raster_lane(RasterShared<S>& s, const FrameArgs& a, const DScene& sc,
+template <int S, int T>
+__device__ __forceinline__ void raster_lane(RasterShared<S, T>& s, const FrameArgs& a, const DScene& sc,
                                             const PacketLanes& L, uint32_t pk, float w1, float w2, int32_t lx,
                                             int32_t ly) {
     const float b1 = w1 * L.ooa, b2 = w2 * L.ooa;
@@ -1634,8 +1640,8 @@ __device__ __forceinline__ int32_t geom_ox(uint32_t g) { return (int32_t)(int8_t
 __device__ __forceinline__ int32_t geom_oy(uint32_t g) { return (int32_t)(int8_t)(g >> 24); }
 
 // Exact region quad: lane = one quad, evaluated in closed form.
-template <int S>
-__device__ __forceinline__ void raster_exact_quad(RasterShared<S>& s, const FrameArgs& a, const DScene& sc,
+template <int S, int T>
+__device__ __forceinline__ void raster_exact_quad(RasterShared<S, T>& s, const FrameArgs& a, const DScene& sc,
                                                   uint32_t r, uint32_t q, uint32_t g) {
     const uint32_t pi = s.r_pi[r];
     if (pi & kSlowRegion) return;
@@ -1672,8 +1678,8 @@ __device__ __forceinline__ void raster_exact_quad(RasterShared<S>& s, const Fram
 
 // Sequential region: one warp, lane = (quad row, quad lane); each lane walks
 // its row along x with the reference's additions.
-template <int S>
-__device__ __forceinline__ void raster_slow_region(RasterShared<S>& s, const FrameArgs& a, const DScene& sc,
+template <int S, int T>
+__device__ __forceinline__ void raster_slow_region(RasterShared<S, T>& s, const FrameArgs& a, const DScene& sc,
                                                    uint32_t r) {
     const uint32_t lane = threadIdx.x & 31u;
     const int32_t k = (int32_t)(lane & 3u);
@@ -1720,8 +1726,8 @@ __device__ __forceinline__ void raster_slow_region(RasterShared<S>& s, const Fra
 // row w: each load reads whole key rows (16 B a lane, consecutive lanes
 // consecutive keys), so the warp's accesses cover distinct banks; four lanes
 // hold a cell's part of a row and shuffles fold the lanes and rows.
-template <int S>
-__device__ __forceinline__ void cell_depths(RasterShared<S>& s) {
+template <int S, int T>
+__device__ __forceinline__ void cell_depths(RasterShared<S, T>& s) {
     constexpr int CW = S / 8;      // cells per side
     constexpr int LPR = S / 2;     // lanes per key row (two keys a lane)
     constexpr int RPW = 32 / LPR;  // key rows per warp load
@@ -1747,8 +1753,8 @@ __device__ __forceinline__ void cell_depths(RasterShared<S>& s) {
 
 // Farthest key depth over the cells holding pixels [xl, xh] x [yl, yh]
 // clipped to the scheduling tile (all ones when none of them is in it).
-template <int S>
-__device__ __forceinline__ uint32_t cells_far(const RasterShared<S>& s, int32_t xl, int32_t xh, int32_t yl, int32_t yh,
+template <int S, int T>
+__device__ __forceinline__ uint32_t cells_far(const RasterShared<S, T>& s, int32_t xl, int32_t xh, int32_t yl, int32_t yh,
                                               int32_t sx0, int32_t sy0) {
     xl = max(xl, sx0), xh = min(xh, sx0 + S - 1), yl = max(yl, sy0), yh = min(yh, sy0 + S - 1);
     if (xh < xl || yh < yl) return 0xFFFFFFFFu;
@@ -1769,8 +1775,8 @@ __device__ __forceinline__ uint32_t packet_floor(const PacketCtx& c) { return c.
 // either count them (regions, quads; the accepted 16-px blocks of a coarse
 // packet go to bmask) or stage them from the given positions (bmask as the
 // count left it).
-template <int S>
-__device__ __forceinline__ void packet_regions(RasterShared<S>& s, const PacketCtx& c, int32_t sx0, int32_t sy0,
+template <int S, int T>
+__device__ __forceinline__ void packet_regions(RasterShared<S, T>& s, const PacketCtx& c, int32_t sx0, int32_t sy0,
                                                bool write, uint32_t pk, uint32_t& n_r, uint32_t& n_q,
                                                uint32_t& bmask) {
     auto region = [&](int32_t ox, int32_t oy, int32_t ex, int32_t ey) {
@@ -1847,10 +1853,10 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
 // regions (a block-wide scan places them), pass 2 rasterizes the exact
 // regions' quads flattened over all lanes, pass 3 the sequential regions.
 // GI and MODE: the fused shading's variant (see k_shade); unused without FUSE.
-template <int S, bool FUSE, bool GI, int MODE>
-__global__ void __launch_bounds__(RasterShared<S>::kThreads, RasterShared<S>::kMinBlocks) k_raster(FrameArgs a) {
+template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads>
+__global__ void __launch_bounds__(T, RasterShared<S, T>::kMinBlocks) k_raster(FrameArgs a) {
     frame_kernel_entry();
-    using Sh = RasterSmem<S, FUSE>;
+    using Sh = RasterSmem<S, FUSE, T>;
     constexpr int NT = Sh::kThreads, R = Sh::kRegions, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char raster_smem[];
     Sh& s = *reinterpret_cast<Sh*>(raster_smem);
@@ -2840,10 +2846,10 @@ __global__ void __launch_bounds__(kResolveThreads) k_resolve(FrameArgs a) {
 // --------------------------------------------------------------------------
 static uint64_t g_const_init_mask = 0;  // one bit per device
 
-template <int S, bool FUSE, bool GI, int MODE>
+template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads>
 static cudaError_t raster_smem_attr() {
-    return cudaFuncSetAttribute(k_raster<S, FUSE, GI, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(RasterSmem<S, FUSE>));
+    return cudaFuncSetAttribute(k_raster<S, FUSE, GI, MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(RasterSmem<S, FUSE, T>));
 }
 template <int S>
 static cudaError_t fused_smem_attr() {
@@ -2869,9 +2875,9 @@ static void launch_kernel(void (*k)(FrameArgs), uint32_t grid, uint32_t threads,
     cudaLaunchKernelEx(&c, k, a);
 }
 
-template <int S, bool FUSE, bool GI, int MODE>
+template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads>
 static void launch_raster(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
-    launch_kernel(k_raster<S, FUSE, GI, MODE>, grid, RasterShared<S>::kThreads, sizeof(RasterSmem<S, FUSE>), a, s);
+    launch_kernel(k_raster<S, FUSE, GI, MODE, T>, grid, T, sizeof(RasterSmem<S, FUSE, T>), a, s);
 }
 // The fused shading compiled for what the frame needs: the variant for baked
 // grids of any rsqrt mode spills 250-450 B a thread against 0-130 B, and
@@ -2897,27 +2903,31 @@ cudaError_t init_kernel_constants() {
     if (e == cudaSuccess) e = fused_smem_attr<16>();
     if (e == cudaSuccess) e = fused_smem_attr<32>();
     if (e == cudaSuccess) e = raster_smem_attr<32, false, false, kModeAny>();
+    if (e == cudaSuccess) e = raster_smem_attr<32, false, false, kModeAny, 128>();
     if (e == cudaSuccess) e = raster_smem_attr<64, false, false, kModeAny>();
     if (e == cudaSuccess && dev < 64) g_const_init_mask |= 1ull << dev;
     return e;
 }
 
-template <int S, bool FUSE>
+template <int S, bool FUSE, int T = RasterShared<S>::kThreads>
 static int raster_blocks_per_sm() {
     int rb = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rb, k_raster<S, FUSE, false, FUSE ? kModeArm : kModeAny>,
-                                                  RasterShared<S>::kThreads, sizeof(RasterSmem<S, FUSE>));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rb, k_raster<S, FUSE, false, FUSE ? kModeArm : kModeAny, T>, T,
+                                                  sizeof(RasterSmem<S, FUSE, T>));
     return rb;
 }
 
 bool shade_fused(uint32_t S, bool fuse32) { return S <= kFusedShadeMaxTile || (S == 32 && fuse32); }
 
-void frame_grids(int num_sms, uint32_t S, bool fuse32, uint32_t* raster_grid, uint32_t* shade_grid) {
+void frame_grids(int num_sms, uint32_t S, bool fuse32, bool narrow, uint32_t* raster_grid, uint32_t* shade_grid) {
     int rb = 1, sb = 1;
     switch (S) {
         case 8: rb = raster_blocks_per_sm<8, true>(); break;
         case 16: rb = raster_blocks_per_sm<16, true>(); break;
-        case 32: rb = fuse32 ? raster_blocks_per_sm<32, true>() : raster_blocks_per_sm<32, false>(); break;
+        case 32:
+            rb = fuse32 ? raster_blocks_per_sm<32, true>()
+                        : (narrow ? raster_blocks_per_sm<32, false, 128>() : raster_blocks_per_sm<32, false>());
+            break;
         default: rb = raster_blocks_per_sm<64, false>(); break;
     }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sb, k_shade<false, kModeArm>, ShadeShape<false>::kThreads, 0);
@@ -2986,6 +2996,7 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
         case 16: launch_fused<16>(a, rg, s); break;
         case 32:
             if (a.fused_shade) launch_fused<32>(a, rg, s);
+            else if (a.narrow_raster) launch_raster<32, false, false, kModeAny, 128>(a, rg, s);
             else launch_raster<32, false, false, kModeAny>(a, rg, s);
             break;
         default: launch_raster<64, false, false, kModeAny>(a, rg, s); break;

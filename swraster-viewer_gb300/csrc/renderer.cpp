@@ -174,8 +174,10 @@ swr_status FrameEngine::init(std::string& err) {
 }
 
 void FrameEngine::release() {
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    graph_exec = nullptr;
+    for (cudaGraphExec_t& g : graph_exec) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
     if (capture_stream) cudaStreamDestroy(capture_stream);
     capture_stream = nullptr;
     for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &rec_t, &fan_base, &clip_queue, &wide_queue, &tile_count, &tile_offset,
@@ -325,11 +327,13 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     std::memcpy(hs + lay.o_views, vws.data(), vws.size() * sizeof(DView));
     if (!h_order.empty()) std::memcpy(hs + lay.o_order, h_order.data(), h_order.size() * sizeof(uint32_t));
     const bool fused32 = fuse32 && sched_tile == 32;
-    if (grid_tile != sched_tile || grid_fused32 != fused32 || grid_cap != raster_cta_cap) {
-        frame_grids(num_sms, sched_tile, fused32, &raster_grid, &shade_grid);
+    const bool narrow = sched_tile == 32 && !fused32 && !raster_cta_cap && stile_cursor >= kNarrowTiles * (uint32_t)num_sms;
+    if (grid_tile != sched_tile || grid_fused32 != fused32 || grid_narrow != narrow || grid_cap != raster_cta_cap) {
+        frame_grids(num_sms, sched_tile, fused32, narrow, &raster_grid, &shade_grid);
         if (raster_cta_cap) raster_grid = std::min<uint32_t>(raster_grid, (uint32_t)num_sms * raster_cta_cap);
         grid_tile = sched_tile;
         grid_fused32 = fused32;
+        grid_narrow = narrow;
         grid_cap = raster_cta_cap;
     }
     uint8_t* tb = static_cast<uint8_t*>(tables.p);
@@ -347,6 +351,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     a.skip_unsampled = 1u;
     a.overlap = 0u;
     a.fused_shade = fused32 ? 1u : 0u;
+    a.narrow_raster = narrow ? 1u : 0u;
     a.chunk_cap = chunk_cap;
     a.tri_cap = tri_cap;
     a.extra_cap = (uint32_t)extra_cap;
@@ -403,37 +408,38 @@ swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string
         stage_pending[slot] = true;
         stage_slot = (slot + 1) % kStageRing;
     }
-    const bool same = graph_exec && std::memcmp(&graph_args, &args, sizeof(args)) == 0;
+    const uint32_t gi = args.narrow_raster;
+    const bool same = graph_exec[gi] && std::memcmp(&graph_args[gi], &args, sizeof(args)) == 0;
     if (auto_graph) {
         same_frames = std::memcmp(&prev_args, &args, sizeof(args)) == 0 ? same_frames + 1 : 0;
         prev_args = args;
     }
     if (e == cudaSuccess && !ev && (use_graph || (auto_graph && (same || same_frames >= kGraphAfter)))) {
         if (!same) {
-            if (graph_exec) cudaGraphExecDestroy(graph_exec);
-            graph_exec = nullptr;
+            if (graph_exec[gi]) cudaGraphExecDestroy(graph_exec[gi]);
+            graph_exec[gi] = nullptr;
             if (!capture_stream) e = cudaStreamCreateWithFlags(&capture_stream, cudaStreamNonBlocking);
             cudaGraph_t g = nullptr;
             // Capture on the engine's own stream; the graph is then launched
             // into the caller's stream (which may be the legacy default one).
             if (e == cudaSuccess) e = cudaStreamBeginCapture(capture_stream, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
-                graph_kernels = launch_frame(args, capture_stream, num_sms, nullptr);
+                graph_kernels[gi] = launch_frame(args, capture_stream, num_sms, nullptr);
                 e = cudaStreamEndCapture(capture_stream, &g);
             }
-            if (e == cudaSuccess) e = cudaGraphInstantiate(&graph_exec, g, 0);
+            if (e == cudaSuccess) e = cudaGraphInstantiate(&graph_exec[gi], g, 0);
             if (g) cudaGraphDestroy(g);
             if (e != cudaSuccess) {
                 err = std::string("graph capture failed: ") + cudaGetErrorString(e);
                 cudaGetLastError();
-                graph_exec = nullptr;
+                graph_exec[gi] = nullptr;
                 return SWR_CUDA_ERROR;
             }
-            graph_args = args;
+            graph_args[gi] = args;
             graph_stream = stream;
         }
-        e = cudaGraphLaunch(graph_exec, stream);
-        if (e == cudaSuccess) kernel_launches += graph_kernels;
+        e = cudaGraphLaunch(graph_exec[gi], stream);
+        if (e == cudaSuccess) kernel_launches += graph_kernels[gi];
     } else if (e == cudaSuccess) {
         kernel_launches += launch_frame(args, stream, num_sms, ev);
         e = cudaGetLastError();

@@ -84,7 +84,12 @@ struct FrameEngine {
     uint32_t raster_grid = 0, shade_grid = 0, grid_tile = 0;
     uint32_t raster_cta_cap = 0, grid_cap = 0;  // raster CTAs per SM (0: as many as fit; batch autotuner's choice)
     bool fuse32 = false;        // 32-px tiles shade inside the raster kernel (batch autotuner's choice)
-    bool grid_fused32 = false;
+    bool grid_fused32 = false, grid_narrow = false;
+    // Tiles per SM from which 32-px tiles shaded apart are rasterized by CTAs
+    // of 128 threads, not 256. Raster us with 256 -> 128: 349 tiles an SM 479
+    // -> 411, 64 424 -> 368, 13 138 -> 135, 7 67 -> 103 (too few CTAs wide
+    // enough for the heaviest tiles). A capped CTA count keeps 256.
+    static constexpr uint32_t kNarrowTiles = 12;
     DBuf tables, tri_state, rec_r, rec_s, rec_t, fan_base, clip_queue, wide_queue;
     DBuf tile_count, tile_offset, tile_cursor, work, sky_tab, bins, keys, counters, rsqrt_tab;
     DBuf color;                // linear colour of views that need it (padded tile grids)
@@ -99,7 +104,6 @@ struct FrameEngine {
     int stage_slot = 0;
     uint32_t retries = 0;
     uint64_t kernel_launches = 0;  // kernels enqueued (graph replays count the graph's kernels)
-    uint32_t graph_kernels = 0;    // kernels in the captured graph
     DCounters last{};
     DFrameDyn dyn{};
     FrameArgs args{};
@@ -112,8 +116,11 @@ struct FrameEngine {
     static constexpr uint32_t kGraphAfter = 4;
     uint32_t same_frames = 0;
     FrameArgs prev_args{};
-    cudaGraphExec_t graph_exec = nullptr;
-    FrameArgs graph_args{};
+    // One graph for each width of the raster's CTAs: batches of one engine
+    // vary in size.
+    cudaGraphExec_t graph_exec[2] = {};
+    FrameArgs graph_args[2] = {};
+    uint32_t graph_kernels[2] = {};  // kernels in the captured graph
     cudaStream_t graph_stream = nullptr;
     cudaStream_t capture_stream = nullptr;  // legacy default streams cannot be captured
 

@@ -35,3 +35,19 @@ def test_ties_and_culling_in_32px_tiles(n, fused):
         assert (r.stats().culled_pairs > 0) == (n == 300)
     r.close()
     s.close()
+
+
+@pytest.mark.parametrize("views,cap", [(75, 0), (77, 0), (77, 3)])
+def test_many_32px_tiles(views, cap):
+    """24 tiles a view: 12 tiles per SM of 152 lie between 75 and 77 views, where
+    the raster's CTA width changes; every view must equal the oracle's."""
+    s = swr.Scene(tie_across_rounds_scene(300))
+    w, h = 190, 127
+    cam = swr.make_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 1.0, w, h, 40.0)
+    _, ovis, _, _ = oracle.render(s, cam, w, h, rsqrt_mode=swr.RSQRT_AARCH64, threads=1)
+    b = swr.Batch(sched_tile=32, raster_ctas_per_sm=cap)
+    b.render(swr.Batch.views([(s, cam, w, h, 2.0, swr.RSQRT_AARCH64)] * views))
+    for i in range(views):
+        assert np.array_equal(b.output(i, w, h)[1], ovis)
+    b.close()
+    s.close()
