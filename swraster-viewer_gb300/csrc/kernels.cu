@@ -1831,18 +1831,18 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
                                             int32_t qy, int32_t k, bool needed, unsigned long long key);
 
 // Occlusion culling is on for 64-px scheduling tiles and for the 32-px tiles
-// that take more than one round (SWR_CULL_FROM packets). It pays where many
+// that take more than one round (one packet per thread). It pays where many
 // packets of a tile lie behind near geometry drawn first: eight uneven scenes
 // in a batch, 32-px raster 1,454 -> 1,080 us with the fused shading, 830 ->
 // 442 apart. From 100, 192, 256, 320 or 384 packets on, that raster takes
 // 448, 443, 442, 442 and 443 us, and the fused one of 64 batched views (small
-// spheres, seldom hidden) 2,373, 2,333, 2,323, 2,320 and 2,315. Lighter tiles
-// would pay a short first round's barriers for it.
+// spheres, seldom hidden) 2,373, 2,333, 2,323, 2,320 and 2,315 (rounds of
+// 256). With rounds of 128, from 64, 128, 192 or 256 packets on: 2M triangles
+// at 1920x1080 222, 218, 234 and 252 us, eight scenes 368, 372, 368 and 375,
+// 64 views 433, 418, 416 and 412. Lighter tiles would pay a short first
+// round's barriers for it.
 // A first round of 64 packets: 4K raster 0.444 ms, against 0.461 (32),
 // 0.460 (128) and 0.477 (a full round of 256).
-#ifndef SWR_CULL_FROM
-#define SWR_CULL_FROM 256
-#endif
 #ifndef SWR_CULL_FIRST
 #define SWR_CULL_FIRST 64
 #endif
@@ -1869,7 +1869,7 @@ __global__ void __launch_bounds__(T, RasterShared<S, T>::kMinBlocks) k_raster(Fr
     // of packets, whole instead: 4K 718 against 728 frames/s).
     constexpr bool kCull = S >= SWR_CULL_MIN_TILE;
     constexpr uint32_t kFirst = (kCull && SWR_CULL_FIRST > 0 && SWR_CULL_FIRST < NT) ? SWR_CULL_FIRST : NT;
-    constexpr uint32_t kCullFrom = S >= 64 ? 0u : SWR_CULL_FROM;
+    constexpr uint32_t kCullFrom = S >= 64 ? 0u : (uint32_t)NT;
     if constexpr (kFuse)
         for (int i = threadIdx.x; i < 512; i += NT) s.tab[i] = a.rsqrt_table[i];
     uint32_t n_culled = 0, held = 0xFFFFFFFFu;

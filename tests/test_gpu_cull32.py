@@ -1,8 +1,9 @@
-"""Occlusion culling in 32-px scheduling tiles: bins of more than one round
-(256 packets) are culled against the depths of earlier rounds, lighter ones are
-not. Stacks of screen-filling quads with a tie that arrives last, with bins on
-both sides of the line, shaded apart and in the raster kernel, against the
-oracle: visibility must be equal and the last of the tied quads must win."""
+"""Occlusion culling in 32-px scheduling tiles: bins of more than one round (a
+packet per thread of the CTA) are culled against the depths of earlier rounds,
+lighter ones are not. Stacks of screen-filling quads with a tie that arrives
+last, with bins on both sides of the line, shaded apart and in the raster
+kernel, against the oracle: visibility must be equal and the last of the tied
+quads must win."""
 import numpy as np
 import pytest
 
