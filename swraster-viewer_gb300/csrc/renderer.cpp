@@ -397,6 +397,15 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     return SWR_OK;
 }
 
+// Whether the caller is capturing the stream: a graph cannot be launched into
+// a capture, kernels can.
+static bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string& err) {
     // The staging copy runs ahead of the kernels (graph or not) and is the
     // only reader of its staging buffer; with a ring of them the host stages
@@ -414,7 +423,8 @@ swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string
         same_frames = std::memcmp(&prev_args, &args, sizeof(args)) == 0 ? same_frames + 1 : 0;
         prev_args = args;
     }
-    if (e == cudaSuccess && !ev && (use_graph || (auto_graph && (same || same_frames >= kGraphAfter)))) {
+    bool replay = !ev && (use_graph || (auto_graph && (same || same_frames >= kGraphAfter) && !capturing(stream)));
+    if (e == cudaSuccess && replay) {
         if (!same) {
             if (graph_exec[gi]) cudaGraphExecDestroy(graph_exec[gi]);
             graph_exec[gi] = nullptr;
@@ -433,14 +443,20 @@ swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string
                 err = std::string("graph capture failed: ") + cudaGetErrorString(e);
                 cudaGetLastError();
                 graph_exec[gi] = nullptr;
-                return SWR_CUDA_ERROR;
+                if (use_graph) return SWR_CUDA_ERROR;
+                auto_graph = replay = false;  // not asked for: plain launches do
+                err.clear();
+                e = cudaSuccess;
             }
             graph_args[gi] = args;
             graph_stream = stream;
         }
-        e = cudaGraphLaunch(graph_exec[gi], stream);
-        if (e == cudaSuccess) kernel_launches += graph_kernels[gi];
-    } else if (e == cudaSuccess) {
+        if (replay) {
+            e = cudaGraphLaunch(graph_exec[gi], stream);
+            if (e == cudaSuccess) kernel_launches += graph_kernels[gi];
+        }
+    }
+    if (e == cudaSuccess && !replay) {
         kernel_launches += launch_frame(args, stream, num_sms, ev);
         e = cudaGetLastError();
     }

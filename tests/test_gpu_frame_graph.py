@@ -66,3 +66,23 @@ def test_exposure_and_blit_target_between_replays(three):
         want_rgba, want_vis = fresh(three[0], cam)
         assert np.array_equal(rgba, want_rgba) and np.array_equal(r.visbuffer(), want_vis), i
     r.close()
+
+
+@pytest.mark.parametrize("warm", [2, 8])
+def test_frame_captured_by_the_caller(three, warm):
+    """A stream that the caller captures gets the kernels themselves, before and after the renderer replays."""
+    torch = pytest.importorskip("torch")
+    r, s = swr.Renderer(W, H), torch.cuda.Stream()
+    for i in range(warm):
+        r.render(three[0], camera(three[0], i), stream=s.cuda_stream)
+        r.blit(stream=s.cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    cam = camera(three[0], 3)
+    with torch.cuda.graph(graph, stream=s, capture_error_mode="relaxed"):
+        r.render(three[0], cam, stream=s.cuda_stream)
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    want_rgba, want_vis = fresh(three[0], cam)
+    assert np.array_equal(r.visbuffer(), want_vis) and np.array_equal(r.blit(), want_rgba)
+    r.close()
