@@ -13,12 +13,15 @@
 //               vertex transform (src/renderer.rs:470-574), trivial clip
 //               classification, triangle setup (bin_triangle,
 //               src/renderer.rs:668-831), per-tile pair counts with
-//               warp-aggregated atomics.
+//               warp-aggregated atomics; triangles over many tiles go to a
+//               queue in segments.
 //   k_clip      Sutherland-Hodgman for triangles with a vertex outside a plane
-//               (clip_against_frustum, src/renderer.rs:579-665), fan setup.
-//   k_scan      exclusive scan of tile counts -> bin offsets, overflow check.
-//   k_scatter   record indices into per-tile bins (warp-aggregated cursors);
-//               replaces BumpQueue::push (src/bumpqueue.rs:96-112).
+//               (clip_against_frustum, src/renderer.rs:579-665), fan setup;
+//               counts of the queued segments.
+//   k_scan      places the bins, overflow check, the raster's visiting order.
+//   k_scatter   record indices into per-tile bins (warp-aggregated cursors;
+//               replaces BumpQueue::push, src/bumpqueue.rs:96-112), the
+//               raster's work items, the views' sky tables.
 //   k_raster    one CTA per scheduling tile: the reference's coarse/fine
 //               traversal and f32 edge stepping (src/tilerasterizer.rs:114-383)
 //               with a 64-bit (depth, sequence) atomicMin per pixel in shared
@@ -2497,11 +2500,12 @@ __device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* 
 // CTA shape of the grid-stride shading kernel. Without voxel GI, eight
 // 128-thread CTAs per SM (64 registers): 4K shade 442 us, against 451 at seven
 // (72), 450 at six and 471 at five; 64 views 1,478, 1,490, 1,555 and 1,720.
-// The GI variant keeps three 256-thread CTAs: at 72 registers its cone-tracing
-// loop spills 216 B per thread.
+// With the baked voxel grid seven (72 registers): 288 us at 4K, 114 at 1080p, 63
+// at 720p; eight 285, 120 and 66, six 293, 120 and 65, five 307, 124 and 65,
+// three of 256 threads 298, 121 and 66.
 template <bool GI> struct ShadeShape {
-    static constexpr int kThreads = GI ? 256 : 128;
-    static constexpr int kMinBlocks = GI ? 3 : 8;
+    static constexpr int kThreads = 128;
+    static constexpr int kMinBlocks = GI ? 7 : 8;
 };
 // GI: the frame has scenes with a baked voxel grid. MODE: see shade_pixel.
 template <bool GI, int MODE>
