@@ -364,6 +364,7 @@ struct FrameArgs {
     // (4K 1062 -> 1088: the next kernel's waiting CTAs take up places).
     uint32_t overlap;
     uint32_t narrow_raster;    // 32-px tiles shaded apart: rasterized by 128-thread CTAs
+    uint32_t cull16;           // 16-px tiles: occlusion culling
     uint32_t pair_limit;       // (triangle, 64-px tile) pairs past which a frame counts as overflowed, 0 = none
     uint32_t skip_unsampled;   // triangles that hold no pixel centre are not binned
     uint32_t rsqrt_uniform;    // 1 + the rsqrt mode all views share, 0 = per view

@@ -447,11 +447,6 @@ __device__ __forceinline__ bool push_wide(const FrameArgs& a, uint32_t* counter,
     return ok;
 }
 
-// Occlusion culling runs for scheduling tiles of at least this many pixels
-// a side (the raster drops packets hidden behind the depths of earlier rounds).
-#ifndef SWR_CULL_MIN_TILE
-#define SWR_CULL_MIN_TILE 32
-#endif
 
 // Whether no pixel centre can pass the raster's edge tests for a front-facing
 // triangle with subpixel vertices (x0, y0) .. (x2, y2) inside the screen,
@@ -538,7 +533,7 @@ __device__ __forceinline__ void store_raster(const FrameArgs& a, uint32_t slot, 
     r.material = material;
     r.view = view_idx;
     r.zfloor = 0u;
-    if ((int32_t)a.sched_tile >= SWR_CULL_MIN_TILE && !(material & kRecTransBit)) {
+    if ((a.sched_tile >= 32u || a.cull16) && !(material & kRecTransBit)) {
         const float zc[3] = {v0.cz, v1.cz, v2.cz}, wc[3] = {v0.cw, v1.cw, v2.cw};
         float zl;
         if (depth_floor(r.p, t.area, r.zow, r.oow, zc, wc, t.mxx * kSubpixelScale, t.mxy * kSubpixelScale, zl))
@@ -1834,7 +1829,9 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
                                             int32_t qy, int32_t k, bool needed, unsigned long long key);
 
 // Occlusion culling is on for 64-px scheduling tiles and for the 32-px tiles
-// that take more than one round (one packet per thread). It pays where many
+// that take more than one round (one packet per thread); for 16-px tiles it is
+// a variant of its own (FrameArgs.cull16), since the plain one is faster where
+// bins are light. It pays where many
 // packets of a tile lie behind near geometry drawn first: eight uneven scenes
 // in a batch, 32-px raster 1,454 -> 1,080 us with the fused shading, 830 ->
 // 442 apart. From 100, 192, 256, 320 or 384 packets on, that raster takes
@@ -1856,7 +1853,8 @@ __device__ __forceinline__ void shade_pixel(const FrameArgs& a, const uint8_t* t
 // regions (a block-wide scan places them), pass 2 rasterizes the exact
 // regions' quads flattened over all lanes, pass 3 the sequential regions.
 // GI and MODE: the fused shading's variant (see k_shade); unused without FUSE.
-template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads>
+// CULL: with occlusion culling.
+template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads, bool CULL = (S >= 32)>
 __global__ void __launch_bounds__(T, RasterShared<S, T>::kMinBlocks) k_raster(FrameArgs a) {
     frame_kernel_entry();
     using Sh = RasterSmem<S, FUSE, T>;
@@ -1866,11 +1864,10 @@ __global__ void __launch_bounds__(T, RasterShared<S, T>::kMinBlocks) k_raster(Fr
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t n_tiles = FUSE ? a.dyn->n_stiles : a.counters->filled;
     constexpr bool kFuse = FUSE;
-    // Occlusion culling for tiles of at least SWR_CULL_MIN_TILE px; the first
-    // round of a tile takes at most kFirst packets, so that later rounds
+    // With occlusion culling the first round of a tile takes at most kFirst packets, so that later rounds
     // meet the nearest depths sooner (taking light tiles, at most one round
     // of packets, whole instead: 4K 718 against 728 frames/s).
-    constexpr bool kCull = S >= SWR_CULL_MIN_TILE;
+    constexpr bool kCull = CULL;
     constexpr uint32_t kFirst = (kCull && SWR_CULL_FIRST > 0 && SWR_CULL_FIRST < NT) ? SWR_CULL_FIRST : NT;
     constexpr uint32_t kCullFrom = S >= 64 ? 0u : (uint32_t)NT;
     if constexpr (kFuse)
@@ -2850,17 +2847,17 @@ __global__ void __launch_bounds__(kResolveThreads) k_resolve(FrameArgs a) {
 // --------------------------------------------------------------------------
 static uint64_t g_const_init_mask = 0;  // one bit per device
 
-template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads>
+template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads, bool CULL = (S >= 32)>
 static cudaError_t raster_smem_attr() {
-    return cudaFuncSetAttribute(k_raster<S, FUSE, GI, MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_raster<S, FUSE, GI, MODE, T, CULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(RasterSmem<S, FUSE, T>));
 }
-template <int S>
+template <int S, bool CULL = (S >= 32)>
 static cudaError_t fused_smem_attr() {
-    cudaError_t e = raster_smem_attr<S, true, false, kModeArm>();
-    if (e == cudaSuccess) e = raster_smem_attr<S, true, false, kModeAny>();
-    if (e == cudaSuccess) e = raster_smem_attr<S, true, true, kModeArm>();
-    if (e == cudaSuccess) e = raster_smem_attr<S, true, true, kModeAny>();
+    cudaError_t e = raster_smem_attr<S, true, false, kModeArm, RasterShared<S>::kThreads, CULL>();
+    if (e == cudaSuccess) e = raster_smem_attr<S, true, false, kModeAny, RasterShared<S>::kThreads, CULL>();
+    if (e == cudaSuccess) e = raster_smem_attr<S, true, true, kModeArm, RasterShared<S>::kThreads, CULL>();
+    if (e == cudaSuccess) e = raster_smem_attr<S, true, true, kModeAny, RasterShared<S>::kThreads, CULL>();
     return e;
 }
 // Launches a frame kernel, with FrameArgs.overlap as a programmatic dependent
@@ -2879,22 +2876,22 @@ static void launch_kernel(void (*k)(FrameArgs), uint32_t grid, uint32_t threads,
     cudaLaunchKernelEx(&c, k, a);
 }
 
-template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads>
+template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads, bool CULL = (S >= 32)>
 static void launch_raster(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
-    launch_kernel(k_raster<S, FUSE, GI, MODE, T>, grid, T, sizeof(RasterSmem<S, FUSE, T>), a, s);
+    launch_kernel(k_raster<S, FUSE, GI, MODE, T, CULL>, grid, T, sizeof(RasterSmem<S, FUSE, T>), a, s);
 }
 // The fused shading compiled for what the frame needs: the variant for baked
 // grids of any rsqrt mode spills 250-450 B a thread against 0-130 B, and
 // every fused frame ran it (64 batched views 5% slower, 1280x720 2%).
-template <int S>
+template <int S, bool CULL = (S >= 32)>
 static void launch_fused(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
     const bool arm = a.rsqrt_uniform == 1u + kModeArm;
     if (a.has_gi) {
-        if (arm) launch_raster<S, true, true, kModeArm>(a, grid, s);
-        else launch_raster<S, true, true, kModeAny>(a, grid, s);
+        if (arm) launch_raster<S, true, true, kModeArm, RasterShared<S>::kThreads, CULL>(a, grid, s);
+        else launch_raster<S, true, true, kModeAny, RasterShared<S>::kThreads, CULL>(a, grid, s);
     } else {
-        if (arm) launch_raster<S, true, false, kModeArm>(a, grid, s);
-        else launch_raster<S, true, false, kModeAny>(a, grid, s);
+        if (arm) launch_raster<S, true, false, kModeArm, RasterShared<S>::kThreads, CULL>(a, grid, s);
+        else launch_raster<S, true, false, kModeAny, RasterShared<S>::kThreads, CULL>(a, grid, s);
     }
 }
 
@@ -2905,6 +2902,7 @@ cudaError_t init_kernel_constants() {
     if (dev < 64 && (g_const_init_mask >> dev) & 1ull) return cudaSuccess;
     e = fused_smem_attr<8>();
     if (e == cudaSuccess) e = fused_smem_attr<16>();
+    if (e == cudaSuccess) e = fused_smem_attr<16, true>();
     if (e == cudaSuccess) e = fused_smem_attr<32>();
     if (e == cudaSuccess) e = raster_smem_attr<32, false, false, kModeAny>();
     if (e == cudaSuccess) e = raster_smem_attr<32, false, false, kModeAny, 128>();
@@ -2997,7 +2995,10 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
     const uint32_t rg = a.raster_grid > 0 ? a.raster_grid : (uint32_t)num_sms;
     switch (a.sched_tile) {
         case 8: launch_fused<8>(a, rg, s); break;
-        case 16: launch_fused<16>(a, rg, s); break;
+        case 16:
+            if (a.cull16) launch_fused<16, true>(a, rg, s);
+            else launch_fused<16>(a, rg, s);
+            break;
         case 32:
             if (a.fused_shade) launch_fused<32>(a, rg, s);
             else if (a.narrow_raster) launch_raster<32, false, false, kModeAny, 128>(a, rg, s);

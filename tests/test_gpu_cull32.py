@@ -1,4 +1,4 @@
-"""Occlusion culling in 32-px scheduling tiles: bins of more than one round (a
+"""Occlusion culling in 16- and 32-px scheduling tiles: bins of more than one round (a
 packet per thread of the CTA) are culled against the depths of earlier rounds,
 lighter ones are not. Stacks of screen-filling quads with a tie that arrives
 last, with bins on both sides of the line, shaded apart and in the raster
@@ -51,4 +51,24 @@ def test_many_32px_tiles(views, cap):
     for i in range(views):
         assert np.array_equal(b.output(i, w, h)[1], ovis)
     b.close()
+    s.close()
+
+
+@pytest.mark.parametrize("n", [480, 520, 1000])
+@pytest.mark.parametrize("gi", [False, True])
+def test_ties_and_culling_in_16px_tiles(n, gi):
+    """16 tiles of 16 px: from 1,024 triangles on they are culled."""
+    s = swr.Scene(tie_across_rounds_scene(n), gi=gi)
+    w, h = 61, 45
+    cam = swr.make_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 1.0, w, h, 40.0)
+    for mode in (swr.RSQRT_AARCH64, swr.RSQRT_IEEE):
+        orgba, ovis, _, _ = oracle.render(s, cam, w, h, rsqrt_mode=mode, threads=1)
+        r = swr.Renderer(w, h, rsqrt_mode=mode, sched_tile=16)
+        r.render(s, cam)
+        assert np.array_equal(r.visbuffer(), ovis)
+        rgba = r.blit()
+        d = np.abs(rgba[:h & ~1].view(np.uint8).astype(np.int32) - orgba[:h & ~1].view(np.uint8).astype(np.int32))
+        assert d.max() <= 1
+        assert (r.stats().culled_pairs > 0) == (n > 500)
+        r.close()
     s.close()
