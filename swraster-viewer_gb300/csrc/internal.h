@@ -365,6 +365,7 @@ struct FrameArgs {
     uint32_t overlap;
     uint32_t narrow_raster;    // 32-px tiles shaded apart: rasterized by 128-thread CTAs
     uint32_t cull16;           // 16-px tiles: occlusion culling
+    uint32_t wide_shade;       // k_shade in one CTA an SM (frames without baked grids)
     uint32_t pair_limit;       // (triangle, 64-px tile) pairs past which a frame counts as overflowed, 0 = none
     uint32_t skip_unsampled;   // triangles that hold no pixel centre are not binned
     uint32_t rsqrt_uniform;    // 1 + the rsqrt mode all views share, 0 = per view

@@ -2494,25 +2494,29 @@ __device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* 
     shade_pixel<GI, MODE>(a, tab, c, qx, qy, k, needed, key);
 }
 
-// CTA shape of the grid-stride shading kernel. Without voxel GI, eight
-// 128-thread CTAs per SM (64 registers): 4K shade 442 us, against 451 at seven
-// (72), 450 at six and 471 at five; 64 views 1,478, 1,490, 1,555 and 1,720.
-// With the baked voxel grid seven (72 registers): 288 us at 4K, 114 at 1080p, 63
-// at 720p; eight 285, 120 and 66, six 293, 120 and 65, five 307, 124 and 65,
-// three of 256 threads 298, 121 and 66.
-template <bool GI> struct ShadeShape {
-    static constexpr int kThreads = 128;
-    static constexpr int kMinBlocks = GI ? 7 : 8;
-};
+// CTA shape of the grid-stride shading kernel, 64 registers a thread. Where
+// every SM has some 1,024 pixels several times over (FrameArgs.wide_shade),
+// one CTA of 1,024 threads an SM: its warps shade a strip of 256x4 pixels, so
+// the lines of keys and outputs and the records and texels at their borders
+// stay with one SM. us at 128, 256, 512 and 1,024 threads (1,024 an SM): 4K
+// 446, 434, 417 and 393, 1M triangles at 2560x1440 201, 199, 191 and 179,
+// 1367x769 89, 90, 88 and 89, eight scenes 508, 502, 475 and 461, 64 views
+// 1,437, 1,389, 1,392 and 1,409. (CTAs in 32x32 or 64x16 pixels: 4K 413 and
+// 411.) With fewer pixels, eight CTAs of 128 spread over more SMs.
+// With the baked voxel grid seven of 128 (72 registers): 288 us at 4K, 114 at
+// 1080p, 63 at 720p; eight 285, 120 and 66, six 293, 120 and 65, five 307, 124
+// and 65, three of 256 threads 298, 121 and 66.
+constexpr int kShadeThreads = 128, kShadeWide = 1024;
+template <bool GI, int T> constexpr int kShadeBlocks = T == kShadeWide ? 1 : (GI ? 7 : 8);
 // GI: the frame has scenes with a baked voxel grid. MODE: see shade_pixel.
-template <bool GI, int MODE>
-__global__ void __launch_bounds__(ShadeShape<GI>::kThreads, ShadeShape<GI>::kMinBlocks) k_shade(FrameArgs a) {
+template <bool GI, int MODE, int T = kShadeThreads>
+__global__ void __launch_bounds__(T, kShadeBlocks<GI, T>) k_shade(FrameArgs a) {
     frame_kernel_entry();
     __shared__ uint8_t tab[512];
     __shared__ ShadeConst sc;
     for (int i = threadIdx.x; i < 512; i += blockDim.x) tab[i] = a.rsqrt_table[i];
     // Every view's quad count is a multiple of 1024 (a 64-px tile), so the
-    // CTA's 32 or 64 quads are one view's and all live.
+    // CTA's 32 or 256 quads are one view's and all live.
     const uint32_t total = a.dyn->total_quads;
     const uint32_t stride = gridDim.x * blockDim.x;
     // Quads [q0, q1) are the held view's (a search per iteration took six
@@ -2932,7 +2936,7 @@ void frame_grids(int num_sms, uint32_t S, bool fuse32, bool narrow, uint32_t* ra
             break;
         default: rb = raster_blocks_per_sm<64, false>(); break;
     }
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sb, k_shade<false, kModeArm>, ShadeShape<false>::kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sb, k_shade<false, kModeArm>, kShadeThreads, 0);
     cudaGetLastError();
     *raster_grid = (uint32_t)(num_sms * (rb > 0 ? rb : 1));
     *shade_grid = (uint32_t)(num_sms * (sb > 0 ? sb : 1));
@@ -3014,21 +3018,28 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
             // CTAs per SM are taken once (the same on every GB300).
             static const uint32_t gi_blocks = [] {
                 int b = 0;
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<true, kModeArm>, ShadeShape<true>::kThreads, 0);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<true, kModeArm>, kShadeThreads, 0);
                 cudaGetLastError();
                 return (uint32_t)(b > 0 ? b : 1);
             }();
             const uint32_t sg = (uint32_t)num_sms * gi_blocks;
-            const uint32_t T = ShadeShape<true>::kThreads;
+            const uint32_t T = kShadeThreads;
             if (a.rsqrt_uniform == 1u + kModeArm) launch_kernel(k_shade<true, kModeArm>, sg, T, 0, a, s);
             else if (a.rsqrt_uniform == 1u + kModeIeee) launch_kernel(k_shade<true, kModeIeee>, sg, T, 0, a, s);
             else launch_kernel(k_shade<true, kModeAny>, sg, T, 0, a, s);
         } else {
-            const uint32_t sg = a.shade_grid > 0 ? a.shade_grid : (uint32_t)num_sms;
-            const uint32_t T = ShadeShape<false>::kThreads;
-            if (a.rsqrt_uniform == 1u + kModeArm) launch_kernel(k_shade<false, kModeArm>, sg, T, 0, a, s);
-            else if (a.rsqrt_uniform == 1u + kModeIeee) launch_kernel(k_shade<false, kModeIeee>, sg, T, 0, a, s);
-            else launch_kernel(k_shade<false, kModeAny>, sg, T, 0, a, s);
+            const bool arm = a.rsqrt_uniform == 1u + kModeArm, ieee = a.rsqrt_uniform == 1u + kModeIeee;
+            if (a.wide_shade) {
+                const uint32_t sg = (uint32_t)num_sms, T = kShadeWide;
+                if (arm) launch_kernel(k_shade<false, kModeArm, kShadeWide>, sg, T, 0, a, s);
+                else if (ieee) launch_kernel(k_shade<false, kModeIeee, kShadeWide>, sg, T, 0, a, s);
+                else launch_kernel(k_shade<false, kModeAny, kShadeWide>, sg, T, 0, a, s);
+            } else {
+                const uint32_t sg = a.shade_grid > 0 ? a.shade_grid : (uint32_t)num_sms, T = kShadeThreads;
+                if (arm) launch_kernel(k_shade<false, kModeArm>, sg, T, 0, a, s);
+                else if (ieee) launch_kernel(k_shade<false, kModeIeee>, sg, T, 0, a, s);
+                else launch_kernel(k_shade<false, kModeAny>, sg, T, 0, a, s);
+            }
         }
         launches++;
     }

@@ -352,6 +352,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     a.overlap = 0u;
     a.fused_shade = fused32 ? 1u : 0u;
     a.narrow_raster = narrow ? 1u : 0u;
+    a.wide_shade = !shares_device && !shade_fused(sched_tile, fused32) && 4ull * quad_cursor >= kWideShadeRounds * 1024u * num_sms ? 1u : 0u;
     a.cull16 = sched_tile == 16 && tri_bound >= kCullTris * stile_cursor ? 1u : 0u;
     a.chunk_cap = chunk_cap;
     a.tri_cap = tri_cap;
@@ -418,7 +419,7 @@ swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string
         stage_pending[slot] = true;
         stage_slot = (slot + 1) % kStageRing;
     }
-    const uint32_t gi = args.narrow_raster | args.cull16;
+    const uint32_t gi = (args.narrow_raster | args.cull16) + 2u * args.wide_shade;
     const bool same = graph_exec[gi] && std::memcmp(&graph_args[gi], &args, sizeof(args)) == 0;
     if (auto_graph) {
         same_frames = std::memcmp(&prev_args, &args, sizeof(args)) == 0 ? same_frames + 1 : 0;

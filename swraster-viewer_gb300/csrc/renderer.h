@@ -96,6 +96,12 @@ struct FrameEngine {
     // 60k at 480x300 (94) 121 -> 117, 150k at 1280x720 (39) 215 -> 218, 82k
     // (21) 98 -> 101.
     static constexpr uint64_t kCullTris = 64;
+    // The engine's launches usually run beside other streams' (the server's
+    // batches): a CTA that needs a whole SM would wait there until one is empty
+    // (24 requests 1,137 us with k_shade in such CTAs, 1,088 without).
+    bool shares_device = false;
+    // Pixels per SM (in rounds of 1,024) from which k_shade takes one CTA an SM.
+    static constexpr uint64_t kWideShadeRounds = 4;
     DBuf tables, tri_state, rec_r, rec_s, rec_t, fan_base, clip_queue, wide_queue;
     DBuf tile_count, tile_offset, tile_cursor, work, sky_tab, bins, keys, counters, rsqrt_tab;
     DBuf color;                // linear colour of views that need it (padded tile grids)
@@ -122,11 +128,11 @@ struct FrameEngine {
     static constexpr uint32_t kGraphAfter = 4;
     uint32_t same_frames = 0;
     FrameArgs prev_args{};
-    // One graph for each form of the raster kernel: batches of one engine
-    // vary in size.
-    cudaGraphExec_t graph_exec[2] = {};
-    FrameArgs graph_args[2] = {};
-    uint32_t graph_kernels[2] = {};  // kernels in the captured graph
+    // One graph for each form of the raster and shading kernels: batches of
+    // one engine vary in size.
+    cudaGraphExec_t graph_exec[4] = {};
+    FrameArgs graph_args[4] = {};
+    uint32_t graph_kernels[4] = {};  // kernels in the captured graph
     cudaStream_t graph_stream = nullptr;
     cudaStream_t capture_stream = nullptr;  // legacy default streams cannot be captured
 

@@ -314,6 +314,7 @@ swr_status swr_server_create(const swr_server_opts* opts, swr_server** out) {
         e->b->opts.sched_tile = o.sched_tile;
         e->b->opt_fuse32 = e->b->base_fuse32 = (o.flags & SWR_BATCH_FUSED_SHADE) != 0u;
         e->b->eng.use_graph = o.use_graph != 0;
+        e->b->eng.shares_device = true;
         std::string err;
         swr_status st = e->b->eng.init(err);
         if (st == SWR_OK && (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess ||
