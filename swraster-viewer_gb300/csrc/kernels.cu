@@ -2496,9 +2496,10 @@ __device__ __forceinline__ void shade_thread(const FrameArgs& a, const uint8_t* 
 
 // CTA shape of the grid-stride shading kernel, 64 registers a thread. Where
 // every SM has some 1,024 pixels several times over (FrameArgs.wide_shade),
-// one CTA of 1,024 threads an SM: its warps shade a strip of 256x4 pixels, so
-// the lines of keys and outputs and the records and texels at their borders
-// stay with one SM. us at 128, 256, 512 and 1,024 threads (1,024 an SM): 4K
+// one CTA of 1,024 threads an SM: its warps go through the kernel's long code
+// more nearly together (stalls for instructions 1.30 -> 0.28 an issue) over
+// one strip of 256x4 pixels (L1 hits 60 -> 68%), and 80% of the issue slots
+// are busy instead of 69%. us at 128, 256, 512 and 1,024 threads (1,024 an SM): 4K
 // 446, 434, 417 and 393, 1M triangles at 2560x1440 201, 199, 191 and 179,
 // 1367x769 89, 90, 88 and 89, eight scenes 508, 502, 475 and 461, 64 views
 // 1,437, 1,389, 1,392 and 1,409. (CTAs in 32x32 or 64x16 pixels: 4K 413 and
