@@ -412,7 +412,15 @@ void swr_renderer_destroy(swr_renderer* r);
  * once the frame is enqueued (and, when dt > 0, after the exposure step's
  * host callback is enqueued). Bin overflow is detected on the device and
  * the frame is re-rendered with a larger capacity on the next call to
- * swr_renderer_sync, swr_blit or swr_read_visbuffer. */
+ * swr_renderer_sync, swr_blit or swr_read_visbuffer.
+ * A stream that the caller captures (cudaStreamBeginCapture, relaxed mode)
+ * records the frame instead: each launch of the caller's graph renders it
+ * again (with dt > 0: advances the exposure by dt again) until the renderer or
+ * the scene is destroyed. The renderer can render other frames between
+ * launches, in stream order or after waiting for them. Frames of that size and
+ * scene should have been rendered before, so that their capacities have grown:
+ * a recorded frame that overflows does so at every launch. Batches likewise
+ * (without use_graph). */
 swr_status swr_render_frame(swr_renderer* r, const swr_scene* scene, const swr_camera* camera,
                             float dt, void* stream);
 

@@ -83,12 +83,21 @@ swr_status BatchImpl::enqueue(const swr_view_desc* vd, int32_t n, cudaStream_t s
     }
     swr_status st = eng.prepare(scenes, views, cams, err);
     if (st != SWR_OK) return st;
-    cudaEventRecord(ev_start, stream);
-    st = eng.launch(stream, nullptr, err);
-    cudaEventRecord(ev_end, stream);
-    if (st == SWR_OK && (h_counters.ensure(sizeof(DCounters)) != cudaSuccess ||
-                         cudaMemcpyAsync(h_counters.p, eng.counters.p, sizeof(DCounters), cudaMemcpyDeviceToHost,
-                                         stream) != cudaSuccess)) {
+    // A batch that the caller captures records no events (they could not be
+    // read), and its graph's launches write the outputs it names.
+    const bool captured = stream_captured(stream);
+    if (!captured) cudaEventRecord(ev_start, stream);
+    st = eng.launch(stream, captured, nullptr, err);
+    if (!captured) cudaEventRecord(ev_end, stream);
+    if (captured) {
+        tile_lum.in_graph = true;
+        for (int32_t i = 0; i < n; ++i) owned[i].rgba8.in_graph = owned[i].vis.in_graph = true;
+    }
+    const bool fresh = !h_counters.p;
+    if (st == SWR_OK && h_counters.ensure(sizeof(DCounters)) == cudaSuccess && fresh)
+        std::memset(h_counters.p, 0, sizeof(DCounters));
+    if (st == SWR_OK && (!h_counters.p || cudaMemcpyAsync(h_counters.p, eng.counters.p, sizeof(DCounters),
+                                                          cudaMemcpyDeviceToHost, stream) != cudaSuccess)) {
         cudaGetLastError();
         err = "counter readback failed";
         st = SWR_CUDA_ERROR;

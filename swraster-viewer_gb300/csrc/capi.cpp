@@ -240,6 +240,7 @@ swr_status swr_renderer_create(int32_t width, int32_t height, const swr_renderer
         return cuda_fail(e, "renderer allocation");
     }
     *r->h_expo = r->expo.exposure;
+    std::memset(r->h_counters, 0, sizeof(DCounters));  // read before any frame ran where the first one is only captured
     *out = r;
     return SWR_OK;
 }
@@ -283,11 +284,12 @@ void prof_collect(swr_renderer* r, int slot) {
 }
 
 void CUDART_CB exposure_callback(void* p) {
-    swr_renderer* r = static_cast<swr_renderer*>(p);
+    const auto* step = static_cast<const swr_renderer::ExposureStep*>(p);
+    swr_renderer* r = step->r;
     // A frame that overflowed its bins is re-rendered; it must not advance
     // the exposure state.
     if (r->h_counters->status & kStRetry) return;
-    r->expo.update(r->h_lum, (size_t)r->tiles_x * r->tiles_y, r->pending_dt);
+    r->expo.update(r->h_lum, (size_t)r->tiles_x * r->tiles_y, step->dt);
     *r->h_expo = r->expo.exposure;
 }
 
@@ -326,7 +328,10 @@ swr_status enqueue_frame(swr_renderer* r, const swr_scene* scene, const swr_came
     std::vector<const swr_camera*> cams = {cam};
     cudaEvent_t* ev = nullptr;
     int slot = -1;
-    if (r->profiling) {
+    // Events recorded in a capture can be neither queried nor waited for: a
+    // captured frame records none and is not profiled.
+    const bool captured = stream_captured(stream);
+    if (r->profiling && !captured) {
         slot = r->prof_next;
         r->prof_next = (r->prof_next + 1) % swr_renderer::kProfRing;
         prof_collect(r, slot);
@@ -335,25 +340,36 @@ swr_status enqueue_frame(swr_renderer* r, const swr_scene* scene, const swr_came
         r->prof_resolve[slot] = deferred;
     }
     FrameArgs a{};
-    swr_status st = r->eng.run(scenes, views, cams, stream, &a, err, ev);
+    swr_status st = r->eng.run(scenes, views, cams, stream, captured, &a, err, ev);
     if (st != SWR_OK) return fail(st, err);
     // The counters are final here (the resolve does not touch them).
     cudaMemcpyAsync(r->h_counters, r->eng.counters.p, sizeof(DCounters), cudaMemcpyDeviceToHost, stream);
     if (deferred) {
         const size_t nt = (size_t)r->tiles_x * r->tiles_y;
         cudaMemcpyAsync(r->h_lum, r->tile_lum.p, nt * sizeof(float), cudaMemcpyDeviceToHost, stream);
-        r->pending_dt = dt;
-        cudaLaunchHostFunc(stream, exposure_callback, r);
+        swr_renderer::ExposureStep* step = &r->step;
+        if (captured) {
+            step = nullptr;
+            for (auto& g : r->graph_steps)
+                if (g.dt == dt) step = &g;
+            if (!step) step = &r->graph_steps.emplace_back();
+        }
+        *step = {r, dt};
+        cudaLaunchHostFunc(stream, exposure_callback, step);
         a.exposure_dev = r->d_expo;
         if (ev) cudaEventRecord(ev[8], stream);
         launch_resolve(a, stream);
         r->eng.kernel_launches++;
         if (ev) cudaEventRecord(ev[9], stream);
-        cudaEventRecord(r->expo_done, stream);
-        r->expo_pending = true;
+        if (!captured) {
+            cudaEventRecord(r->expo_done, stream);
+            r->expo_pending = true;
+        }
     }
-    cudaEventRecord(r->status_ev, stream);
-    r->status_pending = true;
+    if (!captured) {
+        cudaEventRecord(r->status_ev, stream);
+        r->status_pending = true;
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
     r->last_args = a;

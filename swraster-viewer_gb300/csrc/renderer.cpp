@@ -180,9 +180,9 @@ void FrameEngine::release() {
     }
     if (capture_stream) cudaStreamDestroy(capture_stream);
     capture_stream = nullptr;
-    for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &rec_t, &fan_base, &clip_queue, &wide_queue, &tile_count, &tile_offset,
-                    &tile_cursor, &work, &sky_tab, &bins, &keys, &counters, &rsqrt_tab, &color})
-        b->release();
+    each_buffer([](DBuf& b) { b.release(); });
+    for (GraphStage& g : graph_stages) g.buf.release();
+    graph_stages.clear();
     for (int i = 0; i < kStageRing; ++i) {
         h_stage[i].release();
         if (stage_done[i]) cudaEventDestroy(stage_done[i]);
@@ -305,6 +305,11 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
         stage_pending[stage_slot] = false;
     }
     HBuf& h_stage_cur = h_stage[stage_slot];
+    for (size_t i = 0; i < graph_stages.size() && !h_stage_cur.p; ++i)
+        if (graph_stages[i].gone->load()) {
+            h_stage_cur = graph_stages[i].buf;
+            graph_stages.erase(graph_stages.begin() + (ptrdiff_t)i);
+        }
     if (h_stage_cur.ensure(lay.staged) != cudaSuccess) {
         err = "pinned allocation failed";
         return SWR_NO_MEMORY;
@@ -399,25 +404,62 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     return SWR_OK;
 }
 
-// Whether the caller is capturing the stream: a graph cannot be launched into
-// a capture, kernels can.
-static bool capturing(cudaStream_t stream) {
+bool stream_captured(cudaStream_t stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
     cudaGetLastError();
     return true;
 }
 
-swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string& err) {
+// A frame that the caller captures: its graph reads the slot's staging buffer
+// and the device buffers at every launch, whatever this engine renders until
+// then. An event recorded in a capture cannot be waited for, so the staging
+// buffer is not marked in flight but taken out of the ring.
+void FrameEngine::keep_for_graph(cudaStream_t stream, int slot) {
+    each_buffer([](DBuf& b) { b.in_graph = true; });
+    GraphStage g{h_stage[slot], std::make_shared<std::atomic<bool>>(false)};
+    h_stage[slot] = HBuf{};
+    graph_stages.push_back(g);
+    // The graph and its executable forms own a user object; its destructor
+    // (which may not call CUDA) marks the buffer free. Without one the buffer
+    // stays until the engine is released.
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    cudaUserObject_t obj = nullptr;
+    auto* flag = new std::shared_ptr<std::atomic<bool>>(g.gone);
+    auto done = [](void* p) {
+        auto* f = static_cast<std::shared_ptr<std::atomic<bool>>*>(p);
+        (*f)->store(true);
+        delete f;
+    };
+    if (cudaStreamGetCaptureInfo(stream, &st, nullptr, &graph) != cudaSuccess || !graph ||
+        cudaUserObjectCreate(&obj, flag, done, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        cudaGetLastError();
+        delete flag;
+        return;
+    }
+    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        // The graph does not hold the object, so its end says nothing.
+        cudaGetLastError();
+        graph_stages.back().gone = std::make_shared<std::atomic<bool>>(false);
+        cudaUserObjectRelease(obj, 1);
+    }
+}
+
+swr_status FrameEngine::launch(cudaStream_t stream, bool captured, cudaEvent_t* ev, std::string& err) {
     // The staging copy runs ahead of the kernels (graph or not) and is the
     // only reader of its staging buffer; with a ring of them the host stages
     // up to kStageRing frames ahead of the device.
     const int slot = stage_slot;
     cudaError_t e = cudaMemcpyAsync(tables.p, h_stage[slot].p, lay.staged, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaEventRecord(stage_done[slot], stream);
-    if (e == cudaSuccess) {
-        stage_pending[slot] = true;
-        stage_slot = (slot + 1) % kStageRing;
+    if (e == cudaSuccess && captured) {
+        keep_for_graph(stream, slot);
+    } else {
+        if (e == cudaSuccess) e = cudaEventRecord(stage_done[slot], stream);
+        if (e == cudaSuccess) {
+            stage_pending[slot] = true;
+            stage_slot = (slot + 1) % kStageRing;
+        }
     }
     const uint32_t gi = (args.narrow_raster | args.cull16) + 2u * args.wide_shade;
     const bool same = graph_exec[gi] && std::memcmp(&graph_args[gi], &args, sizeof(args)) == 0;
@@ -425,7 +467,8 @@ swr_status FrameEngine::launch(cudaStream_t stream, cudaEvent_t* ev, std::string
         same_frames = std::memcmp(&prev_args, &args, sizeof(args)) == 0 ? same_frames + 1 : 0;
         prev_args = args;
     }
-    bool replay = !ev && (use_graph || (auto_graph && (same || same_frames >= kGraphAfter) && !capturing(stream)));
+    // A graph cannot be launched into a capture, kernels can.
+    bool replay = !ev && (use_graph || (auto_graph && (same || same_frames >= kGraphAfter) && !captured));
     if (e == cudaSuccess && replay) {
         if (!same) {
             if (graph_exec[gi]) cudaGraphExecDestroy(graph_exec[gi]);
@@ -491,11 +534,11 @@ swr_status FrameEngine::grow_for(const DCounters& c, std::string& err) {
 }
 
 swr_status FrameEngine::run(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& vws,
-                            const std::vector<const swr_camera*>& cams, cudaStream_t stream, FrameArgs* out,
-                            std::string& err, cudaEvent_t* ev) {
+                            const std::vector<const swr_camera*>& cams, cudaStream_t stream, bool captured,
+                            FrameArgs* out, std::string& err, cudaEvent_t* ev) {
     swr_status st = prepare(scenes, vws, cams, err);
     if (st != SWR_OK) return st;
-    st = launch(stream, ev, err);
+    st = launch(stream, captured, ev, err);
     if (out) *out = args;
     return st;
 }

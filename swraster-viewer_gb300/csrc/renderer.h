@@ -4,7 +4,10 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
+#include <deque>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -18,11 +21,17 @@ namespace swr {
 struct DBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    // A graph that the caller captured holds this address and may be launched
+    // at any time: a buffer that grows past it keeps it until release().
+    bool in_graph = false;
+    std::vector<void*> outgrown;
     cudaError_t ensure(size_t n) {
         if (n <= bytes) return cudaSuccess;
-        if (p) cudaFree(p);
+        if (p && in_graph) outgrown.push_back(p);
+        else if (p) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        in_graph = false;
         size_t want = n + n / 4;
         cudaError_t e = cudaMalloc(&p, want);
         if (e == cudaSuccess) bytes = want;
@@ -30,8 +39,11 @@ struct DBuf {
     }
     void release() {
         if (p) cudaFree(p);
+        for (void* o : outgrown) cudaFree(o);
+        outgrown.clear();
         p = nullptr;
         bytes = 0;
+        in_graph = false;
     }
     template <typename T>
     T* as() const { return static_cast<T*>(p); }
@@ -136,6 +148,22 @@ struct FrameEngine {
     cudaStream_t graph_stream = nullptr;
     cudaStream_t capture_stream = nullptr;  // legacy default streams cannot be captured
 
+    // Staging buffers of frames that a caller captured: the graph's upload reads
+    // its buffer at every launch, so the buffer leaves the ring until the graph
+    // is gone (its user object tells) or the engine is released.
+    struct GraphStage {
+        HBuf buf;
+        std::shared_ptr<std::atomic<bool>> gone;
+    };
+    std::vector<GraphStage> graph_stages;
+    template <typename F>
+    void each_buffer(F f) {
+        for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &rec_t, &fan_base, &clip_queue, &wide_queue, &tile_count,
+                        &tile_offset, &tile_cursor, &work, &sky_tab, &bins, &keys, &counters, &rsqrt_tab, &color})
+            f(*b);
+    }
+    void keep_for_graph(cudaStream_t stream, int slot);
+
     swr_status init(std::string& err);
     // Grows what a frame's counters report as overflowed (bins, clip slots)
     // or, when a tile held too many translucent packets, halves the
@@ -144,12 +172,17 @@ struct FrameEngine {
     void release();
     swr_status prepare(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& views,
                        const std::vector<const swr_camera*>& cams, std::string& err);
-    swr_status launch(cudaStream_t stream, cudaEvent_t* ev, std::string& err);
+    // captured: the caller captures the stream (stream_captured), so nothing
+    // here waits for what is enqueued and what it reads stays as it is.
+    swr_status launch(cudaStream_t stream, bool captured, cudaEvent_t* ev, std::string& err);
     // prepare + launch (the plain renderer's path).
     swr_status run(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& views,
-                   const std::vector<const swr_camera*>& cams, cudaStream_t stream, FrameArgs* out_args,
+                   const std::vector<const swr_camera*>& cams, cudaStream_t stream, bool captured, FrameArgs* out_args,
                    std::string& err, cudaEvent_t* ev = nullptr);
 };
+
+// Whether the caller is capturing the stream.
+bool stream_captured(cudaStream_t stream);
 
 // compute_nodes_by_distance (src/renderer.rs:201-210): appends the scene's
 // node indices, nearest first, to `out`.
@@ -197,7 +230,15 @@ struct swr_renderer {
     float* d_expo = nullptr;
     cudaEvent_t expo_done = nullptr;
     bool expo_pending = false;
-    float pending_dt = 0.0f;
+    // What the exposure callback of a frame advances: one step for frames in
+    // flight (a frame waits for the step before it), and one for each dt that a
+    // caller captured, which its graph's launches read again.
+    struct ExposureStep {
+        swr_renderer* r;
+        float dt;
+    };
+    ExposureStep step{};
+    std::deque<ExposureStep> graph_steps;
     // Last frame, kept for overflow re-runs.
     const swr_scene* last_scene = nullptr;
     swr_camera last_cam{};
