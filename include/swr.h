@@ -650,6 +650,10 @@ swr_status swr_selftest_srgb_pow(const float* in, float* out, uint64_t n, uint32
  * counterpart in the reference, whose raster tests every packet. */
 swr_status swr_selftest_depth_floor(const int32_t* p, const float* zow, const float* oow, int32_t xe, int32_t ye,
                                     float* zlo);
+/* The same with the vertices' clip-space depths z[3] and w[3], which the front
+ * end passes; the call above takes them from the interpolants. */
+swr_status swr_selftest_depth_floor_vertices(const int32_t* p, const float* zow, const float* oow, const float* z,
+                                             const float* w, int32_t xe, int32_t ye, float* zlo);
 
 /* Allocation-free frame. No counterpart in the reference: an addition for
  * callers that cannot allocate device memory while they render (processes

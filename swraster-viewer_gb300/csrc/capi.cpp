@@ -636,7 +636,15 @@ swr_status swr_selftest_depth_floor(const int32_t* p, const float* zow, const fl
                                     float* zlo) {
     if (!p || !zow || !oow || !zlo) return fail(SWR_INVALID_ARG, "null argument");
     float z = 0.0f;
-    *zlo = depth_floor_host(p, zow, oow, xe, ye, z) ? z : -std::numeric_limits<float>::infinity();
+    *zlo = depth_floor_host(p, zow, oow, nullptr, nullptr, xe, ye, z) ? z : -std::numeric_limits<float>::infinity();
+    return SWR_OK;
+}
+
+swr_status swr_selftest_depth_floor_vertices(const int32_t* p, const float* zow, const float* oow, const float* z,
+                                             const float* w, int32_t xe, int32_t ye, float* zlo) {
+    if (!p || !zow || !oow || !z || !w || !zlo) return fail(SWR_INVALID_ARG, "null argument");
+    float f = 0.0f;
+    *zlo = depth_floor_host(p, zow, oow, z, w, xe, ye, f) ? f : -std::numeric_limits<float>::infinity();
     return SWR_OK;
 }
 

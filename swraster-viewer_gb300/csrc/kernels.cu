@@ -3064,15 +3064,16 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
     return launches;
 }
 
-bool depth_floor_host(const int32_t p[6], const float zow[3], const float oow[3], int32_t xe, int32_t ye, float& zlo) {
-    // Vertex depths and w from the interpolants' corners, the area wrapped as
-    // the front end's.
+bool depth_floor_host(const int32_t p[6], const float zow[3], const float oow[3], const float* z, const float* w,
+                      int32_t xe, int32_t ye, float& zlo) {
+    // Without the vertices' depths and w: those of the interpolants' corners.
+    // The area is wrapped as the front end's.
     float zc[3], wc[3];
     for (int v = 0; v < 3; ++v) {
-        const float o = v == 0 ? oow[0] : oow[0] + oow[v], z = v == 0 ? zow[0] : zow[0] + zow[v];
-        if (!(o > 0.0f)) return false;
-        zc[v] = z / o;
-        wc[v] = 1.0f / o;
+        const float o = v == 0 ? oow[0] : oow[0] + oow[v], n = v == 0 ? zow[0] : zow[0] + zow[v];
+        if (!z && !(o > 0.0f)) return false;
+        zc[v] = z ? z[v] : n / o;
+        wc[v] = z ? w[v] : 1.0f / o;
     }
     auto d = [&](int i, int j) { return (uint32_t)p[i] - (uint32_t)p[j]; };
     const int32_t area = (int32_t)(d(2, 0) * d(5, 1) - d(4, 0) * d(3, 1));

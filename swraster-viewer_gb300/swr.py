@@ -190,6 +190,7 @@ EXPORTS = [
     "swr_camera_update", "swr_renderer_create", "swr_renderer_destroy", "swr_render_frame", "swr_renderer_sync",
     "swr_blit", "swr_renderer_set_blit_target", "swr_read_visbuffer", "swr_renderer_device_outputs", "swr_renderer_get_exposure",
     "swr_renderer_set_exposure", "swr_renderer_get_stats", "swr_renderer_get_tile_luminance", "swr_last_error",
+    "swr_selftest_depth_floor_vertices",
     "swr_abi_version", "swr_renderer_set_profiling", "swr_renderer_get_profile", "swr_render_frame_noalloc",
     "swr_batch_create", "swr_batch_destroy", "swr_batch_render", "swr_batch_sync", "swr_batch_output",
     "swr_batch_autotune", "swr_batch_last_ms", "swr_batch_get_tuning", "swr_server_create", "swr_server_destroy", "swr_server_add_scene",
@@ -234,6 +235,8 @@ def lib():
         "swr_renderer_get_profile": ([vp, f32p, C.c_int32, C.POINTER(C.c_uint32)], C.c_int),
         "swr_selftest_rsqrt": ([f32p, f32p, C.c_uint64, C.c_uint32], C.c_int),
         "swr_selftest_depth_floor": ([C.c_void_p, f32p, f32p, C.c_int32, C.c_int32, f32p], C.c_int),
+        "swr_selftest_depth_floor_vertices": ([C.c_void_p, f32p, f32p, f32p, f32p, C.c_int32, C.c_int32, f32p],
+                                              C.c_int),
         "swr_scene_load_gltf": ([C.c_char_p, C.POINTER(GltfOpts), C.POINTER(vp)], C.c_int),
         "swr_render_frame_noalloc": ([vp, C.POINTER(Camera), C.c_int32, C.c_int32, C.c_float, C.c_uint32, vp, vp, vp],
                                      C.c_int),
@@ -543,6 +546,16 @@ def selftest_depth_floor(p, zow, oow, xe, ye):
     check(lib().swr_selftest_depth_floor(p.ctypes.data, zow.ctypes.data_as(f32p), oow.ctypes.data_as(f32p), xe, ye,
                                          z.ctypes.data_as(f32p)))
     return float(z[0])
+
+
+def selftest_depth_floor_vertices(p, zow, oow, z, w, xe, ye):
+    """The floor as the front end takes it, with the vertices' clip-space z and w."""
+    p = np.ascontiguousarray(p, np.int32)
+    a = [np.ascontiguousarray(x, np.float32) for x in (zow, oow, z, w)]
+    out = np.zeros(1, np.float32)
+    check(lib().swr_selftest_depth_floor_vertices(p.ctypes.data, *(x.ctypes.data_as(f32p) for x in a), xe, ye,
+                                                  out.ctypes.data_as(f32p)))
+    return float(out[0])
 
 
 def copy_device_to_host(dev_ptr, nbytes, out, stream=None):
