@@ -508,7 +508,7 @@ def measure_plain(args, name, world=1, rank=0, local=0, with_e2e=True):
     prof, nprof = r.profile()
     r.set_profiling(False)
     clk = clocks.stop()
-    st2 = r.stats()
+    st2, detail = r.stats(), r.detail()
     # A frame that overflowed its bins is rendered again with grown buffers
     # when its result is read; none may have happened in the timed region.
     if st2.overflow_retries != st.overflow_retries:
@@ -525,6 +525,7 @@ def measure_plain(args, name, world=1, rank=0, local=0, with_e2e=True):
                            "clip_path_fraction": st.triangles_clip_path / max(1, st.triangles_in),
                            "clipped": st.triangles_clipped,
                            "setup_triangles": st.setup_triangles, "bin_pairs": st.bin_pairs,
+                           "unsampled_triangles": detail.unsampled_triangles,
                            "culled_pairs": st.culled_pairs},
            "clocks": clk, "gpu_launches": launches, "kernels_per_frame": launches / steps}
     if with_e2e:
@@ -564,10 +565,15 @@ def measure_plain(args, name, world=1, rank=0, local=0, with_e2e=True):
     # and writes 4-B RGBA8 + 8-B visibility ID per pixel).
     dom = max(("raster", "shade", "frontend"), key=lambda k: prof[k])
     px = W * H
-    # raster: bins read (4 B/pair), raster records read (80 B/emitted triangle),
-    # depth keys written (8 B per pixel of the 64-px tile grid).
-    alg = {"shade": 20.0 * px, "raster": 4.0 * st.bin_pairs + 80.0 * st.setup_triangles + 8.0 * st.tiles * 4096,
-           "frontend": 12.0 * st.triangles_in + 48.0 * 3 * st.triangles_in + 256.0 * st.setup_triangles}[dom]
+    # Triangles that hold no pixel centre have no record and no bin entry.
+    # raster: bins read (4 B/pair), raster records read (80 B each), depth keys
+    # written (8 B per pixel of the 64-px tile grid). front end: indices and
+    # positions of every triangle, the rest of the vertices (16 B of 48 stay
+    # unread without a normal map) and the records (208 B) of recorded ones.
+    records = float(st.setup_triangles - detail.unsampled_triangles)
+    pairs = float(st.bin_pairs - detail.unsampled_pairs)
+    alg = {"shade": 20.0 * px, "raster": 4.0 * pairs + 80.0 * records + 8.0 * st.tiles * 4096,
+           "frontend": (12.0 + 3 * 16) * st.triangles_in + (3 * 16 + 208.0) * records}[dom]
     peak, peak_kind = peaks()
     achieved = alg / (prof[dom] / 1000.0) / 1e9
     traffic, issue = None, None

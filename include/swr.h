@@ -482,6 +482,18 @@ typedef struct swr_frame_stats {
 
 swr_status swr_renderer_get_stats(swr_renderer* r, swr_frame_stats* out);
 
+/* What the last frame left out, and the kernel forms it took. */
+typedef struct swr_frame_detail {
+    uint64_t unsampled_triangles; /* of setup_triangles: hold no pixel centre, so have no record and no bin entry */
+    uint64_t unsampled_pairs;     /* of bin_pairs: theirs */
+    uint32_t raster_threads;      /* threads of the raster's CTAs */
+    uint32_t shade_threads;       /* threads of the shading kernel's CTAs, 0 where the raster shades */
+    uint32_t culling;             /* 1: the raster drops hidden packets */
+    uint32_t reserved;
+} swr_frame_detail;
+
+swr_status swr_renderer_get_frame_detail(swr_renderer* r, swr_frame_detail* out);
+
 /* Per-tile centre luminance of the last frame (tiles_x * tiles_y floats,
  * 64-pixel reference tiles), the auto-exposure meter input
  * (src/tilerasterizer.rs:103-106). */

@@ -38,13 +38,15 @@ def build(force=False):
 
 
 class Opts(C.Structure):
-    _fields_ = [("rsqrt_mode", C.c_uint32), ("threads", C.c_uint32), ("dt", C.c_float), ("ev", C.c_float)]
+    _fields_ = [("rsqrt_mode", C.c_uint32), ("threads", C.c_uint32), ("dt", C.c_float), ("ev", C.c_float),
+                ("counts", C.c_uint32)]
 
 
 class Result(C.Structure):
     _fields_ = [("ev", C.c_float), ("exposure", C.c_float), ("target", C.c_float), ("tiles", C.c_uint32),
                 ("packets", C.c_uint64), ("triangles_in", C.c_uint64), ("quads_tested", C.c_uint64),
-                ("fragments", C.c_uint64), ("depth_passed", C.c_uint64)]
+                ("fragments", C.c_uint64), ("depth_passed", C.c_uint64), ("setup", C.c_uint64),
+                ("pairs", C.c_uint64 * 4), ("unsampled", C.c_uint64), ("unsampled_pairs", C.c_uint64 * 4)]
 
 
 _lib = None
@@ -147,18 +149,18 @@ def camera(position, look_at, fov, width, height, far_plane):
     return cam
 
 
-def render(scene, cam, width, height, rsqrt_mode=swr.RSQRT_AARCH64, threads=1, dt=0.0, ev=1.0):
+def render(scene, cam, width, height, rsqrt_mode=swr.RSQRT_AARCH64, threads=1, dt=0.0, ev=1.0, counts=False):
     """Renders `scene` (an oracle Scene, or a product scene whose scene dict
     the oracle rebuilds) from `cam` (rebuilt by the oracle from the
     parameters it was made with). Returns (rgba8 (H,W) u32, vis (H,W) u64,
-    tile_lum, Result)."""
+    tile_lum, Result). counts: also fill the result's triangle counts."""
     view = scene_of(scene).view
     cam = camera(*cam.args)
     rgba = np.zeros((height, width), np.uint32)
     vis = np.zeros((height, width), np.uint64)
     tl = np.zeros(((width + 63) // 64) * ((height + 63) // 64), np.float32)
     res = Result()
-    o = Opts(rsqrt_mode, threads, dt, ev)
+    o = Opts(rsqrt_mode, threads, dt, ev, 1 if counts else 0)
     rc = lib().oracle_render(C.byref(view), C.byref(cam), width, height, C.byref(o),
                              rgba.ctypes.data_as(C.c_void_p), vis.ctypes.data_as(C.c_void_p),
                              tl.ctypes.data_as(C.c_void_p), C.byref(res))

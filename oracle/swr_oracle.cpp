@@ -1030,6 +1030,7 @@ typedef struct oracle_opts {
     uint32_t threads;     /* 1 = canonical sequential order */
     float dt;
     float ev;             /* exposure state in: log2 of the current exposure (1.0 fresh) */
+    uint32_t counts;      /* 1: fill the last four fields of the result */
 } oracle_opts;
 
 typedef struct oracle_result {
@@ -1042,7 +1043,43 @@ typedef struct oracle_result {
     uint64_t quads_tested;   /* quad coverage tests in fine_raster */
     uint64_t fragments;      /* lanes inside a triangle */
     uint64_t depth_passed;   /* lanes passing the depth test in queue order */
+    /* Opaque triangles with a packet, their (triangle, tile) pairs for tiles
+     * of 8, 16, 32 and 64 px, and those of them that hold no pixel centre by
+     * exact integer edge tests (see count_unsampled) with their pairs. Holds
+     * for scenes without triangles that reach across the whole width. */
+    uint64_t setup;
+    uint64_t pairs[4];
+    uint64_t unsampled;
+    uint64_t unsampled_pairs[4];
 } oracle_result;
+
+// The triangle's bounding box lies inside the screen and holds at most 2x2
+// pixel centres, none of which is inside all three edges, and no term of the
+// tile raster's f32 edge arithmetic on it reaches 2^24.
+static bool holds_no_centre(const orc::Packet& k, int64_t w, int64_t h) {
+    const int64_t x[3] = {k.p[0].x, k.p[1].x, k.p[2].x}, y[3] = {k.p[0].y, k.p[1].y, k.p[2].y};
+    const int64_t lx = std::min({x[0], x[1], x[2]}), hx = std::max({x[0], x[1], x[2]});
+    const int64_t ly = std::min({y[0], y[1], y[2]}), hy = std::max({y[0], y[1], y[2]});
+    if (lx < 0 || ly < 0 || hx > 16 * w || hy > 16 * h) return false;
+    if (2 * ((hy - ly) * (hx + 64) + (hx - lx) * (hy + 64)) + 1 + 256 * (hx - lx + hy - ly) > (1 << 24)) return false;
+    int64_t nx = 0, ny = 0, inside = 0;
+    for (int64_t c = 8; c <= hx; c += 16) nx += c >= lx;
+    for (int64_t c = 8; c <= hy; c += 16) ny += c >= ly;
+    if (nx > 2 || ny > 2) return false;
+    for (int64_t cy = 8; cy <= hy; cy += 16)
+        for (int64_t cx = lx / 16 * 16 - 8; cx <= hx; cx += 16) {
+            if (cx < lx || cy < ly) continue;
+            bool in = true;
+            for (int i = 0; i < 3; ++i) {
+                const int j = (i + 1) % 3;
+                const int64_t a = y[j] - y[i], b = x[i] - x[j];
+                const int64_t top_left = (a < 0 || (a == 0 && b > 0)) ? 0 : -1;
+                in = in && a * (cx - x[i]) + b * (cy - y[i]) + top_left >= 0;
+            }
+            inside += in;
+        }
+    return inside == 0;
+}
 
 // Renderer::render_scene + update_auto_exposure + blit_to_buffer for a fresh
 // Renderer (its vbuffer bary/packet index start at zero). rgba8 (height rows
@@ -1231,6 +1268,28 @@ int oracle_render(const swr_scene_host_view* s, const swr_camera* cam, int32_t w
         res->packets = packets;
         res->triangles_in = tri_in;
         res->quads_tested = res->fragments = res->depth_passed = 0;
+        if (o->counts) {
+            res->setup = res->unsampled = 0;
+            for (int i = 0; i < 4; ++i) res->pairs[i] = res->unsampled_pairs[i] = 0;
+            for (Tile* t : f.tiles)
+                for (size_t i = 0; i < t->opaque.size(); ++i) {
+                    const Packet& k = t->opaque.get(i);
+                    const bool none = holds_no_centre(k, width, height);
+                    // Once per triangle: at the packet that holds its first pixel.
+                    const bool first =
+                        k.min.x == std::max(std::min({k.p[0].x, k.p[1].x, k.p[2].x}), 0) >> 4 &&
+                        k.min.y == std::max(std::min({k.p[0].y, k.p[1].y, k.p[2].y}), 0) >> 4;
+                    res->setup += first;
+                    res->unsampled += first && none;
+                    for (int s = 0; s < 4; ++s) {
+                        const int S = 8 << s;
+                        const uint64_t n = (uint64_t)((k.max.x - 1) / S - k.min.x / S + 1) *
+                                           (uint64_t)((k.max.y - 1) / S - k.min.y / S + 1);
+                        res->pairs[s] += n;
+                        if (none) res->unsampled_pairs[s] += n;
+                    }
+                }
+        }
         for (Tile* t : f.tiles) {
             res->quads_tested += t->quads_tested;
             res->fragments += t->fragments;

@@ -554,7 +554,7 @@ swr_status swr_renderer_get_stats(swr_renderer* r, swr_frame_stats* o) {
     o->triangles_in = c.draw_tris;
     o->triangles_clipped = c.clip_queue;
     o->setup_triangles = c.setup_tris;
-    o->bin_pairs = c.pairs + c.unsampled;
+    o->bin_pairs = c.pairs + (uint32_t)c.unsampled;
     o->bin_capacity = r->eng.bin_cap;
     o->tiles = r->tiles_x * r->tiles_y;
     o->overflow_retries = r->eng.retries;
@@ -564,6 +564,22 @@ swr_status swr_renderer_get_stats(swr_renderer* r, swr_frame_stats* o) {
     o->culled_pairs = c.culled;
     o->kernel_launches = r->eng.kernel_launches;
     o->triangles_clip_path = c.clip_path;
+    return SWR_OK;
+}
+
+swr_status swr_renderer_get_frame_detail(swr_renderer* r, swr_frame_detail* o) {
+    if (!r || !o) return fail(SWR_INVALID_ARG, "null argument");
+    swr_status st = check_frame(r);
+    if (st != SWR_OK) return st;
+    std::memset(o, 0, sizeof(*o));
+    if (!r->have_frame) return SWR_OK;
+    const DCounters& c = r->eng.last;
+    const FrameArgs& a = r->last_args;
+    o->unsampled_triangles = c.unsampled >> 32;
+    o->unsampled_pairs = (uint32_t)c.unsampled;
+    o->raster_threads = raster_threads(a);
+    o->shade_threads = shade_threads(a);
+    o->culling = a.sched_tile >= 32u || a.cull16 ? 1u : 0u;
     return SWR_OK;
 }
 

@@ -269,7 +269,7 @@ struct alignas(16) DCounters {
     uint32_t status;
     uint32_t clip_queue;       // triangles queued for clipping
     uint32_t extra_used;       // extra record slots taken by fans 1..6
-    uint32_t setup_tris;       // records written
+    uint32_t setup_tris;       // triangles that touch a tile (records written, and unsampled ones)
     unsigned long long pairs;  // (triangle, tile) pairs counted
     uint32_t work_next;        // persistent raster work cursor
     uint32_t trans_next;       // translucent pass work cursor
@@ -281,8 +281,10 @@ struct alignas(16) DCounters {
     uint32_t culled;           // (triangle, tile) pairs the raster dropped as hidden
     uint32_t clip_path;        // triangles of draws whose sphere intersects the frustum (the clip path)
     uint32_t ref_pairs;        // (triangle, 64-px tile) pairs of a frame with a pair limit
-    uint32_t unsampled;        // (triangle, tile) pairs of triangles that hold no pixel centre (not binned)
     uint32_t scan_done;        // k_scan's CTAs done
+    // Triangles that hold no pixel centre (no record, not binned), their
+    // number in the high half and their (triangle, tile) pairs in the low one.
+    unsigned long long unsampled;
     uint32_t filled;           // scheduling tiles with opaque packets, first in the visiting order
     uint32_t bucket[kOrderBuckets];  // opaque bins per size bucket; then the next place in the visiting order
     uint32_t wide_main;        // wide-queue segments appended by k_frontend
@@ -390,5 +392,9 @@ cudaError_t init_kernel_constants();
 void frame_grids(int num_sms, uint32_t sched_tile, bool fuse32, bool narrow, uint32_t* raster_grid, uint32_t* shade_grid);
 // Whether frames with this scheduling tile shade inside the raster kernel.
 bool shade_fused(uint32_t sched_tile, bool fuse32);
+// Threads of the CTAs that a frame's raster and shading kernels take (shading
+// inside the raster: 0).
+uint32_t raster_threads(const FrameArgs& a);
+uint32_t shade_threads(const FrameArgs& a);
 
 }  // namespace swr

@@ -393,6 +393,15 @@ __device__ __forceinline__ void warp_sum(uint32_t* counter, uint32_t v) {
     if ((int)(threadIdx.x & 31u) == __ffs(active) - 1 && s) atomicAdd(counter, s);
 }
 
+// One atomic per warp: counts the active lanes' unsampled triangles and their
+// tiles (none: 0; at most four, since such a box is under 64 subpixels wide).
+__device__ __forceinline__ void warp_unsampled(unsigned long long* counter, uint32_t tiles) {
+    const uint32_t active = __activemask();
+    const uint32_t s = __reduce_add_sync(active, tiles ? (1u << 16) | tiles : 0u);
+    if ((int)(threadIdx.x & 31u) == __ffs(active) - 1 && s)
+        atomicAdd(counter, ((unsigned long long)(s >> 16) << 32) | (s & 0xFFFFu));
+}
+
 // Warp-aggregated atomicAdd of 1 on counter[idx].
 __device__ __forceinline__ void agg_inc(uint32_t* counter, uint32_t idx) {
     const uint32_t active = __activemask();
@@ -865,7 +874,7 @@ __global__ void __launch_bounds__(256) k_reset(FrameArgs a) {
         a.counters->culled = 0u;
         a.counters->clip_path = 0u;
         a.counters->ref_pairs = 0u;
-        a.counters->unsampled = 0u;
+        a.counters->unsampled = 0ull;
         a.counters->scan_done = 0u;
         a.counters->wide_main = 0u;
         a.counters->wide_clip = 0u;
@@ -971,7 +980,7 @@ __device__ __forceinline__ void frontend_triangle(const FrameArgs& a, uint32_t p
     }
     a.tri_state[g] = res == kSetupRecord ? 1 : 0;
     warp_count(&a.counters->setup_tris, res != kSetupNone);
-    warp_sum(&a.counters->unsampled, res == kSetupUnsampled ? t.tiles.count() : 0u);
+    warp_unsampled(&a.counters->unsampled, res == kSetupUnsampled ? t.tiles.count() : 0u);
     if (a.pair_limit) warp_sum(&a.counters->ref_pairs, pairs64);
 }
 
@@ -1143,7 +1152,7 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(FrameArgs a) {
             ok = res == kSetupRecord;
             if (res == kSetupUnsampled) {
                 atomicAdd(&a.counters->setup_tris, 1u);
-                atomicAdd(&a.counters->unsampled, tiles.count());
+                atomicAdd(&a.counters->unsampled, (1ull << 32) | tiles.count());
             }
             if (ok) {
                 const Vtx &v0 = pl[0], &v1 = pl[i + 1], &v2 = pl[i + 2];
@@ -2925,6 +2934,14 @@ static int raster_blocks_per_sm() {
 }
 
 bool shade_fused(uint32_t S, bool fuse32) { return S <= kFusedShadeMaxTile || (S == 32 && fuse32); }
+uint32_t raster_threads(const FrameArgs& a) {
+    const bool narrow = a.sched_tile == 32u && !a.fused_shade && a.narrow_raster;
+    return a.sched_tile <= 16u || narrow ? 128u : 256u;
+}
+uint32_t shade_threads(const FrameArgs& a) {
+    if (shade_fused(a.sched_tile, a.fused_shade != 0)) return 0u;
+    return a.wide_shade && !a.has_gi ? kShadeWide : kShadeThreads;
+}
 
 void frame_grids(int num_sms, uint32_t S, bool fuse32, bool narrow, uint32_t* raster_grid, uint32_t* shade_grid) {
     int rb = 1, sb = 1;
@@ -3006,7 +3023,7 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
             break;
         case 32:
             if (a.fused_shade) launch_fused<32>(a, rg, s);
-            else if (a.narrow_raster) launch_raster<32, false, false, kModeAny, 128>(a, rg, s);
+            else if (raster_threads(a) == 128u) launch_raster<32, false, false, kModeAny, 128>(a, rg, s);
             else launch_raster<32, false, false, kModeAny>(a, rg, s);
             break;
         default: launch_raster<64, false, false, kModeAny>(a, rg, s); break;
@@ -3030,7 +3047,7 @@ uint32_t launch_frame(const FrameArgs& a, void* stream, int num_sms, cudaEvent_t
             else launch_kernel(k_shade<true, kModeAny>, sg, T, 0, a, s);
         } else {
             const bool arm = a.rsqrt_uniform == 1u + kModeArm, ieee = a.rsqrt_uniform == 1u + kModeIeee;
-            if (a.wide_shade) {
+            if (shade_threads(a) == kShadeWide) {
                 const uint32_t sg = (uint32_t)num_sms, T = kShadeWide;
                 if (arm) launch_kernel(k_shade<false, kModeArm, kShadeWide>, sg, T, 0, a, s);
                 else if (ieee) launch_kernel(k_shade<false, kModeIeee, kShadeWide>, sg, T, 0, a, s);

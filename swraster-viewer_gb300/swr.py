@@ -147,6 +147,11 @@ class FrameStats(C.Structure):
                 ("kernel_launches", C.c_uint64), ("triangles_clip_path", C.c_uint64)]
 
 
+class FrameDetail(C.Structure):
+    _fields_ = [("unsampled_triangles", C.c_uint64), ("unsampled_pairs", C.c_uint64), ("raster_threads", C.c_uint32),
+                ("shade_threads", C.c_uint32), ("culling", C.c_uint32), ("reserved", C.c_uint32)]
+
+
 class BatchTuning(C.Structure):
     _fields_ = [("batch_class", C.c_uint32), ("tuned", C.c_uint32), ("sched_tile", C.c_uint32),
                 ("fused_shade", C.c_uint32), ("raster_ctas_per_sm", C.c_uint32), ("reserved", C.c_uint32),
@@ -190,7 +195,7 @@ EXPORTS = [
     "swr_camera_update", "swr_renderer_create", "swr_renderer_destroy", "swr_render_frame", "swr_renderer_sync",
     "swr_blit", "swr_renderer_set_blit_target", "swr_read_visbuffer", "swr_renderer_device_outputs", "swr_renderer_get_exposure",
     "swr_renderer_set_exposure", "swr_renderer_get_stats", "swr_renderer_get_tile_luminance", "swr_last_error",
-    "swr_selftest_depth_floor_vertices",
+    "swr_renderer_get_frame_detail", "swr_selftest_depth_floor_vertices",
     "swr_abi_version", "swr_renderer_set_profiling", "swr_renderer_get_profile", "swr_render_frame_noalloc",
     "swr_batch_create", "swr_batch_destroy", "swr_batch_render", "swr_batch_sync", "swr_batch_output",
     "swr_batch_autotune", "swr_batch_last_ms", "swr_batch_get_tuning", "swr_server_create", "swr_server_destroy", "swr_server_add_scene",
@@ -230,6 +235,7 @@ def lib():
         "swr_renderer_get_exposure": ([vp, f32p], C.c_int),
         "swr_renderer_set_exposure": ([vp, C.c_float], C.c_int),
         "swr_renderer_get_stats": ([vp, C.POINTER(FrameStats)], C.c_int),
+        "swr_renderer_get_frame_detail": ([vp, C.POINTER(FrameDetail)], C.c_int),
         "swr_renderer_get_tile_luminance": ([vp, f32p, C.c_uint32], C.c_int),
         "swr_renderer_set_profiling": ([vp, C.c_int32], C.c_int),
         "swr_renderer_get_profile": ([vp, f32p, C.c_int32, C.POINTER(C.c_uint32)], C.c_int),
@@ -498,6 +504,11 @@ class Renderer:
         s = FrameStats()
         check(lib().swr_renderer_get_stats(self.handle, C.byref(s)))
         return s
+
+    def detail(self):
+        d = FrameDetail()
+        check(lib().swr_renderer_get_frame_detail(self.handle, C.byref(d)))
+        return d
 
     def tile_luminance(self):
         tx = (self.width + 63) // 64
