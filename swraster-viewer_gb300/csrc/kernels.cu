@@ -1558,8 +1558,8 @@ __device__ __forceinline__ void load_shade_const(ShadeConst& c, const FrameArgs&
 // and 256 views' small frames: a heavy tile of a small frame is one CTA's
 // latency), but 32-px tiles shaded apart 128 where there are many tiles per
 // SM: less of the CTA waits at each round's barriers (64 views, 32-px raster
-// 479 -> 411 us, eight scenes 424 -> 368, 1080p 138 -> 135; 1367x769 with 7
-// tiles an SM 67 -> 103).
+// 479 -> 411 us, eight scenes 424 -> 368; with few tiles the heaviest ones take
+// longer, 1367x769 67 -> 103; see FrameEngine::kNarrowTiles).
 template <int S, int T = (S <= 16 ? 128 : 256)>
 struct RasterShared {
     static constexpr int kThreads = T;

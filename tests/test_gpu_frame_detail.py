@@ -11,6 +11,7 @@ import pytest
 import oracle
 import scenes
 import swr
+from test_gpu_parity import tie_across_rounds_scene
 from test_gpu_unsampled import specks_scene
 
 pytestmark = pytest.mark.gpu
@@ -48,6 +49,36 @@ def frame(s, w, h, tile):
     return out
 
 
+@pytest.mark.parametrize("below", [0, 1])
+def test_crowded_tiles_take_the_narrow_raster(below):
+    """12 tiles of 32 px per SM: the raster's CTAs are narrow from 256 triangles a tile on."""
+    n = sms()
+    count = -(-256 * 12 * n // 20480) - below
+    s = swr.Scene(scenes.spheres_scene(seed=8, count=count, subdiv=5, tex_size=16, cube_size=16, voxel=16))
+    rgba, vis, d = frame(s, 64 * n - 3, 64 * 3 - 1, 32)
+    assert d.raster_threads == (256 if below else 128)
+    want_rgba, want_vis, _ = frame(s, 64 * n - 3, 64 * 3 - 1, 8)
+    assert np.array_equal(vis, want_vis) and np.array_equal(rgba[:190], want_rgba[:190])
+    s.close()
+
+
+@pytest.mark.parametrize("extra", [-1, 1])
+def test_culling_with_many_32px_tiles(extra):
+    """24 tiles a view, on both sides of the number of tiles from which the raster's CTAs are narrow; bins of several
+    rounds of either width, with a tie that the last of the tied triangles wins."""
+    s = swr.Scene(tie_across_rounds_scene(300))
+    w, h = 190, 127
+    cam = swr.make_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 1.0, w, h, 40.0)
+    _, ovis, _, _ = oracle.render(s, cam, w, h, rsqrt_mode=swr.RSQRT_AARCH64, threads=1)
+    views = 56 * sms() // 24 + extra
+    b = swr.Batch(sched_tile=32)
+    b.render(swr.Batch.views([(s, cam, w, h, 2.0, swr.RSQRT_AARCH64)] * views))
+    for i in range(views):
+        assert np.array_equal(b.output(i, w, h)[1], ovis), i
+    b.close()
+    s.close()
+
+
 @pytest.fixture(scope="module")
 def spheres():
     s = swr.Scene(scenes.spheres_scene(seed=8, count=20, subdiv=3, tex_size=16, cube_size=16, voxel=16))  # 25,600
@@ -59,7 +90,8 @@ def spheres():
 def forms(n):
     return {"wide shading below": ((n - 1) // 8, 8, 64, "shade_threads", 128),
             "wide shading": (-(-n // 8), 8, 64, "shade_threads", 1024),
-            "narrow raster below": (n - 1, 3, 32, "raster_threads", 256), "narrow raster": (n, 3, 32, "raster_threads", 128),
+            "narrow raster below": (n - 1, 14, 32, "raster_threads", 256),
+            "narrow raster": (n, 14, 32, "raster_threads", 128),
             "16-px culling below": (13, 2, 16, "culling", 0), "16-px culling": (5, 5, 16, "culling", 1)}
 
 
