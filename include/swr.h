@@ -527,7 +527,7 @@ typedef struct swr_view_desc {
 
 typedef struct swr_batch_opts {
     uint32_t sched_tile;        /* 8, 16, 32, 64; 0 = autotuned choice for the batch's class, else chosen
-                                   from the view sizes (several views: at most 32 px, shaded apart) */
+                                   from the views (several: at most 32 px, small ones with fused shading) */
     uint32_t use_graph;         /* replay the frame as a CUDA graph */
     uint64_t bin_capacity;      /* initial pair capacity, 0 = auto */
     uint32_t flags;             /* SWR_BATCH_* */
@@ -590,7 +590,8 @@ typedef struct swr_server_opts {
     uint32_t max_batch_views;   /* views per batch (default 64) */
     uint32_t max_queue;         /* pending requests before submit returns SWR_BUSY (default 4096) */
     uint32_t inflight;          /* batches in flight on separate streams (default 2) */
-    uint32_t sched_tile;        /* 0 = chosen per batch (several views: at most 32 px, shaded apart) */
+    uint32_t sched_tile;        /* 0 = chosen per batch (several views: at most 32 px, small ones with fused
+                                   shading) */
     uint32_t rsqrt_mode;
     uint32_t use_graph;
     uint32_t flags;             /* SWR_BATCH_* for every batch (SWR_BATCH_FUSED_SHADE) */

@@ -169,14 +169,28 @@ uint32_t BatchImpl::tuned_tile(const swr_view_desc* vd, int32_t n) const {
         h[(size_t)i] = vd[i].height;
     }
     const uint32_t S = auto_sched_tile(w.data(), h.data(), n, eng.num_sms);
+    if (n == 1 || S < 32u) return S;
     // Several views: at most 32-px tiles, which balance better over the
     // persistent CTAs where views and tiles are uneven. Shaded apart they take
     // 2,364 us for 64 views of one scene, 1,374 for eight uneven scenes and
     // 1,093 for a burst of 24 requests, fused into the raster kernel (the
     // autotuner's other form) 2,631, 1,504 and 1,083; 64-px tiles took 2,377,
     // 1,340 and 1,359 (before tiles without packets were left out).
-    if (n > 1 && S >= 32u) return 32u;
-    return S;
+    // Views of at most kSmallView 64-px tiles are shaded in the raster: a
+    // shading CTA's next pixels are then another view's each time, and it
+    // fetches that view's constants for them. us apart and fused, 30k triangles
+    // of all sizes and 82k of spheres: 96 views of 320x240 469 and 358, 1,150
+    // and 1,113; 64 of 480x360 482 and 400, 1,191 and 1,131; 64 of 560x420 567
+    // and 498, 1,290 and 1,340; 40 of 640x480 447 and 408, 994 and 1,042. With
+    // kCrowded triangles to a 32-px tile and more, apart: 400k in 96 views of
+    // 320x240 1,747 and 1,844, in 64 of 480x360 1,735 and 1,891.
+    constexpr uint64_t kSmallView = 48, kCrowded = 2000;
+    uint64_t tiles = 0, tris = 0;
+    for (int32_t i = 0; i < n; ++i) {
+        tiles += (uint64_t)((vd[i].width + kRefTile - 1) / kRefTile) * (uint64_t)((vd[i].height + kRefTile - 1) / kRefTile);
+        tris += vd[i].scene->impl.tri_total;
+    }
+    return tiles <= kSmallView * (uint64_t)n && tris < kCrowded * 4u * tiles ? 32u | 0x100u : 32u;
 }
 
 }  // namespace swr
