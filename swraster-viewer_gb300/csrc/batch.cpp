@@ -178,19 +178,21 @@ uint32_t BatchImpl::tuned_tile(const swr_view_desc* vd, int32_t n) const {
     // 1,340 and 1,359 (before tiles without packets were left out).
     // Views of at most kSmallView 64-px tiles are shaded in the raster: a
     // shading CTA's next pixels are then another view's each time, and it
-    // fetches that view's constants for them. us apart and fused, 30k triangles
-    // of all sizes and 82k of spheres: 96 views of 320x240 469 and 358, 1,150
-    // and 1,113; 64 of 480x360 482 and 400, 1,191 and 1,131; 64 of 560x420 567
-    // and 498, 1,290 and 1,340; 40 of 640x480 447 and 408, 994 and 1,042. With
-    // kCrowded triangles to a 32-px tile and more, apart: 400k in 96 views of
-    // 320x240 1,747 and 1,844, in 64 of 480x360 1,735 and 1,891.
-    constexpr uint64_t kSmallView = 48, kCrowded = 2000;
+    // fetches that view's constants for them. us apart and fused, a scene of 30k
+    // triangles in 96 views of 320x240 486 and 358, in 64 of 480x360 502 and
+    // 400, in 40 of 640x480 470 and 408; spheres of 20k 577 and 451, 679 and 508,
+    // 546 and 491; 60k triangles with every texture slot, 96 views of 320x240 and
+    // 32 of 480x360, 679 and 517, 399 and 298. Pictures filled by 20k triangles
+    // lose, 30 views of each size 455 and 478, 686 and 717, 861 and 994. From
+    // kLargeScene triangles a view on they are shaded apart: 400k 1,747 and
+    // 1,844, 1,735 and 1,891.
+    constexpr uint64_t kSmallView = 48, kLargeScene = 100000;
     uint64_t tiles = 0, tris = 0;
     for (int32_t i = 0; i < n; ++i) {
         tiles += (uint64_t)((vd[i].width + kRefTile - 1) / kRefTile) * (uint64_t)((vd[i].height + kRefTile - 1) / kRefTile);
         tris += vd[i].scene->impl.tri_total;
     }
-    return tiles <= kSmallView * (uint64_t)n && tris < kCrowded * 4u * tiles ? 32u | 0x100u : 32u;
+    return tiles <= kSmallView * (uint64_t)n && tris < kLargeScene * (uint64_t)n ? 32u | 0x100u : 32u;
 }
 
 }  // namespace swr

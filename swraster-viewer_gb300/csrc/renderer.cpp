@@ -334,7 +334,7 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     const bool fused32 = fuse32 && sched_tile == 32;
     const bool crowded = tri_bound >= kCrowdedTris * stile_cursor;
     const bool narrow = sched_tile == 32 && !fused32 && !raster_cta_cap &&
-                        stile_cursor >= (crowded ? kNarrowCrowded : kNarrowTiles) * (uint32_t)num_sms;
+                        stile_cursor >= (crowded || shares_device ? kNarrowLow : kNarrowTiles) * (uint32_t)num_sms;
     if (grid_tile != sched_tile || grid_fused32 != fused32 || grid_narrow != narrow || grid_cap != raster_cta_cap) {
         frame_grids(num_sms, sched_tile, fused32, narrow, &raster_grid, &shade_grid);
         if (raster_cta_cap) raster_grid = std::min<uint32_t>(raster_grid, (uint32_t)num_sms * raster_cta_cap);

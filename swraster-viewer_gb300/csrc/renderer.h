@@ -98,20 +98,24 @@ struct FrameEngine {
     bool fuse32 = false;        // 32-px tiles shade inside the raster kernel (batch autotuner's choice)
     bool grid_fused32 = false, grid_narrow = false;
     // 32-px tiles shaded apart are rasterized by CTAs of 128 threads, not 256,
-    // from kNarrowTiles tiles per SM on, and from kNarrowCrowded on where
+    // from kNarrowTiles tiles per SM on, and from kNarrowLow on where
     // kCrowdedTris triangles (of the scenes, drawn or not) come to a tile. With
     // few tiles the kernel waits for the heaviest ones, and those take the narrow
-    // CTAs longer. us of a frame or batch with 256 -> 128 threads at so many tiles
-    // an SM: spheres of 82k triangles 12: 155 -> 177, 24: 166 -> 180, 38: 344 ->
-    // 355, 54: 382 -> 378, 76: 591 -> 579, 126: 930 -> 910, 358: 2,399 -> 2,327;
-    // of 307k 13: 190 -> 228, 54: 430 -> 450, 76: 762 -> 749; frames filled by
-    // 400k triangles of all sizes 13: 381 -> 379, 24: 478 -> 457, 54: 715 -> 679,
-    // 126: 1,712 -> 1,617. Where tiles are crowded it depends on the picture:
-    // filled ones gain (700k triangles at 1920x1080 459 -> 442, 1.5M 584 -> 549,
-    // 2M at 2560x1440 811 -> 741), spheres before a sky lose (1.2M at 1920x1080
-    // 250 -> 288). A capped CTA count keeps 256.
-    static constexpr uint32_t kNarrowTiles = 56, kNarrowCrowded = 12;
-    static constexpr uint64_t kCrowdedTris = 256;
+    // CTAs longer; with many, less of a CTA waits at each round's barriers. us of
+    // a frame or batch with 256 -> 128 threads at so many tiles an SM: spheres of
+    // 82k triangles before a sky 12: 155 -> 177, 24: 166 -> 180, 38: 344 -> 355,
+    // 54: 382 -> 378, 126: 930 -> 910, 358: 2,399 -> 2,327; of 307k 12: 202 ->
+    // 243, 54: 430 -> 450, 126: 1,231 -> 1,207; pictures filled by 400k triangles
+    // 13: 381 -> 379, 24: 478 -> 457, 54: 715 -> 679, 126: 1,712 -> 1,617. With
+    // 128 below 44 some light ones were slower than they had been before these
+    // CTAs and that culling (30k triangles in twelve views of 640x480, 25: 198,
+    // 194 with 256 and 206 with 128). Crowded tiles, 256 -> 128:
+    // filled pictures of 1920x1080 gain (700k triangles 459 -> 442, 1.5M 584 ->
+    // 549), spheres lose (1.2M 250 -> 288). The server's batches, beside which
+    // others run, take the lower line (a burst of six frames of 54k triangles 322
+    // -> 307). A capped CTA count keeps 256.
+    static constexpr uint32_t kNarrowTiles = 44, kNarrowLow = 12;
+    static constexpr uint64_t kCrowdedTris = 176;
     // Triangles (of the scenes, drawn or not) per tile from which 16-px tiles
     // are culled. Device time of a frame without -> with culling: 1.5M at
     // 640x400 (938 a tile) 739 -> 407 us, 1M at 1280x720 (260) 531 -> 411,

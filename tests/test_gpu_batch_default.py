@@ -1,6 +1,6 @@
 """The form a batch of several views takes by itself: 32-px tiles shaded in the
-raster kernel for small views, shaded apart for larger ones and where many
-triangles come to a tile; 16-px tiles for few. Either form gives the frames of
+raster kernel for small views, shaded apart for larger ones and for scenes of
+many triangles; 16-px tiles for few. Either form gives the frames of
 a renderer."""
 import numpy as np
 import pytest
@@ -14,16 +14,17 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture(scope="module")
 def made():
     s = {"light": swr.Scene(scenes.small_scene(seed=4)),  # 1,920 triangles
-         "heavy": swr.Scene(scenes.spheres_scene(seed=4, count=5, subdiv=6, tex_size=16, cube_size=16, voxel=16))}
+         "heavy": swr.Scene(scenes.spheres_scene(seed=4, count=79, subdiv=3, tex_size=16, cube_size=16, voxel=16)),
+         "below": swr.Scene(scenes.spheres_scene(seed=4, count=78, subdiv=3, tex_size=16, cube_size=16, voxel=16))}
     yield s
     for x in s.values():
         x.close()
 
 
 # Scene, size and number of views; tile and form. 48 tiles of 64 px a view is
-# 8x6; 409,600 triangles are 2,133 to a 32-px tile there and 1,463 with 10x7.
+# 8x6; the scenes have 1,920, 101,120 and 99,840 triangles.
 CASES = [("light", 512, 384, 40, 32, 1), ("light", 513, 384, 40, 32, 0), ("light", 320, 240, 100, 32, 1),
-         ("heavy", 512, 384, 40, 32, 0), ("heavy", 640, 448, 30, 32, 0), ("light", 512, 384, 2, 16, 0),
+         ("heavy", 512, 384, 40, 32, 0), ("below", 512, 384, 40, 32, 1), ("light", 512, 384, 2, 16, 0),
          ("light", 1920, 1080, 2, 32, 0)]
 
 

@@ -51,9 +51,9 @@ def frame(s, w, h, tile):
 
 @pytest.mark.parametrize("below", [0, 1])
 def test_crowded_tiles_take_the_narrow_raster(below):
-    """12 tiles of 32 px per SM: the raster's CTAs are narrow from 256 triangles a tile on."""
+    """12 tiles of 32 px per SM: the raster's CTAs are narrow from 176 triangles a tile on."""
     n = sms()
-    count = -(-256 * 12 * n // 20480) - below
+    count = -(-176 * 12 * n // 20480) - below
     s = swr.Scene(scenes.spheres_scene(seed=8, count=count, subdiv=5, tex_size=16, cube_size=16, voxel=16))
     rgba, vis, d = frame(s, 64 * n - 3, 64 * 3 - 1, 32)
     assert d.raster_threads == (256 if below else 128)
@@ -70,7 +70,7 @@ def test_culling_with_many_32px_tiles(extra):
     w, h = 190, 127
     cam = swr.make_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 1.0, w, h, 40.0)
     _, ovis, _, _ = oracle.render(s, cam, w, h, rsqrt_mode=swr.RSQRT_AARCH64, threads=1)
-    views = 56 * sms() // 24 + extra
+    views = 44 * sms() // 24 + extra
     b = swr.Batch(sched_tile=32)
     b.render(swr.Batch.views([(s, cam, w, h, 2.0, swr.RSQRT_AARCH64)] * views))
     for i in range(views):
@@ -90,8 +90,8 @@ def spheres():
 def forms(n):
     return {"wide shading below": ((n - 1) // 8, 8, 64, "shade_threads", 128),
             "wide shading": (-(-n // 8), 8, 64, "shade_threads", 1024),
-            "narrow raster below": (n - 1, 14, 32, "raster_threads", 256),
-            "narrow raster": (n, 14, 32, "raster_threads", 128),
+            "narrow raster below": (n - 1, 11, 32, "raster_threads", 256),
+            "narrow raster": (n, 11, 32, "raster_threads", 128),
             "16-px culling below": (13, 2, 16, "culling", 0), "16-px culling": (5, 5, 16, "culling", 1)}
 
 
