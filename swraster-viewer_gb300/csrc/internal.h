@@ -10,8 +10,9 @@
 //
 // Per frame (renderer-owned):
 //   draws      DDraw[D]     (node, primitive) pairs in canonical order, + MVP
-//   chunks     DChunk[]     256-triangle slices of draws, one CTA each
-//   tri_state  u8[T]        0 none, 1 record in slot g, 2 clipped
+//   chunks     DChunk[]     256-triangle slices of draws, two front-end CTAs each
+//   tri_state  u8[T]        0 none, 1 record in slot g, 2 queued for the clipper, 3 clipped away or to fans without a
+//                           first
 //   rec_r      RecRaster[T + extra]   80 B: screen vertices, bbox, z/w, 1/w, depth floor
 //   rec_s      RecShade [T + extra]  128 B: shading interpolators
 //   rec_t      RecTangent[T + extra]  48 B: tangents, written under a normal map only
@@ -30,7 +31,7 @@ namespace swr {
 constexpr int kRefTile = 64;          // reference tile size, src/renderer.rs:14
 constexpr int kSubpixelScale = 16;    // src/tilerasterizer.rs:10
 constexpr int kSubpixelShift = 4;
-constexpr int kChunkTris = 256;       // triangles per front-end CTA
+constexpr int kChunkTris = 256;       // triangles per chunk
 constexpr uint64_t kEmptyKey = 0xFF800000FFFFFFFFull;  // orderable(+inf) << 32 | 0xFFFFFFFF
 
 struct alignas(16) DVertex {
@@ -361,7 +362,7 @@ struct FrameArgs {
     uint32_t has_gi;           // some scene of the frame has a baked voxel grid
     uint32_t gpu_draws;        // build draws and chunks on the device (else the host staged them)
     // Kernels are launched to overlap their predecessor's end: for small frames
-    // launched directly (the allocation-free frame, 96 -> 87 us). Replayed
+    // launched directly (the allocation-free frame, 93 -> 81 us). Replayed
     // graphs gain nothing (1280x720 124 -> 126) and frames of large kernels lose
     // (4K 1062 -> 1088: the next kernel's waiting CTAs take up places).
     uint32_t overlap;

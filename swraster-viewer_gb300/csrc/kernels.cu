@@ -41,16 +41,17 @@
 #include "devmath.cuh"
 #include "internal.h"
 
-// Raster: prefetch into L2 the record each thread will likely load in the next round.
 // Shading fused into the raster kernel (k_raster<S, true>): each CTA shades
 // its tile from the depth keys in shared memory right after rasterizing it,
 // so raster and shading work of different tiles share the SMs and keys reach
 // HBM only for the translucent pass. Always for tiles of 8 and 16 px, on
-// request (FrameArgs.fused_shade, chosen by the batch autotuner) for 32;
+// request (FrameArgs.fused_shade: batches of small views, or the batch
+// autotuner's choice) for 32;
 // 64-px tiles keep the separate shading kernel (fused, a 4K frame was 18%
 // slower: the two code bodies share the instruction cache and the shading
 // part spills).
 constexpr uint32_t kFusedShadeMaxTile = 16;
+// Raster: prefetch into L2 the record each thread will likely load in the next round.
 #ifndef SWR_RASTER_PREFETCH
 #define SWR_RASTER_PREFETCH 1
 #endif
@@ -1772,12 +1773,6 @@ __device__ __forceinline__ uint32_t cells_far(const RasterShared<S, T>& s, int32
     return far;
 }
 
-// Orderable depth floor of the packet (its triangle's, taken by the front
-// end); 0 (below every key) when none is taken. A packet is hidden when its
-// floor is above the farthest depth of every cell its covered lanes can fall
-// in: pixels [x0 & ~1, x1] of its clipped rect.
-__device__ __forceinline__ uint32_t packet_floor(const PacketCtx& c) { return c.r.zfloor; }
-
 // Pass 1 of a round for one packet: classify and split into regions, and
 // either count them (regions, quads; the accepted 16-px blocks of a coarse
 // packet go to bmask) or stage them from the given positions (bmask as the
@@ -1940,9 +1935,13 @@ __global__ void __launch_bounds__(T, RasterShared<S, T>::kMinBlocks) k_raster(Fr
                 }
 #endif
                 if (cull && cells_valid) {
+                    // Hidden when the triangle's depth floor (0, below every
+                    // key, where the front end took none) is above the farthest
+                    // depth of every cell the packet's covered lanes can fall
+                    // in: pixels [x0 & ~1, x1] of its clipped rect.
                     const uint32_t far = cells_far<S>(s, c.xs >> kSubpixelShift, c.xe >> kSubpixelShift,
                                                       c.ys >> kSubpixelShift, c.ye >> kSubpixelShift, sx0, sy0);
-                    hidden = far < 0xFF800000u && packet_floor(c) > far;
+                    hidden = far < 0xFF800000u && c.r.zfloor > far;
                 }
                 if (!hidden) packet_regions<S>(s, c, sx0, sy0, false, threadIdx.x, n_r, n_q, bmask);
             }
@@ -2894,9 +2893,12 @@ template <int S, bool FUSE, bool GI, int MODE, int T = RasterShared<S>::kThreads
 static void launch_raster(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
     launch_kernel(k_raster<S, FUSE, GI, MODE, T, CULL>, grid, T, sizeof(RasterSmem<S, FUSE, T>), a, s);
 }
-// The fused shading compiled for what the frame needs: the variant for baked
-// grids of any rsqrt mode spills 250-450 B a thread against 0-130 B, and
-// every fused frame ran it (64 batched views 5% slower, 1280x720 2%).
+// The fused shading compiled for what the frame needs: the variants for baked
+// grids spill 156-328 B a thread against 84-244 B without, and every fused
+// frame ran one of them (64 batched views 5% slower, 1280x720 2%). Of that the
+// mode's part is small: the Arm variants against those of any mode take 0 to 2%
+// less (600k triangles at 1280x720 363 and 367 us, sixteen views of 300k 513 and
+// 523, spheres and baked grids within 0.6%).
 template <int S, bool CULL = (S >= 32)>
 static void launch_fused(const FrameArgs& a, uint32_t grid, cudaStream_t s) {
     const bool arm = a.rsqrt_uniform == 1u + kModeArm;
