@@ -279,17 +279,11 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     const size_t slots = (size_t)tri_cap + extra_cap;
     chk(tables.ensure(lay.total));
     chk(tri_state.ensure(tri_cap));
-    chk(rec_r.ensure(slots * sizeof(RecRaster)));
-    chk(rec_s.ensure(slots * sizeof(RecShade)));
-    chk(rec_t.ensure(slots * sizeof(RecTangent)));
+    chk(records.ensure(slots * (sizeof(RecShade) + sizeof(RecRaster) + sizeof(RecTangent))));
     chk(fan_base.ensure((size_t)tri_cap * sizeof(uint32_t)));
     chk(clip_queue.ensure((size_t)tri_cap * sizeof(uint2)));
-    chk(wide_queue.ensure(2u * kWideCap * sizeof(uint2)));
-    chk(tile_count.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
-    chk(tile_offset.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
-    chk(tile_cursor.ensure((size_t)(stile_cap + 1) * sizeof(uint32_t)));
-    chk(sky_tab.ensure((size_t)view_cap * 256));
-    chk(work.ensure((size_t)(stile_cap / 2 + 1) * sizeof(uint4)));
+    const TileLayout tl(stile_cap, view_cap);
+    chk(tile_block.ensure(tl.total));
     chk(bins.ensure(bin_cap * sizeof(uint32_t)));
     chk(keys.ensure(std::max<uint64_t>(1, key_cap) * sizeof(unsigned long long)));
     if (color_floats > 0) chk(color.ensure(color_floats * sizeof(float)));
@@ -372,18 +366,19 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
     a.bin_cap = bin_cap;
     a.sched_tile = sched_tile;
     a.tri_state = tri_state.as<uint8_t>();
-    a.rec_r = rec_r.as<RecRaster>();
-    a.rec_s = rec_s.as<RecShade>();
-    a.rec_t = rec_t.as<RecTangent>();
+    a.rec_s = records.as<RecShade>();
+    a.rec_r = reinterpret_cast<RecRaster*>(a.rec_s + slots);
+    a.rec_t = reinterpret_cast<RecTangent*>(a.rec_r + slots);
     a.fan_base = fan_base.as<uint32_t>();
     a.clip_queue = clip_queue.as<uint2>();
-    a.wide_queue = wide_queue.as<uint2>();
+    uint8_t* tiles = static_cast<uint8_t*>(tile_block.p);
+    a.wide_queue = reinterpret_cast<uint2*>(tiles + tl.o_wide);
     a.wide_cap = kWideCap;
-    a.tile_count = tile_count.as<uint32_t>();
-    a.tile_offset = tile_offset.as<uint32_t>();
-    a.work = work.as<uint4>();
-    a.sky_tab = sky_tab.as<uint8_t>();
-    a.tile_cursor = tile_cursor.as<uint32_t>();
+    a.tile_count = reinterpret_cast<uint32_t*>(tiles + tl.o_count);
+    a.tile_offset = reinterpret_cast<uint32_t*>(tiles + tl.o_offset);
+    a.work = reinterpret_cast<uint4*>(tiles + tl.o_work);
+    a.sky_tab = tiles + tl.o_sky;
+    a.tile_cursor = reinterpret_cast<uint32_t*>(tiles + tl.o_cursor);
     a.bins = bins.as<uint32_t>();
     a.keys = keys.as<unsigned long long>();
     a.counters = counters.as<DCounters>();

@@ -80,6 +80,22 @@ struct TableLayout {
 TableLayout table_layout(uint32_t scene_cap, uint32_t view_cap, uint32_t order_cap, uint32_t draw_cap,
                          uint32_t chunk_cap);
 
+// Byte offsets of FrameEngine::tile_block.
+struct TileLayout {
+    size_t o_count, o_offset, o_cursor, o_work, o_sky, o_wide, total;
+    TileLayout(uint32_t stile_cap, uint32_t view_cap) {
+        auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+        const size_t bins = al((size_t)(stile_cap + 1) * sizeof(uint32_t));
+        o_count = 0;
+        o_offset = bins;
+        o_cursor = 2 * bins;
+        o_work = 3 * bins;
+        o_sky = o_work + al((size_t)(stile_cap / 2 + 1) * sizeof(uint4));
+        o_wide = o_sky + al((size_t)view_cap * 256);
+        total = o_wide + 2u * kWideCap * sizeof(uint2);
+    }
+};
+
 // Reusable frame engine: everything a batch of views needs on the device.
 // prepare() builds the per-frame tables on the host and grows capacities;
 // launch() uploads the tables with one copy and runs the frame, either as
@@ -131,8 +147,11 @@ struct FrameEngine {
     // us, 2560x1440 448 -> 430, three of 1600x900 275 -> 272, but four of
     // 1920x1080 63 -> 65 where most is sky.
     static constexpr uint64_t kWideShadeRounds = 4;
-    DBuf tables, tri_state, rec_r, rec_s, rec_t, fan_base, clip_queue, wide_queue;
-    DBuf tile_count, tile_offset, tile_cursor, work, sky_tab, bins, keys, counters, rsqrt_tab;
+    // A renderer's first frame waits for each allocation: the three records of a
+    // triangle are one (rec_s, rec_r, rec_t by slots), and the buffers sized by
+    // tiles and views are one (TileLayout).
+    DBuf tables, tri_state, records, fan_base, clip_queue, tile_block;
+    DBuf bins, keys, counters, rsqrt_tab;
     DBuf color;                // linear colour of views that need it (padded tile grids)
     bool defer_resolve = false;// the caller resolves (renderer frames with dt > 0)
     static constexpr int kStageRing = 4;
@@ -175,8 +194,8 @@ struct FrameEngine {
     std::vector<GraphStage> graph_stages;
     template <typename F>
     void each_buffer(F f) {
-        for (DBuf* b : {&tables, &tri_state, &rec_r, &rec_s, &rec_t, &fan_base, &clip_queue, &wide_queue, &tile_count,
-                        &tile_offset, &tile_cursor, &work, &sky_tab, &bins, &keys, &counters, &rsqrt_tab, &color})
+        for (DBuf* b : {&tables, &tri_state, &records, &fan_base, &clip_queue, &tile_block, &bins, &keys, &counters,
+                        &rsqrt_tab, &color})
             f(*b);
     }
     void keep_for_graph(cudaStream_t stream, int slot);

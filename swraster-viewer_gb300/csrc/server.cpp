@@ -133,9 +133,8 @@ struct swr_server {
     static uint64_t one_engine_bytes(const Engine& e) {
         const FrameEngine& f = e.b->eng;
         uint64_t t = e.b->tile_lum.bytes;
-        for (const DBuf* d : {&f.tables, &f.tri_state, &f.rec_r, &f.rec_s, &f.rec_t, &f.fan_base, &f.clip_queue, &f.wide_queue,
-                              &f.tile_count, &f.tile_offset, &f.tile_cursor, &f.work, &f.sky_tab, &f.bins, &f.keys, &f.counters,
-                              &f.rsqrt_tab, &f.color})
+        for (const DBuf* d : {&f.tables, &f.tri_state, &f.records, &f.fan_base, &f.clip_queue, &f.tile_block, &f.bins,
+                              &f.keys, &f.counters, &f.rsqrt_tab, &f.color})
             t += d->bytes;
         for (const OwnedOutput& o : e.b->owned) t += o.rgba8.bytes + o.vis.bytes;
         return t;
