@@ -413,7 +413,7 @@ void swr_renderer_destroy(swr_renderer* r);
  * host callback is enqueued). Bin overflow is detected on the device and
  * the frame is re-rendered with a larger capacity on the next call to
  * swr_renderer_sync, swr_blit or swr_read_visbuffer.
- * A stream that the caller captures (cudaStreamBeginCapture, relaxed mode)
+ * A stream that the caller captures (cudaStreamBeginCapture, any mode)
  * records the frame instead: each launch of the caller's graph renders it
  * again (with dt > 0: advances the exposure by dt again) until the renderer or
  * the scene is destroyed. The renderer can render other frames between

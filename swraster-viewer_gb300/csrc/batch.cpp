@@ -32,6 +32,15 @@ uint32_t batch_class(const swr_view_desc* v, int32_t n) {
 }
 
 swr_status BatchImpl::enqueue(const swr_view_desc* vd, int32_t n, cudaStream_t stream, std::string& err) {
+    // A batch that the caller captures records no events (they could not be
+    // read), and its graph's launches write the outputs it names.
+    const bool captured = stream_captured(stream);
+    const CaptureGuard guard(captured);
+    auto hold = [&] {
+        tile_lum.in_graph = true;
+        for (OwnedOutput& o : owned) o.rgba8.in_graph = o.vis.in_graph = true;
+    };
+    if (captured) hold();  // what grows here is kept, not freed
     // Unique scenes of this batch.
     std::vector<const SceneImpl*> scenes;
     std::vector<DView> views((size_t)n);
@@ -81,18 +90,12 @@ swr_status BatchImpl::enqueue(const swr_view_desc* vd, int32_t n, cudaStream_t s
         cudaGetLastError();
         return SWR_NO_MEMORY;
     }
-    swr_status st = eng.prepare(scenes, views, cams, err);
+    swr_status st = eng.prepare(scenes, views, cams, captured, err);
     if (st != SWR_OK) return st;
-    // A batch that the caller captures records no events (they could not be
-    // read), and its graph's launches write the outputs it names.
-    const bool captured = stream_captured(stream);
     if (!captured) cudaEventRecord(ev_start, stream);
     st = eng.launch(stream, captured, nullptr, err);
     if (!captured) cudaEventRecord(ev_end, stream);
-    if (captured) {
-        tile_lum.in_graph = true;
-        for (int32_t i = 0; i < n; ++i) owned[i].rgba8.in_graph = owned[i].vis.in_graph = true;
-    }
+    if (captured) hold();
     const bool fresh = !h_counters.p;
     if (st == SWR_OK && h_counters.ensure(sizeof(DCounters)) == cudaSuccess && fresh)
         std::memset(h_counters.p, 0, sizeof(DCounters));

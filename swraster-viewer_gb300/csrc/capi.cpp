@@ -294,7 +294,7 @@ void CUDART_CB exposure_callback(void* p) {
 }
 
 swr_status enqueue_frame(swr_renderer* r, const swr_scene* scene, const swr_camera* cam, float dt,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, bool captured) {
     std::string err;
     if (r->expo_pending) {
         cudaEventSynchronize(r->expo_done);
@@ -330,7 +330,6 @@ swr_status enqueue_frame(swr_renderer* r, const swr_scene* scene, const swr_came
     int slot = -1;
     // Events recorded in a capture can be neither queried nor waited for: a
     // captured frame records none and is not profiled.
-    const bool captured = stream_captured(stream);
     if (r->profiling && !captured) {
         slot = r->prof_next;
         r->prof_next = (r->prof_next + 1) % swr_renderer::kProfRing;
@@ -418,7 +417,7 @@ swr_status check_frame(swr_renderer* r) {
         swr_status gs = grow_for_overflow(r, c);
         if (gs != SWR_OK) return gs;
         // The overflowed frame's exposure step was skipped by the callback.
-        swr_status st = enqueue_frame(r, r->last_scene, &r->last_cam, r->last_dt, r->last_stream);
+        swr_status st = enqueue_frame(r, r->last_scene, &r->last_cam, r->last_dt, r->last_stream, false);
         if (st != SWR_OK) return st;
     }
     return fail(SWR_OVERFLOW, "bin capacity could not be grown enough");
@@ -430,6 +429,8 @@ swr_status swr_render_frame(swr_renderer* r, const swr_scene* scene, const swr_c
     if (!r || !scene || !cam) return fail(SWR_INVALID_ARG, "null argument");
     if (!scene->impl.d_scene) return fail(SWR_INVALID_ARG, "scene was created host-only");
     if (!(dt >= 0.0f) && !(dt < 0.0f)) return fail(SWR_INVALID_ARG, "dt is NaN");
+    const bool captured = stream_captured((cudaStream_t)stream);
+    const CaptureGuard guard(captured);
     // The previous frame is replaced, so it is not waited for: a frame is
     // checked (and re-rendered after an overflow) when its result is read.
     swr_status st = poll_frame(r);
@@ -438,7 +439,7 @@ swr_status swr_render_frame(swr_renderer* r, const swr_scene* scene, const swr_c
     r->last_cam = *cam;
     r->last_dt = dt;
     r->last_stream = (cudaStream_t)stream;
-    st = enqueue_frame(r, scene, cam, dt, (cudaStream_t)stream);
+    st = enqueue_frame(r, scene, cam, dt, (cudaStream_t)stream, captured);
     if (st != SWR_OK) return st;
     r->checked = false;
     r->have_frame = true;

@@ -200,7 +200,8 @@ inline uint32_t grow(uint32_t cur, uint64_t need) {
 }  // namespace
 
 swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& vws,
-                                const std::vector<const swr_camera*>& cams, std::string& err) {
+                                const std::vector<const swr_camera*>& cams, bool captured, std::string& err) {
+    if (captured) each_buffer([](DBuf& b) { b.in_graph = true; });
     // Per view: the node order (the host's part of the draw list) and the
     // camera the device builds the draws with; capacities from the scenes'
     // bounds (every primitive in the frustum), since the draw list itself is
@@ -299,8 +300,12 @@ swr_status FrameEngine::prepare(const std::vector<const SceneImpl*>& scenes, std
         stage_pending[stage_slot] = false;
     }
     HBuf& h_stage_cur = h_stage[stage_slot];
+    if (captured && h_stage_cur.bytes < lay.staged && h_stage_cur.p) {  // grown without a free
+        graph_stages.push_back({h_stage_cur, std::make_shared<std::atomic<bool>>(true)});
+        h_stage_cur = HBuf{};
+    }
     for (size_t i = 0; i < graph_stages.size() && !h_stage_cur.p; ++i)
-        if (graph_stages[i].gone->load()) {
+        if (graph_stages[i].gone->load() && (!captured || graph_stages[i].buf.bytes >= lay.staged)) {
             h_stage_cur = graph_stages[i].buf;
             graph_stages.erase(graph_stages.begin() + (ptrdiff_t)i);
         }
@@ -533,7 +538,7 @@ swr_status FrameEngine::grow_for(const DCounters& c, std::string& err) {
 swr_status FrameEngine::run(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& vws,
                             const std::vector<const swr_camera*>& cams, cudaStream_t stream, bool captured,
                             FrameArgs* out, std::string& err, cudaEvent_t* ev) {
-    swr_status st = prepare(scenes, vws, cams, err);
+    swr_status st = prepare(scenes, vws, cams, captured, err);
     if (st != SWR_OK) return st;
     st = launch(stream, captured, ev, err);
     if (out) *out = args;

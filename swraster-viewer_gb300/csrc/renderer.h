@@ -206,10 +206,11 @@ struct FrameEngine {
     // scheduling tile; SWR_OVERFLOW when nothing is left to grow.
     swr_status grow_for(const DCounters& c, std::string& err);
     void release();
-    swr_status prepare(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& views,
-                       const std::vector<const swr_camera*>& cams, std::string& err);
     // captured: the caller captures the stream (stream_captured), so nothing
-    // here waits for what is enqueued and what it reads stays as it is.
+    // here waits for what is enqueued, nothing is freed, and what the frame
+    // reads stays as it is.
+    swr_status prepare(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& views,
+                       const std::vector<const swr_camera*>& cams, bool captured, std::string& err);
     swr_status launch(cudaStream_t stream, bool captured, cudaEvent_t* ev, std::string& err);
     // prepare + launch (the plain renderer's path).
     swr_status run(const std::vector<const SceneImpl*>& scenes, std::vector<DView>& views,
@@ -219,6 +220,22 @@ struct FrameEngine {
 
 // Whether the caller is capturing the stream.
 bool stream_captured(cudaStream_t stream);
+
+// While a caller's capture is fed: its mode may forbid this thread the queries
+// and allocations that a frame makes beside its launches; they touch nothing
+// that is captured, so they are made in relaxed mode.
+struct CaptureGuard {
+    bool on;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    explicit CaptureGuard(bool captured) : on(captured) {
+        if (on) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    ~CaptureGuard() {
+        if (on) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    CaptureGuard(const CaptureGuard&) = delete;
+    CaptureGuard& operator=(const CaptureGuard&) = delete;
+};
 
 // compute_nodes_by_distance (src/renderer.rs:201-210): appends the scene's
 // node indices, nearest first, to `out`.

@@ -40,9 +40,9 @@ def fresh(s, cam):
     return out
 
 
-def captured(torch, stream, call):
+def captured(torch, stream, call, mode="relaxed"):
     g = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(g, stream=stream, capture_error_mode="relaxed"):
+    with torch.cuda.graph(g, stream=stream, capture_error_mode=mode):
         call()
     return g
 
@@ -142,6 +142,28 @@ def test_captured_exposure_steps(small):
         assert r.exposure() == p.exposure(), i
     for x in (r, p):
         x.close()
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_capture_modes_and_growth_while_captured(small, large, mode):
+    """Captures of a new renderer, of one whose buffers have to grow, and two frames in one capture."""
+    torch = pytest.importorskip("torch")
+    r, s = swr.Renderer(W, H), torch.cuda.Stream()
+    a = captured(torch, s, lambda: r.render(small, camera(small, 1), stream=s.cuda_stream), mode)
+    b = captured(torch, s, lambda: r.render(large, camera(large, 2), stream=s.cuda_stream), mode)
+
+    def two():
+        r.render(large, camera(large, 3), stream=s.cuda_stream)
+        r.render(small, camera(small, 4), stream=s.cuda_stream)
+
+    c = captured(torch, s, two, mode)
+    for _ in range(2):
+        for graph, (sc, i) in ((a, (small, 1)), (b, (large, 2)), (c, (small, 4))):
+            assert same(replayed(torch, r, graph), fresh(sc, camera(sc, i))), i
+        for i in range(6):
+            r.render(small, camera(small, 10 + i), stream=s.cuda_stream)
+        assert same((r.blit(), r.visbuffer()), fresh(small, camera(small, 15)))
+    r.close()
 
 
 def test_captured_batch(small, large):
