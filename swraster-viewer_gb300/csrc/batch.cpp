@@ -180,7 +180,7 @@ uint32_t BatchImpl::tuned_tile(const swr_view_desc* vd, int32_t n) const {
     // autotuner's other form) 2,631, 1,504 and 1,083; 64-px tiles took 2,377,
     // 1,340 and 1,359 (before tiles without packets were left out).
     // Views of at most kSmallView 64-px tiles are shaded in the raster: a
-    // shading CTA's next pixels are then another view's each time, and it
+    // shading CTA's next pixels are then nearly always another view's, and it
     // fetches that view's constants for them. us apart and fused, a scene of 30k
     // triangles in 96 views of 320x240 486 and 358, in 64 of 480x360 502 and
     // 400, in 40 of 640x480 470 and 408; spheres of 20k 577 and 451, 679 and 508,
