@@ -88,8 +88,11 @@ void init_view(DView& v, const swr_camera& cam, int32_t width, int32_t height, u
 }
 
 uint32_t auto_sched_tile(const int32_t* widths, const int32_t* heights, int32_t n, int num_sms) {
-    // 64 px from 8 tiles an SM, 32 px from 7 (1367x769 frame with 7.07: 32 px
-    // 217 us against 239 with 16; 1280x720 with 6.05: 113 against 103).
+    // 64 px from 8 tiles an SM, 32 px from 7. us of a frame with 32 and 16 px at
+    // 7 to 8 tiles an SM (1440x810): pictures filled by 30k triangles 176 and 177,
+    // 150k 215 and 268, 600k 355 and 406; spheres before a sky of 20k 115 and 80,
+    // 82k 128 and 103, 307k 165 and 131. At 6 (1280x720) 150k 191 and 228, spheres
+    // of 82k 128 and 95.
     for (uint32_t S : {64u, 32u}) {
         const uint64_t want = (S == 64u ? 8ull : 7ull) * (uint64_t)(num_sms > 0 ? num_sms : 1);
         uint64_t tiles = 0;
